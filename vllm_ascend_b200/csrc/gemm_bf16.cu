@@ -24,9 +24,7 @@
 // All waits are bounded (see common.cuh / comm.cuh).
 #include "comm.cuh"
 #include "common.cuh"
-
-#include <mutex>
-#include <unordered_map>
+#include "tmap_cache.cuh"
 
 namespace b200 {
 
@@ -452,50 +450,6 @@ done:
 }
 
 // ---------------------------------------------------------------- host
-struct TmapKey {
-  const void* ptr;
-  uint64_t rows, cols, ld;
-  uint32_t box_rows;
-  bool operator==(const TmapKey& o) const {
-    return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld &&
-           box_rows == o.box_rows;
-  }
-};
-struct TmapKeyHash {
-  size_t operator()(const TmapKey& k) const {
-    size_t h = (size_t)k.ptr;
-    h = h * 1000003u ^ k.rows;
-    h = h * 1000003u ^ k.cols;
-    h = h * 1000003u ^ k.ld;
-    h = h * 1000003u ^ k.box_rows;
-    return h;
-  }
-};
-
-// Tensor map of a row-major bf16 [rows, cols] matrix with row stride ld, box
-// = [box_rows, 64 cols], 128-byte swizzle.  Cached: encoding costs a few us.
-static int get_tmap_2d_bf16(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t cols,
-                            uint64_t ld, uint32_t box_rows) {
-  static std::unordered_map<TmapKey, CUtensorMap, TmapKeyHash> cache;
-  static std::mutex mu;
-  TmapKey key{ptr, rows, cols, ld, box_rows};
-  std::lock_guard<std::mutex> g(mu);
-  auto it = cache.find(key);
-  if (it != cache.end()) {
-    *out = it->second;
-    return 0;
-  }
-  uint64_t dims[2] = {cols, rows};
-  uint64_t strides[1] = {ld * 2};
-  uint32_t box[2] = {64, box_rows};
-  int rc = make_tmap(out, ptr, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, dims, strides, box,
-                     CU_TENSOR_MAP_SWIZZLE_128B);
-  if (rc) return rc;
-  if (cache.size() > 8192) cache.clear();
-  cache.emplace(key, *out);
-  return 0;
-}
-
 template <int BN>
 static int launch_gemm(const void* A, const void* W, GemmParams& p, int lda, int ldw,
                        long a_rows, long w_rows, int max_ctas, cudaStream_t stream) {

@@ -120,7 +120,8 @@ class Linear:
         else:
             if isinstance(x, ops.QuantAct):
                 x = x.dequant()
-            y = ops.linear(x, self.weight, self.bias, residual)
+            # with adapters in the engine a plain request's rows keep the bits they have without adapter neighbours
+            y = (ops.linear_step if self.lora is None else ops.linear)(x, self.weight, self.bias, residual)
         if self._lora_on():
             y = self.lora.apply(x, y)
         return y
@@ -244,7 +245,7 @@ class ParallelLMHead:
         self.comm = embed.comm
 
     def __call__(self, hidden: torch.Tensor) -> torch.Tensor:
-        logits = ops.linear(hidden, self.weight)
+        logits = ops.linear_step(hidden, self.weight)
         if self.comm.size > 1:
             logits = self.comm.all_gather(logits, dim=-1)
         return logits[..., :self.embed.vocab]
@@ -253,7 +254,7 @@ class ParallelLMHead:
         """Arg-max over the full vocabulary without gathering the logits: every rank reduces its
         own vocabulary shard to (max value, index) and only those pairs are all-gathered — the
         "reduce sample" path of vllm_ascend/sample/sampler.py:87-107, 168-204."""
-        logits = ops.linear(hidden, self.weight)                       # [B, V / tp]
+        logits = ops.linear_step(hidden, self.weight)                  # [B, V / tp]
         n, r = self.comm.size, self.comm.rank
         shard = logits.shape[-1]
         first = r * shard
@@ -494,10 +495,10 @@ class SwiGLUMLP:
         if self.limit is not None:
             if gu.quant is not None or gu._lora_on():
                 raise NotImplementedError("the clamped gate takes plain projections")
-            return self.down_proj(ops.linear_swiglu(x, gu.weight, limit=self.limit))
+            return self.down_proj(ops.linear_swiglu_step(x, gu.weight, limit=self.limit))
         if gu.quant is None and gu.bias is None and not gu.gather_output and not gu._lora_on() \
                 and _plan().enabled("gemm_swiglu"):
-            return self.down_proj(ops.linear_swiglu(x, gu.weight))
+            return self.down_proj((ops.linear_swiglu_step if gu.lora is None else ops.linear_swiglu)(x, gu.weight))
         if wants_quant_act(self.down_proj):
             return self.down_proj(ops.silu_and_mul_quant_fp8(gu(x)))
         return self.down_proj(ops.silu_and_mul(gu(x)))

@@ -303,6 +303,66 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Ten
     return out.view(*x.shape[:-1], I)
 
 
+#: most rows and, beyond 128 rows, most output columns of the few-row GEMM.  Measured on a B200, old kernel -> few-row kernel, us
+#: with cold caches: 4096 x 4096 with 1 / 128 / 256 rows 32 -> 17 / 32 -> 23 / 34 -> 26; 4096 x 12288 71 -> 32 / 72 -> 39 / 75 -> 46;
+#: gate / up 24576 x 4096 80 -> 53 / 64 -> 62 / 77 -> 100.  Beyond 128 rows every stage carries twice as many activations as
+#: weights, which pays only where the tiles of the other kernels leave most SMs idle.
+_FEW_ROWS, _FEW_ROWS_MAX_COLS = 256, 5120
+
+
+def _few_rows(M: int, N: int, K: int) -> bool:
+    """Whether a step's product runs in the kernel that splits K over blocks.  Its rows may differ in the last bit from
+    those of a larger batch, so batch-invariant mode never takes it."""
+    if M > _FEW_ROWS or (M > 128 and N > _FEW_ROWS_MAX_COLS) or K % 8 or N % 8 or envs.VLLM_B200_GEMM == "cublas":
+        return False
+    from ..batch_invariant import is_batch_invariant
+    return not is_batch_invariant()
+
+
+def _gemm_small(x2, weight, out, bias, res2, N: int, glu: bool, alpha: float = 0.0, limit: float = 0.0) -> None:
+    M, K = x2.shape
+    rc = _native.lib().b200_gemm_small_bf16(
+        x2.data_ptr(), weight.data_ptr(), out.data_ptr(), _native.ptr(bias), _native.ptr(res2), M, N, K, x2.stride(0),
+        weight.stride(0), out.stride(0), int(glu), alpha, limit, 0, _native.status_word(x2.device).data_ptr(),
+        _native.stream_ptr())
+    _native.check(rc, "gemm_small")
+    launch_counter[0] += 1
+
+
+def linear_step(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
+                residual: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``linear`` for the products of an engine's step: batches of few rows sum K in parts (fp32) so that all SMs stream
+    weights.  ``linear`` itself gives a row the same bits in every batch."""
+    K, N = x.shape[-1], weight.shape[0]
+    M = x.numel() // K if K else 0
+    if M == 0 or not _use_native(x) or weight.dtype != _BF16 or not _few_rows(M, N, K):
+        return linear(x, weight, bias, residual)
+    x2 = x.reshape(-1, K)
+    if x2.stride(-1) != 1 or (x2.stride(0) % 8) != 0:
+        x2 = x2.contiguous()
+    out = torch.empty((M, N), dtype=x.dtype, device=x.device)
+    res2 = None
+    if residual is not None:
+        res2 = residual.view(M, N)
+        assert res2.stride(0) == out.stride(0) and res2.stride(1) == 1
+    _gemm_small(x2, weight, out, bias, res2, N, False)
+    return out.view(*x.shape[:-1], N)
+
+
+def linear_swiglu_step(x: torch.Tensor, weight: torch.Tensor, limit: Optional[float] = None) -> torch.Tensor:
+    """``linear_swiglu`` for the products of an engine's step (see ``linear_step``)."""
+    K, I = x.shape[-1], weight.shape[0] // 2
+    M = x.numel() // K if K else 0
+    if M == 0 or not _use_native(x) or weight.dtype != _BF16 or not _few_rows(M, 2 * I, K) or I % 8:
+        return linear_swiglu(x, weight, limit=limit)
+    x2 = x.reshape(-1, K)
+    if x2.stride(-1) != 1 or (x2.stride(0) % 8) != 0:
+        x2 = x2.contiguous()
+    out = torch.empty((M, I), dtype=x.dtype, device=x.device)
+    _gemm_small(x2, weight, out, None, None, I, True, *((0.0, 0.0) if limit is None else (CLAMPED_GATE_ALPHA, float(limit))))
+    return out.view(*x.shape[:-1], I)
+
+
 # ---------------------------------------------------------------- attention
 _scratch: dict = {}
 
