@@ -1,0 +1,95 @@
+"""Sampling kernel against its definition in numpy: kept set by sorting in fp64, random numbers by Philox4x32-10, race of
+p / Exp(1).  Rows of every storage form (in the cluster's shared memory, too long for it, unaligned) and of every shape
+that chooses another cut (peaked, flat, masked, fewer large elements than top-k)."""
+import numpy as np
+import pytest
+import torch
+
+from vllm_ascend_b200 import _native, ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _philox(ctr, key):
+    M0, M1, W0, W1 = (np.uint64(v) for v in (0xD2511F53, 0xCD9E8D57, 0x9E3779B9, 0xBB67AE85))
+    m = np.uint64(0xFFFFFFFF)
+    x, y, z, w = (np.asarray(c, dtype=np.uint64) for c in ctr)
+    k0, k1 = np.uint64(key & 0xFFFFFFFF), np.uint64(key >> 32)
+    for _ in range(10):
+        a, b = M0 * x, M1 * z
+        x, y, z, w = (b >> np.uint64(32)) ^ y ^ k0, b & m, (a >> np.uint64(32)) ^ w ^ k1, a & m
+        k0, k1 = (k0 + W0) & m, (k1 + W1) & m
+    return np.stack([x, y, z, w], -1)
+
+
+#: largest error of the fast logarithm between 0.5 and 2, as CUDA documents it: where u is near 1, -log u has no more digits
+LOG_ERROR = 2.0 ** -21
+
+
+def _expected(row, T, k, p, min_p, seed, offset):
+    """(tokens that the race may give, distance of the cut from the nearest alternative)."""
+    x = row.astype(np.float64)
+    if T < 1e-5:
+        return [int(np.argmax(x))], 1.0
+    e = np.exp((x - x.max()) / T)
+    order = np.argsort(-e, kind="stable")
+    keep, gap = np.ones(len(x), bool), 1.0
+    if 0 < k < len(x):
+        keep &= e >= e[order[k - 1]]
+    if p < 1:
+        ks = order[keep[order]]
+        cum = np.cumsum(e[ks])
+        n = int(np.searchsorted(cum, p * cum[-1]))
+        gap = np.abs(cum / (p * cum[-1]) - 1).min()
+        keep &= e >= e[ks[min(n, len(ks) - 1)]]
+    if min_p > 0:
+        keep &= e >= min_p
+        gap = min(gap, np.abs(e / min_p - 1).min())
+    V = len(x)
+    g = np.arange(0, V, 4)
+    r = _philox((g, np.full_like(g, offset & 0xFFFFFFFF), np.full_like(g, offset >> 32), np.zeros_like(g)), seed).reshape(-1)[:V]
+    ex = -np.log(((r >> np.uint64(8)).astype(np.float64) + 1) / 16777216)
+    on = keep & (e > 0)
+    low = np.where(on, e / (ex + LOG_ERROR) * (1 - 1e-5), -1)
+    high = np.where(on, e / np.maximum(ex - LOG_ERROR, 1e-20) * (1 + 1e-5), -1)
+    return np.nonzero(high >= low.max())[0].tolist(), gap
+
+
+def _rows(kind, B, V, rng):
+    x = rng.standard_normal((B, V)).astype(np.float32)
+    if kind == "peaked":
+        x *= 4
+    elif kind == "flat":
+        x *= 1e-2
+    elif kind == "masked":
+        x = np.where(rng.random((B, V)) < 0.98, -np.inf, x * 3).astype(np.float32)
+        x[:, V // 2] = 1.0
+    elif kind == "spikes":                       # three large elements, the rest below every cut
+        x -= 60
+        x[:, [0, V // 3, V - 1]] += 60
+    return x
+
+
+@pytest.mark.parametrize("V,pad", [(5, 3), (31, 1), (4096, 0), (32000, 0), (50257, 3), (151936, 0), (409601, 1), (420004, 4)])
+@pytest.mark.parametrize("kind", ["peaked", "flat", "masked", "spikes"])
+def test_sample_is_the_race_over_the_kept_set(V, pad, kind):
+    rng = np.random.default_rng(V)
+    B = 6
+    wide = torch.zeros((B, V + pad))
+    wide[:, :V] = torch.from_numpy(_rows(kind, B, V, rng))
+    logits = wide.cuda()[:, :V]
+    T = [0.0, 0.7, 1.0, 1.3, 0.9, 1.0]
+    k = [5, 3, min(50, V), 0, 0, V]
+    p = [0.9, 1.0, 0.9, 0.8, 0.97, 1.0]
+    mp = [0.0, 0.0, 0.0, 0.0, 0.013, 0.0]
+    seeds = rng.integers(0, 1 << 62, B)
+    offsets = rng.integers(0, 1 << 34, B)
+    host = logits.cpu().numpy()
+    got = ops.sample(logits, torch.tensor(T).cuda(), torch.tensor(k, dtype=torch.int32).cuda(), torch.tensor(p).cuda(),
+                     torch.tensor(mp).cuda(), torch.from_numpy(seeds).cuda(), torch.from_numpy(offsets).cuda()).cpu().tolist()
+    _native.check_status(torch.device("cuda"))
+    for b in range(B):
+        want, gap = _expected(host[b], T[b], k[b], p[b], mp[b], int(seeds[b]), int(offsets[b]))
+        # the fast exponential and fp32 sums are off by up to 1e-5; where the cut is closer, both sides of it are right
+        if gap > 1e-5:
+            assert got[b] in want, (b, got[b], want)

@@ -3,9 +3,11 @@
 // top-p (-> min-p) -> exponential-race sampling argmax(p / Exp(1)); greedy rows
 // take argmax of the raw logits.  Instead of the reference's full sort, the
 // top-k and top-p cut-offs are found with a 3-pass radix select over the float
-// bit patterns (count histograms for top-k, mass histograms for top-p), so a row
-// costs a handful of streaming passes over the vocabulary.
+// bit patterns (count histograms for top-k, mass histograms for top-p) on a row
+// that stays in the shared memory of a cluster.
 #include "common.cuh"
+
+#include <type_traits>
 
 namespace b200 {
 
@@ -146,128 +148,285 @@ __global__ void penalties_kernel(float* logits, long ld, int V, const long* prom
 }
 
 // ---------------------------------------------------------------- top-k/top-p sampling
-// Radix select helper state lives in shared memory.
-struct RadixSmem {
-  float hist[2048];
-  float red[32];
-  int redi[32];
-  uint32_t prefix;      // selected high bits so far
-  float remaining;      // remaining count / mass to find inside the selected bin
-  float total;
+// A row of 150k fp32 logits is walked about ten times (maximum, exponentials, three digits of a radix select for
+// top-k and three for top-p, the race), so the row is spread over a cluster of eight blocks and stays in their shared memory
+// after one read of HBM.  What bounds it then is instructions and the cluster's meetings, so a walk touches as little as it can:
+//   * the select passes only look at elements above a cut that already holds enough of them (2^-6 to 2^-24 of the
+//     maximum, counted while the exponentials are taken): with peaked rows that leaves a few thousand shared-memory
+//     atomics where there were V per pass;
+//   * bins are integers (mass in units of 2^-40: shared memory adds 64-bit integers by itself, floats in a loop, and the
+//     sum has no order), added and searched in parallel (256 per block, then one warp);
+//   * random numbers are drawn only for groups of four that hold a kept element.
+// 192 rows of 151936: one block per row with thread-serial bins 738 us, this 267 us.
+constexpr int SAMP_C = 8;              // blocks per row
+constexpr int SAMP_T = 512;
+constexpr int SAMP_BINS = 2048;
+constexpr int SAMP_MAX_SLICE = 50 * 1024;        // elements of a row that a block keeps in shared memory
+constexpr int SAMP_CUTS = 5;
+using samp_n = unsigned long long;     // elements, or mass in units of 2^-40 (e <= 1, so a row's mass fits)
+constexpr float SAMP_UNIT = 1099511627776.f;
+
+struct SampXch { float v[1 + SAMP_CUTS]; uint32_t n[SAMP_CUTS]; int i; };
+
+struct SampSmem {
+  samp_n hist[SAMP_BINS];
+  samp_n own[SAMP_BINS / SAMP_C];      // this block's bins, summed over the cluster
+  samp_n tot[6];                       // sum of `own`, one slot per select pass
+  samp_n remaining;
+  SampXch xch[4];                      // what a block tells the others: one slot per meeting
+  float red[SAMP_T / 32][1 + 2 * SAMP_CUTS];
+  float sv[32];
+  int si[32];
+  samp_n sn[SAMP_T / 32];
+  uint32_t prefix;
 };
 
-// One pass: histogram (count or mass) of the `bits`-wide digit at `shift` over elements
-// whose higher bits equal `prefix` and which pass the `floor_key` filter, then walk
-// bins from the top to find where the cumulative quantity reaches `remaining`.
-__device__ void radix_pass(const float* __restrict__ e, int V, RadixSmem* s, int shift, int bits,
-                           uint32_t hi_mask, bool by_mass, uint32_t floor_key) {
-  const int nb = 1 << bits;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) s->hist[i] = 0.f;
+__device__ __forceinline__ void samp_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// the address of `p` (shared memory of this block) in block r of the cluster
+template <typename U>
+__device__ __forceinline__ U samp_peek(const U* p, int r) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(r));
+  U out;
+  if constexpr (sizeof(U) == 8) {
+    unsigned long long v;
+    asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+    memcpy(&out, &v, 8);
+  } else {
+    uint32_t v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    memcpy(&out, &v, 4);
+  }
+  return out;
+}
+// sum of v over the block, in every thread
+__device__ __forceinline__ float samp_block_sum(float v, float* red) {
+  v = warp_reduce_sum(v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = threadIdx.x % 32 < SAMP_T / 32 ? red[threadIdx.x % 32] : 0.f;
+  v = warp_reduce_sum(v);
+  __syncthreads();
+  return v;
+}
+__device__ __forceinline__ samp_n samp_warp_sum(samp_n v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ void samp_better(float& v, int& i, float ov, int oi) {
+  if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
+}
+// argmax over the cluster, lowest index on ties
+__device__ void samp_cluster_argmax(float& v, int& idx, SampSmem* s, SampXch* x) {
+  block_argmax(v, idx, s->sv, s->si);
+  if (threadIdx.x == 0) { x->v[0] = v; x->i = idx; }
+  samp_cluster_sync();
+  v = -INFINITY;
+  idx = 0x7fffffff;
+  for (int r = 0; r < SAMP_C; r++) samp_better(v, idx, samp_peek(&x->v[0], r), samp_peek(&x->i, r));
+}
+
+// One digit of the select: histogram (elements or their mass) of the `bits`-wide digit at `shift` over the elements whose
+// higher bits equal the prefix and whose key reaches floor_key, then the bin, walking down from the top, at which the
+// running sum reaches `remaining`.  Every block of the cluster ends with the same prefix and remaining.
+template <bool MASS>
+__device__ void samp_pass(const float* e, int n, SampSmem* s, int pass, int shift, int bits, uint32_t hi_mask, uint32_t floor_key, int rank) {
+  const int nb = 1 << bits, per = nb / SAMP_C;
+  for (int i = threadIdx.x; i < nb; i += SAMP_T) s->hist[i] = 0;
   __syncthreads();
   const uint32_t prefix = s->prefix;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) {
+  const samp_n rem0 = s->remaining;
+  for (int i = threadIdx.x; i < n; i += SAMP_T) {
     const float v = e[i];
     const uint32_t k = __float_as_uint(v);
-    if (k < floor_key) continue;
-    if ((k & hi_mask) != prefix) continue;
-    atomicAdd(&s->hist[(k >> shift) & (nb - 1)], by_mass ? v : 1.f);
+    if (k < floor_key || (k & hi_mask) != prefix) continue;
+    atomicAdd(&s->hist[(k >> shift) & (nb - 1)], MASS ? __float2ull_rn(v * SAMP_UNIT) : 1ull);
   }
+  samp_cluster_sync();
+  samp_n b = 0;
+  if ((int)threadIdx.x < per) {
+#pragma unroll
+    for (int r = 0; r < SAMP_C; r++) b += samp_peek(&s->hist[rank * per + threadIdx.x], r);
+    s->own[threadIdx.x] = b;
+  }
+  b = samp_warp_sum(b);
+  if ((threadIdx.x & 31) == 0) s->sn[threadIdx.x >> 5] = b;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float rem = s->remaining;
-    int sel = 0;
-    for (int bin = nb - 1; bin >= 0; bin--) {
-      const float hval = s->hist[bin];
-      if (hval >= rem || bin == 0) { sel = bin; break; }
-      rem -= hval;
+  if (threadIdx.x < 32) {
+    b = samp_warp_sum(threadIdx.x < SAMP_T / 32 ? s->sn[threadIdx.x] : 0);
+    if (threadIdx.x == 0) s->tot[pass] = b;
+  }
+  samp_cluster_sync();
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    const samp_n t_lane = samp_peek(&s->tot[pass], lane % SAMP_C);
+    samp_n rem = rem0;
+    int r = SAMP_C - 1;
+    for (; r > 0; r--) {
+      const samp_n t = __shfl_sync(0xffffffffu, t_lane, r);
+      if (t >= rem) break;
+      rem -= t;
     }
-    // fp rounding can leave every bin below rem: fall back to the lowest non-empty bin
-    s->prefix = prefix | ((uint32_t)sel << shift);
-    s->remaining = rem;
+    // lane l owns bins [top - w (l + 1), top - w l) of block r
+    constexpr int W = SAMP_BINS / SAMP_C / 32;
+    const int w = per / 32;
+    samp_n mine[W], sum = 0;
+#pragma unroll
+    for (int j = 0; j < W; j++) {
+      mine[j] = j < w ? samp_peek(&s->own[per - 1 - (lane * w + j)], r) : 0;
+      sum += mine[j];
+    }
+    samp_n upto = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const samp_n t = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += t;
+    }
+    const uint32_t hit = __ballot_sync(0xffffffffu, upto >= rem);
+    const int who = hit ? __ffs(hit) - 1 : 31;                     // rounding can leave every sum below rem: the lowest bin
+    if (lane == who) {
+      rem -= upto - sum;
+      int sel = w - 1;
+#pragma unroll
+      for (int j = 0; j < W; j++)
+        if (j < w - 1 && sel == w - 1) {
+          if (mine[j] >= rem) sel = j;
+          else rem -= mine[j];
+        }
+      s->prefix = prefix | ((uint32_t)(r * per + per - 1 - (lane * w + sel)) << shift);
+      s->remaining = rem;
+    }
   }
   __syncthreads();
 }
 
-// logits: fp32 [B, V] (already penalised), overwritten with exp((x - max)/T).
+// logits: fp32 [B, V] (already penalised); overwritten where a row does not fit the cluster's shared memory.
 // temperature/top_k/top_p/min_p: per row (top_k <= 0 or >= V: off; top_p >= 1: off).
 // seeds: per-row uint64 seed, offsets: per-row counter (e.g. number of tokens generated).
-__global__ void __launch_bounds__(SAMP_THREADS)
-sample_kernel(float* logits, long ld, int V, const float* __restrict__ temperature,
+__global__ void __launch_bounds__(SAMP_T)
+sample_kernel(float* logits, long ld, int V, int slice, int resident, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p,
               const float* __restrict__ min_p, const unsigned long long* __restrict__ seeds,
               const long* __restrict__ offsets, long* __restrict__ out) {
-  __shared__ RadixSmem s;
-  const int b = blockIdx.x;
-  float* row = logits + (long)b * ld;
+  __shared__ SampSmem s;
+  extern __shared__ __align__(16) float kept_row[];
+  const int rank = blockIdx.x, b = blockIdx.y;
+  const int first = rank * slice, n = max(0, min(V - first, slice));
+  float* row = logits + (long)b * ld + first;
+  float* e = resident ? kept_row : row;
   const float T = temperature ? temperature[b] : 1.f;
-  // ---- max (also the greedy answer)
+  // ---- the row comes in; its maximum (also the greedy answer)
   float best = -INFINITY;
   int bi = 0x7fffffff;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) {
-    const float v = row[i];
-    if (v > best) { best = v; bi = i; }
+  if (resident && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+    const int nv = n >> 2;
+#pragma unroll 4
+    for (int c = threadIdx.x; c < nv; c += SAMP_T) {
+      const float4 q = reinterpret_cast<const float4*>(row)[c];
+      reinterpret_cast<float4*>(e)[c] = q;
+      if (q.x > best) { best = q.x; bi = first + 4 * c; }
+      if (q.y > best) { best = q.y; bi = first + 4 * c + 1; }
+      if (q.z > best) { best = q.z; bi = first + 4 * c + 2; }
+      if (q.w > best) { best = q.w; bi = first + 4 * c + 3; }
+    }
+    for (int i = 4 * nv + threadIdx.x; i < n; i += SAMP_T) {
+      const float v = row[i];
+      e[i] = v;
+      if (v > best) { best = v; bi = first + i; }
+    }
+  } else {
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += SAMP_T) {
+      const float v = row[i];
+      if (resident) e[i] = v;
+      if (v > best) { best = v; bi = first + i; }
+    }
   }
-  block_argmax(best, bi, s.red, s.redi);
+  samp_cluster_argmax(best, bi, &s, &s.xch[0]);
   if (T < 1e-5f) {
-    if (threadIdx.x == 0) out[b] = bi;
+    if (rank == 0 && threadIdx.x == 0) out[b] = bi;
+    samp_cluster_sync();               // nobody leaves while another reads its memory
     return;
   }
-  // ---- e = exp((x - max)/T), Z
+  // ---- e = exp((x - max)/T), their sum, and how much lies above each cut
+  const uint32_t cuts[SAMP_CUTS] = {0x3C800000u, 0x3A800000u, 0x38800000u, 0x36800000u, 0x33800000u};   // 2^-6, -10, -14, -18, -24
   const float invT = 1.f / T;
-  float z = 0.f;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) {
-    const float ev = __expf((row[i] - best) * invT);
-    row[i] = ev;
-    z += ev;
+  float part[1 + 2 * SAMP_CUTS];       // sum, sum and number above each cut
+#pragma unroll
+  for (int j = 0; j < 1 + 2 * SAMP_CUTS; j++) part[j] = 0.f;
+  for (int i = threadIdx.x; i < n; i += SAMP_T) {
+    const float ev = __expf((e[i] - best) * invT);
+    e[i] = ev;
+    part[0] += ev;
+#pragma unroll
+    for (int j = 0; j < SAMP_CUTS; j++)
+      if (__float_as_uint(ev) >= cuts[j]) { part[1 + j] += ev; part[1 + SAMP_CUTS + j] += 1.f; }
   }
-  z = warp_reduce_sum(z);
-  if ((threadIdx.x & 31) == 0) s.red[threadIdx.x >> 5] = z;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    float t = threadIdx.x < (blockDim.x >> 5) ? s.red[threadIdx.x] : 0.f;
-    t = warp_reduce_sum(t);
-    if (threadIdx.x == 0) s.total = t;
+#pragma unroll
+  for (int j = 0; j < 1 + 2 * SAMP_CUTS; j++) {
+    part[j] = warp_reduce_sum(part[j]);
+    if ((threadIdx.x & 31) == 0) s.red[threadIdx.x >> 5][j] = part[j];
   }
   __syncthreads();
-  float mass = s.total;
-  uint32_t thr_key = 0;  // keep elements with key >= thr_key
+  if (threadIdx.x < 1 + 2 * SAMP_CUTS) {
+    float t = 0.f;
+    for (int w = 0; w < SAMP_T / 32; w++) t += s.red[w][threadIdx.x];
+    if (threadIdx.x <= SAMP_CUTS) s.xch[1].v[threadIdx.x] = t;
+    else s.xch[1].n[threadIdx.x - 1 - SAMP_CUTS] = (uint32_t)t;
+  }
+  samp_cluster_sync();
+  float z = 0.f, zc[SAMP_CUTS];
+  uint32_t nc[SAMP_CUTS];
+#pragma unroll
+  for (int r = 0; r < SAMP_C; r++) z += samp_peek(&s.xch[1].v[0], r);
+#pragma unroll
+  for (int j = 0; j < SAMP_CUTS; j++) {
+    zc[j] = 0.f;
+    nc[j] = 0;
+#pragma unroll
+    for (int r = 0; r < SAMP_C; r++) { zc[j] += samp_peek(&s.xch[1].v[1 + j], r); nc[j] += samp_peek(&s.xch[1].n[j], r); }
+  }
+  float mass = z;
+  uint32_t thr_key = 0;                // keep elements with key >= thr_key
 
   const int k = top_k ? top_k[b] : 0;
   if (k > 0 && k < V) {
-    if (threadIdx.x == 0) { s.prefix = 0; s.remaining = (float)k; }
+    uint32_t cut = 0;
+#pragma unroll
+    for (int j = SAMP_CUTS - 1; j >= 0; j--) if (nc[j] >= (uint32_t)k) cut = cuts[j];
+    if (threadIdx.x == 0) { s.prefix = 0; s.remaining = (samp_n)k; }
     __syncthreads();
-    radix_pass(row, V, &s, 21, 11, 0x00000000u, false, 0);
-    radix_pass(row, V, &s, 10, 11, 0xFFE00000u, false, 0);
-    radix_pass(row, V, &s, 0, 10, 0xFFFFFC00u, false, 0);
+    samp_pass<false>(e, n, &s, 0, 21, 11, 0x00000000u, cut, rank);
+    samp_pass<false>(e, n, &s, 1, 10, 11, 0xFFE00000u, cut, rank);
+    samp_pass<false>(e, n, &s, 2, 0, 10, 0xFFFFFC00u, cut, rank);
     thr_key = s.prefix;
-    __syncthreads();
     // mass of the kept set
     float mk = 0.f;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
-      const float v = row[i];
+    for (int i = threadIdx.x; i < n; i += SAMP_T) {
+      const float v = e[i];
       if (__float_as_uint(v) >= thr_key) mk += v;
     }
-    mk = warp_reduce_sum(mk);
-    if ((threadIdx.x & 31) == 0) s.red[threadIdx.x >> 5] = mk;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      float t = threadIdx.x < (blockDim.x >> 5) ? s.red[threadIdx.x] : 0.f;
-      t = warp_reduce_sum(t);
-      if (threadIdx.x == 0) s.total = t;
-    }
-    __syncthreads();
-    mass = s.total;
+    mk = samp_block_sum(mk, s.sv);
+    if (threadIdx.x == 0) s.xch[2].v[0] = mk;
+    samp_cluster_sync();
+    mass = 0.f;
+    for (int r = 0; r < SAMP_C; r++) mass += samp_peek(&s.xch[2].v[0], r);
   }
   const float pth = top_p ? top_p[b] : 1.f;
   if (pth < 1.f) {
-    if (threadIdx.x == 0) { s.prefix = 0; s.remaining = pth * mass; }
+    uint32_t cut = 0;                  // a margin for the order of the sums
+#pragma unroll
+    for (int j = SAMP_CUTS - 1; j >= 0; j--) if (zc[j] >= pth * mass * 1.001f) cut = cuts[j];
+    if (thr_key > cut) cut = thr_key;
+    if (threadIdx.x == 0) { s.prefix = 0; s.remaining = __float2ull_rn(pth * mass * SAMP_UNIT); }
     __syncthreads();
-    radix_pass(row, V, &s, 21, 11, 0x00000000u, true, thr_key);
-    radix_pass(row, V, &s, 10, 11, 0xFFE00000u, true, thr_key);
-    radix_pass(row, V, &s, 0, 10, 0xFFFFFC00u, true, thr_key);
-    const uint32_t tp = s.prefix;
-    if (tp > thr_key) thr_key = tp;
-    __syncthreads();
+    samp_pass<true>(e, n, &s, 3, 21, 11, 0x00000000u, cut, rank);
+    samp_pass<true>(e, n, &s, 4, 10, 11, 0xFFE00000u, cut, rank);
+    samp_pass<true>(e, n, &s, 5, 0, 10, 0xFFFFFC00u, cut, rank);
+    if (s.prefix > thr_key) thr_key = s.prefix;
   }
   const float mp = min_p ? min_p[b] : 0.f;
   if (mp > 0.f) {
@@ -280,32 +439,47 @@ sample_kernel(float* logits, long ld, int V, const float* __restrict__ temperatu
   const uint2 key = make_uint2((uint32_t)seed, (uint32_t)(seed >> 32));
   float bestv = -INFINITY;
   int besti = bi;
-  for (int i0 = threadIdx.x * 4; i0 < V; i0 += blockDim.x * 4) {
-    const uint4 rnd = philox4x32(
-        make_uint4((uint32_t)i0, (uint32_t)offset, (uint32_t)((unsigned long long)offset >> 32), 0u), key);
-    const uint32_t rr[4] = {rnd.x, rnd.y, rnd.z, rnd.w};
+  for (int i0 = threadIdx.x * 4; i0 < n; i0 += SAMP_T * 4) {     // slices start at multiples of four
+    float v[4];
+    bool any = false;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      const int i = i0 + j;
-      if (i < V) {
-        const float v = row[i];
-        if (__float_as_uint(v) >= thr_key && v > 0.f) {
-          const float ex = -__logf(u32_to_unit(rr[j]));  // Exp(1)
-          const float sc = v / fmaxf(ex, 1e-20f);
-          if (sc > bestv || (sc == bestv && i < besti)) { bestv = sc; besti = i; }
-        }
-      }
+      v[j] = i0 + j < n ? e[i0 + j] : 0.f;
+      any |= __float_as_uint(v[j]) >= thr_key && v[j] > 0.f;
     }
+    if (!any) continue;
+    const uint4 rnd = philox4x32(
+        make_uint4((uint32_t)(first + i0), (uint32_t)offset, (uint32_t)((unsigned long long)offset >> 32), 0u), key);
+    const uint32_t rr[4] = {rnd.x, rnd.y, rnd.z, rnd.w};
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (__float_as_uint(v[j]) >= thr_key && v[j] > 0.f) {
+        const float ex = -__logf(u32_to_unit(rr[j]));  // Exp(1)
+        samp_better(bestv, besti, v[j] / fmaxf(ex, 1e-20f), first + i0 + j);
+      }
   }
-  block_argmax(bestv, besti, s.red, s.redi);
-  if (threadIdx.x == 0) out[b] = besti;
+  samp_cluster_argmax(bestv, besti, &s, &s.xch[3]);
+  if (rank == 0 && threadIdx.x == 0) out[b] = besti;
+  samp_cluster_sync();
 }
 
-__global__ void cast_bf16_to_f32_kernel(const __nv_bfloat16* __restrict__ in, long ld_in,
-                                        float* __restrict__ out, long ld_out, int V) {
-  const __nv_bfloat16* r = in + (long)blockIdx.x * ld_in;
-  float* o = out + (long)blockIdx.x * ld_out;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) o[i] = __bfloat162float(r[i]);
+// Rows of 16-byte aligned storage go eight elements at a time: 192 x 151936 81 us with single elements, 33 us so.
+__global__ void __launch_bounds__(256) cast_bf16_to_f32_kernel(const __nv_bfloat16* __restrict__ in, long ld_in,
+                                                               float* __restrict__ out, long ld_out, int V) {
+  const __nv_bfloat16* r = in + (long)blockIdx.y * ld_in;
+  float* o = out + (long)blockIdx.y * ld_out;
+  const int step = gridDim.x * blockDim.x, i0 = blockIdx.x * blockDim.x + threadIdx.x;
+  int done = 0;
+  if (((reinterpret_cast<uintptr_t>(r) | reinterpret_cast<uintptr_t>(o)) & 15) == 0) {
+    for (int c = i0; c < V >> 3; c += step) {
+      const uint4 q = reinterpret_cast<const uint4*>(r)[c];
+      const float2 f0 = unpack_bf16x2(q.x), f1 = unpack_bf16x2(q.y), f2 = unpack_bf16x2(q.z), f3 = unpack_bf16x2(q.w);
+      reinterpret_cast<float4*>(o)[2 * c] = make_float4(f0.x, f0.y, f1.x, f1.y);
+      reinterpret_cast<float4*>(o)[2 * c + 1] = make_float4(f2.x, f2.y, f3.x, f3.y);
+    }
+    done = V & ~7;
+  }
+  for (int i = done + i0; i < V; i += step) o[i] = __bfloat162float(r[i]);
 }
 
 }  // namespace b200
@@ -327,8 +501,9 @@ B200_API int b200_argmax(const void* logits, int dtype, long ld, int B, int V, v
 B200_API int b200_cast_bf16_f32(const void* in, long ld_in, void* out, long ld_out, int B, int V,
                                 cudaStream_t stream) {
   if (B <= 0) return 0;
-  cast_bf16_to_f32_kernel<<<B, 1024, 0, stream>>>((const __nv_bfloat16*)in, ld_in, (float*)out,
-                                                  ld_out, V);
+  // 64 elements a thread
+  cast_bf16_to_f32_kernel<<<dim3((unsigned)((V + 16383) / 16384), (unsigned)B), 256, 0, stream>>>(
+      (const __nv_bfloat16*)in, ld_in, (float*)out, ld_out, V);
   return B200_CHECK_LAUNCH();
 }
 
@@ -356,9 +531,34 @@ B200_API int b200_sample(void* logits_f32, long ld, int B, int V, const void* te
                          const void* seeds, const void* offsets, void* out,
                          cudaStream_t stream) {
   if (B <= 0) return 0;
-  sample_kernel<<<B, SAMP_THREADS, 0, stream>>>(
-      (float*)logits_f32, ld, V, (const float*)temperature, (const int*)top_k,
-      (const float*)top_p, (const float*)min_p, (const unsigned long long*)seeds,
-      (const long*)offsets, (long*)out);
-  return B200_CHECK_LAUNCH();
+  const int slice = ((V + SAMP_C - 1) / SAMP_C + 3) / 4 * 4;
+  const int resident = slice <= SAMP_MAX_SLICE;
+  const size_t smem = resident ? (size_t)slice * 4 : 0;
+  static size_t smem_set = 0;
+  if (smem > smem_set) {
+    cudaError_t e = cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    smem_set = smem;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(SAMP_T);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = SAMP_C;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  for (int b0 = 0; b0 < B; b0 += 65535) {
+    const int nb = B - b0 < 65535 ? B - b0 : 65535;
+    cfg.gridDim = dim3(SAMP_C, (unsigned)nb);
+    cudaError_t e = cudaLaunchKernelEx(
+        &cfg, sample_kernel, (float*)logits_f32 + (long)b0 * ld, ld, V, slice, resident,
+        temperature ? (const float*)temperature + b0 : nullptr, top_k ? (const int*)top_k + b0 : nullptr,
+        top_p ? (const float*)top_p + b0 : nullptr, min_p ? (const float*)min_p + b0 : nullptr,
+        seeds ? (const unsigned long long*)seeds + b0 : nullptr, offsets ? (const long*)offsets + b0 : nullptr, (long*)out + b0);
+    if (e != cudaSuccess) return (int)e;
+  }
+  return 0;
 }
