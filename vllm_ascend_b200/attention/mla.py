@@ -10,6 +10,7 @@ Cache layout contract: two paged tensors per layer, latent
 """
 from __future__ import annotations
 
+import functools
 from typing import Optional
 
 import torch
@@ -36,14 +37,24 @@ def _split_scratch(dev, numel: int) -> torch.Tensor:
     return buf
 
 
+def _most_splits(sms: int, ctas: int) -> int:
+    return min(_MAX_SPLITS, max(1, (2 * sms + ctas - 1) // max(ctas, 1)))
+
+
+@functools.lru_cache(maxsize=4096)
+def _best_splits(sms: int, ctas: int, tiles: int) -> int:
+    return min(range(1, min(tiles, _most_splits(sms, ctas)) + 1), key=lambda s: (-(-ctas * s // sms)) * (-(-tiles // s) + 2))
+
+
 def _num_splits(dev, ctas: int, max_keys: int) -> int:
-    """Splits of the key range that give about two CTAs per SM, at most one per 128-key tile."""
+    """Splits of the key range: at most one per 128-key tile and two CTAs per SM.  A CTA has an SM to itself, so what a split
+    count costs is its waves times the tiles that a CTA walks one after the other, and two more for its start and end (32 sequences
+    of 2500 to 5700 tokens, 32 heads: ten splits in three waves 137 us)."""
     from ..batch_invariant import is_batch_invariant
     if is_batch_invariant():
         return 1
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
-    tiles = max(1, (max_keys + 127) // 128)
-    return max(1, min(tiles, (2 * sms + ctas - 1) // max(ctas, 1), _MAX_SPLITS))
+    return _best_splits(sms, max(ctas, 1), max(1, (max_keys + 127) // 128))
 
 
 def _tc_sizes_ok(q_lat: torch.Tensor, q_pe: torch.Tensor, lat_cache: torch.Tensor) -> bool:
@@ -155,7 +166,9 @@ def reserve_mla_scratch(device, rows: int, heads: int, width: int = 512, max_key
     """Allocate the split-KV scratch of decode batches of up to ``rows`` rows up front (before graph
     capture, whose batches all use it)."""
     hb = (heads + 31) // 32 if heads > 16 else 1
-    worst = max(r * _num_splits(device, r * hb, max_keys or _MAX_SPLITS * 128) for r in range(1, rows + 1))
+    sms = torch.cuda.get_device_properties(device).multi_processor_count
+    tiles = max(1, ((max_keys or _MAX_SPLITS * 128) + 127) // 128)
+    worst = max(r * min(tiles, _most_splits(sms, r * hb)) for r in range(1, rows + 1))
     _split_scratch(device, worst * heads * (width + 1))
 
 
@@ -216,6 +229,64 @@ def mla_paged_attention(q_lat: torch.Tensor, q_pe: torch.Tensor, lat_cache: torc
         p = torch.softmax(s, dim=-1)[..., :sl]
         out[qs:qe] = torch.einsum("hqk,kc->qhc", p, lat).to(out.dtype)
     return out
+
+
+#: query-key pairs per key from which prompts attend over up-projected keys and values: per head a pair costs 2 x 1088
+#: operations in the latent space (at the 110 TFLOP/s its kernel reaches on prompts) and 2 x 320 over them, a key 2 x 512 x 256 to
+#: project up; level at about 12 pairs per key.  And the most memory the projected rows may take.
+_EXPAND_PAIRS_PER_KEY, _EXPAND_BYTES = 16, 1 << 30
+
+
+def expanded_prompts(meta, heads: int, dn: int, dr: int, dv: int, q: torch.Tensor, lat_cache: torch.Tensor,
+                     pe_cache: torch.Tensor) -> Optional[tuple[int, int]]:
+    """(sequences, keys): the step's prompts that attend over up-projected latents are all sequences behind the first
+    ``sequences`` (those have one token each), ``keys`` is the number of their keys; None where the latent space is the better
+    place (decode steps, few new tokens behind long contexts) or the only one (captured or batch-invariant steps)."""
+    import numpy as np
+    from .. import envs
+    from ..batch_invariant import is_batch_invariant
+    if not (q.is_cuda and q.dtype == lat_cache.dtype == torch.bfloat16 and meta.max_query_len > 1
+            and envs.VLLM_B200_MLA_ATTN == "tcgen05") or is_batch_invariant() or torch.cuda.is_current_stream_capturing():
+        return None
+    if dn != 128 or dv % 8 or not 8 <= dv <= 128 or dr % 8 or not 8 <= dr <= 64 or lat_cache.shape[-1] % 8 \
+            or not (q.is_contiguous() and lat_cache.is_contiguous() and pe_cache.is_contiguous()):
+        return None
+    B = meta.num_reqs
+    new = np.diff(np.asarray(meta.query_start_loc_cpu[:B + 1], dtype=np.int64))
+    seen = np.asarray(meta.seq_lens_cpu[:B], dtype=np.int64)
+    first = int(np.argmax(new != 1))                       # max_query_len > 1: there is one
+    new, seen = new[first:], seen[first:]
+    keys = int(seen.sum())
+    pairs = int((new * (seen - new) + new * (new + 1) // 2).sum())
+    if (new < 1).any() or pairs < _EXPAND_PAIRS_PER_KEY * keys or keys * heads * (dn + dv) * 2 > _EXPAND_BYTES:
+        return None
+    return first, keys
+
+
+def prompt_attention_expanded(q: torch.Tensor, kv_b: torch.Tensor, lat_cache: torch.Tensor, pe_cache: torch.Tensor, meta,
+                              scale: float, dv: int, first: int, keys: int, out: torch.Tensor) -> None:
+    """Causal attention of the sequences behind the first ``first`` over keys and values projected up from their latents:
+    q [T, H, dn + dr] (rotated), kv_b [H (dn + dv), dc], out [T, H, dv] (those sequences' rows are written)."""
+    from .. import ops
+    T, H, D = q.shape
+    dc, dr = lat_cache.shape[-1], pe_cache.shape[-1]
+    n, dev = meta.num_reqs - first, q.device
+    lat = torch.empty((keys, dc), dtype=q.dtype, device=dev)
+    pe = torch.empty((keys, dr), dtype=q.dtype, device=dev)
+    starts = torch.empty(n + 1, dtype=torch.int32, device=dev)
+    table, lens = meta.block_table[first:], meta.seq_lens[first:]
+    status = _native.status_word(dev).data_ptr()
+    rc = _native.lib().b200_gather_latents(
+        lat_cache.data_ptr(), pe_cache.data_ptr(), dc, dr, lat_cache.shape[1], lat_cache.shape[0], lens.data_ptr(),
+        table.data_ptr(), table.stride(0), n, keys, starts.data_ptr(), lat.data_ptr(), pe.data_ptr(), status, _native.stream_ptr())
+    _native.check(rc, "gather_latents")
+    _native.count_launch(2)
+    kv = ops.linear(lat, kv_b)
+    rc = _native.lib().b200_attn_prefill_latent(
+        q.data_ptr(), q.stride(0), T, kv.data_ptr(), pe.data_ptr(), keys, meta.query_start_loc[first:].data_ptr(),
+        starts.data_ptr(), lens.data_ptr(), n, T - first, H, D - dr, dr, dv, scale, out.data_ptr(), status, _native.stream_ptr())
+    _native.check(rc, "attn_prefill_latent")
+    _native.count_launch()
 
 
 class B200MLABackend:

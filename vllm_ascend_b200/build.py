@@ -80,16 +80,17 @@ def _compile_one(src: str, hdr_digest: str, verbose: bool) -> tuple[str, bool]:
 
 #: sources a model needs, for builds that compile no more than that (architecture -> names; others: all)
 MODEL_SOURCES = {
-    "Vofelix": ("activations", "attention_decode", "attention_mla_decode", "cache_ops", "gemm_bf16", "gemm_bf16_2cta",
-                "latent_attention", "linear_attention", "mla_preprocess", "sampler", "stream_norm"),
+    "Vofelix": ("activations", "attention_decode", "attention_mla_decode", "attention_prefill", "cache_ops",
+                "gemm_bf16", "gemm_bf16_2cta", "gemm_small", "latent_attention", "linear_attention", "mla_preprocess", "sampler",
+                "stream_norm"),
     "Pegopel": ("activations", "attention_decode", "attention_decode_tc", "attention_tc", "attention_variant", "cache_ops",
-                "gemm_bf16", "gemm_bf16_2cta", "qkv_prep", "sampler", "stream_norm"),
-    "Dubizen": ("activations", "attention_decode", "attention_decode_tc", "attention_mla_decode", "attention_tc",
-                "attention_variant", "cache_ops", "elementwise", "gemm_bf16", "gemm_bf16_2cta", "latent_attention",
-                "mla_preprocess", "moe", "qkv_prep", "sampler", "stream_norm"),
+                "gemm_bf16", "gemm_bf16_2cta", "gemm_small", "qkv_prep", "sampler", "stream_norm"),
+    "Dubizen": ("activations", "attention_decode", "attention_decode_tc", "attention_mla_decode", "attention_prefill",
+                "attention_tc", "attention_variant", "cache_ops", "elementwise", "gemm_bf16", "gemm_bf16_2cta", "gemm_small",
+                "latent_attention", "mla_preprocess", "moe", "qkv_prep", "sampler", "stream_norm"),
     "Nevotar": ("activations", "attention_decode", "attention_decode_tc", "attention_tc", "attention_variant",
-                "attention_wide", "cache_ops", "elementwise", "gemm_bf16", "gemm_bf16_2cta", "group_norm", "linear_attention",
-                "linear_recurrence", "moe", "qkv_prep", "sampler", "stream_norm"),
+                "attention_wide", "cache_ops", "elementwise", "gemm_bf16", "gemm_bf16_2cta", "gemm_small",
+                "group_norm", "linear_attention", "linear_recurrence", "moe", "qkv_prep", "sampler", "stream_norm"),
 }
 
 

@@ -345,6 +345,9 @@ class MLAAttention:
             ops.mla_preprocess(q, kv, self.kv_a_norm.weight, self.kv_a_norm.eps, meta.positions, self.cos_sin,
                                meta.slot_mapping, lat_cache, pe_cache, self.dn, self.dr)
             q_pe = q[..., self.dn:]
+            o = self._attend_expanded(q, lat_cache, pe_cache, meta)
+            if o is not None:
+                return self.o_proj(o)
         else:
             latent = self.kv_a_norm(kv[:, :self.dc].contiguous())[0]
             k_pe = kv[:, self.dc:].reshape(T, 1, self.dr)
@@ -385,6 +388,9 @@ class MLAAttention:
                              self.q_a_norm.eps, meta.positions, self.cos_sin, meta.slot_mapping, lat_cache, pe_cache)
         q = self.q_b_proj(qr).view(T, self.H, self.dn + self.dr)
         nope = ops.latent_query(q, meta.positions, self.cos_sin)
+        o = self._attend_expanded(q, lat_cache, pe_cache, meta)
+        if o is not None:
+            return self.o_proj(o)
         q_lat = self._per_head_matmul(nope, self.W_UK, self.W_UK_nk)
         dcp = pstate.get_dcp_group()
         if dcp.world_size > 1:
@@ -397,6 +403,34 @@ class MLAAttention:
                                         window=self.window, sink=self.sink, out=o_lat)
         o = self._per_head_matmul(o_lat, self.W_UV, self.W_UV_nk)
         return self.o_proj(o.reshape(T, self.H * self.dv))
+
+    def _attend_expanded(self, q: torch.Tensor, lat_cache, pe_cache, meta) -> Optional[torch.Tensor]:
+        """Attention output [T, H dv] of a step with prompts that attend over up-projected keys and values; the one-token
+        sequences in front of them stay in the latent space.  None: the whole step does.  q [T, H, dn + dr] is rotated."""
+        from ..attention import mla as mla_ops
+        if self.window or self.sink is not None or self.index_topk or pstate.get_dcp_group().world_size > 1 \
+                or self.kv_b_proj.weight.dtype != q.dtype or self.kv_b_proj.weight.device != q.device:
+            return None
+        plan = mla_ops.expanded_prompts(meta, self.H, self.dn, self.dr, self.dv, q, lat_cache, pe_cache)
+        if plan is None:
+            return None
+        first, keys = plan
+        T = q.shape[0]
+        out = torch.empty((T, self.H, self.dv), dtype=q.dtype, device=q.device)
+        if first:
+            import copy
+            dm = copy.copy(meta)
+            dm.num_reqs, dm.max_query_len = first, 1
+            dm.query_start_loc, dm.seq_lens, dm.block_table = (meta.query_start_loc[:first + 1], meta.seq_lens[:first],
+                                                               meta.block_table[:first])
+            dm.max_seq_len = int(meta.seq_lens_cpu[:first].max())
+            qd = q[:first]
+            q_lat = self._per_head_matmul(qd[..., :self.dn], self.W_UK, self.W_UK_nk)
+            o_lat = torch.empty((self.H, first, self.dc), dtype=q.dtype, device=q.device).transpose(0, 1)
+            mla_ops.mla_paged_attention(q_lat, qd[..., self.dn:], lat_cache, pe_cache, dm, self.scale, out=o_lat)
+            out[:first] = self._per_head_matmul(o_lat, self.W_UV, self.W_UV_nk)
+        mla_ops.prompt_attention_expanded(q, self.kv_b_proj.weight, lat_cache, pe_cache, meta, self.scale, self.dv, first, keys, out)
+        return out.view(T, self.H * self.dv)
 
     def load_part(self, part: str, w: torch.Tensor) -> None:
         """One un-fused tensor: q (or, through a latent, dq, dq.norm, uq), dkv (joint down-projection), dkv.norm,
