@@ -62,3 +62,26 @@ def test_rows_do_not_depend_on_the_row_count_within_a_tile():
     full = ops.linear_step(x, w)
     for m in (1, 16, 33, 100):
         assert torch.equal(ops.linear_step(x[:m], w), full[:m])
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 2048), (256, 4096, 2048), (130, 1000, 4096)])
+def test_row_statistics_are_those_of_the_stored_rows(M, N, K):
+    g = torch.Generator(device=DEV).manual_seed(N)
+    x = torch.randn(M, K, device=DEV, generator=g).bfloat16()
+    w = (torch.randn(N, K, device=DEV, generator=g) * 0.05).bfloat16()
+    res = torch.randn(M, N, device=DEV, generator=g).bfloat16()
+    ss = ops.alloc_row_stats(300, 4096, torch.device(DEV))
+    want = ops.linear_step(x, w, None, res)
+    out = ops.linear_norm_folded(x, w, residual=res, out=res, ss_out=ss)       # in place on the stream
+    assert out is res and torch.equal(out, want)
+    parts = int(ss[32 * 300:32 * 300 + 1].view(torch.int32))
+    assert parts == (N + 127) // 128
+    got = ss[:parts * 300].view(parts, 300)[:, :M]
+    sq = torch.nn.functional.pad(out.double() ** 2, (0, parts * 128 - N)).view(M, parts, 128).sum(-1).t()
+    assert ((got.double() - sq).abs() <= sq * 2.0 ** -20).all()
+    # the next product reads them
+    w2 = (torch.randn(256, N, device=DEV, generator=g) * 0.05).bfloat16()
+    y = ops.linear_norm_folded(out, w2, ss_in=ss, norm_dim=N, eps=1e-6)
+    ref = (out.double() @ w2.double().t()) * torch.rsqrt((out.double() ** 2).mean(-1, keepdim=True) + 1e-6)
+    assert ((y.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-3).all()
+    _native.check_status(torch.device(DEV))

@@ -37,6 +37,9 @@ struct SmallGemmParams {
   const __nv_bfloat16* bias;
   const __nv_bfloat16* residual;
   __nv_bfloat16* C;
+  float* ss_out;                   // [tile][ss_stride]: sum of squares of each stored output row within the tile, or null
+  long ss_stride;
+  int ss_parts_max;                // behind that many parts: how many there are
   int* status;
 };
 
@@ -185,6 +188,8 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   if (*abort_word == 0) {
     if (!p.glu) {
       const int col = tile * SG_ROWS + lane * 4;
+      if (p.ss_out && tile == 0 && split == 0 && threadIdx.x == 0)
+        *reinterpret_cast<int*>(p.ss_out + (long)p.ss_parts_max * p.ss_stride) = gridDim.y;
       for (int t = t0 + warp; t < t1; t += SG_THREADS / 32) {
         float4 v = sg_sum(part, p.splits, (uint32_t)(t * SG_ROWS + lane * 4) * 4);
         if (col < p.N) {                                  // N is a multiple of 8
@@ -198,7 +203,16 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
             const float2 b0 = unpack_bf16x2(b.x), b1 = unpack_bf16x2(b.y);
             v.x += b0.x; v.y += b0.y; v.z += b1.x; v.w += b1.y;
           }
-          *reinterpret_cast<uint2*>(p.C + (size_t)t * p.ldc + col) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+          const uint2 o = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+          *reinterpret_cast<uint2*>(p.C + (size_t)t * p.ldc + col) = o;
+          const float2 f0 = unpack_bf16x2(o.x), f1 = unpack_bf16x2(o.y);       // of the values as stored
+          v = make_float4(f0.x, f0.y, f1.x, f1.y);
+        } else {
+          v = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        if (p.ss_out) {
+          const float ss = warp_reduce_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w);
+          if (lane == 0) p.ss_out[(long)tile * p.ss_stride + t] = ss;
         }
       }
     } else {
@@ -304,4 +318,25 @@ B200_API int b200_gemm_small_bf16(const void* A, const void* W, void* C, const v
   p.C = (__nv_bfloat16*)C;
   p.status = status;
   return launch_small(A, W, p, lda, ldw, splits, stream);
+}
+
+// The same with the row statistics of the output (b200_gemm_bf16_2cta_norm's row_ss_out): ss_out holds ss_parts_max parts of
+// ss_stride rows and the part count; one part per 128 columns.
+B200_API int b200_gemm_small_stats(const void* A, const void* W, void* C, const void* bias, const void* residual, int M, int N,
+                                   int K, int lda, int ldw, int ldc, void* ss_out, long ss_stride, int ss_parts_max, int* status,
+                                   cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (M > 256 || K <= 0 || (K & 7) || (N & 7) || (lda & 7) || (ldw & 7) || (ldc & 7)) return 9100;
+  if (!ss_out || ss_stride < M || (long)ss_parts_max * SG_ROWS < N) return 9135;
+  SmallGemmParams p;
+  memset(&p, 0, sizeof(p));
+  p.M = M; p.N = N; p.K = K; p.ldc = ldc;
+  p.bias = (const __nv_bfloat16*)bias;
+  p.residual = (const __nv_bfloat16*)residual;
+  p.C = (__nv_bfloat16*)C;
+  p.ss_out = (float*)ss_out;
+  p.ss_stride = ss_stride;
+  p.ss_parts_max = ss_parts_max;
+  p.status = status;
+  return launch_small(A, W, p, lda, ldw, 0, stream);
 }
