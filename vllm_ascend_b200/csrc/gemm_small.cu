@@ -16,12 +16,12 @@
 // (gate / up) 80 -> 53, 151936 x 4096 282 -> 204 (6.1 TB/s).
 // Roles: warps 0..3 read the accumulator (one TMEM lane quarter each), warp 4 issues TMA, warp 5 issues
 // tcgen05.mma (cta_group::1, M = 128, N = tokens, K = 16, f32 in TMEM); all six reduce and store.
+#include "cluster_sum.cuh"
 #include "common.cuh"
 #include "tmap_cache.cuh"
 
 namespace b200 {
 
-constexpr int SG_ROWS = 128;       // weight rows per tile
 constexpr int SG_BK = 64;          // columns per stage (128 bytes: one swizzle row)
 constexpr int SG_THREADS = 192;
 constexpr int SG_WBYTES = SG_ROWS * SG_BK * 2;
@@ -42,33 +42,6 @@ struct SmallGemmParams {
   int ss_parts_max;                // behind that many parts: how many there are
   int* status;
 };
-
-__device__ __forceinline__ uint32_t sg_map(uint32_t saddr, uint32_t rank) {
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
-  return a;
-}
-__device__ __forceinline__ float4 sg_ld(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(addr)
-               : "memory");
-  return v;
-}
-__device__ __forceinline__ void sg_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-
-// Sum of four neighbouring rows of one token over the blocks of the cluster, in block order.
-__device__ __forceinline__ float4 sg_sum(const uint32_t part, int splits, uint32_t off) {
-  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int r = 0; r < splits; r++) {
-    const float4 v = sg_ld(sg_map(part + off, r));
-    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-  }
-  return s;
-}
 
 __device__ __forceinline__ float sg_gate(float g, float u, float alpha, float limit) {
   if (alpha > 0.f) {

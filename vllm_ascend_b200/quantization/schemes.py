@@ -111,6 +111,7 @@ def _declare_native():
     from ctypes import c_int, c_long, c_void_p
     P, I, L = c_void_p, c_int, c_long
     _native.register_signature("b200_gemm_fp8_block", [P, P, P, P, P, P, I, I, I, I, I, I, P, P])
+    _native.register_signature("b200_gemm_small_fp8", [P, P, P, P, P, P, I, I, I, I, I, I, I, P, P])
     _native.register_signature("b200_grouped_gemm_fp8_block",
                                [P, P, P, P, P, P, I, L, I, I, I, I, I, P, P])
     _native.register_signature("b200_gemm_fp8_channel", [P, P, P, P, P, P, I, I, I, I, I, I, P, P])
@@ -119,6 +120,10 @@ def _declare_native():
 
 
 _declare_native()
+
+
+#: most rows of the few-row GEMM
+_FP8_FEW_ROWS = 128
 
 
 def fp8_block_linear(x: Optional[torch.Tensor], w8: torch.Tensor, w_scale: torch.Tensor,
@@ -132,6 +137,15 @@ def fp8_block_linear(x: Optional[torch.Tensor], w8: torch.Tensor, w_scale: torch
     N = w8.shape[0]
     out = torch.empty((M, N), dtype=torch.bfloat16, device=xq.device)
     if M == 0:
+        return out
+    from ..batch_invariant import is_batch_invariant
+    if M <= _FP8_FEW_ROWS and not is_batch_invariant():
+        # K split over blocks: rows may differ in the last bit from those of a larger batch
+        rc = _native.lib().b200_gemm_small_fp8(
+            xq.data_ptr(), xs.data_ptr(), w8.data_ptr(), w_scale.data_ptr(), out.data_ptr(), _native.ptr(bias), M, N, K,
+            xq.stride(0), w8.stride(0), out.stride(0), 0, _native.status_word(xq.device).data_ptr(), _native.stream_ptr())
+        _native.check(rc, "gemm_small_fp8")
+        ops.launch_counter[0] += 1
         return out
     rc = _native.lib().b200_gemm_fp8_block(
         xq.data_ptr(), xs.data_ptr(), w8.data_ptr(), w_scale.data_ptr(), out.data_ptr(),
