@@ -156,8 +156,10 @@ __global__ void penalties_kernel(float* logits, long ld, int V, const long* prom
 //     atomics where there were V per pass;
 //   * bins are integers (mass in units of 2^-40: shared memory adds 64-bit integers by itself, floats in a loop, and the
 //     sum has no order), added and searched in parallel (256 per block, then one warp);
+//   * where the cut leaves at most 2048 elements (top-k, peaked top-p), one block sorts them and ends the row by itself;
 //   * random numbers are drawn only for groups of four that hold a kept element.
-// 192 rows of 151936: one block per row with thread-serial bins 738 us, this 267 us.
+// 192 rows of 151936: one block per row with thread-serial bins 738 us, 267 us in shared memory of the
+// cluster, 187 us with rows of few candidates finished by one block.
 constexpr int SAMP_C = 8;              // blocks per row
 constexpr int SAMP_T = 512;
 constexpr int SAMP_BINS = 2048;
@@ -179,6 +181,7 @@ struct SampSmem {
   int si[32];
   samp_n sn[SAMP_T / 32];
   uint32_t prefix;
+  uint32_t listed;                     // candidates in hist (rank 0)
 };
 
 __device__ __forceinline__ void samp_cluster_sync() {
@@ -303,6 +306,100 @@ __device__ void samp_pass(const float* e, int n, SampSmem* s, int pass, int shif
   __syncthreads();
 }
 
+// Elements above the cut, gathered from the whole cluster into rank 0's `hist` as (key, inverted index): value descending, index
+// ascending is then one 64-bit order.
+__device__ void samp_gather(const float* e, int n, int first, uint32_t cut, SampSmem* s) {
+  uint32_t list, count;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(list) : "r"(smem_u32(s->hist)));
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(count) : "r"(smem_u32(&s->listed)));
+  const int lane = threadIdx.x & 31;
+  for (int i0 = threadIdx.x - lane; i0 < n; i0 += SAMP_T) {
+    const int i = i0 + lane;
+    const uint32_t k = i < n ? __float_as_uint(e[i]) : 0;
+    const uint32_t on = __ballot_sync(0xffffffffu, i < n && k >= cut);
+    if (on == 0) continue;
+    uint32_t at = 0;
+    if (lane == 0) asm volatile("atom.relaxed.cluster.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(at) : "r"(count), "r"(__popc(on)) : "memory");
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(on & ((1u << lane) - 1));
+    if ((on >> lane & 1) && at < SAMP_BINS) {
+      const samp_n v = (samp_n)k << 32 | (uint32_t)~(first + i);
+      asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(list + at * 8), "l"(v) : "memory");
+    }
+  }
+}
+
+// Rank 0 alone: orders the n gathered candidates, cuts them by rank and by mass, and runs the race.  `mass` is what top-p is a
+// share of where top-k is off.
+__device__ int samp_finish(SampSmem* s, int n, int k, float pth, float mp, float mass, uint2 key, long offset, int fallback) {
+  samp_n* c = s->hist;
+  int size = 32;
+  while (size < n) size *= 2;
+  for (int i = n + threadIdx.x; i < size; i += SAMP_T) c[i] = 0;
+  __syncthreads();
+  for (int len = 2; len <= size; len *= 2)
+    for (int step = len / 2; step > 0; step /= 2) {
+      for (int t = threadIdx.x; t < size / 2; t += SAMP_T) {
+        const int i = 2 * t - (t & (step - 1)), j = i + step;
+        const samp_n a = c[i], b = c[j];
+        if ((a < b) == ((i & len) == 0)) { c[i] = b; c[j] = a; }       // descending
+      }
+      __syncthreads();
+    }
+  auto value = [&](int i) { return (uint32_t)(c[i] >> 32); };
+  uint32_t thr = k > 0 ? value(k - 1) : 0;
+  if (pth < 1.f) {
+    // running mass in units of 2^-40: a thread sums its run of neighbours, then their sums are scanned
+    constexpr int PER = SAMP_BINS / SAMP_T;
+    samp_n run[PER], sum = 0;
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+      const int i = threadIdx.x * PER + j;
+      if (i < n && value(i) >= thr) sum += __float2ull_rn(__uint_as_float(value(i)) * SAMP_UNIT);
+      run[j] = sum;
+    }
+    samp_n upto = sum;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const samp_n t = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += t;
+    }
+    if (lane == 31) s->sn[warp] = upto;
+    if (threadIdx.x == 0) s->prefix = 0;
+    __syncthreads();
+    samp_n before = upto - sum, all = 0;
+    for (int w = 0; w < SAMP_T / 32; w++) {
+      if (w < warp) before += s->sn[w];
+      all += s->sn[w];
+    }
+    const samp_n want = __float2ull_rn(pth * (k > 0 ? (float)all / SAMP_UNIT : mass) * SAMP_UNIT);
+#pragma unroll
+    for (int j = 0; j < PER; j++) {                        // the first element at which the sum reaches what is wanted
+      const int i = threadIdx.x * PER + j;
+      const samp_n prev = before + (j ? run[j - 1] : 0);
+      if (i < n && before + run[j] >= want && (prev < want || i == 0)) s->prefix = value(i);
+    }
+    __syncthreads();
+    if (want == 0) thr = 0xffffffffu;                      // a share of nothing: the largest element
+    else if (s->prefix > thr) thr = s->prefix;
+  }
+  if (mp > 0.f && __float_as_uint(mp) > thr) thr = __float_as_uint(mp);
+  float bestv = -INFINITY;
+  int besti = fallback;
+  for (int i = threadIdx.x; i < n; i += SAMP_T) {
+    const float v = __uint_as_float(value(i));
+    if (value(i) < thr) break;
+    if (!(v > 0.f)) continue;
+    const int idx = (int)~(uint32_t)c[i];
+    const uint4 rnd = philox4x32(make_uint4((uint32_t)(idx & ~3), (uint32_t)offset, (uint32_t)((unsigned long long)offset >> 32), 0u), key);
+    const uint32_t r = (idx & 2) ? ((idx & 1) ? rnd.w : rnd.z) : ((idx & 1) ? rnd.y : rnd.x);
+    const float ex = -__logf(u32_to_unit(r));  // Exp(1)
+    samp_better(bestv, besti, v / fmaxf(ex, 1e-20f), idx);
+  }
+  block_argmax(bestv, besti, s->sv, s->si);
+  return besti;
+}
+
 // logits: fp32 [B, V] (already penalised); overwritten where a row does not fit the cluster's shared memory.
 // temperature/top_k/top_p/min_p: per row (top_k <= 0 or >= V: off; top_p >= 1: off).
 // seeds: per-row uint64 seed, offsets: per-row counter (e.g. number of tokens generated).
@@ -345,6 +442,7 @@ sample_kernel(float* logits, long ld, int V, int slice, int resident, const floa
       if (v > best) { best = v; bi = first + i; }
     }
   }
+  if (threadIdx.x == 0) s.listed = 0;
   samp_cluster_argmax(best, bi, &s, &s.xch[0]);
   if (T < 1e-5f) {
     if (rank == 0 && threadIdx.x == 0) out[b] = bi;
@@ -393,10 +491,25 @@ sample_kernel(float* logits, long ld, int V, int slice, int resident, const floa
   uint32_t thr_key = 0;                // keep elements with key >= thr_key
 
   const int k = top_k ? top_k[b] : 0;
-  if (k > 0 && k < V) {
-    uint32_t cut = 0;
+  const float pth = top_p ? top_p[b] : 1.f, mp = min_p ? min_p[b] : 0.f;
+  const unsigned long long seed = seeds ? seeds[b] : 0ull;
+  const long offset = offsets ? offsets[b] : 0;
+  const uint2 key = make_uint2((uint32_t)seed, (uint32_t)(seed >> 32));
+  const bool by_rank = k > 0 && k < V;
+  uint32_t cut = 0, above = 0;         // the highest cut that holds enough, and how many elements reach it
 #pragma unroll
-    for (int j = SAMP_CUTS - 1; j >= 0; j--) if (nc[j] >= (uint32_t)k) cut = cuts[j];
+  for (int j = SAMP_CUTS - 1; j >= 0; j--)
+    if (by_rank ? nc[j] >= (uint32_t)k : pth < 1.f && zc[j] >= pth * mass * 1.001f) { cut = cuts[j]; above = nc[j]; }
+  if (cut != 0 && above <= SAMP_BINS) {
+    // everything that can be kept fits one block: no more meetings of the cluster
+    samp_gather(e, n, first, cut, &s);
+    samp_cluster_sync();
+    if (rank != 0) return;
+    const int win = samp_finish(&s, (int)above, by_rank ? k : 0, pth, mp, mass, key, offset, bi);
+    if (threadIdx.x == 0) out[b] = win;
+    return;
+  }
+  if (by_rank) {
     if (threadIdx.x == 0) { s.prefix = 0; s.remaining = (samp_n)k; }
     __syncthreads();
     samp_pass<false>(e, n, &s, 0, 21, 11, 0x00000000u, cut, rank);
@@ -415,9 +528,8 @@ sample_kernel(float* logits, long ld, int V, int slice, int resident, const floa
     mass = 0.f;
     for (int r = 0; r < SAMP_C; r++) mass += samp_peek(&s.xch[2].v[0], r);
   }
-  const float pth = top_p ? top_p[b] : 1.f;
   if (pth < 1.f) {
-    uint32_t cut = 0;                  // a margin for the order of the sums
+    cut = 0;                           // a margin for the order of the sums
 #pragma unroll
     for (int j = SAMP_CUTS - 1; j >= 0; j--) if (zc[j] >= pth * mass * 1.001f) cut = cuts[j];
     if (thr_key > cut) cut = thr_key;
@@ -428,15 +540,11 @@ sample_kernel(float* logits, long ld, int V, int slice, int resident, const floa
     samp_pass<true>(e, n, &s, 5, 0, 10, 0xFFFFFC00u, cut, rank);
     if (s.prefix > thr_key) thr_key = s.prefix;
   }
-  const float mp = min_p ? min_p[b] : 0.f;
   if (mp > 0.f) {
     const uint32_t tm = __float_as_uint(mp);  // max e is exactly 1
     if (tm > thr_key) thr_key = tm;
   }
   // ---- exponential race over the kept set
-  const unsigned long long seed = seeds ? seeds[b] : 0ull;
-  const long offset = offsets ? offsets[b] : 0;
-  const uint2 key = make_uint2((uint32_t)seed, (uint32_t)(seed >> 32));
   float bestv = -INFINITY;
   int besti = bi;
   for (int i0 = threadIdx.x * 4; i0 < n; i0 += SAMP_T * 4) {     // slices start at multiples of four
