@@ -225,12 +225,25 @@ __global__ void qknorm_rope_kvwrite_kernel(__nv_bfloat16* qkv, long qkv_stride,
   }
 }
 
-// Fast path for D = 128 with full rotary (rot_dim = 128).  The op moves ~27 KB per token and is
-// limited by instruction issue as much as by bytes, so: a half-warp owns one (token, head) row and
-// lane l holds elements [4l, 4l+4) AND their rotation partners [64+4l, 64+4l+4) (two 8-byte
-// accesses, each half-warp access covers 128 contiguous bytes), which makes the rotation
-// shuffle-free; a warp walks QKN_ROWS_PER_WARP rows and issues all row loads up front.
-constexpr int QKN_ROWS_PER_WARP = 8;     // 4 rows per half-warp
+// Fast path for D = 128 with full rotary (rot_dim = 128).  The op moves ~27 KB per token and is limited by instruction issue
+// as much as by bytes, so: eight lanes own one (token, head) row, lane l holds elements [8l, 8l+8) AND their rotation partners
+// [64+8l, 64+8l+8) (two 16-byte accesses, each covers 128 contiguous bytes of the row), which makes the rotation shuffle-free; a
+// warp walks QKN_ROWS_PER_WARP rows, issues all row loads up front and divides in 32 bits.  8192 tokens of 32 + 2 x 8 heads:
+// 87 us with 8-byte accesses and 64-bit divisions, 65 us so.
+constexpr int QKN_ROWS_PER_WARP = 16;    // 4 rows per group of eight lanes
+
+__device__ __forceinline__ void unpack8(const uint4& q, float* v) {
+  const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const float2 f = unpack_bf16x2(w[j]);
+    v[2 * j] = f.x;
+    v[2 * j + 1] = f.y;
+  }
+}
+__device__ __forceinline__ uint4 pack8(const float* v) {
+  return make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+}
 
 __global__ void __launch_bounds__(256)
 qknorm_rope_kvwrite_d128_kernel(__nv_bfloat16* qkv, long qkv_stride,
@@ -242,101 +255,89 @@ qknorm_rope_kvwrite_d128_kernel(__nv_bfloat16* qkv, long qkv_stride,
                                 const long* __restrict__ slot_mapping, int T, int Hq, int Hkv,
                                 long num_slots, int block_size, int kv_layout, int* status) {
   constexpr int D = 128;
-  constexpr int RPT = QKN_ROWS_PER_WARP / 2;          // rows per thread
-  const int heads_total = Hq + 2 * Hkv;
-  const long total_rows = (long)T * heads_total;
-  const long gw = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  constexpr int RPT = QKN_ROWS_PER_WARP / 4;           // rows per thread
+  const uint32_t heads_total = Hq + 2 * Hkv;
+  const uint32_t total_rows = (uint32_t)T * heads_total;
+  const uint32_t gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  const int hl = lane & 15;                            // lane inside the half-warp
-  const long row0 = gw * QKN_ROWS_PER_WARP + (lane >> 4);
+  const int hl = lane & 7;                             // lane inside the row's group
+  const uint32_t row0 = gw * QKN_ROWS_PER_WARP + (lane >> 3);
   if (gw * QKN_ROWS_PER_WARP >= total_rows) return;
 
-  uint2 lo[RPT], hi[RPT];                              // elements 4hl.. and 64+4hl..
+  uint4 lo[RPT], hi[RPT];                              // elements 8hl.. and 64+8hl..
   int tt[RPT], hh[RPT];
   bool ok[RPT];
 #pragma unroll
   for (int i = 0; i < RPT; i++) {
-    const long r = row0 + 2 * i;
+    const uint32_t r = row0 + 4 * i;
     ok[i] = r < total_rows;
-    const long rc = ok[i] ? r : 0;
+    const uint32_t rc = ok[i] ? r : 0;
     tt[i] = (int)(rc / heads_total);
-    hh[i] = (int)(rc - (long)tt[i] * heads_total);
-    const uint2* src = reinterpret_cast<const uint2*>(qkv + (long)tt[i] * qkv_stride + (long)hh[i] * D);
-    lo[i] = ok[i] ? src[hl] : make_uint2(0u, 0u);
-    hi[i] = ok[i] ? src[16 + hl] : make_uint2(0u, 0u);
-  }
-  // norm weights of this thread's 8 columns (q and k), shared by all of its rows
-  float wq[8], wk[8];
-  {
-    const uint2 z = make_uint2(0u, 0u);
-    const uint2 a0 = q_norm_w ? reinterpret_cast<const uint2*>(q_norm_w)[hl] : z;
-    const uint2 a1 = q_norm_w ? reinterpret_cast<const uint2*>(q_norm_w)[16 + hl] : z;
-    const uint2 b0 = k_norm_w ? reinterpret_cast<const uint2*>(k_norm_w)[hl] : z;
-    const uint2 b1 = k_norm_w ? reinterpret_cast<const uint2*>(k_norm_w)[16 + hl] : z;
-    const uint32_t aw[4] = {a0.x, a0.y, a1.x, a1.y}, bw[4] = {b0.x, b0.y, b1.x, b1.y};
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const float2 fa = unpack_bf16x2(aw[j]), fb = unpack_bf16x2(bw[j]);
-      wq[2 * j] = fa.x; wq[2 * j + 1] = fa.y;
-      wk[2 * j] = fb.x; wk[2 * j + 1] = fb.y;
-    }
+    hh[i] = (int)(rc - (uint32_t)tt[i] * heads_total);
+    const uint4* src = reinterpret_cast<const uint4*>(qkv + (long)tt[i] * qkv_stride + (long)hh[i] * D);
+    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+    lo[i] = ok[i] ? src[hl] : z;
+    hi[i] = ok[i] ? src[8 + hl] : z;
   }
   // rotary angles of the token the previous row belonged to: a thread's rows are heads of one token
   // most of the time, so the table is read once per token instead of once per (token, head)
   int t_cs = -1;
-  float cc[4] = {1.f, 1.f, 1.f, 1.f}, sv[4] = {0.f, 0.f, 0.f, 0.f};
+  float cc[8], sv[8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) { cc[j] = 1.f; sv[j] = 0.f; }
 #pragma unroll
   for (int i = 0; i < RPT; i++) {
     const int t = tt[i], h = hh[i];
     const bool is_q = h < Hq;
     const bool is_k = !is_q && h < Hq + Hkv;
     const bool rot = is_q || is_k;
-    uint2 olo = lo[i], ohi = hi[i];
+    uint4 olo = lo[i], ohi = hi[i];
     // every lane takes part in the reduction shuffles; rows past the end carry zeros
-    float v[8];                                          // v[0..3] first half, v[4..7] partners
-    {
-      const uint32_t w32[4] = {lo[i].x, lo[i].y, hi[i].x, hi[i].y};
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const float2 f = unpack_bf16x2(w32[j]);
-        v[2 * j] = f.x; v[2 * j + 1] = f.y;
-      }
-    }
-    const bool has_norm = is_q ? (q_norm_w != nullptr) : (is_k && k_norm_w != nullptr);
+    float v1[8], v2[8];                                  // first half, rotation partners
+    unpack8(olo, v1);
+    unpack8(ohi, v2);
     float ss = 0.f;
 #pragma unroll
-    for (int j = 0; j < 8; j++) ss += v[j] * v[j];
+    for (int j = 0; j < 8; j++) ss += v1[j] * v1[j] + v2[j] * v2[j];
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    for (int o = 4; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if (rot) {
-      if (has_norm) {
+      const __nv_bfloat16* w = is_q ? q_norm_w : k_norm_w;
+      if (w) {
         const float inv = rsqrtf(ss / (float)D + eps);
+        float w1[8], w2[8];
+        unpack8(reinterpret_cast<const uint4*>(w)[hl], w1);
+        unpack8(reinterpret_cast<const uint4*>(w)[8 + hl], w2);
 #pragma unroll
-        for (int j = 0; j < 8; j++)      // rounded to bf16 like the unfused norm -> rope sequence
-          v[j] = __bfloat162float(__float2bfloat16(v[j] * inv * (is_q ? wq[j] : wk[j])));
+        for (int j = 0; j < 8; j++) {    // rounded to bf16 like the unfused norm -> rope sequence
+          v1[j] = __bfloat162float(__float2bfloat16(v1[j] * inv * w1[j]));
+          v2[j] = __bfloat162float(__float2bfloat16(v2[j] * inv * w2[j]));
+        }
       }
       if (t != t_cs) {
-        const float* cs = cos_sin + positions[t] * (long)D + hl * 4;
-        const float4 c = *reinterpret_cast<const float4*>(cs);
-        const float4 sn = *reinterpret_cast<const float4*>(cs + 64);
-        cc[0] = c.x; cc[1] = c.y; cc[2] = c.z; cc[3] = c.w;
-        sv[0] = sn.x; sv[1] = sn.y; sv[2] = sn.z; sv[3] = sn.w;
+        const float4* cs = reinterpret_cast<const float4*>(cos_sin + positions[t] * (long)D + hl * 8);
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+          const float4 c = cs[j], sn = cs[16 + j];
+          cc[4 * j] = c.x; cc[4 * j + 1] = c.y; cc[4 * j + 2] = c.z; cc[4 * j + 3] = c.w;
+          sv[4 * j] = sn.x; sv[4 * j + 1] = sn.y; sv[4 * j + 2] = sn.z; sv[4 * j + 3] = sn.w;
+        }
         t_cs = t;
       }
-      float x1[4], x2[4];
+      float x1[8], x2[8];
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        x1[j] = v[j] * cc[j] - v[4 + j] * sv[j];
-        x2[j] = v[4 + j] * cc[j] + v[j] * sv[j];
+      for (int j = 0; j < 8; j++) {
+        x1[j] = v1[j] * cc[j] - v2[j] * sv[j];
+        x2[j] = v2[j] * cc[j] + v1[j] * sv[j];
       }
-      olo = make_uint2(pack_bf16x2(x1[0], x1[1]), pack_bf16x2(x1[2], x1[3]));
-      ohi = make_uint2(pack_bf16x2(x2[0], x2[1]), pack_bf16x2(x2[2], x2[3]));
+      olo = pack8(x1);
+      ohi = pack8(x2);
     }
     if (!ok[i]) continue;
     if (rot) {
-      uint2* dst = reinterpret_cast<uint2*>(qkv + (long)t * qkv_stride + (long)h * D);
+      uint4* dst = reinterpret_cast<uint4*>(qkv + (long)t * qkv_stride + (long)h * D);
       dst[hl] = olo;
-      dst[16 + hl] = ohi;
+      dst[8 + hl] = ohi;
     }
     if (!is_q && k_cache) {
       const long slot = slot_mapping[t];
@@ -348,12 +349,12 @@ qknorm_rope_kvwrite_d128_kernel(__nv_bfloat16* qkv, long qkv_stride,
       const int kvh = is_k ? (h - Hq) : (h - Hq - Hkv);
       long row = slot * Hkv + kvh;
       if (kv_layout == 1) {
-        const long blk = slot / block_size, off = slot - blk * block_size;
-        row = (blk * Hkv + kvh) * block_size + off;
+        const uint32_t blk = (uint32_t)slot / (uint32_t)block_size, off = (uint32_t)slot - blk * (uint32_t)block_size;
+        row = ((long)blk * Hkv + kvh) * block_size + off;
       }
-      uint2* dst = reinterpret_cast<uint2*>((is_k ? k_cache : v_cache) + row * (long)D);
+      uint4* dst = reinterpret_cast<uint4*>((is_k ? k_cache : v_cache) + row * (long)D);
       dst[hl] = olo;
-      dst[16 + hl] = ohi;
+      dst[8 + hl] = ohi;
     }
   }
 }
@@ -630,9 +631,9 @@ static int qknorm_rope_impl(void* qkv, long qkv_stride, const void* positions,
       (const __nv_bfloat16*)q_norm_w, (const __nv_bfloat16*)k_norm_w, eps,                    \
       (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, (const long*)slot_mapping, T, Hq, Hkv, \
       num_slots, block_size, kv_layout, status, (const int*)mrope_axis, pos_stride)
-  if (D == 128 && rot_dim == 128 && (qkv_stride & 3) == 0 && !mrope_axis &&
+  if (D == 128 && rot_dim == 128 && (qkv_stride & 7) == 0 && !mrope_axis && warps < (1l << 31) && num_slots < (1l << 31) &&
       (((uintptr_t)qkv | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)q_norm_w |
-        (uintptr_t)k_norm_w) & 7) == 0) {
+        (uintptr_t)k_norm_w | (uintptr_t)cos_sin) & 15) == 0) {
     const long w8 = (warps + QKN_ROWS_PER_WARP - 1) / QKN_ROWS_PER_WARP;
     const unsigned blocks8 = (unsigned)((w8 + wpb - 1) / wpb);
     qknorm_rope_kvwrite_d128_kernel<<<blocks8, wpb * 32, 0, stream>>>(
