@@ -7,14 +7,16 @@
 //
 // The scales change every 128 columns of K, so products of different K blocks cannot
 // be summed inside the tensor core.  Two-level accumulation:
-//   warp 0      TMA producer: 128 x 128 e4m3 tiles of A and W (one 128-byte swizzle row each)
-//   warp 1      tcgen05.mma kind::f8f6f4 (M=128, N=128, K=32 x 4) per K block into one of two
+//   warp 0      TMA producer: 128 x 128 e4m3 tiles of A, BN x 128 of W (one 128-byte swizzle row each)
+//   warp 1      tcgen05.mma kind::f8f6f4 (M=128, N=BN, K=32 x 4) per K block into one of two
 //               TMEM partial buffers (fresh accumulator every block)
-//   warps 2..9  read the partial with tcgen05.ld, scale it by a_scale * w_scale and add it to
-//               fp32 accumulators held in registers; store bf16 at the end.  Two warpgroups
-//               split the tile's 128 columns (64 accumulators per thread, both TMEM loads of a
-//               K block in flight before the one wait): the promotion of a block has to keep up
+//   warps 2..   read the partial with tcgen05.ld, scale it by a_scale * w_scale and add it to
+//               fp32 accumulators held in registers; store bf16 at the end.  A warpgroup per 64
+//               columns of the tile (64 accumulators per thread): the promotion of a block has to keep up
 //               with its MMA, which four warps with 128 accumulators each did not
+// Tiles are 128 x 256 where they fill the GPU as well as 128 x 128 do: a K block of the small tile brings 32 KB for
+// 4.2 MFLOP, and at 1.3 PFLOP/s that is 10 TB/s out of L2, which bounds it (four warpgroups and four buffers for the
+// small tile changed nothing); the wide one brings 24 KB for the same.
 // The MMA of block kb+1 overlaps the promotion of block kb.  Grouped mode (MoE experts)
 // uses per-group row offsets and per-expert weight / scale matrices.  Bounded waits.
 #include "common.cuh"
@@ -24,14 +26,19 @@
 
 namespace b200 {
 
-constexpr int F8_BM = 128, F8_BN = 128, F8_BK = 128;
-constexpr int F8_THREADS = 320;            // producer, MMA issuer, 2 x 4 promotion warps
-constexpr int F8_HALF = F8_BN / 2;         // columns per promotion warpgroup
-constexpr int F8_STAGES = 6;
-constexpr int F8_TILE_BYTES = 128 * 128;                 // 16 KB per operand tile
-constexpr int F8_STAGE_BYTES = 2 * F8_TILE_BYTES;
+constexpr int F8_BM = 128, F8_BK = 128;
+constexpr int F8_BLOCK = 128;              // rows of W that share a scale
+constexpr int F8_COLS = 64;                // columns per promotion warpgroup
+constexpr int F8_TILE_BYTES = 128 * 128;                 // 16 KB per 128 operand rows
 constexpr int F8_MAX_GROUPS = 512;
-constexpr int F8_SMEM_BYTES = F8_STAGES * F8_STAGE_BYTES + 1024 + 256 + (F8_MAX_GROUPS + 1) * 4;
+
+template <int BN>
+struct F8Cfg {
+  static constexpr int kThreads = 64 + 2 * BN;           // producer, MMA issuer, BN / 64 promotion warpgroups
+  static constexpr int kStages = BN == 256 ? 4 : 6;
+  static constexpr int kStageBytes = F8_TILE_BYTES * (1 + BN / 128);
+  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256 + (F8_MAX_GROUPS + 1) * 4;
+};
 
 struct Fp8Params {
   int M, N, K, ldc;
@@ -57,6 +64,7 @@ struct F8Tile {
   int row0, row_end, tn, w_row0, group;
 };
 
+template <int BN>
 __device__ __forceinline__ void f8_tile(const Fp8Params& p, const int* grp_tiles, int t, F8Tile& c) {
   if (p.num_groups > 0) {
     const int total_m = grp_tiles[p.num_groups];
@@ -71,19 +79,21 @@ __device__ __forceinline__ void f8_tile(const Fp8Params& p, const int* grp_tiles
     c.row0 = p.group_offsets[lo] + (tm_global - grp_tiles[lo]) * F8_BM;
     c.row_end = p.group_offsets[lo + 1];
     c.tn = tn;
-    c.w_row0 = lo * p.w_rows_per_group + tn * F8_BN;
+    c.w_row0 = lo * p.w_rows_per_group + tn * BN;
   } else {
     c.group = 0;
     c.row0 = (t % p.tiles_m) * F8_BM;
     c.row_end = p.M;
     c.tn = t / p.tiles_m;
-    c.w_row0 = c.tn * F8_BN;
+    c.w_row0 = c.tn * BN;
   }
 }
 
-__global__ void __launch_bounds__(F8_THREADS, 1)
+template <int BN>
+__global__ void __launch_bounds__(F8Cfg<BN>::kThreads, 1)
 gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a,
                       const __grid_constant__ CUtensorMap tmap_b, const Fp8Params p) {
+  constexpr int F8_STAGES = F8Cfg<BN>::kStages, F8_STAGE_BYTES = F8Cfg<BN>::kStageBytes;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* tiles = smem;
@@ -105,7 +115,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
     for (int b = 0; b < 2; b++) {
       mbar_init(&part_full[b], 1);
-      mbar_init(&part_empty[b], 8);
+      mbar_init(&part_empty[b], 4 * (BN / F8_COLS));
     }
     *abort_word = 0;
     mbar_fence_init();
@@ -128,7 +138,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
   }
   if (warp == 1) {
-    tmem_alloc(tmem_ptr, 256);
+    tmem_alloc(tmem_ptr, 2 * BN);
     tmem_relinquish();
   }
   if (warp == 0 && lane == 0) {
@@ -147,14 +157,16 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a,
     uint32_t phase = 0;
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
       F8Tile c;
-      f8_tile(p, grp_tiles, t, c);
+      f8_tile<BN>(p, grp_tiles, t, c);
       for (int kb = 0; kb < num_kb; kb++) {
         if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_word)) goto done;
         if (lane == 0) {
           uint8_t* sa = tiles + stage * F8_STAGE_BYTES;
           mbar_expect_tx(&full_bar[stage], F8_STAGE_BYTES);
           tma_load_2d(sa, &tmap_a, &full_bar[stage], kb * F8_BK, c.row0);
-          tma_load_2d(sa + F8_TILE_BYTES, &tmap_b, &full_bar[stage], kb * F8_BK, c.w_row0);
+#pragma unroll
+          for (int h = 0; h < BN / 128; h++)
+            tma_load_2d(sa + (1 + h) * F8_TILE_BYTES, &tmap_b, &full_bar[stage], kb * F8_BK, c.w_row0 + h * 128);
         }
         __syncwarp();
         if (++stage == F8_STAGES) { stage = 0; phase ^= 1; }
@@ -162,7 +174,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    constexpr uint32_t idesc = make_idesc_e4m3(F8_BM, F8_BN);
+    constexpr uint32_t idesc = make_idesc_e4m3(F8_BM, BN);
     int stage = 0;
     uint32_t phase = 0;
     uint32_t it = 0;          // K blocks issued so far (selects the partial buffer)
@@ -179,7 +191,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a,
           for (int kk = 0; kk < F8_BK / 32; kk++) {       // 32 e4m3 = 32 bytes per MMA
             const uint64_t da = make_smem_desc(sa + kk * 32, 16, 1024, kLayoutSw128);
             const uint64_t db = make_smem_desc(sb + kk * 32, 16, 1024, kLayoutSw128);
-            umma_f8_ss(tmem_base + b * F8_BN, da, db, idesc, kk > 0 ? 1u : 0u);
+            umma_f8_ss(tmem_base + b * BN, da, db, idesc, kk > 0 ? 1u : 0u);
           }
           umma_commit(&empty_bar[stage]);
           umma_commit(&part_full[b]);
@@ -191,21 +203,22 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a,
   } else {
     // ------------------------------------------------------------ promotion + epilogue
     const int q = warp & 3;                              // TMEM lane quarter this warp may read
-    const int half = (warp - 2) >> 2;                    // which 64 columns of the tile
+    const int wg = (warp - 2) >> 2;                      // which 64 columns of the tile
     const int kblocks = p.K / F8_BK;                     // columns of the scale matrices
-    const int n_blocks = (p.N + F8_BN - 1) / F8_BN;
+    const int n_blocks = (p.N + F8_BLOCK - 1) / F8_BLOCK;
     uint32_t it = 0;
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
       F8Tile c;
-      f8_tile(p, grp_tiles, t, c);
+      f8_tile<BN>(p, grp_tiles, t, c);
       const int row = c.row0 + q * 32 + lane;
       const bool row_ok = row < c.row_end;
       const bool per_channel = p.row_scale != nullptr;
       const float* as_row = per_channel ? nullptr : p.a_scale + (size_t)(row_ok ? row : 0) * kblocks;
-      const float* ws_row = per_channel ? nullptr : p.w_scale + ((size_t)c.group * n_blocks + c.tn) * kblocks;
-      float acc[F8_HALF];
+      const int blk = min(c.tn * (BN / F8_BLOCK) + wg * F8_COLS / F8_BLOCK, n_blocks - 1);     // columns beyond N have no scale
+      const float* ws_row = per_channel ? nullptr : p.w_scale + ((size_t)c.group * n_blocks + blk) * kblocks;
+      float acc[F8_COLS];
 #pragma unroll
-      for (int i = 0; i < F8_HALF; i++) acc[i] = 0.f;
+      for (int i = 0; i < F8_COLS; i++) acc[i] = 0.f;
       float sc_next = per_channel ? 1.f : as_row[0] * ws_row[0];
       for (int kb = 0; kb < num_kb; kb++, it++) {
         const int b = it & 1;
@@ -213,27 +226,44 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a,
         if (!per_channel && kb + 1 < num_kb) sc_next = as_row[kb + 1] * ws_row[kb + 1];
         if (!mbar_wait(&part_full[b], (it >> 1) & 1u, abort_word)) goto done;
         tc_fence_after();
-        const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + b * F8_BN + half * F8_HALF;
-        uint32_t r0[32], r1[32];
-        tmem_ld_32x32b_x32(t_row, r0);
-        tmem_ld_32x32b_x32(t_row + 32, r1);
-        tmem_ld_wait();
-        // the partial is in registers: the MMA warp may overwrite the buffer
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&part_empty[b]);
+        const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + b * BN + wg * F8_COLS;
+        if constexpr (BN == 128) {
+          uint32_t r0[32], r1[32];
+          tmem_ld_32x32b_x32(t_row, r0);
+          tmem_ld_32x32b_x32(t_row + 32, r1);
+          tmem_ld_wait();
+          // the partial is in registers: the MMA warp may overwrite the buffer
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&part_empty[b]);
 #pragma unroll
-        for (int i = 0; i < 32; i++) acc[i] = fmaf(__uint_as_float(r0[i]), sc, acc[i]);
+          for (int i = 0; i < 32; i++) acc[i] = fmaf(__uint_as_float(r0[i]), sc, acc[i]);
 #pragma unroll
-        for (int i = 0; i < 32; i++) acc[32 + i] = fmaf(__uint_as_float(r1[i]), sc, acc[32 + i]);
+          for (int i = 0; i < 32; i++) acc[32 + i] = fmaf(__uint_as_float(r1[i]), sc, acc[32 + i]);
+        } else {
+          // 576 threads: 16 columns at a time keep the accumulators in registers
+#pragma unroll
+          for (int c0 = 0; c0 < F8_COLS; c0 += 16) {
+            uint32_t r[16];
+            tmem_ld_32x32b_x16(t_row + c0, r);
+            tmem_ld_wait();
+            if (c0 + 16 == F8_COLS) {
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&part_empty[b]);
+            }
+#pragma unroll
+            for (int i = 0; i < 16; i++) acc[c0 + i] = fmaf(__uint_as_float(r[i]), sc, acc[c0 + i]);
+          }
+        }
       }
       if (row_ok) {
         __nv_bfloat16* crow = p.C + (size_t)row * p.ldc;
         const float rs = per_channel ? p.row_scale[row] : 1.f;
         const float* cs = per_channel ? p.col_scale + (size_t)c.group * p.N : nullptr;
 #pragma unroll
-        for (int g = 0; g < F8_HALF / 8; g++) {
-          const int col = c.tn * F8_BN + half * F8_HALF + g * 8;
+        for (int g = 0; g < F8_COLS / 8; g++) {
+          const int col = c.tn * BN + wg * F8_COLS + g * 8;
           if (col < p.N) {
             float v[8];
 #pragma unroll
@@ -274,7 +304,7 @@ done:
   }
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 256);
+    tmem_dealloc(tmem_base, 2 * BN);
   }
 }
 
@@ -319,28 +349,36 @@ static int get_tmap_u8(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_
   return 0;
 }
 
-static int launch_fp8(const void* A, const void* W, Fp8Params& p, int lda, int ldw, long a_rows,
-                      long w_rows, cudaStream_t stream) {
+template <int BN>
+static int launch_fp8_bn(const CUtensorMap& ta, const CUtensorMap& tb, Fp8Params& p, cudaStream_t stream) {
+  using Cfg = F8Cfg<BN>;
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_block_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         F8_SMEM_BYTES);
+    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_block_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
     if (e != cudaSuccess) return (int)e;
     attr_set = true;
   }
+  p.tiles_n = (p.N + BN - 1) / BN;
+  int grid = num_sms();
+  if (p.num_groups == 0 && p.tiles_m * p.tiles_n < grid) grid = p.tiles_m * p.tiles_n;
+  gemm_fp8_block_kernel<BN><<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(ta, tb, p);
+  return B200_CHECK_LAUNCH();
+}
+
+static int launch_fp8(const void* A, const void* W, Fp8Params& p, int lda, int ldw, long a_rows,
+                      long w_rows, cudaStream_t stream) {
   CUtensorMap ta, tb;
   int rc = get_tmap_u8(&ta, A, (uint64_t)a_rows, (uint64_t)p.K, (uint64_t)lda);
   if (rc) return rc;
   rc = get_tmap_u8(&tb, W, (uint64_t)w_rows, (uint64_t)p.K, (uint64_t)ldw);
   if (rc) return rc;
   p.tiles_m = (p.M + F8_BM - 1) / F8_BM;
-  p.tiles_n = (p.N + F8_BN - 1) / F8_BN;
   p.num_kb = p.K / F8_BK;
-  int grid = num_sms();
-  if (p.num_groups == 0 && p.tiles_m * p.tiles_n < grid) grid = p.tiles_m * p.tiles_n;
-  gemm_fp8_block_kernel<<<grid, F8_THREADS, F8_SMEM_BYTES, stream>>>(ta, tb, p);
-  return B200_CHECK_LAUNCH();
+  // waves times width: a wide tile counts 1.6 narrow ones.  Groups keep the narrow tile (their rows are not known here).
+  const long sms = num_sms();
+  auto waves = [&](int bn) { return ((long)p.tiles_m * ((p.N + bn - 1) / bn) + sms - 1) / sms; };
+  if (p.num_groups == 0 && waves(256) * 16 < waves(128) * 10) return launch_fp8_bn<256>(ta, tb, p, stream);
+  return launch_fp8_bn<128>(ta, tb, p, stream);
 }
 
 }  // namespace b200
