@@ -80,7 +80,7 @@ def _compile_one(src: str, hdr_digest: str, verbose: bool) -> tuple[str, bool]:
 
 #: sources a model needs, for builds that compile no more than that (architecture -> names; others: all)
 MODEL_SOURCES = {
-    "Vofelix": ("activations", "attention_decode", "attention_mla_decode", "attention_prefill", "cache_ops",
+    "Vofelix": ("activations", "attention_decode", "attention_mla_decode", "attention_prefill", "cache_ops", "delta_chunk",
                 "gemm_bf16", "gemm_bf16_2cta", "gemm_small", "latent_attention", "linear_attention", "mla_preprocess", "sampler",
                 "stream_norm"),
     "Pegopel": ("activations", "attention_decode", "attention_decode_tc", "attention_tc", "attention_variant", "cache_ops",
@@ -89,7 +89,7 @@ MODEL_SOURCES = {
                 "attention_tc", "attention_variant", "cache_ops", "elementwise", "gemm_bf16", "gemm_bf16_2cta", "gemm_small",
                 "latent_attention", "mla_preprocess", "moe", "qkv_prep", "sampler", "stream_norm"),
     "Nevotar": ("activations", "attention_decode", "attention_decode_tc", "attention_tc", "attention_variant",
-                "attention_wide", "cache_ops", "elementwise", "gemm_bf16", "gemm_bf16_2cta", "gemm_small",
+                "attention_wide", "cache_ops", "delta_chunk", "elementwise", "gemm_bf16", "gemm_bf16_2cta", "gemm_small",
                 "group_norm", "linear_attention", "linear_recurrence", "moe", "qkv_prep", "sampler", "stream_norm"),
 }
 

@@ -9,6 +9,7 @@
 // Counterparts of the reference's causal_conv1d and recurrent / chunked gated-delta-rule ops
 // (csrc/moe/causal_conv1d*, csrc/attention/recurrent_gated_delta_rule*, ops/triton/fla/*).
 #include "common.cuh"
+#include "delta_chunk.h"
 #include "dtypes.cuh"
 
 namespace b200 {
@@ -195,6 +196,7 @@ struct DeltaParams {
   int l2norm;
   long num_slots;
   int* status;
+  int max_len;            // sequences with at least this many tokens are left alone (0: none are)
 };
 
 constexpr int DELTA_CHUNK = 16;      // tokens per stage: eight of the 128 threads work on each
@@ -219,7 +221,7 @@ __global__ void __launch_bounds__(128) gated_delta_rule_kernel(const DeltaParams
     if (threadIdx.x == 0 && p.status) atomicExch(p.status, B200_BAD_INDEX);
     return;
   }
-  if (t0 >= t1) return;
+  if (t0 >= t1 || (p.max_len > 0 && t1 - t0 >= p.max_len)) return;
   const int DK = p.DK, DV = p.DV;
   float* sp = p.state + ((long)slot * p.Hv + hv) * DK * DV;
   auto row_of = [&](int r) { return (r >> 2) * 32 + gl * 4 + (r & 3); };
@@ -601,19 +603,21 @@ B200_API int b200_causal_conv1d(const void* x, long x_stride, const void* w, con
   return dtype ? launch_conv<float>(p, T, stream) : launch_conv<__nv_bfloat16>(p, T, stream);
 }
 
-// uniform: every sequence of the step has exactly one token.  z (optional, with norm_w [DV] and eps, uniform
+// chunk_min > 0: sequences of at least that many tokens run in chunks where the sizes allow it (delta_chunk.cu); any_short:
+// there are shorter ones.  uniform: every sequence of the step has exactly one token.  z (optional, with norm_w [DV] and eps, uniform
 // steps only): the output is the gated RMS norm of the read-out; returns -1 when the sizes do not allow that.
 B200_API int b200_gated_delta_rule(const void* q, const void* k, const void* v, long qk_stride,
                                    long v_stride, const void* g, const void* beta, void* state,
                                    const void* cu, const void* slots, const void* has_init, void* out,
                                    long out_stride, int B, int Hk, int Hv, int DK, int DV, float scale,
                                    int l2norm, long num_slots, int dtype, int uniform, const void* z, long z_stride,
-                                   const void* norm_w, float eps, int* status, cudaStream_t stream) {
+                                   const void* norm_w, float eps, int chunk_min, int any_short, int* status,
+                                   cudaStream_t stream) {
   if (B <= 0) return 0;
   if (Hk <= 0 || Hv % Hk || Hv > 65535) return 9801;
   DeltaParams p{q, k, v, qk_stride, v_stride, (const float*)g, (const float*)beta, (float*)state, (const int*)cu,
                 (const int*)slots, (const int*)has_init, out, out_stride, Hk, Hv, DK, DV, scale, l2norm, num_slots,
-                status};
+                status, 0};
   if (uniform) {
     DeltaDecodeExtra x{z, z_stride, norm_w, eps};
     int rc = 0;
@@ -622,5 +626,15 @@ B200_API int b200_gated_delta_rule(const void* q, const void* k, const void* v, 
       return rc;
   }
   if (z) return -1;
+  if (chunk_min > 0 && dtype == 0) {
+    const DeltaChunkArgs a{q, k, v, qk_stride, v_stride, (const float*)g, (const float*)beta, (float*)state, (const int*)cu,
+                           (const int*)slots, (const int*)has_init, out, out_stride, Hk, Hv, DV, scale, l2norm, num_slots,
+                           chunk_min, status};
+    int rc = 0;
+    if (launch_delta_chunk(a, B, DK, stream, &rc)) {
+      if (rc || !any_short) return rc;
+      p.max_len = chunk_min;
+    }
+  }
   return dtype ? launch_delta<float>(p, B, stream) : launch_delta<__nv_bfloat16>(p, B, stream);
 }

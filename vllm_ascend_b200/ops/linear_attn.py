@@ -15,7 +15,7 @@ P, I, L, Fl = c_void_p, c_int, c_long, c_float
 _native.register_signature("b200_causal_conv1d", [P, L, P, P, P, P, P, P, P, L, L, I, I, I, I, I, L, I, P, L, P, P, I, P, P,
                                                   P, P])
 _native.register_signature("b200_gated_delta_rule", [P, P, P, L, L, P, P, P, P, P, P, P, L, I, I, I, I, I, Fl, I,
-                                                     L, I, I, P, L, P, Fl, P, P])
+                                                     L, I, I, P, L, P, Fl, I, I, P, P])
 _DTYPES = {torch.bfloat16: 0, torch.float32: 1}
 
 
@@ -199,14 +199,27 @@ def gated_delta_rule_chunked(q, k, v, g, beta, state, cu_cpu, slots, has_init, s
 
 
 def _chunk_min(on_cuda: bool = False) -> int:
-    """Fewest new tokens of a sequence that take the chunk-parallel form; 0 = never.  Unset, the
-    form serves host tensors only: on a B200 the recurrence kernel runs 4 x 2048 tokens of 32 heads in
-    1.3 ms, the chunk-parallel form built from fp32 matrix products in 10.3 ms."""
+    """Fewest new tokens of a sequence that take the chunk-parallel form built from fp32 matrix products; 0 = never.
+    Unset, the form serves host tensors only: on a B200 it takes 10.3 ms for 4 x 2048 tokens of 32 heads, the kernels 1.3 ms token
+    by token (three prompts of 2000 tokens: 1.6 ms, and 0.8 ms in chunks: ``_kernel_chunk_min``)."""
     import os
     from .. import envs
     if "VLLM_B200_GDN_CHUNK_MIN" not in os.environ and on_cuda:
         return 0
     return int(envs.VLLM_B200_GDN_CHUNK_MIN)
+
+
+#: new tokens of a sequence from which the kernel that works in chunks of 64 tokens is the faster one: a chunk, full or not, takes
+#: 19 us, a token of the token-serial kernel 0.7 us
+_KERNEL_CHUNK_MIN = 32
+
+
+def _kernel_chunk_min() -> int:
+    """0: token by token only (asked for with VLLM_B200_GDN_CHUNK_MIN=0, or batch-invariant mode: a portion's split into
+    chunks must not show)."""
+    import os
+    from ..batch_invariant import is_batch_invariant
+    return 0 if is_batch_invariant() or os.environ.get("VLLM_B200_GDN_CHUNK_MIN") == "0" else _KERNEL_CHUNK_MIN
 
 
 def gated_delta_rule(q, k, v, g, beta, state, cu, slots, has_init, scale, l2norm=True, cu_cpu=None, uniform=False,
@@ -250,17 +263,27 @@ def gated_delta_rule(q, k, v, g, beta, state, cu, slots, has_init, scale, l2norm
     uniform = bool(uniform and T == cu.numel() - 1)
     fused = uniform and gate is not None and gate[0].dtype == q.dtype and gate[1].dtype == q.dtype \
         and gate[0].stride(1) == 1
+    chunk_min = any_short = 0
+    if cu_cpu is not None and not uniform:
+        import numpy as np
+        lens = np.diff(np.asarray(cu_cpu)[:cu.numel()])
+        chunk_min = _kernel_chunk_min()
+        if chunk_min and (lens >= chunk_min).any():
+            any_short = int(((lens > 0) & (lens < chunk_min)).any())
+        else:
+            chunk_min = 0
     for z in ((gate[0], None) if fused else (None,)):
         rc = _native.lib().b200_gated_delta_rule(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), v.stride(0), g.data_ptr(), beta.data_ptr(),
             state.data_ptr(), cu.data_ptr(), slots.data_ptr(), has_init.data_ptr(), out.data_ptr(), out.stride(0),
             cu.numel() - 1, Hk, Hv, DK, DV, scale, int(l2norm), state.shape[0], _DTYPES[q.dtype], int(uniform),
             _native.ptr(z), 0 if z is None else z.stride(0), None if z is None else gate[1].data_ptr(),
-            0.0 if z is None else float(gate[2]), _native.status_word(q.device).data_ptr(), _native.stream_ptr())
+            0.0 if z is None else float(gate[2]), chunk_min, any_short, _native.status_word(q.device).data_ptr(),
+            _native.stream_ptr())
         if rc != -1:                  # -1: these sizes have no fused form, nothing was launched
             break
     _native.check(rc, "gated_delta_rule")
-    _native.count_launch()
+    _native.count_launch(1 + any_short)
     return out.view(T, Hv * DV) if z is not None else _gate(out, gate)
 
 
