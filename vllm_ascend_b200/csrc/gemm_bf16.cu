@@ -100,17 +100,21 @@ __device__ __forceinline__ bool tile_coord(const GemmParams& p, const int* grp_t
                                            TileCoord& c) {
   constexpr int BN_OUT = BN;  // columns of W consumed per tile
   if (p.mode & GEMM_GROUPED) {
-    // grp_tiles[e] = first tile (in units of M tiles) of group e
+    // grp_tiles[e] = M tiles of the groups before e.  Group after group, so that what is in flight are the rows and weights
+    // of few groups, each from HBM once.  All groups' rows for one column of tiles after another read rows that L2 does not hold once
+    // per column: 128 groups, 32000 rows, the two products of an expert layer together 458 us so and 372 us group by group; 384 rows
+    // 232 and 222 us.
     int lo = 0, hi = p.num_groups;
-    const int tm_global = t % grp_tiles[p.num_groups];
-    const int tn = t / grp_tiles[p.num_groups];
+    const int at = t / p.tiles_n;
     while (hi - lo > 1) {
       const int mid = (lo + hi) >> 1;
-      if (grp_tiles[mid] <= tm_global) lo = mid; else hi = mid;
+      if (grp_tiles[mid] <= at) lo = mid; else hi = mid;
     }
     const int e = lo;
+    const int local = t - grp_tiles[e] * p.tiles_n, tiles_m = grp_tiles[e + 1] - grp_tiles[e];
+    const int tn = local / tiles_m;
     const int g0 = p.group_offsets[e], g1 = p.group_offsets[e + 1];
-    c.row0 = g0 + (tm_global - grp_tiles[e]) * GEMM_BM;
+    c.row0 = g0 + (local - tn * tiles_m) * GEMM_BM;
     c.row_end = g1;
     c.tn = tn;
     const int ncols = (p.mode & GEMM_SWIGLU) ? BN_OUT / 2 : BN_OUT;
@@ -163,25 +167,34 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
     *abort_word = 0;
     mbar_fence_init();
-    if (p.mode & GEMM_GROUPED) {
-      // offsets come from device memory the caller filled: a table that is not ascending inside
-      // [0, M] (stale or overwritten) is reported and yields no tiles instead of addresses
-      int acc = 0;
-      bool ok = p.group_offsets[0] >= 0;
-      for (int e = 0; e < p.num_groups; e++) {
-        grp_tiles[e] = acc;
-        const int g0 = p.group_offsets[e], g1 = p.group_offsets[e + 1];
-        if (g1 < g0 || g1 > p.M) ok = false;
-        const int cnt = ok ? g1 - g0 : 0;
-        acc += (cnt + GEMM_BM - 1) / GEMM_BM;
+  }
+  if (warp == 0 && (p.mode & GEMM_GROUPED)) {
+    // offsets come from device memory the caller filled: a table that is not ascending inside
+    // [0, M] (stale or overwritten) is reported and yields no tiles instead of addresses
+    int acc = 0;
+    bool ok = true;
+    for (int base = 0; base < p.num_groups; base += 32) {       // 32 groups at a time: one by one, 128 groups took 5 us
+      const int e = base + lane;
+      const bool in = e < p.num_groups;
+      const int g0 = in ? p.group_offsets[e] : 0, g1 = in ? p.group_offsets[e + 1] : 0;
+      const bool bad = g0 < 0 || g1 < g0 || g1 > p.M;
+      ok = ok && !__any_sync(0xffffffffu, bad);
+      const int cnt = bad ? 0 : (g1 - g0 + GEMM_BM - 1) / GEMM_BM;
+      int incl = cnt;
+      for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += o;
       }
-      if (!ok) {
-        for (int e = 0; e <= p.num_groups; e++) grp_tiles[e] = 0;
-        acc = 0;
-        if (p.status) atomicCAS(p.status, 0, B200_BAD_INDEX);
-      }
-      grp_tiles[p.num_groups] = acc;
+      if (in) grp_tiles[e] = acc + incl - cnt;
+      acc += __shfl_sync(0xffffffffu, incl, 31);
     }
+    if (!ok) {
+      __syncwarp();
+      for (int e = lane; e < p.num_groups; e += 32) grp_tiles[e] = 0;
+      acc = 0;
+      if (lane == 0 && p.status) atomicCAS(p.status, 0, B200_BAD_INDEX);
+    }
+    if (lane == 0) grp_tiles[p.num_groups] = acc;
   }
   if (warp == 1) {
     tmem_alloc(tmem_ptr, Cfg::kTmemCols);
