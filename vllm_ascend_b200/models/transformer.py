@@ -100,9 +100,10 @@ class SparseMoeBlock:
         elif x.is_cuda and x.dtype == torch.bfloat16 and cfg.scoring_func == "softmax" and not cfg.use_mla:
             # softmax routers of bf16 checkpoints run their gate in the model dtype (as the
             # original implementation does): one tensor-core GEMM instead of an fp32 SIMT one
+            # (48 rows, 128 experts, K = 2048: one block's tile 18.4 us, K split over a cluster 6.0 us)
             if self._gate_bf16 is None:
                 self._gate_bf16 = self.gate_weight.to(torch.bfloat16)
-            logits = ops.linear(x, self._gate_bf16).float()
+            logits = ops.linear_step(x, self._gate_bf16).float()
         else:
             logits = torch.nn.functional.linear(x.float(), self.gate_weight)
         w, ids = fused_moe.gating_topk(logits, cfg.num_experts_per_tok, cfg.scoring_func,

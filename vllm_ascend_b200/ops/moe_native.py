@@ -69,7 +69,7 @@ class Permutation:
             self.cursor.data_ptr(), self.offsets.data_ptr(), self.pos.data_ptr(),
             self.src_token.data_ptr(), _native.stream_ptr())
         _native.check(rc, "moe_permute")
-        launch_counter[0] += 3
+        launch_counter[0] += 1 if T * k <= 8192 else 3       # few pairs are one block's work
         self.max_rows = T * k                      # rows beyond offsets[E] stay unused
 
     def row_weights(self, topk_w: torch.Tensor) -> torch.Tensor:
