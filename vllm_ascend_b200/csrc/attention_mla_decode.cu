@@ -67,7 +67,8 @@ struct MlaCfg {
   static constexpr int Q_SLAB = NQ * 128;
   static constexpr int P_HALF = NQ * 128;           // NQ rows x 64 keys
   static constexpr int P_BYTES = 2 * P_HALF;
-  static constexpr int MISC_BYTES = 2048;           // barriers, tmem pointer, reduction scratch
+  static constexpr int COL_OFF = 2048;              // barriers, tmem pointer, reduction scratch; then per column and warp
+  static constexpr int MISC_BYTES = COL_OFF + 2 * 4 * 32 * 4;
   static constexpr int smem_bytes(int slabs) {
     return slabs * (MLA_SLAB + Q_SLAB) + 2 * P_BYTES + MISC_BYTES + 1024;
   }
@@ -169,6 +170,8 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   volatile int* abort_word = (volatile int*)(tmem_ptr + 1);
   int* redi = (int*)(tmem_ptr + 4);        // [2 tiles][4 warps][NQ]
   float* redf = (float*)(redi + 2 * 4 * NQ);   // [4 warps][NQ]
+  float* col_max = (float*)(Ps + 2 * Cfg::P_BYTES + Cfg::COL_OFF);   // [4 warps][NQ] reference of the exponentials, log2 units
+  float* col_alpha = col_max + 4 * NQ;                               // [4 warps][NQ] factor of what has been summed
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
@@ -303,12 +306,15 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     const int tid = qd * 32 + lane;                 // key inside the tile; d inside a value block
     const uint32_t t_lane = tmem_base + ((uint32_t)(qd * 32) << 16);
     const float sl2 = p.scale_log2;
-    float m[NQ], lsum[NQ];
+    // A thread has one key and all columns for the scores, one column (its lane's) for the maxima: 128 keys took 7600 clocks between
+    // scores and probabilities with maxima and masks of all columns in every thread, of 17400 for the tile (PV takes as many, behind
+    // it).  32 heads, one block over 4096 keys 302 -> 203 us, 32 sequences of 4096 keys in four splits 122 -> 94 us.
+    const int col = lane & (NQ - 1);
+    col_max += qd * NQ;
+    col_alpha += qd * NQ;
+    float m = -INFINITY, lsum[NQ];
 #pragma unroll
-    for (int c = 0; c < NQ; c++) {
-      m[c] = -INFINITY;
-      lsum[c] = 0.f;
-    }
+    for (int c = 0; c < NQ; c++) lsum[c] = 0.f;
     for (int j = 0; j < n; j++) {
       const int b = j & 1;
       if (!mbar_wait(&s_ready[b], ((uint32_t)j >> 1) & 1u, abort_word)) goto done;
@@ -321,40 +327,48 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       if (lane == 0) mbar_arrive(&s_free[b]);
       const int key = ((t0 + j) << 7) + tid;
       float s[NQ];
-      int tok = 0, left = p.HC;                       // column c = (token c / HC, head c % HC)
-      int* rj = redi + (j & 1) * 4 * NQ + qd * NQ;
+      if (((t0 + j + 1) << 7) <= kv0 && p.window <= 0) {       // every row sees the whole tile
+#pragma unroll
+        for (int c = 0; c < NQ; c++) s[c] = __uint_as_float(r[c]);
+      } else {
+        int tok = 0, left = p.HC;                     // column c = (token c / HC, head c % HC)
+#pragma unroll
+        for (int c = 0; c < NQ; c++) {
+          const int kv_c = kv0 + tok;
+          const bool visible = tok < ntok && key < kv_c && (p.window <= 0 || key >= kv_c - p.window);
+          if (--left == 0) { left = p.HC; tok++; }
+          s[c] = visible ? __uint_as_float(r[c]) : -INFINITY;
+        }
+      }
+      int* rj = redi + (j & 1) * 4 * NQ;
+      int warp_max = 0;
 #pragma unroll
       for (int c = 0; c < NQ; c++) {
-        const int kv_c = kv0 + tok;
-        const bool visible = tok < ntok && key < kv_c && (p.window <= 0 || key >= kv_c - p.window);
-        if (--left == 0) { left = p.HC; tok++; }
-        s[c] = visible ? __uint_as_float(r[c]) : -INFINITY;
         int ob = __float_as_int(s[c]);
         ob ^= (ob >> 31) & 0x7fffffff;              // order-preserving float -> int
         const int wm = __reduce_max_sync(0xffffffffu, ob);
-        if (lane == 0) rj[c] = wm;
+        if (col == c) warp_max = wm;
       }
+      rj[qd * NQ + col] = warp_max;
       mla_softmax_bar();
-      const int* ra = redi + (j & 1) * 4 * NQ;
-      bool any_change = false;
-      float alpha[NQ];
-#pragma unroll
-      for (int c = 0; c < NQ; c++) {
-        int t = max(max(ra[c], ra[NQ + c]), max(ra[2 * NQ + c], ra[3 * NQ + c]));
-        t ^= (t >> 31) & 0x7fffffff;
-        const float mn = fmaxf(m[c], __int_as_float(t));
-        alpha[c] = 1.f;
-        if (mn > m[c] && (m[c] == -INFINITY || (mn - m[c]) * sl2 > kMlaRescaleLog2)) {
-          alpha[c] = (m[c] == -INFINITY) ? 0.f : mla_exp2((m[c] - mn) * sl2);
-          any_change = any_change || (m[c] != -INFINITY);
-          m[c] = mn;
-        }
-        lsum[c] *= alpha[c];
+      int t = max(max(rj[col], rj[NQ + col]), max(rj[2 * NQ + col], rj[3 * NQ + col]));
+      t ^= (t >> 31) & 0x7fffffff;
+      const float mn = fmaxf(m, __int_as_float(t));
+      float alpha = 1.f;
+      if (mn > m && (m == -INFINITY || (mn - m) * sl2 > kMlaRescaleLog2)) {
+        if (m != -INFINITY) alpha = mla_exp2((m - mn) * sl2);      // nothing has been summed before the first maximum
+        m = mn;
       }
+      col_max[col] = m == -INFINITY ? 0.f : m * sl2;
+      col_alpha[col] = alpha;
+      const bool any_change = __any_sync(0xffffffffu, alpha != 1.f);      // the same in the four warps
+      __syncwarp();
       if (j >= 2) {      // P buffer j&1 was last read by PV(j-2)
         if (!mbar_wait(&pv_done[j & 1], (((uint32_t)j - 2) >> 1) & 1u, abort_word)) goto done;
       }
       if (j > 0 && any_change) {    // uniform over the 128 threads: O^T must be quiescent
+#pragma unroll
+        for (int c = 0; c < NQ; c++) lsum[c] *= col_alpha[c];
         if (!mbar_wait(&pv_done[(j - 1) & 1], (((uint32_t)j - 1) >> 1) & 1u, abort_word)) goto done;
         tc_fence_after();
 #pragma unroll 1
@@ -363,7 +377,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           mla_tmem_ld<NQ>(t_lane + Cfg::O_COL + blk * NQ, o);
           tmem_ld_wait();
 #pragma unroll
-          for (int c = 0; c < NQ; c++) o[c] = __float_as_uint(__uint_as_float(o[c]) * alpha[c]);
+          for (int c = 0; c < NQ; c++) o[c] = __float_as_uint(__uint_as_float(o[c]) * col_alpha[c]);
           mla_tmem_st<NQ>(t_lane + Cfg::O_COL + blk * NQ, o);
         }
         tmem_st_wait();
@@ -371,10 +385,11 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       // probabilities of this key for every head -> P[head][key] (K-major, swizzled)
       uint8_t* pbase = Ps + (j & 1) * Cfg::P_BYTES + (tid >> 6) * Cfg::P_HALF;
       const int kin = tid & 63;
+      alignas(16) float mb[4];
 #pragma unroll
       for (int c = 0; c < NQ; c++) {
-        const float mb = (m[c] == -INFINITY) ? 0.f : m[c] * sl2;
-        const float pv = mla_exp2(s[c] * sl2 - mb);
+        if ((c & 3) == 0) *reinterpret_cast<float4*>(mb) = *reinterpret_cast<const float4*>(col_max + c);
+        const float pv = mla_exp2(s[c] * sl2 - mb[c & 3]);
         lsum[c] += pv;
         const int chunk = (kin >> 3) ^ (c & 7);
         *reinterpret_cast<__nv_bfloat16*>(pbase + c * 128 + (chunk << 4) + (kin & 7) * 2) =
@@ -388,6 +403,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     // ---- epilogue
     if (!mbar_wait(&pv_done[(n - 1) & 1], (((uint32_t)n - 1) >> 1) & 1u, abort_word)) goto done;
     tc_fence_after();
+    col_max[col] = m * sl2;
     mla_softmax_bar();
 #pragma unroll
     for (int c = 0; c < NQ; c++) {
@@ -400,7 +416,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 #pragma unroll
     for (int c = 0; c < NQ; c++) {
       float l = redf[c] + redf[NQ + c] + redf[2 * NQ + c] + redf[3 * NQ + c];
-      float m2 = m[c] * sl2, f = 1.f;                 // row maximum in log2 units
+      float m2 = col_max[c], f = 1.f;                 // row maximum in log2 units
       if (p.sink != nullptr && split == 0 && hb * p.HC + hd < p.H) {      // counted once, keys or not
         const float sk = p.sink[hb * p.HC + hd] * 1.4426950408889634f;
         if (sk > m2) {
