@@ -66,3 +66,67 @@ def test_engine_in_batch_invariant_mode_gives_a_request_the_same_tokens_alone_an
             assert alone.outputs[0].logprobs == together[i].outputs[0].logprobs
     finally:
         batch_invariant.disable_batch_invariant_mode()
+
+
+@pytest.mark.parametrize("Hkv,G,decodes", [(8, 4, 0), (8, 4, 3), (4, 8, 0)])
+def test_prompt_attention_rows_do_not_depend_on_the_rows_beside_them(monkeypatch, Hkv, G, decodes):
+    """A prompt alone, below the row count from which steps may take the kernel of two query tiles per block, and beside others far above it."""
+    from vllm_ascend_b200.attention.metadata import metadata_from_tensors
+    monkeypatch.setenv("VLLM_B200_BATCH_INVARIANT", "1")
+    g = torch.Generator(device="cpu").manual_seed(3)
+    D, page = 128, 128
+    new, old = [1] * decodes + [300, 2600, 77], [50] * decodes + [40, 0, 513]
+    pages = [-(-(n + o) // page) for n, o in zip(new, old)]
+    k, v = (ops.alloc_kv_cache(sum(pages), page, Hkv, D, torch.bfloat16, DEV) for _ in range(2))
+    for c in (k, v):
+        c.copy_(torch.randn(c.shape, generator=g).to(DEV))
+    q = torch.randn(sum(new), Hkv * G, D, generator=g).bfloat16().to(DEV)
+    table = torch.zeros(len(new), max(pages), dtype=torch.int32)
+    at = 0
+    for b, n in enumerate(pages):
+        table[b, :n] = torch.arange(at, at + n)
+        at += n
+    starts = np.cumsum([0] + new)
+
+    def run(seqs):
+        rows = torch.cat([torch.arange(starts[b], starts[b + 1]) for b in seqs]).to(DEV)
+        cu = torch.tensor(np.cumsum([0] + [new[b] for b in seqs]), dtype=torch.int32, device=DEV)
+        lens = torch.tensor([new[b] + old[b] for b in seqs], dtype=torch.int32, device=DEV)
+        meta = metadata_from_tensors(cu, lens, table[seqs].to(DEV), max(new[b] for b in seqs), int(lens.max()), Hkv * G, Hkv, D)
+        return rows, ops.paged_attention(q[rows], k, v, meta, D ** -0.5)
+    _, together = run(list(range(len(new))))
+    for b in range(len(new)):
+        rows, alone = run([b])
+        assert torch.equal(alone, together[rows]), b
+    _native.check_status(torch.device(DEV))
+
+
+def _logprobs_alone_and_together(cfg, **kw):
+    """Greedy log-probabilities of requests whose steps hold 2048 rows together, and of each by itself."""
+    from vllm_ascend_b200.engine.llm import LLM
+    from vllm_ascend_b200.engine.request import SamplingParams
+    rng = np.random.default_rng(8)
+    prompts = [rng.integers(0, 2048, size=n).tolist() for n in (300, 900, 130, 700, 20)]
+    sp = SamplingParams(temperature=0.0, max_tokens=4, ignore_eos=True, logprobs=3)
+    llm = LLM(cfg, device="cuda", max_model_len=1024, max_num_seqs=8, max_num_batched_tokens=2048, num_gpu_blocks_override=64,
+              enforce_eager=True, enable_prefix_caching=False, **kw)
+    together = llm.generate(prompts, sp)
+    return [(llm.generate([p], sp)[0].outputs[0].logprobs, t.outputs[0].logprobs) for p, t in zip(prompts, together)]
+
+
+def _wide_cfg():
+    """Heads that fill the GPU with prompt tiles, products with enough columns of K to be split."""
+    from vllm_ascend_b200.config import ModelConfig
+    return ModelConfig(name="t", architecture="Qwen3ForCausalLM", vocab_size=2048, hidden_size=2048, intermediate_size=4096,
+                       num_hidden_layers=2, num_attention_heads=32, num_key_value_heads=8, head_dim=128, qk_norm=True,
+                       rope_theta=1e6, dtype="bfloat16", init_std=0.05)
+
+
+def test_engine_in_batch_invariant_mode_with_prompts_that_fill_the_gpu(monkeypatch):
+    from vllm_ascend_b200 import batch_invariant
+    monkeypatch.setenv("VLLM_B200_BATCH_INVARIANT", "1")
+    try:
+        for alone, together in _logprobs_alone_and_together(_wide_cfg()):
+            assert alone == together
+    finally:
+        batch_invariant.disable_batch_invariant_mode()

@@ -1,12 +1,21 @@
 """Batch-invariant (run-to-run and batch-size independent) execution mode.
 
-What changes a result with the batch composition here is the reduction order, and only two
-places choose it from the batch: the split-KV factor of decode attention and the collective
-algorithm.  The GEMM kernels accumulate every output element over K in one fixed order
-whatever the tile shape, the norm/activation kernels reduce per row.  So the mode pins the
-split factor to 1 and the collectives to a fixed algorithm; the reference reaches the same
-goal by swapping aten matmul/softmax/mean/rmsnorm for batch-invariant kernels and setting
-deterministic collective variables (vllm_ascend/batch_invariant.py:76-162).
+What changes a result with the batch composition here is the reduction order.  The places that
+choose it from the batch, and what the mode does there:
+
+* the split-KV factor of decode attention: 1;
+* the collective algorithm: a fixed one;
+* products of few rows, which split K over the blocks of a cluster (bf16 and block-scaled fp8): not
+  taken.  The other GEMM kernels accumulate every output element over K in one fixed order whatever
+  the tile shape;
+* prompt attention with two query tiles per block, and latent prompts over up-projected keys and
+  values: not taken;
+* gated delta rule in chunks of 64 tokens: token by token;
+* norms folded into the GEMMs around them: not folded.
+
+The norm / activation / sampling kernels reduce per row.  The reference reaches the same goal by
+swapping aten matmul/softmax/mean/rmsnorm for batch-invariant kernels and setting deterministic
+collective variables (vllm_ascend/batch_invariant.py:76-162).
 """
 from __future__ import annotations
 

@@ -445,7 +445,11 @@ def paged_prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: tor
 def _prefill_pairs(q: torch.Tensor, Hkv: int, first_row: int) -> bool:
     """Whether a step's prompts run in the kernel that gives a block two query tiles: where those blocks can fill the GPU.
     Fewer tiles are better off one to a block (137 tokens of 32 / 8 heads: 11.3 us in pairs, 9.2 us one by one; 2048 tokens of
-    64 / 8 heads 103 us in pairs, 122 us)."""
+    64 / 8 heads 103 us in pairs, 122 us).  The kernels add a row's probabilities in different orders, so batch-invariant mode,
+    where a prompt gets the same bits whatever shares its step, never takes it."""
+    from ..batch_invariant import is_batch_invariant
+    if is_batch_invariant():
+        return False
     pair = 2 * (128 // (q.shape[1] // Hkv))
     return ((q.shape[0] - first_row) // pair) * Hkv >= torch.cuda.get_device_properties(q.device).multi_processor_count
 
