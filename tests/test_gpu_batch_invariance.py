@@ -130,3 +130,58 @@ def test_engine_in_batch_invariant_mode_with_prompts_that_fill_the_gpu(monkeypat
             assert alone == together
     finally:
         batch_invariant.disable_batch_invariant_mode()
+
+
+def test_training_consistent_products_do_not_depend_on_the_row_count():
+    """The switch by itself, without batch-invariant mode: products of a decode step and of the full sequence agree."""
+    from vllm_ascend_b200.attention.backend import set_training_consistent_attention
+    from vllm_ascend_b200.ops import linear_attn
+    from vllm_ascend_b200.quantization import schemes
+    g = torch.Generator(device="cpu").manual_seed(2)
+    K, N = 4096, 2048
+    x = (torch.randn(600, K, generator=g) * 0.5).bfloat16().to(DEV)
+    w = (torch.randn(N, K, generator=g) * 0.05).bfloat16().to(DEV)
+    w8 = torch.randn(N, K, generator=g).to(DEV).to(torch.float8_e4m3fn)
+    ws = torch.rand(N // 128, K // 128, generator=g).to(DEV)
+    cu, H = [0, 100, 140], 2
+    rows = torch.randn(140, 3 * H * 128, generator=g).bfloat16().to(DEV)
+    q, k, v = (r.view(140, H, 128) for r in rows.split(H * 128, 1))
+    decay, beta = (torch.rand(140, H, generator=g).to(DEV) for _ in range(2))
+
+    def delta(parts):
+        out, state = [], torch.zeros(1, H, 128, 128, device=DEV)
+        for i, (a, b) in enumerate(zip(parts, parts[1:])):
+            t, has = torch.tensor([0, b - a], dtype=torch.int32, device=DEV), torch.tensor([i > 0], dtype=torch.int32, device=DEV)
+            out.append(linear_attn.gated_delta_rule(q[a:b], k[a:b], v[a:b], -decay[a:b], beta[a:b], state, t, torch.zeros_like(has), has,
+                                                    128 ** -0.5, True, cu_cpu=np.array([0, b - a])))
+        return torch.cat(out), state
+    set_training_consistent_attention(True)
+    try:
+        for step in (lambda x: ops.linear_step(x, w), lambda x: ops.linear_swiglu_step(x, w),
+                     lambda x: schemes.fp8_block_linear(x, w8, ws)):
+            full = step(x)
+            for m in (1, 128, 256, 300):
+                assert torch.equal(step(x[:m]), full[:m]), m
+        whole, parts = delta([0, 140]), delta([0, 70, 71, 140])
+        assert torch.equal(whole[0], parts[0]) and torch.equal(whole[1], parts[1])
+    finally:
+        set_training_consistent_attention(False)
+    _native.check_status(torch.device(DEV))
+
+
+def test_engine_with_training_consistency_alone():
+    import os
+    from vllm_ascend_b200.attention.backend import set_training_consistent_attention
+    from vllm_ascend_b200.batch_invariant import is_batch_invariant
+    from vllm_ascend_b200.platform_config import clear_b200_config
+    saved = dict(os.environ)
+    try:
+        pairs = _logprobs_alone_and_together(_wide_cfg(), additional_config={"rl_config": {"enabled": True, "enable_training_consistency": True}})
+        assert not is_batch_invariant()
+        for alone, together in pairs:
+            assert alone == together
+    finally:
+        set_training_consistent_attention(False)
+        clear_b200_config()
+        os.environ.clear()
+        os.environ.update(saved)

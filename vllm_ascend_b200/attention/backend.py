@@ -10,7 +10,7 @@ from __future__ import annotations
 
 import torch
 
-from .. import _native, ops
+from .. import _native, batch_invariant, ops
 from .metadata import AttentionMetadata, AttentionState  # noqa: F401  (re-exported)
 
 
@@ -128,16 +128,12 @@ def _swap_blocks(src: torch.Tensor, dst: torch.Tensor, src_to_dst: torch.Tensor)
     _native.count_launch()
 
 
-_TRAINING_CONSISTENT = False
-
-
 def set_training_consistent_attention(on: bool) -> None:
-    global _TRAINING_CONSISTENT
-    _TRAINING_CONSISTENT = bool(on)
+    batch_invariant.set_training_consistent(on)
 
 
 def training_consistent_attention() -> bool:
-    return _TRAINING_CONSISTENT
+    return batch_invariant.is_training_consistent()
 
 
 class B200FAImpl(B200AttentionImpl):

@@ -241,12 +241,12 @@ def expanded_prompts(meta, heads: int, dn: int, dr: int, dv: int, q: torch.Tenso
                      pe_cache: torch.Tensor) -> Optional[tuple[int, int]]:
     """(sequences, keys): the step's prompts that attend over up-projected latents are all sequences behind the first
     ``sequences`` (those have one token each), ``keys`` is the number of their keys; None where the latent space is the better
-    place (decode steps, few new tokens behind long contexts) or the only one (captured or batch-invariant steps)."""
+    place (decode steps, few new tokens behind long contexts) or the only one (captured steps, modes that fix the order of sums)."""
     import numpy as np
     from .. import envs
-    from ..batch_invariant import is_batch_invariant
+    from ..batch_invariant import fixed_sums
     if not (q.is_cuda and q.dtype == lat_cache.dtype == torch.bfloat16 and meta.max_query_len > 1
-            and envs.VLLM_B200_MLA_ATTN == "tcgen05") or is_batch_invariant() or torch.cuda.is_current_stream_capturing():
+            and envs.VLLM_B200_MLA_ATTN == "tcgen05") or fixed_sums() or torch.cuda.is_current_stream_capturing():
         return None
     if dn != 128 or dv % 8 or not 8 <= dv <= 128 or dr % 8 or not 8 <= dr <= 64 or lat_cache.shape[-1] % 8 \
             or not (q.is_contiguous() and lat_cache.is_contiguous() and pe_cache.is_contiguous()):

@@ -22,6 +22,22 @@ from __future__ import annotations
 import os
 
 _enabled = False
+_training_consistent = False
+
+
+def fixed_sums() -> bool:
+    """Whether a row's sums have one order whatever shares its step: batch-invariant mode, or training-consistent attention
+    (``attention.backend``), whose decode steps have to agree with the trainer's full-sequence pass in every kernel."""
+    return _training_consistent or is_batch_invariant()
+
+
+def set_training_consistent(on: bool) -> None:
+    global _training_consistent
+    _training_consistent = bool(on)
+
+
+def is_training_consistent() -> bool:
+    return _training_consistent
 
 
 def is_batch_invariant() -> bool:

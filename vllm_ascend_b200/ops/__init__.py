@@ -322,11 +322,11 @@ _FEW_ROWS, _FEW_ROWS_MAX_COLS = 256, 5120
 
 def _few_rows(M: int, N: int, K: int) -> bool:
     """Whether a step's product runs in the kernel that splits K over blocks.  Its rows may differ in the last bit from
-    those of a larger batch, so batch-invariant mode never takes it."""
+    those of a larger batch, so modes that fix the order of sums never take it."""
     if M > _FEW_ROWS or (M > 128 and N > _FEW_ROWS_MAX_COLS) or K % 8 or N % 8 or envs.VLLM_B200_GEMM == "cublas":
         return False
-    from ..batch_invariant import is_batch_invariant
-    return not is_batch_invariant()
+    from ..batch_invariant import fixed_sums
+    return not fixed_sums()
 
 
 def _pair_rows(M: int) -> bool:
@@ -445,10 +445,10 @@ def paged_prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: tor
 def _prefill_pairs(q: torch.Tensor, Hkv: int, first_row: int) -> bool:
     """Whether a step's prompts run in the kernel that gives a block two query tiles: where those blocks can fill the GPU.
     Fewer tiles are better off one to a block (137 tokens of 32 / 8 heads: 11.3 us in pairs, 9.2 us one by one; 2048 tokens of
-    64 / 8 heads 103 us in pairs, 122 us).  The kernels add a row's probabilities in different orders, so batch-invariant mode,
-    where a prompt gets the same bits whatever shares its step, never takes it."""
-    from ..batch_invariant import is_batch_invariant
-    if is_batch_invariant():
+    64 / 8 heads 103 us in pairs, 122 us).  The kernels add a row's probabilities in different orders, so modes in
+    which a prompt gets the same bits whatever shares its step never take it."""
+    from ..batch_invariant import fixed_sums
+    if fixed_sums():
         return False
     pair = 2 * (128 // (q.shape[1] // Hkv))
     return ((q.shape[0] - first_row) // pair) * Hkv >= torch.cuda.get_device_properties(q.device).multi_processor_count

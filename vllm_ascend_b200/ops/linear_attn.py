@@ -215,11 +215,11 @@ _KERNEL_CHUNK_MIN = 32
 
 
 def _kernel_chunk_min() -> int:
-    """0: token by token only (asked for with VLLM_B200_GDN_CHUNK_MIN=0, or batch-invariant mode: a portion's split into
-    chunks must not show)."""
+    """0: token by token only (asked for with VLLM_B200_GDN_CHUNK_MIN=0, or in modes that fix the order of sums: a portion's
+    split into chunks must not show)."""
     import os
-    from ..batch_invariant import is_batch_invariant
-    return 0 if is_batch_invariant() or os.environ.get("VLLM_B200_GDN_CHUNK_MIN") == "0" else _KERNEL_CHUNK_MIN
+    from ..batch_invariant import fixed_sums
+    return 0 if fixed_sums() or os.environ.get("VLLM_B200_GDN_CHUNK_MIN") == "0" else _KERNEL_CHUNK_MIN
 
 
 def gated_delta_rule(q, k, v, g, beta, state, cu, slots, has_init, scale, l2norm=True, cu_cpu=None, uniform=False,

@@ -138,8 +138,8 @@ def fp8_block_linear(x: Optional[torch.Tensor], w8: torch.Tensor, w_scale: torch
     out = torch.empty((M, N), dtype=torch.bfloat16, device=xq.device)
     if M == 0:
         return out
-    from ..batch_invariant import is_batch_invariant
-    if M <= _FP8_FEW_ROWS and not is_batch_invariant():
+    from ..batch_invariant import fixed_sums
+    if M <= _FP8_FEW_ROWS and not fixed_sums():
         # K split over blocks: rows may differ in the last bit from those of a larger batch
         rc = _native.lib().b200_gemm_small_fp8(
             xq.data_ptr(), xs.data_ptr(), w8.data_ptr(), w_scale.data_ptr(), out.data_ptr(), _native.ptr(bias), M, N, K,
