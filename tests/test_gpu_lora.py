@@ -128,3 +128,31 @@ def test_expert_lora_on_gpu():
     assert base[0] != mixed[0] and base[2] != mixed[2]
     from vllm_ascend_b200 import _native
     _native.check_status(torch.device("cuda"))
+
+
+@pytest.mark.parametrize("kind", ["dense", "fp8", "moe", "mla"])
+def test_plain_rows_of_an_adapter_engine_do_not_depend_on_the_row_count(kind):
+    """Steps without an active adapter: a row has the same bits in a step of any size, through every product of the model (split sums
+    would change at 129 and 257 rows)."""
+    from vllm_ascend_b200.config import ModelConfig
+    from vllm_ascend_b200.engine.llm import LLM
+    more = {"dense": {}, "fp8": dict(quantization="fp8"),
+            "moe": dict(architecture="Qwen3MoeForCausalLM", num_experts=8, num_experts_per_tok=2, moe_intermediate_size=256),
+            "mla": dict(architecture="DeepseekV3ForCausalLM", use_mla=True, q_lora_rank=2048, kv_lora_rank=512, qk_nope_head_dim=128,
+                        qk_rope_head_dim=64, v_head_dim=128)}[kind]
+    cfg = ModelConfig(**{**dict(name="t", architecture="Qwen3ForCausalLM", vocab_size=2048, hidden_size=2048, intermediate_size=2048,
+                                num_hidden_layers=1, num_attention_heads=8, num_key_value_heads=2, head_dim=128, rope_theta=1e6,
+                                dtype="bfloat16", init_std=0.05), **more})
+    llm = LLM(cfg, device="cuda", max_model_len=512, max_num_seqs=8, max_num_batched_tokens=512, num_gpu_blocks_override=16,
+              enforce_eager=True, enable_lora=True, max_loras=1, max_lora_rank=8)
+    model = llm.engine.runner.model
+    L = model.layers[0]
+    products = [model.compute_logits, L.mlp] + [getattr(L.self_attn, n) for n in ("qkv_proj", "q_a_proj", "q_b_proj", "kv_a_proj", "o_proj")
+                                                if getattr(L.self_attn, n, None) is not None]
+    g = torch.Generator().manual_seed(4)
+    for f in products:
+        K = f.weight.shape[1] if hasattr(f, "weight") else cfg.hidden_size
+        x = torch.randn(400, K, generator=g).bfloat16().cuda()
+        full = f(x)
+        for m in (1, 128, 129, 256, 300):
+            assert torch.equal(f(x[:m]), full[:m]), (f, m)

@@ -49,6 +49,21 @@ class LoRALayerState:
         return self.punica.add_lora_linear(y, x, self.a, self.b, self.scale, self.output_slices, self.rank)
 
 
+def _model_parts(root):
+    """``root`` and the objects of the model packages that are reached from it through attributes and containers."""
+    seen, todo = set(), [root]
+    while todo:
+        o = todo.pop()
+        if isinstance(o, (list, tuple)):
+            todo.extend(o)
+        elif isinstance(o, dict):
+            todo.extend(o.values())
+        elif id(o) not in seen and type(o).__module__.startswith(("vllm_ascend_b200.models", "vllm_ascend_b200.parallel.finegrained")):
+            seen.add(id(o))
+            yield o
+            todo.extend(vars(o).values())
+
+
 class LoRAManager:
     def __init__(self, model, max_loras: int, max_rank: int, max_tokens: int, max_seqs: int, device, dtype):
         self.model = model
@@ -63,6 +78,10 @@ class LoRAManager:
         self._attach()
 
     def _attach(self) -> None:
+        # a plain request's rows keep the bits they have without adapter neighbours, whose products take other kernels
+        for part in _model_parts(self.model):
+            if hasattr(type(part), "fixed_rows"):
+                part.fixed_rows = True
         r = self.max_rank
         for L in self.model.layers:
             mods = {"qkv_proj": getattr(L.self_attn, "qkv_proj", None), "o_proj": getattr(L.self_attn, "o_proj", None)}

@@ -104,6 +104,9 @@ class TPComm:
 class Linear:
     """y = x W^T (+b).  ``weight`` is [N_local, K_local]."""
 
+    #: a row has the same bits in a step of any size (set in engines with adapters: ``lora.manager``)
+    fixed_rows = False
+
     def __init__(self, weight: torch.Tensor, bias: Optional[torch.Tensor] = None, name: str = ""):
         self.weight = weight
         self.bias = bias
@@ -120,8 +123,7 @@ class Linear:
         else:
             if isinstance(x, ops.QuantAct):
                 x = x.dequant()
-            # with adapters in the engine a plain request's rows keep the bits they have without adapter neighbours
-            y = (ops.linear_step if self.lora is None else ops.linear)(x, self.weight, self.bias, residual)
+            y = (ops.linear if self.fixed_rows else ops.linear_step)(x, self.weight, self.bias, residual)
         if self._lora_on():
             y = self.lora.apply(x, y)
         return y
@@ -239,13 +241,18 @@ class VocabParallelEmbedding:
 class ParallelLMHead:
     """Logits = hidden @ W^T with the vocab sharded over TP and gathered."""
 
+    fixed_rows = False          # see Linear
+
     def __init__(self, embed: VocabParallelEmbedding, weight: Optional[torch.Tensor] = None):
         self.embed = embed
         self.weight = weight if weight is not None else embed.weight
         self.comm = embed.comm
 
+    def _local(self, hidden: torch.Tensor) -> torch.Tensor:
+        return (ops.linear if self.fixed_rows else ops.linear_step)(hidden, self.weight)
+
     def __call__(self, hidden: torch.Tensor) -> torch.Tensor:
-        logits = ops.linear_step(hidden, self.weight)
+        logits = self._local(hidden)
         if self.comm.size > 1:
             logits = self.comm.all_gather(logits, dim=-1)
         return logits[..., :self.embed.vocab]
@@ -254,7 +261,7 @@ class ParallelLMHead:
         """Arg-max over the full vocabulary without gathering the logits: every rank reduces its
         own vocabulary shard to (max value, index) and only those pairs are all-gathered — the
         "reduce sample" path of vllm_ascend/sample/sampler.py:87-107, 168-204."""
-        logits = ops.linear_step(hidden, self.weight)                  # [B, V / tp]
+        logits = self._local(hidden)                                   # [B, V / tp]
         n, r = self.comm.size, self.comm.rank
         shard = logits.shape[-1]
         first = r * shard
@@ -490,15 +497,16 @@ class SwiGLUMLP:
 
     def __call__(self, x: torch.Tensor) -> torch.Tensor:
         gu = self.gate_up_proj
+        swiglu = ops.linear_swiglu if gu.fixed_rows else ops.linear_swiglu_step
         if self.act is not None:
             return self.down_proj(ops.activation(gu(x).contiguous(), self.act, gated=True))
         if self.limit is not None:
             if gu.quant is not None or gu._lora_on():
                 raise NotImplementedError("the clamped gate takes plain projections")
-            return self.down_proj(ops.linear_swiglu_step(x, gu.weight, limit=self.limit))
+            return self.down_proj(swiglu(x, gu.weight, limit=self.limit))
         if gu.quant is None and gu.bias is None and not gu.gather_output and not gu._lora_on() \
                 and _plan().enabled("gemm_swiglu"):
-            return self.down_proj((ops.linear_swiglu_step if gu.lora is None else ops.linear_swiglu)(x, gu.weight))
+            return self.down_proj(swiglu(x, gu.weight))
         if wants_quant_act(self.down_proj):
             return self.down_proj(ops.silu_and_mul_quant_fp8(gu(x)))
         return self.down_proj(ops.silu_and_mul(gu(x)))

@@ -28,6 +28,8 @@ class SparseMoeBlock:
     """Router + routed experts (+ shared experts).  Experts are sharded over the EP
     group when expert parallelism is on, else over TP along the intermediate dim."""
 
+    fixed_rows = False          # the router's products: see layers.Linear
+
     def __init__(self, pf: ParamFactory, cfg: ModelConfig, layer_idx: int, comm: TPComm,
                  ep_group: Optional[pstate.GroupCoordinator], moe_runtime=None):
         self.cfg = cfg
@@ -103,7 +105,7 @@ class SparseMoeBlock:
             # (48 rows, 128 experts, K = 2048: one block's tile 18.4 us, K split over a cluster 6.0 us)
             if self._gate_bf16 is None:
                 self._gate_bf16 = self.gate_weight.to(torch.bfloat16)
-            logits = ops.linear_step(x, self._gate_bf16).float()
+            logits = (ops.linear if self.fixed_rows else ops.linear_step)(x, self._gate_bf16).float()
         else:
             logits = torch.nn.functional.linear(x.float(), self.gate_weight)
         w, ids = fused_moe.gating_topk(logits, cfg.num_experts_per_tok, cfg.scoring_func,

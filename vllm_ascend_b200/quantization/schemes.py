@@ -84,7 +84,8 @@ class Fp8BlockLinear(LinearScheme):
         if isinstance(x, ops.QuantAct):
             N = layer.weight.shape[0]
             if x.q.is_cuda and N % 8 == 0:
-                y = fp8_block_linear(None, layer.weight, layer.weight_scale_inv, bias, quant=(x.q, x.scales))
+                y = fp8_block_linear(None, layer.weight, layer.weight_scale_inv, bias, quant=(x.q, x.scales),
+                                     fixed_rows=getattr(layer, "fixed_rows", False))
             else:
                 y = ref.block_fp8_linear(x.dequant(), layer.weight, layer.weight_scale_inv, self.block, x.dtype)
                 if bias is not None:
@@ -94,7 +95,7 @@ class Fp8BlockLinear(LinearScheme):
         N = layer.weight.shape[0]
         x2 = x.reshape(-1, K)
         if x2.is_cuda and x2.dtype == torch.bfloat16 and K % 128 == 0 and N % 8 == 0:
-            y = fp8_block_linear(x2, layer.weight, layer.weight_scale_inv, bias)
+            y = fp8_block_linear(x2, layer.weight, layer.weight_scale_inv, bias, fixed_rows=getattr(layer, "fixed_rows", False))
         else:
             y = ref.block_fp8_linear(x2, layer.weight, layer.weight_scale_inv, self.block, x.dtype)
             if bias is not None:
@@ -127,8 +128,9 @@ _FP8_FEW_ROWS = 128
 
 
 def fp8_block_linear(x: Optional[torch.Tensor], w8: torch.Tensor, w_scale: torch.Tensor,
-                     bias: Optional[torch.Tensor] = None, quant: Optional[tuple] = None) -> torch.Tensor:
-    """bf16 activations [M,K] -> dynamic 1x128 e4m3 quantisation -> block-scaled GEMM."""
+                     bias: Optional[torch.Tensor] = None, quant: Optional[tuple] = None, fixed_rows: bool = False) -> torch.Tensor:
+    """bf16 activations [M,K] -> dynamic 1x128 e4m3 quantisation -> block-scaled GEMM.  ``fixed_rows``: a row has the same
+    bits whatever M is."""
     if quant is not None:
         xq, xs = quant
     else:
@@ -139,7 +141,7 @@ def fp8_block_linear(x: Optional[torch.Tensor], w8: torch.Tensor, w_scale: torch
     if M == 0:
         return out
     from ..batch_invariant import fixed_sums
-    if M <= _FP8_FEW_ROWS and not fixed_sums():
+    if M <= _FP8_FEW_ROWS and not fixed_rows and not fixed_sums():
         # K split over blocks: rows may differ in the last bit from those of a larger batch
         rc = _native.lib().b200_gemm_small_fp8(
             xq.data_ptr(), xs.data_ptr(), w8.data_ptr(), w_scale.data_ptr(), out.data_ptr(), _native.ptr(bias), M, N, K,
