@@ -73,6 +73,35 @@ def test_paged_prompts(G, page, layout, window):
         at += n
 
 
+@pytest.mark.parametrize("causal", [True, False])
+def test_sequences_without_keys_leave_their_rows_alone(causal):
+    """Query rows of sequences that have no keys (padding, an encoder without output) between ones that have; and fewer keys than
+    queries, where causal rows in front of the first key see none."""
+    g = torch.Generator().manual_seed(9)
+    Hkv, G, D, page = 8, 4, 128, 128
+    new, keys = [300, 700, 40, 1500], [0, 650, 0, 1500]
+    table, cu, lens, blocks = _batch([1] * 4, [max(n - 1, 0) for n in keys], page, g)
+    cu, lens = (torch.tensor(x, dtype=torch.int32, device=DEV) for x in ([0] + list(np.cumsum(new)), keys))
+    k, v = (ops.alloc_kv_cache(blocks, page, Hkv, D, torch.bfloat16, DEV) for _ in range(2))
+    for c in (k, v):
+        c.copy_(torch.randn(c.shape, generator=g).to(DEV))
+    q = torch.randn((sum(new), Hkv * G, D), generator=g).to(DEV).bfloat16()
+    meta = metadata_from_tensors(cu, lens, table, max(new), max(keys), Hkv * G, Hkv, D, decode_kernel=False)
+    out = torch.full(q.shape, 7.0, device=DEV, dtype=torch.bfloat16)
+    ops.paged_prefill_attention(q, k, v, meta, D ** -0.5, out, causal)
+    _native.check_status(torch.device(DEV))
+    at = 0
+    for b, (n, m) in enumerate(zip(new, keys)):
+        got = out[at:at + n]
+        if m == 0:
+            assert (got == 7.0).all(), b
+        else:
+            first = max(n - m, 0) if causal else 0             # rows that see a key
+            want = _want(q[at:at + n], _rows(k, table[b], m, page), _rows(v, table[b], m, page), m - n, D ** -0.5, causal=causal)[first:]
+            assert ((got[first:].double() - want).abs() <= 3 * 2.0 ** -8 * (1 + want.abs())).all(), b
+        at += n
+
+
 def test_mixed_step_gives_decodes_and_prompts_their_rows():
     g = torch.Generator().manual_seed(5)
     new, old = [1, 1, 1, 4700, 130], [300, 5, 129, 0, 64]         # enough tiles for the kernel of pairs

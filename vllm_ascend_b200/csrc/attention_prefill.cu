@@ -91,6 +91,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   }
   const int t_lo = (p.window > 0 ? max(0, ctx + tok0 - p.window + 1) : 0) >> 7;
   const int n0 = t_hi[0] - t_lo, n = max(t_hi[0], t_hi[1]) - t_lo, n1 = ntok[1] > 0 ? n : 0;    // key tiles of each query tile
+  if (n <= 0) return;                        // no keys: nothing would arrive that the roles below wait for; rows stay as they are
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   extern __shared__ uint8_t smem_raw[];
