@@ -93,3 +93,10 @@ def test_sample_is_the_race_over_the_kept_set(V, pad, kind):
         # the fast exponential and fp32 sums are off by up to 1e-5; where the cut is closer, both sides of it are right
         if gap > 1e-5:
             assert got[b] in want, (b, got[b], want)
+
+
+@pytest.mark.parametrize("B,V,pad", [(65535, 8, 0), (65536, 3, 5), (131073, 9, 7), (3, 16385, 7), (4, 0, 0)])
+def test_logits_become_fp32_row_by_row(B, V, pad):
+    """More rows than a grid has in y, no columns, columns around a block's share."""
+    x = torch.randn(B, V + pad, generator=torch.Generator().manual_seed(B)).bfloat16().cuda()[:, :V]
+    assert torch.equal(ops.to_float_logits(x), x.float())

@@ -608,10 +608,11 @@ B200_API int b200_argmax(const void* logits, int dtype, long ld, int B, int V, v
 
 B200_API int b200_cast_bf16_f32(const void* in, long ld_in, void* out, long ld_out, int B, int V,
                                 cudaStream_t stream) {
-  if (B <= 0) return 0;
-  // 64 elements a thread
-  cast_bf16_to_f32_kernel<<<dim3((unsigned)((V + 16383) / 16384), (unsigned)B), 256, 0, stream>>>(
-      (const __nv_bfloat16*)in, ld_in, (float*)out, ld_out, V);
+  if (B <= 0 || V <= 0) return 0;
+  const unsigned blocks = (unsigned)((V + 16383) / 16384);           // 64 elements a thread
+  for (int b0 = 0; b0 < B; b0 += 65535)                              // rows are the grid's y
+    cast_bf16_to_f32_kernel<<<dim3(blocks, (unsigned)(B - b0 < 65535 ? B - b0 : 65535)), 256, 0, stream>>>(
+        (const __nv_bfloat16*)in + (long)b0 * ld_in, ld_in, (float*)out + (long)b0 * ld_out, ld_out, V);
   return B200_CHECK_LAUNCH();
 }
 
