@@ -100,3 +100,20 @@ def test_logits_become_fp32_row_by_row(B, V, pad):
     """More rows than a grid has in y, no columns, columns around a block's share."""
     x = torch.randn(B, V + pad, generator=torch.Generator().manual_seed(B)).bfloat16().cuda()[:, :V]
     assert torch.equal(ops.to_float_logits(x), x.float())
+
+
+def test_threads_may_sample_rows_of_different_lengths():
+    """Each thread on a stream of its own; how much shared memory the kernel may use does not depend on who asks first."""
+    from concurrent.futures import ThreadPoolExecutor
+    rows = [torch.randn(3, V, generator=torch.Generator().manual_seed(V)).cuda() for V in (700, 409601, 30000, 151936, 64, 262144) * 4]
+
+    def sample(x):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            n = x.shape[0]
+            out = ops.sample(x.clone(), torch.ones(n).cuda(), torch.full((n,), 40, dtype=torch.int32).cuda(), torch.full((n,), 0.9).cuda(),
+                             torch.zeros(n).cuda(), torch.arange(n).cuda(), torch.zeros(n, dtype=torch.int64).cuda())
+            return out.cpu().tolist()
+    torch.cuda.synchronize()
+    with ThreadPoolExecutor(8) as pool:
+        together = list(pool.map(sample, rows))
+    assert together == [sample(x) for x in rows]

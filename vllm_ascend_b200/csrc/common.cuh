@@ -8,6 +8,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <atomic>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -383,6 +384,20 @@ inline int make_tmap(CUtensorMap* out, const void* base, CUtensorMapDataType dt,
     return 9000 + (int)r;
   }
   return 0;
+}
+
+// Lets a kernel use that much dynamic shared memory; the driver is asked once per device.
+template <auto Kernel>
+inline cudaError_t allow_smem(int bytes) {
+  static std::atomic<uint64_t> done{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+  if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return e;
 }
 
 inline int num_sms() {

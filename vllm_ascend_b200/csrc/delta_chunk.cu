@@ -486,12 +486,8 @@ __global__ void __launch_bounds__(DC_THREADS, 1) delta_chunk_kernel(const DeltaC
 
 template <int COLS>
 static int launch_dc(const DeltaChunkArgs& p, int B, cudaStream_t stream) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(delta_chunk_kernel<COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, DcCfg<COLS>::SMEM);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  const cudaError_t e = allow_smem<delta_chunk_kernel<COLS>>(DcCfg<COLS>::SMEM);
+  if (e != cudaSuccess) return (int)e;
   delta_chunk_kernel<COLS><<<dim3((unsigned)B, (unsigned)p.Hv, (unsigned)(p.DV / COLS)), DC_THREADS, DcCfg<COLS>::SMEM, stream>>>(p);
   return B200_CHECK_LAUNCH();
 }

@@ -643,12 +643,8 @@ B200_API int b200_sample(void* logits_f32, long ld, int B, int V, const void* te
   const int slice = ((V + SAMP_C - 1) / SAMP_C + 3) / 4 * 4;
   const int resident = slice <= SAMP_MAX_SLICE;
   const size_t smem = resident ? (size_t)slice * 4 : 0;
-  static size_t smem_set = 0;
-  if (smem > smem_set) {
-    cudaError_t e = cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    smem_set = smem;
-  }
+  const cudaError_t allowed = allow_smem<sample_kernel>(SAMP_MAX_SLICE * 4);
+  if (allowed != cudaSuccess) return (int)allowed;
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(SAMP_T);
   cfg.dynamicSmemBytes = smem;
