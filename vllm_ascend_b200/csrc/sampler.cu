@@ -347,7 +347,7 @@ __device__ int samp_finish(SampSmem* s, int n, int k, float pth, float mp, float
     }
   auto value = [&](int i) { return (uint32_t)(c[i] >> 32); };
   uint32_t thr = k > 0 ? value(k - 1) : 0;
-  if (pth < 1.f) {
+  if (pth < 1.f && value(0) <= 0x7F800000u) {              // a row with a NaN has no mass to take a share of
     // running mass in units of 2^-40: a thread sums its run of neighbours, then their sums are scanned
     constexpr int PER = SAMP_BINS / SAMP_T;
     samp_n run[PER], sum = 0;
@@ -528,7 +528,7 @@ sample_kernel(float* logits, long ld, int V, int slice, int resident, const floa
     mass = 0.f;
     for (int r = 0; r < SAMP_C; r++) mass += samp_peek(&s.xch[2].v[0], r);
   }
-  if (pth < 1.f) {
+  if (pth < 1.f && mass == mass) {
     cut = 0;                           // a margin for the order of the sums
 #pragma unroll
     for (int j = SAMP_CUTS - 1; j >= 0; j--) if (zc[j] >= pth * mass * 1.001f) cut = cuts[j];
