@@ -102,6 +102,19 @@ def test_sample_is_the_race_over_the_kept_set(V, pad, kind):
     _check(wide, V, T, k, p, mp, rng)
 
 
+@pytest.mark.parametrize("B,V,pad", [(38, 4099, 2), (75, 22000, 0), (80, 70, 0), (149, 3, 5), (150, 5003, 1), (150, 23000, 0)])
+def test_more_rows_take_fewer_blocks_each(B, V, pad):
+    """Row counts from which a row has four, two and one block, with all shapes of rows and of requests mixed."""
+    rng = np.random.default_rng(B + V)
+    wide = torch.zeros((B, V + pad))
+    for i, kind in enumerate(("peaked", "flat", "masked", "spikes")):
+        wide[i::4, :V] = torch.from_numpy(_rows(kind, len(range(i, B, 4)), V, rng))
+    pick = [(0.0, 5, 0.9, 0.0), (0.7, 3, 1.0, 0.0), (1.0, min(50, V), 0.9, 0.0), (1.3, 0, 0.8, 0.0), (0.9, 0, 0.97, 0.013), (1.0, V, 1.0, 0.0),
+            (1.0, max(V * 2 // 3, 1), 0.999, 0.0)]
+    T, k, p, mp = (list(c) for c in zip(*(pick[(b // 4) % len(pick)] for b in range(B))))
+    _check(wide, V, T, k, p, mp, rng)
+
+
 @pytest.mark.parametrize("B,V", [(6, 70), (6, 151936), (160, 5000)])
 def test_nan_and_infinite_logits(B, V):
     """NaN is never chosen, an infinite logit always; what else a row asks for still ends, and other rows are not touched."""

@@ -149,33 +149,38 @@ __global__ void penalties_kernel(float* logits, long ld, int V, const long* prom
 
 // ---------------------------------------------------------------- top-k/top-p sampling
 // A row of 150k fp32 logits is walked about ten times (maximum, exponentials, three digits of a radix select for
-// top-k and three for top-p, the race), so the row is spread over a cluster of eight blocks and stays in their shared memory
+// top-k and three for top-p, the race), so the row is spread over a cluster of up to eight blocks and stays in their shared memory
 // after one read of HBM.  What bounds it then is instructions and the cluster's meetings, so a walk touches as little as it can:
 //   * the select passes only look at elements above a cut that already holds enough of them (2^-6 to 2^-24 of the
 //     maximum, counted while the exponentials are taken): with peaked rows that leaves a few thousand shared-memory
-//     atomics where there were V per pass;
+//     atomics where there were V per pass.  Rows without top-k and top-p skip sums, cuts and their meeting;
 //   * bins are integers (mass in units of 2^-40: shared memory adds 64-bit integers by itself, floats in a loop, and the
-//     sum has no order), added and searched in parallel (256 per block, then one warp);
+//     sum has no order), added and searched in parallel;
 //   * where the cut leaves at most 2048 elements (top-k, peaked top-p), one block sorts them and ends the row by itself;
-//   * random numbers are drawn only for groups of four that hold a kept element.
-// 192 rows of 151936: one block per row with thread-serial bins 738 us, 267 us in shared memory of the
-// cluster, 187 us with rows of few candidates finished by one block.
-constexpr int SAMP_C = 8;              // blocks per row
+//   * random numbers are drawn only for groups of four that hold a kept element;
+//   * what the other blocks of the cluster say is read once per block: read by every thread, 192 x 32000 without top-k and top-p
+//     took 115 us of which 88 reads per thread were most, 56 us so (37 us with two blocks a row, 66 us one block with the row in L2).
+// 192 rows of 151936, top-k 50: one block per row with thread-serial bins 849 us, 131 us so.
 constexpr int SAMP_T = 512;
 constexpr int SAMP_BINS = 2048;
 constexpr int SAMP_MAX_SLICE = 50 * 1024;        // elements of a row that a block keeps in shared memory
+constexpr int SAMP_PAIR_SLICE = 23000;           // ... while an SM holds two such blocks
+constexpr int SAMP_TWO_HIST_SLICE = 47000;       // ... beside a second histogram (256 flat rows of 262144, top-p: 4294 -> 2960 us)
 constexpr int SAMP_CUTS = 5;
 using samp_n = unsigned long long;     // elements, or mass in units of 2^-40 (e <= 1, so a row's mass fits)
 constexpr float SAMP_UNIT = 1099511627776.f;
 
 struct SampXch { float v[1 + SAMP_CUTS]; uint32_t n[SAMP_CUTS]; int i; };
 
+// C: blocks per row (a cluster), K: histograms per block (a lane adds to its own, so that fewer lanes meet in a bin)
+template <int C, int K>
 struct SampSmem {
-  samp_n hist[SAMP_BINS];
-  samp_n own[SAMP_BINS / SAMP_C];      // this block's bins, summed over the cluster
+  samp_n hist[K * SAMP_BINS];
+  samp_n own[C > 1 ? SAMP_BINS / C : 1];       // this block's bins, summed over the cluster
   samp_n tot[6];                       // sum of `own`, one slot per select pass
   samp_n remaining;
   SampXch xch[4];                      // what a block tells the others: one slot per meeting
+  SampXch all[4];                      // the same over the cluster
   float red[SAMP_T / 32][1 + 2 * SAMP_CUTS];
   float sv[32];
   int si[32];
@@ -184,12 +189,15 @@ struct SampSmem {
   uint32_t listed;                     // candidates in hist (rank 0)
 };
 
-__device__ __forceinline__ void samp_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+template <int C>
+__device__ __forceinline__ void samp_meet() {
+  if constexpr (C == 1) __syncthreads();
+  else asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
-// the address of `p` (shared memory of this block) in block r of the cluster
-template <typename U>
+// the value at `p` (shared memory of this block) in block r of the cluster
+template <int C, typename U>
 __device__ __forceinline__ U samp_peek(const U* p, int r) {
+  if constexpr (C == 1) return *(const volatile U*)p;
   uint32_t a;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(r));
   U out;
@@ -223,22 +231,37 @@ __device__ __forceinline__ void samp_better(float& v, int& i, float ov, int oi) 
   if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
 }
 // argmax over the cluster, lowest index on ties
-__device__ void samp_cluster_argmax(float& v, int& idx, SampSmem* s, SampXch* x) {
+template <int C, int K>
+__device__ void samp_cluster_argmax(float& v, int& idx, SampSmem<C, K>* s, int slot) {
   block_argmax(v, idx, s->sv, s->si);
-  if (threadIdx.x == 0) { x->v[0] = v; x->i = idx; }
-  samp_cluster_sync();
-  v = -INFINITY;
-  idx = 0x7fffffff;
-  for (int r = 0; r < SAMP_C; r++) samp_better(v, idx, samp_peek(&x->v[0], r), samp_peek(&x->i, r));
+  if constexpr (C > 1) {
+    if (threadIdx.x == 0) { s->xch[slot].v[0] = v; s->xch[slot].i = idx; }
+    samp_meet<C>();
+    if (threadIdx.x < 32) {
+      v = samp_peek<C>(&s->xch[slot].v[0], threadIdx.x % C);
+      idx = samp_peek<C>(&s->xch[slot].i, threadIdx.x % C);
+#pragma unroll
+      for (int o = C / 2; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, v, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
+        samp_better(v, idx, ov, oi);
+      }
+      if (threadIdx.x == 0) { s->all[slot].v[0] = v; s->all[slot].i = idx; }
+    }
+    __syncthreads();
+    v = s->all[slot].v[0];
+    idx = s->all[slot].i;
+  }
 }
 
 // One digit of the select: histogram (elements or their mass) of the `bits`-wide digit at `shift` over the elements whose
 // higher bits equal the prefix and whose key reaches floor_key, then the bin, walking down from the top, at which the
 // running sum reaches `remaining`.  Every block of the cluster ends with the same prefix and remaining.
-template <bool MASS>
-__device__ void samp_pass(const float* e, int n, SampSmem* s, int pass, int shift, int bits, uint32_t hi_mask, uint32_t floor_key, int rank) {
-  const int nb = 1 << bits, per = nb / SAMP_C;
-  for (int i = threadIdx.x; i < nb; i += SAMP_T) s->hist[i] = 0;
+template <bool MASS, int C, int K>
+__device__ void samp_pass(const float* e, int n, SampSmem<C, K>* s, int pass, int shift, int bits, uint32_t hi_mask, uint32_t floor_key, int rank) {
+  const int nb = 1 << bits;
+  for (int i = threadIdx.x; i < K * nb; i += SAMP_T) s->hist[i] = 0;
+  samp_n* hist = s->hist + (threadIdx.x & (K - 1)) * nb;
   __syncthreads();
   const uint32_t prefix = s->prefix;
   const samp_n rem0 = s->remaining;
@@ -246,40 +269,18 @@ __device__ void samp_pass(const float* e, int n, SampSmem* s, int pass, int shif
     const float v = e[i];
     const uint32_t k = __float_as_uint(v);
     if (k < floor_key || (k & hi_mask) != prefix) continue;
-    atomicAdd(&s->hist[(k >> shift) & (nb - 1)], MASS ? __float2ull_rn(v * SAMP_UNIT) : 1ull);
+    atomicAdd(&hist[(k >> shift) & (nb - 1)], MASS ? __float2ull_rn(v * SAMP_UNIT) : 1ull);
   }
-  samp_cluster_sync();
-  samp_n b = 0;
-  if ((int)threadIdx.x < per) {
-#pragma unroll
-    for (int r = 0; r < SAMP_C; r++) b += samp_peek(&s->hist[rank * per + threadIdx.x], r);
-    s->own[threadIdx.x] = b;
-  }
-  b = samp_warp_sum(b);
-  if ((threadIdx.x & 31) == 0) s->sn[threadIdx.x >> 5] = b;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    b = samp_warp_sum(threadIdx.x < SAMP_T / 32 ? s->sn[threadIdx.x] : 0);
-    if (threadIdx.x == 0) s->tot[pass] = b;
-  }
-  samp_cluster_sync();
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    const samp_n t_lane = samp_peek(&s->tot[pass], lane % SAMP_C);
-    samp_n rem = rem0;
-    int r = SAMP_C - 1;
-    for (; r > 0; r--) {
-      const samp_n t = __shfl_sync(0xffffffffu, t_lane, r);
-      if (t >= rem) break;
-      rem -= t;
-    }
-    // lane l owns bins [top - w (l + 1), top - w l) of block r
-    constexpr int W = SAMP_BINS / SAMP_C / 32;
-    const int w = per / 32;
+  samp_meet<C>();
+  if constexpr (C == 1) {
+    // thread t owns bins [top - w (t + 1), top - w t)
+    constexpr int W = SAMP_BINS / SAMP_T;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w = nb / SAMP_T;
     samp_n mine[W], sum = 0;
 #pragma unroll
     for (int j = 0; j < W; j++) {
-      mine[j] = j < w ? samp_peek(&s->own[per - 1 - (lane * w + j)], r) : 0;
+      mine[j] = 0;
+      for (int h = 0; h < K; h++) mine[j] += j < w ? s->hist[h * nb + nb - 1 - ((int)threadIdx.x * w + j)] : 0;
       sum += mine[j];
     }
     samp_n upto = sum;
@@ -288,10 +289,16 @@ __device__ void samp_pass(const float* e, int n, SampSmem* s, int pass, int shif
       const samp_n t = __shfl_up_sync(0xffffffffu, upto, o);
       if (lane >= o) upto += t;
     }
-    const uint32_t hit = __ballot_sync(0xffffffffu, upto >= rem);
-    const int who = hit ? __ffs(hit) - 1 : 31;                     // rounding can leave every sum below rem: the lowest bin
-    if (lane == who) {
-      rem -= upto - sum;
+    if (lane == 31) s->sn[warp] = upto;
+    __syncthreads();
+    samp_n before = upto - sum, all = 0;
+    for (int v = 0; v < SAMP_T / 32; v++) {
+      if (v < warp) before += s->sn[v];
+      all += s->sn[v];
+    }
+    // rounding can leave the whole sum below rem0: the lowest bin
+    if (rem0 == 0 ? threadIdx.x == 0 : all < rem0 ? threadIdx.x == SAMP_T - 1 : before < rem0 && before + sum >= rem0) {
+      samp_n rem = rem0 - before;
       int sel = w - 1;
 #pragma unroll
       for (int j = 0; j < W; j++)
@@ -299,8 +306,66 @@ __device__ void samp_pass(const float* e, int n, SampSmem* s, int pass, int shif
           if (mine[j] >= rem) sel = j;
           else rem -= mine[j];
         }
-      s->prefix = prefix | ((uint32_t)(r * per + per - 1 - (lane * w + sel)) << shift);
+      s->prefix = prefix | ((uint32_t)(nb - 1 - ((int)threadIdx.x * w + sel)) << shift);
       s->remaining = rem;
+    }
+  } else {
+    const int per = nb / C;
+    samp_n b = 0;
+    for (int i = threadIdx.x; i < per; i += SAMP_T) {
+      samp_n t = 0;
+#pragma unroll
+      for (int r = 0; r < C * K; r++) t += samp_peek<C>(&s->hist[r / C * nb + rank * per + i], r % C);
+      s->own[i] = t;
+      b += t;
+    }
+    b = samp_warp_sum(b);
+    if ((threadIdx.x & 31) == 0) s->sn[threadIdx.x >> 5] = b;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      b = samp_warp_sum(threadIdx.x < SAMP_T / 32 ? s->sn[threadIdx.x] : 0);
+      if (threadIdx.x == 0) s->tot[pass] = b;
+    }
+    samp_meet<C>();
+    if (threadIdx.x < 32) {
+      const int lane = threadIdx.x;
+      const samp_n t_lane = samp_peek<C>(&s->tot[pass], lane % C);
+      samp_n rem = rem0;
+      int r = C - 1;
+      for (; r > 0; r--) {
+        const samp_n t = __shfl_sync(0xffffffffu, t_lane, r);
+        if (t >= rem) break;
+        rem -= t;
+      }
+      // lane l owns bins [top - w (l + 1), top - w l) of block r
+      constexpr int W = SAMP_BINS / C / 32;
+      const int w = per / 32;
+      samp_n mine[W], sum = 0;
+#pragma unroll
+      for (int j = 0; j < W; j++) {
+        mine[j] = j < w ? samp_peek<C>(&s->own[per - 1 - (lane * w + j)], r) : 0;
+        sum += mine[j];
+      }
+      samp_n upto = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const samp_n t = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += t;
+      }
+      const uint32_t hit = __ballot_sync(0xffffffffu, upto >= rem);
+      const int who = hit ? __ffs(hit) - 1 : 31;                     // rounding can leave every sum below rem: the lowest bin
+      if (lane == who) {
+        rem -= upto - sum;
+        int sel = w - 1;
+#pragma unroll
+        for (int j = 0; j < W; j++)
+          if (j < w - 1 && sel == w - 1) {
+            if (mine[j] >= rem) sel = j;
+            else rem -= mine[j];
+          }
+        s->prefix = prefix | ((uint32_t)(r * per + per - 1 - (lane * w + sel)) << shift);
+        s->remaining = rem;
+      }
     }
   }
   __syncthreads();
@@ -308,7 +373,8 @@ __device__ void samp_pass(const float* e, int n, SampSmem* s, int pass, int shif
 
 // Elements above the cut, gathered from the whole cluster into rank 0's `hist` as (key, inverted index): value descending, index
 // ascending is then one 64-bit order.
-__device__ void samp_gather(const float* e, int n, int first, uint32_t cut, SampSmem* s) {
+template <int C, int K>
+__device__ void samp_gather(const float* e, int n, int first, uint32_t cut, SampSmem<C, K>* s) {
   uint32_t list, count;
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(list) : "r"(smem_u32(s->hist)));
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(count) : "r"(smem_u32(&s->listed)));
@@ -330,7 +396,8 @@ __device__ void samp_gather(const float* e, int n, int first, uint32_t cut, Samp
 
 // Rank 0 alone: orders the n gathered candidates, cuts them by rank and by mass, and runs the race.  `mass` is what top-p is a
 // share of where top-k is off.
-__device__ int samp_finish(SampSmem* s, int n, int k, float pth, float mp, float mass, uint2 key, long offset, int fallback) {
+template <int C, int K>
+__device__ int samp_finish(SampSmem<C, K>* s, int n, int k, float pth, float mp, float mass, uint2 key, long offset, int fallback) {
   samp_n* c = s->hist;
   int size = 32;
   while (size < n) size *= 2;
@@ -403,99 +470,110 @@ __device__ int samp_finish(SampSmem* s, int n, int k, float pth, float mp, float
 // logits: fp32 [B, V] (already penalised); overwritten where a row does not fit the cluster's shared memory.
 // temperature/top_k/top_p/min_p: per row (top_k <= 0 or >= V: off; top_p >= 1: off).
 // seeds: per-row uint64 seed, offsets: per-row counter (e.g. number of tokens generated).
-__global__ void __launch_bounds__(SAMP_T)
+template <int C, int K>
+__global__ void __launch_bounds__(SAMP_T, 2)
 sample_kernel(float* logits, long ld, int V, int slice, int resident, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p,
               const float* __restrict__ min_p, const unsigned long long* __restrict__ seeds,
               const long* __restrict__ offsets, long* __restrict__ out) {
-  __shared__ SampSmem s;
+  __shared__ SampSmem<C, K> s;
   extern __shared__ __align__(16) float kept_row[];
   const int rank = blockIdx.x, b = blockIdx.y;
   const int first = rank * slice, n = max(0, min(V - first, slice));
   float* row = logits + (long)b * ld + first;
   float* e = resident ? kept_row : row;
-  const float T = temperature ? temperature[b] : 1.f;
+  const float temp = temperature ? temperature[b] : 1.f;
+  const int k = top_k ? top_k[b] : 0;
+  const float pth = top_p ? top_p[b] : 1.f, mp = min_p ? min_p[b] : 0.f;
+  const bool greedy = temp < 1e-5f, by_rank = k > 0 && k < V;
   // ---- the row comes in; its maximum (also the greedy answer)
   float best = -INFINITY;
   int bi = 0x7fffffff;
-  if (resident && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+  const bool keep = resident && !greedy;
+  int done = 0;
+  if ((reinterpret_cast<uintptr_t>(row) & 15) == 0) {
     const int nv = n >> 2;
 #pragma unroll 4
     for (int c = threadIdx.x; c < nv; c += SAMP_T) {
       const float4 q = reinterpret_cast<const float4*>(row)[c];
-      reinterpret_cast<float4*>(e)[c] = q;
+      if (keep) reinterpret_cast<float4*>(e)[c] = q;
       if (q.x > best) { best = q.x; bi = first + 4 * c; }
       if (q.y > best) { best = q.y; bi = first + 4 * c + 1; }
       if (q.z > best) { best = q.z; bi = first + 4 * c + 2; }
       if (q.w > best) { best = q.w; bi = first + 4 * c + 3; }
     }
-    for (int i = 4 * nv + threadIdx.x; i < n; i += SAMP_T) {
-      const float v = row[i];
-      e[i] = v;
-      if (v > best) { best = v; bi = first + i; }
-    }
-  } else {
+    done = 4 * nv;
+  }
 #pragma unroll 4
-    for (int i = threadIdx.x; i < n; i += SAMP_T) {
-      const float v = row[i];
-      if (resident) e[i] = v;
-      if (v > best) { best = v; bi = first + i; }
-    }
+  for (int i = done + threadIdx.x; i < n; i += SAMP_T) {
+    const float v = row[i];
+    if (keep) e[i] = v;
+    if (v > best) { best = v; bi = first + i; }
   }
   if (threadIdx.x == 0) s.listed = 0;
-  samp_cluster_argmax(best, bi, &s, &s.xch[0]);
-  if (T < 1e-5f) {
+  samp_cluster_argmax(best, bi, &s, 0);
+  if (greedy) {
     if (rank == 0 && threadIdx.x == 0) out[b] = bi;
-    samp_cluster_sync();               // nobody leaves while another reads its memory
+    samp_meet<C>();                    // nobody leaves while another reads its memory
     return;
   }
-  // ---- e = exp((x - max)/T), their sum, and how much lies above each cut
+  // ---- e = exp((x - max)/T); where something is cut by rank or mass, their sum and how much lies above each cut
   const uint32_t cuts[SAMP_CUTS] = {0x3C800000u, 0x3A800000u, 0x38800000u, 0x36800000u, 0x33800000u};   // 2^-6, -10, -14, -18, -24
-  const float invT = 1.f / T;
-  float part[1 + 2 * SAMP_CUTS];       // sum, sum and number above each cut
-#pragma unroll
-  for (int j = 0; j < 1 + 2 * SAMP_CUTS; j++) part[j] = 0.f;
-  for (int i = threadIdx.x; i < n; i += SAMP_T) {
-    const float ev = __expf((e[i] - best) * invT);
-    e[i] = ev;
-    part[0] += ev;
-#pragma unroll
-    for (int j = 0; j < SAMP_CUTS; j++)
-      if (__float_as_uint(ev) >= cuts[j]) { part[1 + j] += ev; part[1 + SAMP_CUTS + j] += 1.f; }
-  }
-#pragma unroll
-  for (int j = 0; j < 1 + 2 * SAMP_CUTS; j++) {
-    part[j] = warp_reduce_sum(part[j]);
-    if ((threadIdx.x & 31) == 0) s.red[threadIdx.x >> 5][j] = part[j];
-  }
-  __syncthreads();
-  if (threadIdx.x < 1 + 2 * SAMP_CUTS) {
-    float t = 0.f;
-    for (int w = 0; w < SAMP_T / 32; w++) t += s.red[w][threadIdx.x];
-    if (threadIdx.x <= SAMP_CUTS) s.xch[1].v[threadIdx.x] = t;
-    else s.xch[1].n[threadIdx.x - 1 - SAMP_CUTS] = (uint32_t)t;
-  }
-  samp_cluster_sync();
+  const float invT = 1.f / temp;
   float z = 0.f, zc[SAMP_CUTS];
   uint32_t nc[SAMP_CUTS];
+  if (by_rank || pth < 1.f) {
+    float part[1 + 2 * SAMP_CUTS];     // sum, sum and number above each cut
 #pragma unroll
-  for (int r = 0; r < SAMP_C; r++) z += samp_peek(&s.xch[1].v[0], r);
+    for (int j = 0; j < 1 + 2 * SAMP_CUTS; j++) part[j] = 0.f;
+    for (int i = threadIdx.x; i < n; i += SAMP_T) {
+      const float ev = __expf((e[i] - best) * invT);
+      e[i] = ev;
+      part[0] += ev;
 #pragma unroll
-  for (int j = 0; j < SAMP_CUTS; j++) {
-    zc[j] = 0.f;
-    nc[j] = 0;
+      for (int j = 0; j < SAMP_CUTS; j++)
+        if (__float_as_uint(ev) >= cuts[j]) { part[1 + j] += ev; part[1 + SAMP_CUTS + j] += 1.f; }
+    }
 #pragma unroll
-    for (int r = 0; r < SAMP_C; r++) { zc[j] += samp_peek(&s.xch[1].v[1 + j], r); nc[j] += samp_peek(&s.xch[1].n[j], r); }
+    for (int j = 0; j < 1 + 2 * SAMP_CUTS; j++) {
+      part[j] = warp_reduce_sum(part[j]);
+      if ((threadIdx.x & 31) == 0) s.red[threadIdx.x >> 5][j] = part[j];
+    }
+    __syncthreads();
+    if (threadIdx.x < 1 + 2 * SAMP_CUTS) {
+      float t = 0.f;
+      for (int w = 0; w < SAMP_T / 32; w++) t += s.red[w][threadIdx.x];
+      if (threadIdx.x <= SAMP_CUTS) s.xch[1].v[threadIdx.x] = t;
+      else s.xch[1].n[threadIdx.x - 1 - SAMP_CUTS] = (uint32_t)t;
+    }
+    samp_meet<C>();
+    if (threadIdx.x <= SAMP_CUTS) {
+      float t = 0.f;
+#pragma unroll
+      for (int r = 0; r < C; r++) t += samp_peek<C>(&s.xch[1].v[threadIdx.x], r);
+      s.all[1].v[threadIdx.x] = t;
+    } else if (threadIdx.x < 1 + 2 * SAMP_CUTS) {
+      uint32_t t = 0;
+#pragma unroll
+      for (int r = 0; r < C; r++) t += samp_peek<C>(&s.xch[1].n[threadIdx.x - 1 - SAMP_CUTS], r);
+      s.all[1].n[threadIdx.x - 1 - SAMP_CUTS] = t;
+    }
+    __syncthreads();
+    z = s.all[1].v[0];
+#pragma unroll
+    for (int j = 0; j < SAMP_CUTS; j++) { zc[j] = s.all[1].v[1 + j]; nc[j] = s.all[1].n[j]; }
+  } else {
+    for (int i = threadIdx.x; i < n; i += SAMP_T) e[i] = __expf((e[i] - best) * invT);
+#pragma unroll
+    for (int j = 0; j < SAMP_CUTS; j++) { zc[j] = 0.f; nc[j] = 0; }
+    __syncthreads();
   }
   float mass = z;
   uint32_t thr_key = 0;                // keep elements with key >= thr_key
 
-  const int k = top_k ? top_k[b] : 0;
-  const float pth = top_p ? top_p[b] : 1.f, mp = min_p ? min_p[b] : 0.f;
   const unsigned long long seed = seeds ? seeds[b] : 0ull;
   const long offset = offsets ? offsets[b] : 0;
   const uint2 key = make_uint2((uint32_t)seed, (uint32_t)(seed >> 32));
-  const bool by_rank = k > 0 && k < V;
   uint32_t cut = 0, above = 0;         // the highest cut that holds enough, and how many elements reach it
 #pragma unroll
   for (int j = SAMP_CUTS - 1; j >= 0; j--)
@@ -503,7 +581,7 @@ sample_kernel(float* logits, long ld, int V, int slice, int resident, const floa
   if (cut != 0 && above <= SAMP_BINS) {
     // everything that can be kept fits one block: no more meetings of the cluster
     samp_gather(e, n, first, cut, &s);
-    samp_cluster_sync();
+    samp_meet<C>();
     if (rank != 0) return;
     const int win = samp_finish(&s, (int)above, by_rank ? k : 0, pth, mp, mass, key, offset, bi);
     if (threadIdx.x == 0) out[b] = win;
@@ -512,9 +590,9 @@ sample_kernel(float* logits, long ld, int V, int slice, int resident, const floa
   if (by_rank) {
     if (threadIdx.x == 0) { s.prefix = 0; s.remaining = (samp_n)k; }
     __syncthreads();
-    samp_pass<false>(e, n, &s, 0, 21, 11, 0x00000000u, cut, rank);
-    samp_pass<false>(e, n, &s, 1, 10, 11, 0xFFE00000u, cut, rank);
-    samp_pass<false>(e, n, &s, 2, 0, 10, 0xFFFFFC00u, cut, rank);
+    samp_pass<false, C, K>(e, n, &s, 0, 21, 11, 0x00000000u, cut, rank);
+    samp_pass<false, C, K>(e, n, &s, 1, 10, 11, 0xFFE00000u, cut, rank);
+    samp_pass<false, C, K>(e, n, &s, 2, 0, 10, 0xFFFFFC00u, cut, rank);
     thr_key = s.prefix;
     // mass of the kept set
     float mk = 0.f;
@@ -524,9 +602,14 @@ sample_kernel(float* logits, long ld, int V, int slice, int resident, const floa
     }
     mk = samp_block_sum(mk, s.sv);
     if (threadIdx.x == 0) s.xch[2].v[0] = mk;
-    samp_cluster_sync();
-    mass = 0.f;
-    for (int r = 0; r < SAMP_C; r++) mass += samp_peek(&s.xch[2].v[0], r);
+    samp_meet<C>();
+    if (threadIdx.x == 0) {
+      mk = 0.f;
+      for (int r = 0; r < C; r++) mk += samp_peek<C>(&s.xch[2].v[0], r);
+      s.all[2].v[0] = mk;
+    }
+    __syncthreads();
+    mass = s.all[2].v[0];
   }
   if (pth < 1.f && mass == mass) {
     cut = 0;                           // a margin for the order of the sums
@@ -535,9 +618,9 @@ sample_kernel(float* logits, long ld, int V, int slice, int resident, const floa
     if (thr_key > cut) cut = thr_key;
     if (threadIdx.x == 0) { s.prefix = 0; s.remaining = __float2ull_rn(pth * mass * SAMP_UNIT); }
     __syncthreads();
-    samp_pass<true>(e, n, &s, 3, 21, 11, 0x00000000u, cut, rank);
-    samp_pass<true>(e, n, &s, 4, 10, 11, 0xFFE00000u, cut, rank);
-    samp_pass<true>(e, n, &s, 5, 0, 10, 0xFFFFFC00u, cut, rank);
+    samp_pass<true, C, K>(e, n, &s, 3, 21, 11, 0x00000000u, cut, rank);
+    samp_pass<true, C, K>(e, n, &s, 4, 10, 11, 0xFFE00000u, cut, rank);
+    samp_pass<true, C, K>(e, n, &s, 5, 0, 10, 0xFFFFFC00u, cut, rank);
     if (s.prefix > thr_key) thr_key = s.prefix;
   }
   if (mp > 0.f) {
@@ -566,9 +649,9 @@ sample_kernel(float* logits, long ld, int V, int slice, int resident, const floa
         samp_better(bestv, besti, v[j] / fmaxf(ex, 1e-20f), first + i0 + j);
       }
   }
-  samp_cluster_argmax(bestv, besti, &s, &s.xch[3]);
+  samp_cluster_argmax(bestv, besti, &s, 3);
   if (rank == 0 && threadIdx.x == 0) out[b] = besti;
-  samp_cluster_sync();
+  samp_meet<C>();
 }
 
 // Rows of 16-byte aligned storage go eight elements at a time: 192 x 151936 81 us with single elements, 33 us so.
@@ -635,35 +718,48 @@ B200_API int b200_apply_penalties(void* logits, long ld, int B, int V, const voi
   return B200_CHECK_LAUNCH();
 }
 
-B200_API int b200_sample(void* logits_f32, long ld, int B, int V, const void* temperature,
-                         const void* top_k, const void* top_p, const void* min_p,
-                         const void* seeds, const void* offsets, void* out,
-                         cudaStream_t stream) {
-  if (B <= 0) return 0;
-  const int slice = ((V + SAMP_C - 1) / SAMP_C + 3) / 4 * 4;
+template <int C, int K>
+static int launch_sample(float* logits, long ld, int B, int V, int slice, const float* temperature, const int* top_k,
+                         const float* top_p, const float* min_p, const unsigned long long* seeds, const long* offsets,
+                         long* out, cudaStream_t stream) {
   const int resident = slice <= SAMP_MAX_SLICE;
-  const size_t smem = resident ? (size_t)slice * 4 : 0;
-  const cudaError_t allowed = allow_smem<sample_kernel>(SAMP_MAX_SLICE * 4);
-  if (allowed != cudaSuccess) return (int)allowed;
+  cudaError_t e = allow_smem<sample_kernel<C, K>>((K == 1 ? SAMP_MAX_SLICE : SAMP_TWO_HIST_SLICE) * 4);
+  if (e != cudaSuccess) return (int)e;
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(SAMP_T);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = resident ? (size_t)slice * 4 : 0;
   cfg.stream = stream;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = SAMP_C;
+  attr.val.clusterDim.x = C;
   attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   for (int b0 = 0; b0 < B; b0 += 65535) {
     const int nb = B - b0 < 65535 ? B - b0 : 65535;
-    cfg.gridDim = dim3(SAMP_C, (unsigned)nb);
-    cudaError_t e = cudaLaunchKernelEx(
-        &cfg, sample_kernel, (float*)logits_f32 + (long)b0 * ld, ld, V, slice, resident,
-        temperature ? (const float*)temperature + b0 : nullptr, top_k ? (const int*)top_k + b0 : nullptr,
-        top_p ? (const float*)top_p + b0 : nullptr, min_p ? (const float*)min_p + b0 : nullptr,
-        seeds ? (const unsigned long long*)seeds + b0 : nullptr, offsets ? (const long*)offsets + b0 : nullptr, (long*)out + b0);
+    cfg.gridDim = dim3(C, (unsigned)nb);
+    e = cudaLaunchKernelEx(&cfg, sample_kernel<C, K>, logits + (long)b0 * ld, ld, V, slice, resident,
+                           temperature ? temperature + b0 : nullptr, top_k ? top_k + b0 : nullptr, top_p ? top_p + b0 : nullptr,
+                           min_p ? min_p + b0 : nullptr, seeds ? seeds + b0 : nullptr, offsets ? offsets + b0 : nullptr, out + b0);
     if (e != cudaSuccess) return (int)e;
   }
   return 0;
+}
+
+B200_API int b200_sample(void* logits_f32, long ld, int B, int V, const void* temperature,
+                         const void* top_k, const void* top_p, const void* min_p,
+                         const void* seeds, const void* offsets, void* out,
+                         cudaStream_t stream) {
+  if (B <= 0) return 0;
+  // Blocks per row: as many as two per SM give every row (a row of 32000 on eight blocks, 192 rows: plain 56 us, top-p 72; on
+  // two 37 and 49), but so few elements to a block that an SM holds two of them (on one 50 and 58); rows too long for that share
+  // an SM with nobody, and clusters of four then leave no SM out (256 rows of 200000, eight blocks 1.2 times as long).
+  auto slice = [&](int c) { return ((V + c - 1) / c + 3) / 4 * 4; };
+  int c = 8;
+  while (c > 1 && (long)B * c > 2l * num_sms() && slice(c / 2) <= SAMP_PAIR_SLICE) c /= 2;
+  if (slice(8) > SAMP_PAIR_SLICE && slice(4) <= SAMP_MAX_SLICE && B * 8l > num_sms()) c = 4;
+  auto* launch = c == 1 ? launch_sample<1, 1> : c == 2 ? launch_sample<2, 1> : c == 4 ? launch_sample<4, 1>
+                 : slice(8) > SAMP_PAIR_SLICE && slice(8) <= SAMP_TWO_HIST_SLICE ? launch_sample<8, 2> : launch_sample<8, 1>;
+  return launch((float*)logits_f32, ld, B, V, slice(c), (const float*)temperature, (const int*)top_k, (const float*)top_p,
+                (const float*)min_p, (const unsigned long long*)seeds, (const long*)offsets, (long*)out, stream);
 }
