@@ -85,3 +85,34 @@ def test_row_statistics_are_those_of_the_stored_rows(M, N, K):
     ref = (out.double() @ w2.double().t()) * torch.rsqrt((out.double() ** 2).mean(-1, keepdim=True) + 1e-6)
     assert ((y.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-3).all()
     _native.check_status(torch.device(DEV))
+
+
+@pytest.mark.parametrize("M,N,K", [(33, 12288, 2048), (40, 5120, 2048), (64, 6144, 2112), (130, 3072, 2048), (250, 2040, 2048)])
+def test_splits_that_fit_one_wave(M, N, K):
+    """Tile counts at which a part more per tile would leave clusters for a second wave."""
+    g = torch.Generator(device=DEV).manual_seed(N)
+    x = torch.randn(M, K, device=DEV, generator=g).bfloat16()
+    w = (torch.randn(N, K, device=DEV, generator=g) * 0.05).bfloat16()
+    assert ops._few_rows(M, N, K) == (N != 12288)
+    out = torch.full((M, N), float("nan"), device=DEV, dtype=torch.bfloat16)
+    ops._gemm_small(x, w, out, None, None, N, False)
+    _check(out, x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t(), K)
+    _native.check_status(torch.device(DEV))
+
+
+def test_splits_and_the_choice_of_kernel():
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for M in (1, 16, 64, 128, 129, 256):
+        for N in (8, 128, 2048, 5120, 6144, 12288, 18944, 60000, 151936):
+            for K in (8, 2040, 2048, 4096, 28672):
+                for glu in (0, 1):
+                    s = _native.lib().b200_gemm_small_splits(M, N, K, glu)
+                    tiles, blocks = -(-N // (64 if glu else 128)), -(-K // 64)
+                    assert 1 <= s <= min(8, max(1, blocks // 4)) and (s == 1 or blocks >= 32)
+                    assert s == 1 or s * tiles <= sms * (2 if M <= 128 else 1), (M, N, K, glu, s)
+    assert _native.lib().b200_gemm_small_splits(257, 128, 4096, 0) < 0
+    # K that is not split, products wide enough for the general kernels, few rows
+    few = ops._few_rows
+    assert few(1, 4096, 512) and few(32, 151936, 2048) and few(128, 4096, 2048) and few(256, 4096, 4096) and few(64, 12288, 4096)
+    assert not few(33, 4096, 1536) and not few(256, 6144, 4096) and not few(128, 12288, 4096) and not few(64, 12288, 2048)
+    assert few(100, 28672, 2048, True) and not few(128, 28672, 2048, True) and not few(200, 768, 1024, True)

@@ -25,6 +25,7 @@ _SIGNATURES = {
     "b200_gemm_bf16_2cta": [P, P, P, P, P, I, I, I, I, I, I, I, P, P],
     "b200_gemm_bf16_2cta_norm": [P, P, P, P, P, I, I, I, I, I, I, I, P, I, ctypes.c_float, P, L, I, P, P],
     "b200_gemm_small_stats": [P, P, P, P, P, I, I, I, I, I, I, P, L, I, P, P],
+    "b200_gemm_small_splits": [I, I, I, I],
     "b200_gemm_small_bf16": [P, P, P, P, P, I, I, I, I, I, I, I, F, F, I, P, P],
     "b200_attn_prefill": [P, L, L, P, P, L, I, P, P, P, I, I, L, I, I, F, I, I, P, L, I, P, P],
     "b200_attn_prefill_latent": [P, L, L, P, P, L, P, P, P, I, L, I, I, I, I, F, P, P, P],

@@ -34,4 +34,31 @@ __device__ __forceinline__ float4 sg_sum(const uint32_t part, int splits, uint32
   return s;
 }
 
+// How many clusters of `blocks` blocks the GPU runs at once with `per_sm` blocks on an SM.  A cluster lies within one group of SMs, and
+// groups leave SMs over that no cluster fits into: one block per SM, 45 clusters of three, where 148 SMs give 49.  A grid that counted
+// SMs ran in two waves (64 rows of 6144 x 4096 in six parts 27 us, in five 21 us).  The driver is asked once per size, about one
+// block per SM (its answer does not double where two fit); the same groups hold twice as many with two.
+using sg_fit_t = std::atomic<int>;
+template <auto Kernel>
+inline int sg_clusters_at_once(sg_fit_t* known, int blocks, int threads, int per_sm) {
+  int n = known[blocks].load(std::memory_order_relaxed);
+  if (n > 0) return n * per_sm;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks, 1);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = 160 * 1024;             // an SM to itself
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = blocks;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, Kernel, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    return 0;
+  }
+  known[blocks].store(n, std::memory_order_relaxed);
+  return n * per_sm;
+}
+
 }  // namespace b200

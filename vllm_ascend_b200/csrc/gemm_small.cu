@@ -215,7 +215,12 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   }
 }
 
-static int launch_small(const void* A, const void* W, SmallGemmParams& p, int lda, int ldw, int splits, cudaStream_t stream) {
+static int small_smem(const SmallGemmParams& p) {
+  return p.stages * p.stage_bytes + (2 * SG_MAX_STAGES + 1) * 8 + 16 + 1024;
+}
+
+// Tokens, stages and (where none are asked for) splits of K.  Nonzero: refused.
+static int plan_small(SmallGemmParams& p, int splits) {
   const int rows = p.glu ? SG_ROWS / 2 : SG_ROWS;
   const int tiles = (p.N + rows - 1) / rows, num_kb = (p.K + SG_BK - 1) / SG_BK;
   p.nt = (p.M + 15) / 16 * 16;
@@ -226,43 +231,44 @@ static int launch_small(const void* A, const void* W, SmallGemmParams& p, int ld
   if (p.stages > SG_MAX_STAGES) p.stages = SG_MAX_STAGES;
   p.tmem_cols = 32;
   while (p.tmem_cols < p.nt) p.tmem_cols *= 2;
+  cudaError_t e = allow_smem<gemm_small_kernel>(227 * 1024);
+  if (e != cudaSuccess) return (int)e;
   if (splits <= 0) {
     // as many blocks as fit in one wave, at least four stages of K each (shorter parts are all prologue).  K below 2048 is
-    // not split: its rows keep the bits they have in the general kernel, for the few us it would save (one row of
-    // 2048 x 1024: 14.4 us whole, 10.3 us in four parts, 16.4 us in the general kernel)
-    const int slots = num_sms() * (pair ? 2 : 1);
-    splits = slots / tiles;
-    if (splits > num_kb / 4) splits = num_kb / 4;
-    if (splits > 8) splits = 8;
-    if (splits < 1 || num_kb < 32) splits = 1;
+    // not split: its rows keep the bits they have in the general kernel
+    splits = 1;
+    if (num_kb >= 32) {
+      static sg_fit_t fit[9];
+      splits = num_kb / 4 < 8 ? num_kb / 4 : 8;
+      while (splits > 1 && tiles > sg_clusters_at_once<gemm_small_kernel>(fit, splits, SG_THREADS, pair ? 2 : 1)) splits--;
+    }
   }
   if (splits > 8 || splits > num_kb) return 9100;
   p.splits = splits;
   // weights asked of L2 ahead of the loads: at most 48 MB over the grid
-  const long per_kb = (long)tiles * splits * SG_WBYTES;
-  p.prefetch_kb = (int)(48l * 1024 * 1024 / per_kb);
-  const int smem = p.stages * p.stage_bytes + (2 * SG_MAX_STAGES + 1) * 8 + 16 + 1024;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  p.prefetch_kb = (int)(48l * 1024 * 1024 / ((long)tiles * splits * SG_WBYTES));
+  return 0;
+}
+
+static int launch_small(const void* A, const void* W, SmallGemmParams& p, int lda, int ldw, int splits, cudaStream_t stream) {
+  const int rows = p.glu ? SG_ROWS / 2 : SG_ROWS;
+  int rc = plan_small(p, splits);
+  if (rc) return rc;
   CUtensorMap tw, ta;
-  int rc = get_tmap_2d_bf16(&tw, W, (uint64_t)p.N * (p.glu ? 2 : 1), (uint64_t)p.K, (uint64_t)ldw, rows);
+  rc = get_tmap_2d_bf16(&tw, W, (uint64_t)p.N * (p.glu ? 2 : 1), (uint64_t)p.K, (uint64_t)ldw, rows);
   if (rc) return rc;
   rc = get_tmap_2d_bf16(&ta, A, (uint64_t)p.M, (uint64_t)p.K, (uint64_t)lda, p.nt);
   if (rc) return rc;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(splits, tiles);
+  cfg.gridDim = dim3(p.splits, (p.N + rows - 1) / rows);
   cfg.blockDim = dim3(SG_THREADS);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = small_smem(p);
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = splits;
+  attr[1].val.clusterDim.x = p.splits;
   attr[1].val.clusterDim.y = 1;
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
@@ -312,4 +318,15 @@ B200_API int b200_gemm_small_stats(const void* A, const void* W, void* C, const 
   p.ss_parts_max = ss_parts_max;
   p.status = status;
   return launch_small(A, W, p, lda, ldw, 0, stream);
+}
+
+// Parts of K that a product of these sizes is split into where none are asked for (rules that choose between kernels); negative:
+// refused.
+B200_API int b200_gemm_small_splits(int M, int N, int K, int glu) {
+  if (M <= 0 || N <= 0 || M > 256 || K <= 0) return -1;
+  SmallGemmParams p;
+  memset(&p, 0, sizeof(p));
+  p.M = M; p.N = N; p.K = K;
+  p.glu = glu;
+  return plan_small(p, 0) ? -1 : p.splits;
 }

@@ -11,6 +11,7 @@ The op set corresponds to the reference's OOT custom-op table
 """
 from __future__ import annotations
 
+import functools
 from typing import Optional
 
 import torch
@@ -313,20 +314,50 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Ten
     return out.view(*x.shape[:-1], I)
 
 
-#: most rows and, beyond 128 rows, most output columns of the few-row GEMM.  Measured on a B200, old kernel -> few-row kernel, us
-#: with cold caches: 4096 x 4096 with 1 / 128 / 256 rows 32 -> 17 / 32 -> 23 / 34 -> 26; 4096 x 12288 71 -> 32 / 72 -> 39 / 75 -> 46;
-#: gate / up 24576 x 4096 80 -> 53 / 64 -> 62 / 77 -> 100.  Beyond 128 rows every stage carries twice as many activations as
-#: weights, which pays only where the tiles of the other kernels leave most SMs idle.
-_FEW_ROWS, _FEW_ROWS_MAX_COLS = 256, 5120
+#: most rows of the few-row GEMM
+_FEW_ROWS = 256
 
 
-def _few_rows(M: int, N: int, K: int) -> bool:
-    """Whether a step's product runs in the kernel that splits K over blocks.  Its rows may differ in the last bit from
-    those of a larger batch, so modes that fix the order of sums never take it."""
-    if M > _FEW_ROWS or (M > 128 and N > _FEW_ROWS_MAX_COLS) or K % 8 or N % 8 or envs.VLLM_B200_GEMM == "cublas":
+@functools.lru_cache(maxsize=8192)
+def _few_rows_faster(M: int, N: int, K: int, glu: bool) -> bool:
+    """Where the few-row kernel beats the general ones.  us per product in a captured chain of norms and products with cold weights on a
+    B200, general -> few-row:
+
+    up to 32 rows     wherever weights are streamed: 4096 x 4096 28 -> 16, 24576 x 4096 62 -> 43, 151936 x 2048 150 -> 100, 2048 x 512 11 -> 9
+    33..64 rows       K unsplit (below 2048) costs its serial sums: 64 rows of 4096 x 1536 16 -> 18.  Three splits: 4096 x 2048 19 -> 13,
+                      10240 x 2048 20.5 -> 20.3.  Fewer: 14336 x 2048 22 -> 23, x 4096 33 -> 32; wider than the GPU in one go 24576 x 2048 34 -> 29
+    65..256 rows      stages carry as many or twice as many activations as weights: four splits, 128 rows of 8192 x 2048 20.0 -> 19.4, 256 of
+                      4096 x 2048 20 -> 18; three, 128 rows of 10240 x 2048 21 -> 23, x 4096 32 -> 30; fewer, 128 rows of 14336 x 4096 34 -> 36, 256
+                      of 6144 x 4096 32 -> 32.  Up to 128 rows of more tiles than SMs but no more than two per SM (one wave here, two in the
+                      general kernel) 24576 x 4096 58 -> 51, 32000 x 4096 60 -> 60
+    gate and up       nearly everywhere: 64 rows of 2 x 12288 x 4096 65 -> 47.  Level or behind: from 113 rows on with more tiles than run at
+                      once (128 rows of 2 x 28672 x 2048 29 -> 31), from 193 rows on with K unsplit (256 of 2 x 768 x 1024 24 -> 26)
+    """
+    splits = _native.lib().b200_gemm_small_splits(M, N, K, int(glu))
+    sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+    if splits < 1:
+        return False
+    if glu:
+        if M <= 128:
+            return M <= 112 or (N + 63) // 64 <= 2 * sms
+        return 2 * N <= 5120 and (M <= 192 or K >= 2048)
+    if M <= 32:
+        return True
+    tiles = (N + 127) // 128
+    if K < 2048:
+        return False
+    if M <= 64:
+        return splits >= 3 or K >= 4096 or tiles > sms
+    return splits >= 4 or (K >= 4096 and (splits == 3 or (M <= 128 and sms < tiles <= 2 * sms)))
+
+
+def _few_rows(M: int, N: int, K: int, glu: bool = False) -> bool:
+    """Whether a step's product (N columns; ``glu``: of gate and up together twice as many) runs in the kernel that splits K over
+    blocks.  Its rows may differ in the last bit from those of a larger batch, so modes that fix the order of sums never take it."""
+    if M > _FEW_ROWS or K % 8 or N % 8 or envs.VLLM_B200_GEMM == "cublas":
         return False
     from ..batch_invariant import fixed_sums
-    return not fixed_sums()
+    return not fixed_sums() and _few_rows_faster(M, N, K, glu)
 
 
 def _pair_rows(M: int) -> bool:
@@ -352,7 +383,7 @@ def linear_step(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
     K, N = x.shape[-1], weight.shape[0]
     M = x.numel() // K if K else 0
     if M == 0 or not _use_native(x) or weight.dtype != _BF16 or not _few_rows(M, N, K):
-        return linear(x, weight, bias, residual, bn=512 if _pair_rows(M) and N > _FEW_ROWS_MAX_COLS else 0)
+        return linear(x, weight, bias, residual, bn=512 if _pair_rows(M) and N > 5120 else 0)
     x2 = x.reshape(-1, K)
     if x2.stride(-1) != 1 or (x2.stride(0) % 8) != 0:
         x2 = x2.contiguous()
@@ -369,7 +400,7 @@ def linear_swiglu_step(x: torch.Tensor, weight: torch.Tensor, limit: Optional[fl
     """``linear_swiglu`` for the products of an engine's step (see ``linear_step``)."""
     K, I = x.shape[-1], weight.shape[0] // 2
     M = x.numel() // K if K else 0
-    if M == 0 or not _use_native(x) or weight.dtype != _BF16 or not _few_rows(M, 2 * I, K) or I % 8:
+    if M == 0 or not _use_native(x) or weight.dtype != _BF16 or not _few_rows(M, I, K, True):
         return linear_swiglu(x, weight, limit=limit, two_cta=_pair_rows(M))
     x2 = x.reshape(-1, K)
     if x2.stride(-1) != 1 or (x2.stride(0) % 8) != 0:
