@@ -47,3 +47,17 @@ def test_every_split(M, splits):
         _native.status_word(a.device).data_ptr(), _native.stream_ptr()), "gemm_small_fp8")
     _check(out, ad @ wd.t(), ad.abs() @ wd.abs().t(), K)
     _native.check_status(torch.device(DEV))
+
+
+@pytest.mark.parametrize("M,N,K,few", [(32, 128, 1024, True), (32, 128, 896, False), (33, 640, 2048, True), (64, 16384, 4096, False), (64, 16384, 8192, True),
+                                       (128, 2048, 4096, True), (128, 28672, 8192, False), (128, 128, 2048, False), (129, 128, 8192, False)])
+def test_which_products_split_k(monkeypatch, M, N, K, few):
+    """The kernel that the rule chooses, and products of a tile, a remainder and a part of K on both sides of the rule's lines."""
+    assert (M <= schemes._FP8_FEW_ROWS and schemes._fp8_few_rows_faster(M, N, K)) == few
+    N = min(N, 264)
+    a, w, sa, sw, ad, wd = _make(M, N, K, M)
+    for choice in (True, False):
+        monkeypatch.setattr(schemes, "_fp8_few_rows_faster", lambda *size: choice)
+        out = schemes.fp8_block_linear(None, w, sw, None, quant=(a, sa))
+        _check(out, ad @ wd.t(), ad.abs() @ wd.abs().t(), K)
+    _native.check_status(torch.device(DEV))

@@ -238,44 +238,55 @@ static int sf_tmap(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t co
 }
 
 template <int NT>
-static int launch_sf(const void* A, const void* W, SmallFp8Params& p, int lda, int ldw, int splits, cudaStream_t stream) {
+static int sf_smem(const SmallFp8Params& p) {
+  return p.stages * p.stage_bytes + SF_SCALE_KB * NT * 4 + (2 * SF_MAX_STAGES + 2 * SfCfg<NT>::NB) * 8 + 16 + 1024;
+}
+
+// Stages and (where none are asked for) splits of K.  Nonzero: refused.
+template <int NT>
+static int plan_sf(SmallFp8Params& p, int splits) {
   using Cfg = SfCfg<NT>;
   const int tiles = (p.N + SG_ROWS - 1) / SG_ROWS;
   p.stage_bytes = SF_WBYTES + NT * 128;
-  const int fixed = SF_SCALE_KB * NT * 4 + (2 * SF_MAX_STAGES + 2 * Cfg::NB) * 8 + 16 + 1024;
-  p.stages = ((Cfg::BLOCKS == 2 ? 112 : 224) * 1024 - fixed) / p.stage_bytes;
+  p.stages = 0;
+  p.stages = ((Cfg::BLOCKS == 2 ? 112 : 224) * 1024 - sf_smem<NT>(p)) / p.stage_bytes;
   if (p.stages > SF_MAX_STAGES) p.stages = SF_MAX_STAGES;
+  cudaError_t e = allow_smem<gemm_small_fp8_kernel<NT>>(227 * 1024);
+  if (e != cudaSuccess) return (int)e;
   if (splits <= 0) {
     // one wave of blocks, at least four K blocks each; K below 2048 is not split (rows keep the general kernel's bits)
-    splits = num_sms() * Cfg::BLOCKS / tiles;
-    if (splits > p.num_kb / 4) splits = p.num_kb / 4;
-    if (splits > 8) splits = 8;
-    if (splits < 1 || p.num_kb < 16) splits = 1;
+    splits = 1;
+    if (p.num_kb >= 16) {
+      static sg_fit_t fit[9];
+      splits = p.num_kb / 4 < 8 ? p.num_kb / 4 : 8;
+      while (splits > 1 && tiles > sg_clusters_at_once<gemm_small_fp8_kernel<NT>>(fit, splits, SF_THREADS, Cfg::BLOCKS)) splits--;
+    }
   }
   if (splits > 8 || splits > p.num_kb) return 9100;
   p.splits = splits;
   p.prefetch_kb = (int)(48l * 1024 * 1024 / ((long)tiles * splits * SF_WBYTES));      // at most 48 MB over the grid
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_small_fp8_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  return 0;
+}
+
+template <int NT>
+static int launch_sf(const void* A, const void* W, SmallFp8Params& p, int lda, int ldw, int splits, cudaStream_t stream) {
+  int rc = plan_sf<NT>(p, splits);
+  if (rc) return rc;
   CUtensorMap tw, ta;
-  int rc = sf_tmap(&tw, W, (uint64_t)p.N, (uint64_t)p.num_kb * 128, (uint64_t)ldw, SG_ROWS);
+  rc = sf_tmap(&tw, W, (uint64_t)p.N, (uint64_t)p.num_kb * 128, (uint64_t)ldw, SG_ROWS);
   if (rc) return rc;
   rc = sf_tmap(&ta, A, (uint64_t)p.M, (uint64_t)p.num_kb * 128, (uint64_t)lda, NT);
   if (rc) return rc;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(splits, tiles);
+  cfg.gridDim = dim3(p.splits, (p.N + SG_ROWS - 1) / SG_ROWS);
   cfg.blockDim = dim3(SF_THREADS);
-  cfg.dynamicSmemBytes = p.stages * p.stage_bytes + fixed;
+  cfg.dynamicSmemBytes = sf_smem<NT>(p);
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = splits;
+  attr[1].val.clusterDim.x = p.splits;
   attr[1].val.clusterDim.y = 1;
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
@@ -303,4 +314,14 @@ B200_API int b200_gemm_small_fp8(const void* A8, const void* a_scale, const void
   if (M <= 32) return launch_sf<32>(A8, W8, p, lda, ldw, splits, stream);
   if (M <= 64) return launch_sf<64>(A8, W8, p, lda, ldw, splits, stream);
   return launch_sf<128>(A8, W8, p, lda, ldw, splits, stream);
+}
+
+// Parts of K that a product of these sizes is split into where none are asked for; negative: refused.
+B200_API int b200_gemm_small_fp8_splits(int M, int N, int K) {
+  if (M <= 0 || N <= 0 || M > 128 || K < 128) return -1;
+  SmallFp8Params p;
+  memset(&p, 0, sizeof(p));
+  p.M = M; p.N = N; p.num_kb = K / 128;
+  const int rc = M <= 32 ? plan_sf<32>(p, 0) : M <= 64 ? plan_sf<64>(p, 0) : plan_sf<128>(p, 0);
+  return rc ? -1 : p.splits;
 }

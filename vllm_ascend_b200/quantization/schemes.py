@@ -13,6 +13,7 @@ FLOAT          unquantized pass-through (a layer the description lists as "FLOAT
 """
 from __future__ import annotations
 
+import functools
 from typing import Optional
 
 import torch
@@ -112,6 +113,7 @@ def _declare_native():
     from ctypes import c_int, c_long, c_void_p
     P, I, L = c_void_p, c_int, c_long
     _native.register_signature("b200_gemm_fp8_block", [P, P, P, P, P, P, I, I, I, I, I, I, P, P])
+    _native.register_signature("b200_gemm_small_fp8_splits", [I, I, I])
     _native.register_signature("b200_gemm_small_fp8", [P, P, P, P, P, P, I, I, I, I, I, I, I, P, P])
     _native.register_signature("b200_grouped_gemm_fp8_block",
                                [P, P, P, P, P, P, I, L, I, I, I, I, I, P, P])
@@ -125,6 +127,27 @@ _declare_native()
 
 #: most rows of the few-row GEMM
 _FP8_FEW_ROWS = 128
+
+
+@functools.lru_cache(maxsize=8192)
+def _fp8_few_rows_faster(M: int, N: int, K: int) -> bool:
+    """Where the few-row kernel beats the general one.  us per quantisation and product in a captured chain with cold weights on a B200,
+    general -> few-row:
+
+    up to 32 rows   K of 1024 and more: 8192 x 2048 14 -> 12, 57344 x 8192 99 -> 84; 8192 x 512 8 -> 8, x 256 7 -> 8
+    33..64 rows     64 rows of 4096 x 4096 20 -> 16, 10240 x 4096 22 -> 21 (three splits), 14336 x 4096 22 -> 24 and x 8192 37 -> 33 (two); of K = 2048
+                    6144 columns 14.8 -> 14.1, 8192 columns 14.6 -> 15
+    65..128 rows    one block per SM, and its promotion takes as long as the general kernel's: 128 rows of 4096 x 4096 22 -> 18 (four), 8192 x 4096
+                    23 -> 23 and x 8192 37 -> 32 (two), 28672 x 8192 55 -> 95 (one)
+    """
+    splits = _native.lib().b200_gemm_small_fp8_splits(M, N, K)
+    if splits < 1:
+        return False
+    if M <= 32:
+        return K >= 1024
+    if M <= 64:
+        return K >= 8192 or (K >= 4096 and splits >= 3) or (K >= 2048 and N <= 6144)
+    return (K >= 4096 and splits >= 3) or (K >= 8192 and splits >= 2)
 
 
 def fp8_block_linear(x: Optional[torch.Tensor], w8: torch.Tensor, w_scale: torch.Tensor,
@@ -141,7 +164,7 @@ def fp8_block_linear(x: Optional[torch.Tensor], w8: torch.Tensor, w_scale: torch
     if M == 0:
         return out
     from ..batch_invariant import fixed_sums
-    if M <= _FP8_FEW_ROWS and not fixed_rows and not fixed_sums():
+    if M <= _FP8_FEW_ROWS and not fixed_rows and not fixed_sums() and _fp8_few_rows_faster(M, N, K):
         # K split over blocks: rows may differ in the last bit from those of a larger batch
         rc = _native.lib().b200_gemm_small_fp8(
             xq.data_ptr(), xs.data_ptr(), w8.data_ptr(), w_scale.data_ptr(), out.data_ptr(), _native.ptr(bias), M, N, K,
