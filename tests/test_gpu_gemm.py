@@ -143,3 +143,18 @@ def test_gemm_2cta_chooses_narrow_tiles_for_few_tiles():
     # automatic choice: same answers as the fixed widths on the shapes where it departs from 256
     for M, N, K in ((768, 4096, 4096), (1024, 3072, 4096), (512, 6144, 4096), (8192, 768, 4096)):
         _check(M, N, K, bn=512, seed=M)
+
+
+def test_which_rows_share_a_paired_tile(monkeypatch):
+    """The rule of 129 to 255 rows, and that a larger VLLM_B200_GEMM_2CTA_MIN_M is not overridden by it; the same bits either way."""
+    pair = ops._pair_rows
+    assert pair(129, 12288, 1024) and pair(255, 151936, 4096) and pair(137, 4096, 2048, True)
+    assert not pair(128, 12288, 4096) and not pair(144, 8192, 4096) and not pair(144, 16384, 768) and not pair(144, 12288, 1024, True)
+    g = torch.Generator().manual_seed(0)
+    x = torch.randn(137, 1024, generator=g).bfloat16().to(DEV)
+    w = (torch.randn(2 * 9728, 1024, generator=g) * 0.05).bfloat16().to(DEV)
+    paired, gated = ops.linear_step(x, w), ops.linear_swiglu_step(x, w)
+    for least in ("0", "300"):
+        monkeypatch.setenv("VLLM_B200_GEMM_2CTA_MIN_M", least)
+        assert not pair(200, 12288, 4096) and not pair(200, 12288, 4096, True)
+        assert torch.equal(ops.linear_step(x, w), paired) and torch.equal(ops.linear_swiglu_step(x, w), gated)

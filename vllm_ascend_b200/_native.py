@@ -8,6 +8,7 @@ loader ``enable_custom_op`` (vllm_ascend/utils.py:397-456).
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from ctypes import c_float, c_int, c_long, c_uint, c_void_p
 from typing import Optional
@@ -120,6 +121,12 @@ def lib() -> ctypes.CDLL:
 
 def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
+
+
+@functools.lru_cache(maxsize=None)
+def sm_count(device) -> int:
+    """SMs of a device (asking torch for the properties takes 2 us, which rules inside an op have not got)."""
+    return torch.cuda.get_device_properties(device).multi_processor_count
 
 
 def stream_ptr(device=None) -> int:

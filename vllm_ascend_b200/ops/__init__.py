@@ -334,7 +334,7 @@ def _few_rows_faster(M: int, N: int, K: int, glu: bool) -> bool:
                       once (128 rows of 2 x 28672 x 2048 29 -> 31), from 193 rows on with K unsplit (256 of 2 x 768 x 1024 24 -> 26)
     """
     splits = _native.lib().b200_gemm_small_splits(M, N, K, int(glu))
-    sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+    sms = _native.sm_count(torch.cuda.current_device())
     if splits < 1:
         return False
     if glu:
@@ -360,10 +360,17 @@ def _few_rows(M: int, N: int, K: int, glu: bool = False) -> bool:
     return not fixed_sums() and _few_rows_faster(M, N, K, glu)
 
 
-def _pair_rows(M: int) -> bool:
-    """Rows that fill more than half of a paired tile of 256: wide products are faster there than in two tiles of 128 (137 rows of
-    24576 x 4096: 87 us in two tiles, 77 us in one), and keep the same bits."""
-    return 128 < M <= 256 and envs.VLLM_B200_GEMM_2CTA_MIN_M > 0
+def _pair_rows(M: int, N: int, K: int, glu: bool = False) -> bool:
+    """129 to 255 rows, which fill more than half of a paired tile of 256: N columns that keep the GPU busy for more than one wave of
+    128 x 128 tiles read their weights once there and twice in those tiles (137 rows of 24576 x 4096: 87 us in two tiles, 77 us in
+    one; 144 rows of 10240 x 1024 20 -> 17 us).  Narrower ones leave half of the pairs without a tile (144 rows of 8192 x 4096 32 -> 34 us), and
+    K below 1024 is all prologue (of 16384 x 512 15 -> 17 us).  Gate and up: K from 2048 on (2 x 4096 x 4096 57 -> 55 us, x 1024 38 -> 39).  The
+    same bits.  A user's larger VLLM_B200_GEMM_2CTA_MIN_M holds."""
+    if not 128 < M <= 256 or not 0 < envs.VLLM_B200_GEMM_2CTA_MIN_M <= 256:
+        return False
+    if glu:
+        return K >= 2048
+    return K >= 1024 and (N + 127) // 128 * 2 > _native.sm_count(torch.cuda.current_device())
 
 
 def _gemm_small(x2, weight, out, bias, res2, N: int, glu: bool, alpha: float = 0.0, limit: float = 0.0) -> None:
@@ -383,7 +390,7 @@ def linear_step(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
     K, N = x.shape[-1], weight.shape[0]
     M = x.numel() // K if K else 0
     if M == 0 or not _use_native(x) or weight.dtype != _BF16 or not _few_rows(M, N, K):
-        return linear(x, weight, bias, residual, bn=512 if _pair_rows(M) and N > 5120 else 0)
+        return linear(x, weight, bias, residual, bn=512 if x.is_cuda and _pair_rows(M, N, K) else 0)
     x2 = x.reshape(-1, K)
     if x2.stride(-1) != 1 or (x2.stride(0) % 8) != 0:
         x2 = x2.contiguous()
@@ -401,7 +408,7 @@ def linear_swiglu_step(x: torch.Tensor, weight: torch.Tensor, limit: Optional[fl
     K, I = x.shape[-1], weight.shape[0] // 2
     M = x.numel() // K if K else 0
     if M == 0 or not _use_native(x) or weight.dtype != _BF16 or not _few_rows(M, I, K, True):
-        return linear_swiglu(x, weight, limit=limit, two_cta=_pair_rows(M))
+        return linear_swiglu(x, weight, limit=limit, two_cta=x.is_cuda and _pair_rows(M, I, K, True))
     x2 = x.reshape(-1, K)
     if x2.stride(-1) != 1 or (x2.stride(0) % 8) != 0:
         x2 = x2.contiguous()
