@@ -104,7 +104,7 @@ def test_sequences_without_keys_leave_their_rows_alone(causal):
 
 def test_mixed_step_gives_decodes_and_prompts_their_rows():
     g = torch.Generator().manual_seed(5)
-    new, old = [1, 1, 1, 4700, 130], [300, 5, 129, 0, 64]         # enough tiles for the kernel of pairs
+    new, old = [1, 1, 1, 7300, 130], [300, 5, 129, 0, 64]         # enough tiles for the kernel of pairs
     Hkv, G, D, page = 2, 4, 128, 128
     table, cu, lens, blocks = _batch(new, old, page, g)
     k, v = (ops.alloc_kv_cache(blocks, page, Hkv, D, torch.bfloat16, DEV) for _ in range(2))
@@ -112,7 +112,7 @@ def test_mixed_step_gives_decodes_and_prompts_their_rows():
     v.copy_(torch.randn(v.shape, generator=g).to(DEV))
     q = torch.randn((sum(new), Hkv * G, D), generator=g).to(DEV).bfloat16()
     meta = metadata_from_tensors(cu, lens, table, max(new), int(lens.max()), Hkv * G, Hkv, D)
-    assert ops._prefill_pairs(q, Hkv, 3) == (torch.cuda.get_device_properties(0).multi_processor_count <= 150)
+    assert ops._prefill_pairs(q, Hkv, 3, meta, 3) == (torch.cuda.get_device_properties(0).multi_processor_count <= 150)
     out = ops.paged_attention(q, k, v, meta, D ** -0.5)
     at = 0
     for b, (n, o) in enumerate(zip(new, old)):
@@ -181,4 +181,26 @@ def test_many_sequences_start_where_the_ones_before_end():
     seq = torch.repeat_interleave(torch.arange(n), lens.long()).to(DEV)
     pos = torch.arange(keys, device=DEV) - starts[:-1].long()[seq]
     assert torch.equal(a, lat[table[seq, 0].long(), pos]) and torch.equal(b, pe[table[seq, 0].long(), pos])
+    _native.check_status(torch.device(DEV))
+
+
+@pytest.mark.parametrize("new,old,Hkv,G,pairs", [([2048], 0, 8, 4, True), ([137], 0, 8, 4, False), ([16] * 100, 4000, 8, 4, False), ([33] * 256, 0, 8, 8, True),
+                                                 ([100] * 20 + [3000], 100, 1, 8, False), ([700] * 8, 0, 1, 8, False), ([700] * 8, 0, 8, 4, True)])
+def test_rule_counts_waves_and_empty_halves(monkeypatch, new, old, Hkv, G, pairs):
+    """What runs in pairs, and the same rows from either kernel: probabilities and results are rounded to bf16 in both."""
+    g = torch.Generator().manual_seed(len(new))
+    D, page = 128, 128
+    table, cu, lens, blocks = _batch(new, [old] * len(new), page, g)
+    k, v = (ops.alloc_kv_cache(blocks, page, Hkv, D, torch.bfloat16, DEV) for _ in range(2))
+    for c in (k, v):
+        c.copy_(torch.randn(c.shape, dtype=torch.bfloat16, generator=g).to(DEV))
+    q = torch.randn((sum(new), Hkv * G, D), generator=g).to(DEV).bfloat16()
+    meta = metadata_from_tensors(cu, lens, table, max(new), int(lens.max()), Hkv * G, Hkv, D)
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert ops._prefill_pairs(q, Hkv, 0, meta) == pairs
+    rows = []
+    for choice in (True, False):
+        monkeypatch.setattr(ops, "_prefill_pairs", lambda *a: choice)
+        rows.append(ops.paged_attention(q, k, v, meta, D ** -0.5).double())
+    assert ((rows[0] - rows[1]).abs() <= 6 * 2.0 ** -8 * (1 + rows[1].abs())).all()
     _native.check_status(torch.device(DEV))

@@ -14,6 +14,7 @@ from __future__ import annotations
 import functools
 from typing import Optional
 
+import numpy as np
 import torch
 
 from .. import _native, envs
@@ -480,16 +481,40 @@ def paged_prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: tor
     return out
 
 
-def _prefill_pairs(q: torch.Tensor, Hkv: int, first_row: int) -> bool:
-    """Whether a step's prompts run in the kernel that gives a block two query tiles: where those blocks can fill the GPU.
-    Fewer tiles are better off one to a block (137 tokens of 32 / 8 heads: 11.3 us in pairs, 9.2 us one by one; 2048 tokens of
-    64 / 8 heads 103 us in pairs, 122 us).  The kernels add a row's probabilities in different orders, so modes in
-    which a prompt gets the same bits whatever shares its step never take it."""
+@functools.lru_cache(maxsize=256)
+def _pairs_faster(cu: bytes, tile: int, Hkv: int, sms: int) -> bool:
+    """Whether sequences that start at these int32 row numbers take less time with two query tiles of ``tile`` tokens per block than with one.
+    Both kernels hold one block per SM; a pair takes one and a half times as long as a tile, 1.2 times where its second tile is empty.
+    One long prompt is better off in pairs wherever they fill the GPU (1500 tokens of 32 / 4 heads, 188 pairs or 376 tiles: 44 us in pairs,
+    48 us one by one).  Otherwise few waves count whole (20 x 100 and 3000 tokens of 8 / 1 heads, 174 pairs or 328 tiles: 72 us, 49 us; 8 x
+    700 tokens of 32 / 8 heads, 704 or 1408: 88 us, 110 us), and many go by their work (100 x 16 tokens behind 4000, 32 / 8 heads,
+    every pair half empty: 413 us, 334 us; 256 x 33 tokens of 64 / 8 heads, half of the pairs: 283 us, 328 us)."""
+    new = np.diff(np.frombuffer(cu, dtype=np.int32))
+    if 10 * int(new.max()) >= 9 * int(new.sum()):
+        return True
+    tiles, pairs = int((-(-new // tile)).sum()), int((-(-new // (2 * tile))).sum())
+    waves = -(-pairs * Hkv // sms)
+    return 9 * pairs < 7 * tiles if waves >= 4 else 3 * waves < 2 * -(-tiles * Hkv // sms)
+
+
+def _prefill_pairs(q: torch.Tensor, Hkv: int, first_row: int, meta=None, first_seq: int = 0) -> bool:
+    """Whether a step's prompts run in the kernel that gives a block two query tiles, for the sequences of ``meta`` from ``first_seq`` on: where its
+    blocks can fill the GPU and take less time.  The kernels add a row's probabilities in different orders, so modes in which a prompt
+    gets the same bits whatever shares its step never take it."""
     from ..batch_invariant import fixed_sums
     if fixed_sums():
         return False
-    pair = 2 * (128 // (q.shape[1] // Hkv))
-    return ((q.shape[0] - first_row) // pair) * Hkv >= torch.cuda.get_device_properties(q.device).multi_processor_count
+    tile, sms = 128 // (q.shape[1] // Hkv), _native.sm_count(q.device)
+    if (q.shape[0] - first_row) // (2 * tile) * Hkv < sms:
+        return False
+    if meta is None:
+        return True
+    cu = np.ascontiguousarray(meta.query_start_loc_cpu, dtype=np.int32)[first_seq:meta.num_reqs + 1]
+    if len(cu) > 1 and cu[-1] > cu[0]:
+        return _pairs_faster(cu.tobytes(), tile, Hkv, sms)
+    # lengths known on the device only: a sequence adds at most half a pair to half of its tiles
+    pairs = (meta.num_tiles + meta.num_reqs - first_seq) // 2
+    return 3 * -(-pairs * Hkv // sms) < 2 * -(-meta.num_tiles * Hkv // sms)
 
 
 _dec_prefetch_set = None
@@ -658,7 +683,7 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
         nd, ndt = meta.num_decodes, meta.num_decode_tokens
         paged_attention_decode_tc(q[:ndt], k_cache, v_cache, meta, scale, out[:ndt], window,
                                   num_splits=1, num_seqs=nd, max_q_len=1)
-        if meta.num_reqs > nd and D == 128 and _prefill_pairs(q, Hkv, ndt):
+        if meta.num_reqs > nd and D == 128 and _prefill_pairs(q, Hkv, ndt, meta, nd):
             paged_prefill_attention(q, k_cache, v_cache, meta, scale, out, causal, window, nd, ndt)
         elif meta.num_tiles > 0:
             paged_attention_tc(q, k_cache, v_cache, meta, scale, out, causal, window)
@@ -674,7 +699,7 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
             return paged_attention_tc(q, k_cache, v_cache, meta, scale, out, causal, window,
                                       num_splits=meta.num_splits)
     if envs.VLLM_B200_PREFILL_ATTN == "tcgen05" and tc_ok:
-        if D == 128 and meta.tile_seq is not None and _prefill_pairs(q, Hkv, 0):
+        if D == 128 and meta.tile_seq is not None and _prefill_pairs(q, Hkv, 0, meta):
             return paged_prefill_attention(q, k_cache, v_cache, meta, scale, out, causal, window)
         return paged_attention_tc(q, k_cache, v_cache, meta, scale, out, causal, window)
     # explicit opt-out: PyTorch path (validation only)
