@@ -106,3 +106,24 @@ def test_other_forms_stay_token_by_token(form):
     out = la.gated_delta_rule(q, k, v, g, beta, S, cu, slot, slot + 1, DK ** -0.5, cu_cpu=[0, T])
     want, S_want = _exact(q, k, v, g, beta, S0, [0, T], [0], [1], DK ** -0.5, True)
     assert _err(S, S_want) < 4e-6 and _err(out, want) < 2.0 ** -8
+
+
+def test_many_short_portions_share_out_between_the_kernels():
+    """A step whose rule sends portions of 40 and more tokens to chunks and shorter ones to the other kernel, and one whose 65-token portions
+    go token by token: the states and read-outs of both kernels side by side, each its own sequences."""
+    gen = torch.Generator(device=DEV).manual_seed(5)
+    for lens in ([39, 40, 64, 3] * 4, [65] * 15 + [76]):
+        Hk, Hv, DV, T, B = 32, 32, 128, sum(lens), len(lens)
+        cu_h = [sum(lens[:i]) for i in range(B + 1)]
+        q, k, v = (torch.randn(T, h, 128, device=DEV, generator=gen).bfloat16() for h in (Hk, Hk, Hv))
+        g, beta = -torch.rand(T, Hv, device=DEV, generator=gen), torch.rand(T, Hv, device=DEV, generator=gen)
+        S0 = torch.randn(B, Hv, 128, DV, device=DEV, generator=gen) * 0.1
+        slots_h, init_h = list(range(B)), [1] * B
+        cu, slots, init = (torch.tensor(x, dtype=torch.int32, device=DEV) for x in (cu_h, slots_h, init_h))
+        want, S_want = _exact(q, k, v, g, beta, S0, cu_h, slots_h, init_h, 128 ** -0.5, True)
+        S = S0.clone()
+        launches = _native.launch_counter[0]
+        out = la.gated_delta_rule(q, k, v, g, beta, S, cu, slots, init, 128 ** -0.5, True, cu_cpu=cu_h)
+        assert _native.launch_counter[0] - launches == 2
+        _native.check_status(torch.device(DEV))
+        assert _err(out, want) < 2.0 ** -8 and _err(S, S_want) < 4e-6

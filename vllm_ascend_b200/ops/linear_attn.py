@@ -4,8 +4,11 @@ delta-rule recurrence; CUDA kernels on GPU tensors, PyTorch definitions otherwis
 csrc/attention/recurrent_gated_delta_rule*)."""
 from __future__ import annotations
 
+import functools
+import os
 from ctypes import c_float, c_int, c_long, c_void_p
 
+import numpy as np
 import torch
 import torch.nn.functional as F
 
@@ -117,7 +120,6 @@ def gated_delta_rule_chunked(q, k, v, g, beta, state, cu_cpu, slots, has_init, s
     products per chunk position (all sequences that have such a chunk batched together), instead
     of one state update per token: the form the reference uses for prefill
     (vllm_ascend/ops/triton/fla/chunk.py:259, chunk_gated_delta_rule)."""
-    import numpy as np
     T, Hv, DV = v.shape
     Hk, DK = q.shape[1], q.shape[2]
     rep = Hv // Hk
@@ -202,24 +204,43 @@ def _chunk_min(on_cuda: bool = False) -> int:
     """Fewest new tokens of a sequence that take the chunk-parallel form built from fp32 matrix products; 0 = never.
     Unset, the form serves host tensors only: on a B200 it takes 10.3 ms for 4 x 2048 tokens of 32 heads, the kernels 1.3 ms token
     by token (three prompts of 2000 tokens: 1.6 ms, and 0.8 ms in chunks: ``_kernel_chunk_min``)."""
-    import os
     from .. import envs
     if "VLLM_B200_GDN_CHUNK_MIN" not in os.environ and on_cuda:
         return 0
     return int(envs.VLLM_B200_GDN_CHUNK_MIN)
 
 
-#: new tokens of a sequence from which the kernel that works in chunks of 64 tokens is the faster one: a chunk, full or not, takes
-#: 19 us, a token of the token-serial kernel 0.7 us
-_KERNEL_CHUNK_MIN = 32
+def _kernel_chunk_min(lens: np.ndarray, Hv: int, DV: int, sms: int) -> int:
+    """New tokens of a sequence from which a step's sequences run in the kernel that works in chunks of 64 tokens.
+
+    A chunk, full or not, takes a block 19 us and keeps an SM to itself; a token takes the token-serial kernel 0.5 to 0.8 us, three of its
+    blocks to an SM.  While a step has no more than two blocks per SM, 32 tokens and more gain (32 tokens 28 us token by token, 24 us in chunks).  Many
+    sequences are bound by what a block costs: 40 tokens are level (64 sequences of 32 heads: 32 tokens 303 us token by token and 353 in
+    chunks, 48 tokens 418 and 369), and 65 to 74 tokens pay for a second chunk that is nearly empty (65 tokens 555 and 608 us, 80 tokens
+    655 and 610), so that the step's sequences between 40 and 75 tokens decide together."""
+    if int((lens >= 32).sum()) * Hv * -(-DV // 128) <= 2 * sms:
+        return 32
+    mid = lens[(lens >= 40) & (lens < 75)]
+    # what a sequence and head cost an SM, us: (6.5 + 0.79 per token) / 1.5 there, 6.7 + 18.5 per chunk here
+    return 40 if float(((6.5 + 0.79 * mid) / 1.5 - 6.7 - 18.5 * -(-mid // 64)).sum()) >= 0 else 75
 
 
-def _kernel_chunk_min() -> int:
-    """0: token by token only (asked for with VLLM_B200_GDN_CHUNK_MIN=0, or in modes that fix the order of sums: a portion's
-    split into chunks must not show)."""
-    import os
+@functools.lru_cache(maxsize=256)
+def _portions(cu: bytes, Hv: int, DV: int, sms: int) -> tuple[int, int]:
+    """(new tokens from which sequences run in chunks, or 0; 1 where there are shorter ones) for int32 token offsets ``cu``.  A step's layers
+    ask the same, and the host has no time for it in each."""
+    lens = np.diff(np.frombuffer(cu, dtype=np.int32))
+    least = _kernel_chunk_min(lens, Hv, DV, sms)
+    if not (lens >= least).any():
+        return 0, 0
+    return least, int(((lens > 0) & (lens < least)).any())
+
+
+def _token_by_token() -> bool:
+    """No chunks on the GPU: asked for with VLLM_B200_GDN_CHUNK_MIN=0, or a mode that fixes the order of sums (a portion's split
+    into chunks must not show)."""
     from ..batch_invariant import fixed_sums
-    return 0 if fixed_sums() or os.environ.get("VLLM_B200_GDN_CHUNK_MIN") == "0" else _KERNEL_CHUNK_MIN
+    return fixed_sums() or os.environ.get("VLLM_B200_GDN_CHUNK_MIN") == "0"
 
 
 def gated_delta_rule(q, k, v, g, beta, state, cu, slots, has_init, scale, l2norm=True, cu_cpu=None, uniform=False,
@@ -231,7 +252,6 @@ def gated_delta_rule(q, k, v, g, beta, state, cu, slots, has_init, scale, l2norm
     per-token recurrence."""
     cmin = _chunk_min(q.is_cuda) if cu_cpu is not None else 0
     if cmin > 0:
-        import numpy as np
         cu_h = np.asarray(cu_cpu, dtype=np.int64)[:cu.numel()]
         lens = np.diff(cu_h)
         long_ = np.nonzero(lens >= cmin)[0]
@@ -264,14 +284,9 @@ def gated_delta_rule(q, k, v, g, beta, state, cu, slots, has_init, scale, l2norm
     fused = uniform and gate is not None and gate[0].dtype == q.dtype and gate[1].dtype == q.dtype \
         and gate[0].stride(1) == 1
     chunk_min = any_short = 0
-    if cu_cpu is not None and not uniform:
-        import numpy as np
-        lens = np.diff(np.asarray(cu_cpu)[:cu.numel()])
-        chunk_min = _kernel_chunk_min()
-        if chunk_min and (lens >= chunk_min).any():
-            any_short = int(((lens > 0) & (lens < chunk_min)).any())
-        else:
-            chunk_min = 0
+    if cu_cpu is not None and not uniform and not _token_by_token():
+        chunk_min, any_short = _portions(np.ascontiguousarray(cu_cpu, dtype=np.int32)[:cu.numel()].tobytes(), Hv, DV,
+                                         _native.sm_count(q.device))
     for z in ((gate[0], None) if fused else (None,)):
         rc = _native.lib().b200_gated_delta_rule(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), v.stride(0), g.data_ptr(), beta.data_ptr(),
@@ -355,7 +370,6 @@ def gated_linear_attention(q, k, v, g, state, cu, slots, has_init, cu_cpu, chunk
     constant g per head, lightning attention.  The reference's kernels for these layers are its
     Triton lightning-attention prefill / decode pair and vLLM's Mamba-2 kernels
     (vllm_ascend/ops/triton/mamba/lightning_attn.py, vllm_ascend/ops/triton/mamba/causal_conv1d.py)."""
-    import numpy as np
     if q.is_cuda:
         from .linear_recurrence import decayed_attention
         return decayed_attention(q, k, v, g, state, cu, slots, has_init, uniform=max(np.diff(cu_cpu), default=0) <= 1)
@@ -473,7 +487,6 @@ def kda_chunked(q, k, v, g, beta, state, cu_cpu, slots, has_init, scale, l2norm=
     contractions over (channel) of k_j k_m e^{gamma_j - gamma_m}, formed exactly (only non-positive
     exponents are ever exponentiated) for a short chunk
     (vllm_ascend/ops/triton/kda/kda.py, chunk_delta_h.py, solve_tril.py are the reference's kernels)."""
-    import numpy as np
     T, H, DV = v.shape
     DK = q.shape[2]
     dev = q.device
