@@ -109,10 +109,10 @@ def test_other_forms_stay_token_by_token(form):
 
 
 def test_many_short_portions_share_out_between_the_kernels():
-    """A step whose rule sends portions of 40 and more tokens to chunks and shorter ones to the other kernel, and one whose 65-token portions
+    """A step whose portions of 32 and more tokens run in chunks and shorter ones in the other kernel, and one whose 65-token portions
     go token by token: the states and read-outs of both kernels side by side, each its own sequences."""
     gen = torch.Generator(device=DEV).manual_seed(5)
-    for lens in ([39, 40, 64, 3] * 4, [65] * 15 + [76]):
+    for lens in ([39, 40, 64, 3] * 4, [65] * 12 + [200] * 3):
         Hk, Hv, DV, T, B = 32, 32, 128, sum(lens), len(lens)
         cu_h = [sum(lens[:i]) for i in range(B + 1)]
         q, k, v = (torch.randn(T, h, 128, device=DEV, generator=gen).bfloat16() for h in (Hk, Hk, Hv))

@@ -171,20 +171,17 @@ def test_kda_chunked_form_equals_the_per_channel_recurrence(chunk):
 
 
 def test_kernel_chunk_rule(monkeypatch):
-    """Which portions run in chunks of 64 on the GPU: by the step's number of blocks, and by what 40 to 74 tokens cost either way."""
-    from vllm_ascend_b200.ops.linear_attn import _kernel_chunk_min, _portions, _token_by_token
+    """Which portions run in chunks of 64 on the GPU: where the step is estimated to take the least time."""
+    from vllm_ascend_b200.ops.linear_attn import _portions, _token_by_token
 
-    def rule(*lens, Hv=32, DV=128):
-        return _kernel_chunk_min(np.array(lens), Hv, DV, 148)
-    assert rule(32) == rule(1, 1, 500) == rule(*[64] * 9) == 32             # at most two blocks per SM
-    assert rule(*[1] * 200, 2000) == 32                                     # one-token sequences are none of them
-    assert rule(*[33] * 10) == rule(*[48] * 64) == rule(*[2000] * 10) == 40
-    assert rule(*[65] * 64) == 75 and rule(*[48] * 20, *[65] * 10) == 40
-    assert rule(*[40] * 6, DV=256) == 40
-
-    def split(*cu):
-        return _portions(np.array(cu, dtype=np.int32).tobytes(), 32, 128, 148)
-    assert split(0, 31, 32) == (0, 0) and split(0, 32, 32) == (32, 0) and split(0, 32, 33, 33) == (32, 1) and split(0) == (0, 0)
+    def split(*lens, Hv=32, DV=128, sms=148):
+        return _portions(np.cumsum([0, *lens]).astype(np.int32).tobytes(), Hv, DV, sms)
+    assert split() == split(31) == split(0, 1, 31) == (0, 0)
+    assert split(32) == split(33) == split(*[2000] * 10) == (32, 0) and split(1, 1, 500) == split(*[1] * 200, 2000) == (32, 1)
+    assert split(*[33] * 10) == split(*[32] * 64) == split(*[65] * 64) == (0, 0)      # many blocks: a chunk has to be full enough
+    assert split(*[48] * 64) == split(*[80] * 64) == (32, 0)
+    assert split(*[33] * 64, *[64] * 10) == (40, 1) and split(*[65] * 64, *[500] * 2) == (75, 1)
+    assert split(64, DV=64) == split(64, DV=192) == (32, 0)
     monkeypatch.delenv("VLLM_B200_GDN_CHUNK_MIN", raising=False)
     assert not _token_by_token()
     monkeypatch.setenv("VLLM_B200_GDN_CHUNK_MIN", "0")

@@ -41,7 +41,7 @@ def is_training_consistent() -> bool:
 
 
 def is_batch_invariant() -> bool:
-    return _enabled or os.getenv("VLLM_B200_BATCH_INVARIANT", "0") == "1"
+    return _enabled or os.environ.get("VLLM_B200_BATCH_INVARIANT") == "1"
 
 
 def enable_batch_invariant_mode() -> None:

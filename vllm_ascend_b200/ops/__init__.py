@@ -12,12 +12,14 @@ The op set corresponds to the reference's OOT custom-op table
 from __future__ import annotations
 
 import functools
+import os
 from typing import Optional
 
 import numpy as np
 import torch
 
 from .. import _native, envs
+from ..batch_invariant import fixed_sums
 from . import reference as ref
 
 _BF16 = torch.bfloat16
@@ -355,9 +357,8 @@ def _few_rows_faster(M: int, N: int, K: int, glu: bool) -> bool:
 def _few_rows(M: int, N: int, K: int, glu: bool = False) -> bool:
     """Whether a step's product (N columns; ``glu``: of gate and up together twice as many) runs in the kernel that splits K over
     blocks.  Its rows may differ in the last bit from those of a larger batch, so modes that fix the order of sums never take it."""
-    if M > _FEW_ROWS or K % 8 or N % 8 or envs.VLLM_B200_GEMM == "cublas":
+    if M > _FEW_ROWS or K % 8 or N % 8 or os.environ.get("VLLM_B200_GEMM") == "cublas":
         return False
-    from ..batch_invariant import fixed_sums
     return not fixed_sums() and _few_rows_faster(M, N, K, glu)
 
 
@@ -367,11 +368,11 @@ def _pair_rows(M: int, N: int, K: int, glu: bool = False) -> bool:
     one; 144 rows of 10240 x 1024 20 -> 17 us).  Narrower ones leave half of the pairs without a tile (144 rows of 8192 x 4096 32 -> 34 us), and
     K below 1024 is all prologue (of 16384 x 512 15 -> 17 us).  Gate and up: K from 2048 on (2 x 4096 x 4096 57 -> 55 us, x 1024 38 -> 39).  The
     same bits.  A user's larger VLLM_B200_GEMM_2CTA_MIN_M holds."""
-    if not 128 < M <= 256 or not 0 < envs.VLLM_B200_GEMM_2CTA_MIN_M <= 256:
+    if not 128 < M <= 256 or K < (2048 if glu else 1024):
         return False
-    if glu:
-        return K >= 2048
-    return K >= 1024 and (N + 127) // 128 * 2 > _native.sm_count(torch.cuda.current_device())
+    if not glu and (N + 127) // 128 * 2 <= _native.sm_count(torch.cuda.current_device()):
+        return False
+    return 0 < envs.VLLM_B200_GEMM_2CTA_MIN_M <= 256
 
 
 def _gemm_small(x2, weight, out, bias, res2, N: int, glu: bool, alpha: float = 0.0, limit: float = 0.0) -> None:
@@ -501,7 +502,6 @@ def _prefill_pairs(q: torch.Tensor, Hkv: int, first_row: int, meta=None, first_s
     """Whether a step's prompts run in the kernel that gives a block two query tiles, for the sequences of ``meta`` from ``first_seq`` on: where its
     blocks can fill the GPU and take less time.  The kernels add a row's probabilities in different orders, so modes in which a prompt
     gets the same bits whatever shares its step never take it."""
-    from ..batch_invariant import fixed_sums
     if fixed_sums():
         return False
     tile, sms = 128 // (q.shape[1] // Hkv), _native.sm_count(q.device)

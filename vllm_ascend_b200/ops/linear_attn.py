@@ -203,35 +203,43 @@ def gated_delta_rule_chunked(q, k, v, g, beta, state, cu_cpu, slots, has_init, s
 def _chunk_min(on_cuda: bool = False) -> int:
     """Fewest new tokens of a sequence that take the chunk-parallel form built from fp32 matrix products; 0 = never.
     Unset, the form serves host tensors only: on a B200 it takes 10.3 ms for 4 x 2048 tokens of 32 heads, the kernels 1.3 ms token
-    by token (three prompts of 2000 tokens: 1.6 ms, and 0.8 ms in chunks: ``_kernel_chunk_min``)."""
+    by token (three prompts of 2000 tokens: 1.6 ms, and 0.8 ms in chunks: ``_portions``)."""
     from .. import envs
     if "VLLM_B200_GDN_CHUNK_MIN" not in os.environ and on_cuda:
         return 0
     return int(envs.VLLM_B200_GDN_CHUNK_MIN)
 
 
-def _kernel_chunk_min(lens: np.ndarray, Hv: int, DV: int, sms: int) -> int:
-    """New tokens of a sequence from which a step's sequences run in the kernel that works in chunks of 64 tokens.
+def _kernel_times(lens: np.ndarray, Hv: int, DV: int, sms: int, least: int) -> float:
+    """Estimated us of a step whose sequences of ``least`` tokens and more run in chunks of 64 and the others token by token.
 
-    A chunk, full or not, takes a block 19 us and keeps an SM to itself; a token takes the token-serial kernel 0.5 to 0.8 us, three of its
-    blocks to an SM.  While a step has no more than two blocks per SM, 32 tokens and more gain (32 tokens 28 us token by token, 24 us in chunks).  Many
-    sequences are bound by what a block costs: 40 tokens are level (64 sequences of 32 heads: 32 tokens 303 us token by token and 353 in
-    chunks, 48 tokens 418 and 369), and 65 to 74 tokens pay for a second chunk that is nearly empty (65 tokens 555 and 608 us, 80 tokens
-    655 and 610), so that the step's sequences between 40 and 75 tokens decide together."""
-    if int((lens >= 32).sum()) * Hv * -(-DV // 128) <= 2 * sms:
-        return 32
-    mid = lens[(lens >= 40) & (lens < 75)]
-    # what a sequence and head cost an SM, us: (6.5 + 0.79 per token) / 1.5 there, 6.7 + 18.5 per chunk here
-    return 40 if float(((6.5 + 0.79 * mid) / 1.5 - 6.7 - 18.5 * -(-mid // 64)).sum()) >= 0 else 75
+    A block of the chunked kernel keeps an SM to itself and takes 18.5 us per chunk, full or not (14.3 us where every block of 64 value columns has
+    its own SM); one of the token-serial kernel, of which three share an SM, takes 0.42 us per token alone and 0.79 us among others.  Blocks
+    run in waves, or packed one behind the other where they differ, whichever is shorter.  16 portions of 32 tokens, 32 heads: 88 us token by
+    token, 104 us in chunks (estimates 89 and 106); 64 of 65 tokens 555 and 608 (563 and 618); one of 128 tokens 68 and 41 (68 and 35)."""
+    def packed(each, blocks, slots):
+        n = len(each) * blocks
+        longest = float(each.max())
+        return min(-(-n // slots) * longest, float(each.sum()) * blocks / slots + longest / 2) if n > slots else longest
+    far, near = lens[lens >= least], lens[(lens > 0) & (lens < least)]
+    us, halves = 0.0, Hv * -(-DV // 64)
+    if len(far):
+        chunks = -(-far // 64)
+        us += 6 + (packed(14.3 * chunks, halves, sms) if DV % 128 or len(lens) * halves <= sms
+                   else packed(6.7 + 18.5 * chunks, Hv * (DV // 128), sms))
+    if len(near):
+        us += packed(14 + 0.42 * near, halves, sms) if len(near) * halves <= sms else packed(6.5 + 0.79 * near, halves, 3 * sms)
+    return us
 
 
 @functools.lru_cache(maxsize=256)
 def _portions(cu: bytes, Hv: int, DV: int, sms: int) -> tuple[int, int]:
-    """(new tokens from which sequences run in chunks, or 0; 1 where there are shorter ones) for int32 token offsets ``cu``.  A step's layers
-    ask the same, and the host has no time for it in each."""
+    """(new tokens from which sequences run in chunks of 64, or 0; 1 where there are shorter ones) for int32 token offsets ``cu``: the share-out
+    that is estimated to take the least time.  A step's layers ask the same, and the host has no time for it in each."""
     lens = np.diff(np.frombuffer(cu, dtype=np.int32))
-    least = _kernel_chunk_min(lens, Hv, DV, sms)
-    if not (lens >= least).any():
+    marks = [n for n in (32, 40, 75) if (lens >= n).any()]
+    least = min(marks + [1 << 30], key=lambda n: _kernel_times(lens, Hv, DV, sms, n)) if marks else 1 << 30
+    if least == 1 << 30:
         return 0, 0
     return least, int(((lens > 0) & (lens < least)).any())
 

@@ -19,6 +19,7 @@ from typing import Optional
 import torch
 
 from .. import _native, ops
+from ..batch_invariant import fixed_sums
 from ..ops import reference as ref
 from .registry import register_scheme
 
@@ -163,7 +164,6 @@ def fp8_block_linear(x: Optional[torch.Tensor], w8: torch.Tensor, w_scale: torch
     out = torch.empty((M, N), dtype=torch.bfloat16, device=xq.device)
     if M == 0:
         return out
-    from ..batch_invariant import fixed_sums
     if M <= _FP8_FEW_ROWS and not fixed_rows and not fixed_sums() and _fp8_few_rows_faster(M, N, K):
         # K split over blocks: rows may differ in the last bit from those of a larger batch
         rc = _native.lib().b200_gemm_small_fp8(
