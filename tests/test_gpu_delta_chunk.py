@@ -3,6 +3,7 @@
 State and sums are 32-bit in both kernels: what the state is off by is a few 2^-24 of its largest terms per chunk or token.  The
 test allows 4e-6 of the state's norm, and no more than one and a half times the token-serial kernel's error where that is
 larger; read-outs are rounded to bf16 (2^-9)."""
+import numpy as np
 import pytest
 import torch
 
@@ -127,3 +128,26 @@ def test_many_short_portions_share_out_between_the_kernels():
         assert _native.launch_counter[0] - launches == 2
         _native.check_status(torch.device(DEV))
         assert _err(out, want) < 2.0 ** -8 and _err(S, S_want) < 4e-6
+
+
+@pytest.mark.parametrize("at", [0, 5, 63, 70])
+def test_a_nan_reaches_no_earlier_token(at):
+    """Causality holds for values that no product with zero removes: rows before a NaN are what they are without it, bit for bit."""
+    gen = torch.Generator(device=DEV).manual_seed(at)
+    T, H = 100, 2
+    q, k, v = (torch.randn(T, H, 128, device=DEV, generator=gen).bfloat16() for _ in range(3))
+    g, beta = -torch.rand(T, H, device=DEV, generator=gen), torch.rand(T, H, device=DEV, generator=gen)
+    cu, slot = torch.tensor([0, T], dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+
+    def run(v):
+        S = torch.zeros(1, H, 128, 128, device=DEV)
+        return la.gated_delta_rule(q, k, v, g, beta, S, cu, slot, slot, 128 ** -0.5, cu_cpu=[0, T]).view(T, H, 128), S
+    assert la._portions(np.asarray([0, T], np.int32).tobytes(), H, 128, _native.sm_count(torch.device(DEV)))[0] > 0
+    clean, _ = run(v)
+    v = v.clone()
+    v[at, 0, 3] = float("nan")
+    out, S = run(v)
+    assert torch.equal(out[:at], clean[:at]) and torch.equal(out[:, 1], clean[:, 1])
+    assert out[at:, 0, 3].isnan().all() and S[0, 0, :, 3].isnan().all()
+    others = [c for c in range(128) if c != 3]
+    assert torch.equal(out[:, 0, others], clean[:, 0, others])

@@ -443,7 +443,26 @@ __global__ void __launch_bounds__(DC_THREADS, 1) delta_chunk_kernel(const DeltaC
 #pragma unroll
         for (int k = 0; k < CW; k++) acc[i][k] = pack2(x[k], y[k]);
       }
-      if (jb < n) dc_tile<4, CW, UP, 1>(acc, pt + jb, us + c, 0, jb + 8);
+      if (jb < n) {
+        dc_tile<4, CW, UP, 1>(acc, pt + jb, us + c, 0, jb);
+        // the tile's own triangle: rows take nothing of later tokens, not even zero times (a NaN there is not theirs)
+#pragma unroll
+        for (int m = 0; m < 8; m++) {
+          float um[CW];
+#pragma unroll
+          for (int k = 0; k < CW; k += 4) load_vec<float, 4>(us + (jb + m) * UP + c + k, um + k);
+          const float* coef = pt + (jb + m) * DC_PITCH + jb;
+#pragma unroll
+          for (int i = m / 2; i < 4; i++) {
+            const float2 a = *reinterpret_cast<const float2*>(coef + 2 * i);
+#pragma unroll
+            for (int k = 0; k < CW; k++) {
+              const float2 f = unpack2(acc[i][k]);
+              acc[i][k] = 2 * i >= m ? fma2(pack2(a.x, a.y), pack2(um[k], um[k]), acc[i][k]) : pack2(f.x, fmaf(a.y, um[k], f.y));
+            }
+          }
+        }
+      }
       __nv_bfloat16* op = (__nv_bfloat16*)p.out + (long)(tc + jb) * p.out_stride + (long)hv * p.DV + j0 + c;
 #pragma unroll
       for (int i = 0; i < 4; i++) {
