@@ -488,3 +488,23 @@ def test_grammar_bitmask_rows_unpack_to_token_masks():
     assert torch.nonzero(out["a"]).flatten().tolist() == [3, 31, 69]
     assert torch.nonzero(out["b"]).flatten().tolist() == list(range(32, 64))
     assert out["a"].shape == (70,)
+
+
+def test_activation_budget_holds_the_prompt_workspace_of_latent_attention(monkeypatch):
+    """Projected keys and values follow the context: the budget grows by them up to the step's limit, and by nothing where prompts
+    stay in the latent space."""
+    import dataclasses
+
+    from vllm_ascend_b200.attention import mla
+    cfg = dataclasses.replace(get_model_config("tiny-deepseek"), qk_nope_head_dim=128, v_head_dim=64)
+    runner = LLM(cfg, device="cpu", max_model_len=256, max_num_seqs=2, max_num_batched_tokens=32, block_size=16).engine.runner
+    H, dc, dr = cfg.num_attention_heads, cfg.kv_lora_rank, cfg.qk_rope_head_dim
+    need = 512 * 2 * (H * (128 + 64) + dc + dr)
+    whole = runner.activation_bytes_estimate()
+    monkeypatch.setattr(mla, "_EXPAND_BYTES", need // 2)
+    assert whole - runner.activation_bytes_estimate() == need - need // 2
+    monkeypatch.setenv("VLLM_B200_MLA_ATTN", "torch")
+    assert whole - runner.activation_bytes_estimate() == need
+    plain = LLM(get_model_config("tiny-moe"), device="cpu", max_model_len=256, max_num_seqs=2, max_num_batched_tokens=32,
+                block_size=16).engine.runner
+    assert plain._prompt_workspace_bytes() == 0

@@ -165,6 +165,30 @@ def test_rule_keeps_decodes_and_long_contexts_in_the_latent_space():
     assert plan([1000], [0], heads=1 << 12) is None              # 2 GB of projected rows
 
 
+@pytest.mark.parametrize("H", [1, 16])
+def test_workspace_stays_within_its_limit(monkeypatch, H):
+    """What a step allocates beside its output is what the plan was allowed: projected rows, dense latents and rotary keys together."""
+    dn, dr, dv, dc, n = 128, 64, 128, 512, 20000
+    monkeypatch.setattr(mla, "_EXPAND_BYTES", n * 2 * (H * (dn + dv) + dc + dr))
+    for keys in (n, n + 1):
+        table, cu, lens, blocks = _batch([keys], [0], 128, torch.Generator().manual_seed(0))
+        meta = metadata_from_tensors(cu, lens, table, keys, keys, H, H, 128, decode_kernel=False)
+        q = torch.zeros((keys, H, dn + dr), device=DEV, dtype=torch.bfloat16)
+        lat, pe = (torch.zeros((blocks, 128, 1, d), device=DEV, dtype=q.dtype) for d in (dc, dr))
+        plan = mla.expanded_prompts(meta, H, dn, dr, dv, q, lat, pe)
+        assert plan == ((0, n) if keys == n else None)
+        if plan is None:
+            continue
+        kv_b = torch.zeros((H * (dn + dv), dc), device=DEV, dtype=q.dtype)
+        out = torch.empty((keys, H, dv), device=DEV, dtype=q.dtype)
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        mla.prompt_attention_expanded(q, kv_b, lat, pe, meta, 0.1, dv, *plan, out)
+        _native.check_status(torch.device(DEV))
+        assert torch.cuda.max_memory_allocated() - before <= mla._EXPAND_BYTES + (4 << 20)     # allocations are rounded up
+
+
 def test_many_sequences_start_where_the_ones_before_end():
     n = 2500
     lens = torch.randint(1, 4, (n,), generator=torch.Generator().manual_seed(1), dtype=torch.int32)

@@ -233,8 +233,26 @@ def mla_paged_attention(q_lat: torch.Tensor, q_pe: torch.Tensor, lat_cache: torc
 
 #: query-key pairs per key from which prompts attend over up-projected keys and values: per head a pair costs 2 x 1088
 #: operations in the latent space (at the 110 TFLOP/s its kernel reaches on prompts) and 2 x 320 over them, a key 2 x 512 x 256 to
-#: project up; level at about 12 pairs per key.  And the most memory the projected rows may take.
+#: project up; level at about 12 pairs per key.  And the most memory that the projected rows and what they are made of may take.
 _EXPAND_PAIRS_PER_KEY, _EXPAND_BYTES = 16, 1 << 30
+
+
+def _expand_sizes_ok(dn: int, dr: int, dv: int, dc: int) -> bool:
+    return dn == 128 and dv % 8 == 0 and 8 <= dv <= 128 and dr % 8 == 0 and 8 <= dr <= 64 and dc % 8 == 0
+
+
+def _expand_row_bytes(heads: int, dn: int, dr: int, dv: int, dc: int) -> int:
+    """Per key: its projected rows of every head, its dense latent and its rotary part."""
+    return 2 * (heads * (dn + dv) + dc + dr)
+
+
+def expanded_workspace(heads: int, dn: int, dr: int, dv: int, dc: int, keys: int) -> int:
+    """Most bytes that a step with up to ``keys`` keys takes for prompts over up-projected keys and values, beside its output: they
+    follow the context, not the step's tokens, so a budget of so much per token does not hold them."""
+    from .. import envs
+    if not _expand_sizes_ok(dn, dr, dv, dc) or envs.VLLM_B200_MLA_ATTN != "tcgen05":
+        return 0
+    return min(_EXPAND_BYTES, keys * _expand_row_bytes(heads, dn, dr, dv, dc))
 
 
 def expanded_prompts(meta, heads: int, dn: int, dr: int, dv: int, q: torch.Tensor, lat_cache: torch.Tensor,
@@ -248,8 +266,8 @@ def expanded_prompts(meta, heads: int, dn: int, dr: int, dv: int, q: torch.Tenso
     if not (q.is_cuda and q.dtype == lat_cache.dtype == torch.bfloat16 and meta.max_query_len > 1
             and envs.VLLM_B200_MLA_ATTN == "tcgen05") or fixed_sums() or torch.cuda.is_current_stream_capturing():
         return None
-    if dn != 128 or dv % 8 or not 8 <= dv <= 128 or dr % 8 or not 8 <= dr <= 64 or lat_cache.shape[-1] % 8 \
-            or not (q.is_contiguous() and lat_cache.is_contiguous() and pe_cache.is_contiguous()):
+    dc = lat_cache.shape[-1]
+    if not _expand_sizes_ok(dn, dr, dv, dc) or not (q.is_contiguous() and lat_cache.is_contiguous() and pe_cache.is_contiguous()):
         return None
     B = meta.num_reqs
     new = np.diff(np.asarray(meta.query_start_loc_cpu[:B + 1], dtype=np.int64))
@@ -258,7 +276,7 @@ def expanded_prompts(meta, heads: int, dn: int, dr: int, dv: int, q: torch.Tenso
     new, seen = new[first:], seen[first:]
     keys = int(seen.sum())
     pairs = int((new * (seen - new) + new * (new + 1) // 2).sum())
-    if (new < 1).any() or pairs < _EXPAND_PAIRS_PER_KEY * keys or keys * heads * (dn + dv) * 2 > _EXPAND_BYTES:
+    if (new < 1).any() or pairs < _EXPAND_PAIRS_PER_KEY * keys or keys * _expand_row_bytes(heads, dn, dr, dv, dc) > _EXPAND_BYTES:
         return None
     return first, keys
 

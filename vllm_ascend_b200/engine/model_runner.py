@@ -259,7 +259,16 @@ class ModelRunner:
         per_tok = (6 * c.hidden_size + 3 * (c.num_attention_heads * c.q_head_dim) // tp
                    + 3 * inter // tp) * 2
         logits = self.max_seqs * c.vocab_size * 6
-        return int(1.3 * (T * per_tok + logits)) + (1 << 30)
+        return int(1.3 * (T * per_tok + logits)) + (1 << 30) + self._prompt_workspace_bytes()
+
+    def _prompt_workspace_bytes(self) -> int:
+        """Latent attention's workspace for prompts: by the keys that a step can look at."""
+        if self.dcp_size > 1:
+            return 0
+        from ..attention.mla import expanded_workspace
+        keys = self.max_seqs * self.max_blocks_per_seq * self.block_size
+        return max((expanded_workspace(a.H, a.dn, a.dr, a.dv, a.dc, keys) for a in (L.self_attn for L in self.model.layers)
+                    if hasattr(a, "kv_b_proj") and not (a.window or a.sink is not None or a.index_topk)), default=0)
 
     def determine_num_blocks(self) -> int:
         cc = self.cfg.cache
