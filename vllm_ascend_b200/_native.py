@@ -129,11 +129,15 @@ def sm_count(device) -> int:
     return torch.cuda.get_device_properties(device).multi_processor_count
 
 
+#: a private entry of torch: builds without it (or without CUDA) go through the Stream object
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def stream_ptr(device=None) -> int:
     """Handle of the current stream, without the Stream object that ``torch.cuda.current_stream`` makes (3 us of the 15 to 20 us
     that the host spends on an op, which is what bounds launch-by-launch steps of a few hundred tokens)."""
-    if device is None:
-        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    if device is None and _raw_stream is not None:
+        return _raw_stream(torch._C._cuda_getDevice())
     return torch.cuda.current_stream(device).cuda_stream
 
 

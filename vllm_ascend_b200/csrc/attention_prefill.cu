@@ -37,7 +37,7 @@ struct PrefillParams {
   const int* seq_lens;         // [num_seqs] keys of each sequence, its new tokens included
   const int* block_table;      // paged
   int num_seqs, max_blocks, block_size, rows_per_load;
-  int G, Hq, tok_per_tile, dn, dv;
+  int G, tok_per_tile, dv;
   float scale_log2, rescale_threshold;
   int causal, window;
   __nv_bfloat16* out;
@@ -506,7 +506,7 @@ B200_API int b200_attn_prefill(const void* q, long q_stride, long q_rows, const 
   p.seq_lens = (const int*)seq_lens;
   p.block_table = (const int*)block_table;
   p.num_seqs = num_seqs; p.max_blocks = max_blocks; p.block_size = block_size; p.rows_per_load = rpl;
-  p.G = G; p.Hq = Hq; p.tok_per_tile = tpt; p.dn = D; p.dv = D;
+  p.G = G; p.tok_per_tile = tpt; p.dv = D;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.rescale_threshold = 8.f;
   p.causal = causal; p.window = window;
@@ -519,7 +519,7 @@ B200_API int b200_attn_prefill(const void* q, long q_stride, long q_rows, const 
 
 // Causal attention over up-projected latents: q [*, H, dn + dr] (token stride q_stride), kv [keys, H, dn + dv] dense, pe [keys, dr]
 // dense, out [*, H, dv] dense.  cu [num_seqs + 1] rows of q / out, kv_start [num_seqs + 1] rows of kv / pe, seq_lens the keys of
-// each sequence.  dn, dv multiples of 64 up to 128, dr a multiple of 8 up to 64.
+// each sequence.  dn = 128, dv a multiple of 8 up to 128, dr a multiple of 8 up to 64.
 B200_API int b200_attn_prefill_latent(const void* q, long q_stride, long q_rows, const void* kv, const void* pe, long keys,
                                       const void* cu, const void* kv_start, const void* seq_lens, int num_seqs, long tokens,
                                       int H, int dn, int dr, int dv, float scale, void* out, int* status, cudaStream_t stream) {
@@ -552,7 +552,7 @@ B200_API int b200_attn_prefill_latent(const void* q, long q_stride, long q_rows,
   p.kv_start = (const int*)kv_start;
   p.seq_lens = (const int*)seq_lens;
   p.num_seqs = num_seqs;
-  p.G = 1; p.Hq = H; p.tok_per_tile = 128; p.dn = dn; p.dv = dv;
+  p.G = 1; p.tok_per_tile = 128; p.dv = dv;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.rescale_threshold = 8.f;
   p.causal = 1;

@@ -59,7 +59,8 @@ struct Gemm2Params {
   int rows_per_owner;
   int raster;                         // M-tiles per raster group (0/1: column-major order)
   int bn;                             // tile width: 128..256 in steps of 16 (32 with the reduce-scatter
-                                      // epilogue, whose staging flushes 64-column pairs; SwiGLU tiles: 256)
+                                      // epilogue, whose staging flushes 64-column pairs; SwiGLU tiles: 256); from 64
+                                      // on with a single row of tiles, no row statistics and no peer memory
   // ---- RMSNorm folded into the GEMMs around it (the norm weight lives in W of the consumer)
   // Row statistics travel as per-column-tile partial sums so that their total does not depend on
   // the order in which tiles finish: buffer [ss_parts_max][ss_stride] fp32 followed by one int32

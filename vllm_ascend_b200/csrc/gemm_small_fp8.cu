@@ -36,7 +36,7 @@ template <int NT>
 struct SfCfg {
   static constexpr int CPW = NT / 2;
   static constexpr int BLOCKS = NT <= 64 ? 2 : 1;            // per SM
-  static constexpr int NB = NT <= 64 ? 4 : 4;                // accumulators in tensor memory
+  static constexpr int NB = 4;                               // accumulators in tensor memory
   static constexpr int TMEM_COLS = NB * NT < 32 ? 32 : NB * NT;      // 128, 256, 512
 };
 

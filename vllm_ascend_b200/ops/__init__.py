@@ -261,7 +261,8 @@ def linear_norm_folded(x: torch.Tensor, weight: torch.Tensor, bias: Optional[tor
         out = torch.empty((M, N), dtype=x.dtype, device=x.device)
     if ss_out is not None and ss_in is None and not swiglu and K % 8 == 0 and _few_rows(M, N, K) \
             and x.stride(0) % 8 == weight.stride(0) % 8 == out.stride(0) % 8 == 0:
-        # output and down projections of steps around 256 rows (34 and 75 us in the paired-CTA kernel, 26 and 46 us here)
+        # output and down projections of steps of 256 rows (34 and 75 us in the paired-CTA kernel, 26 and 46 us here): norms are folded
+        # from VLLM_B200_GEMM_2CTA_MIN_M rows on, 256 unless it says fewer, and the few-row kernel takes no more than 256
         rc = _native.lib().b200_gemm_small_stats(
             x.data_ptr(), weight.data_ptr(), out.data_ptr(), _native.ptr(bias), _native.ptr(residual), M, N, K, x.stride(0),
             weight.stride(0), out.stride(0), ss_out.data_ptr(), rows, parts, _native.status_word(x.device).data_ptr(),
