@@ -34,13 +34,20 @@ __device__ __forceinline__ float4 sg_sum(const uint32_t part, int splits, uint32
   return s;
 }
 
-// How many clusters of `blocks` blocks the GPU runs at once with `per_sm` blocks on an SM.  A cluster lies within one group of SMs, and
-// groups leave SMs over that no cluster fits into: one block per SM, 45 clusters of three, where 148 SMs give 49.  A grid that counted
-// SMs ran in two waves (64 rows of 6144 x 4096 in six parts 27 us, in five 21 us).  The driver is asked once per size, about one
-// block per SM (its answer does not double where two fit); the same groups hold twice as many with two.
+// How many clusters of `blocks` blocks the GPU runs at once with `per_sm` (1 or 2) blocks on an SM.  A cluster lies within one group of SMs,
+// and groups leave SMs over that no cluster fits into: one block per SM, 45 clusters of three, where 148 SMs give 49.  A grid that
+// counted SMs ran in two waves (64 rows of 6144 x 4096 in six parts 27 us, in five 21 us).  The driver is asked once per size, about
+// one block per SM, as its answer does not double where two fit.  With two, a group of n SMs holds as many clusters of six or eight as
+// with one of three or four (33 of eight, where twice the answer for eight says 30 and 32 tiles of 4096 x 12288 took 26.2 us in six
+// parts, 25.0 us in eight; 45 of six).  Four do not come to that (74 tiles of 9472 x 2048, 128 rows: 24.2 us, the general kernel 18.2), and
+// odd sizes have no half: twice the answer is what surely fits.
 using sg_fit_t = std::atomic<int>;
 template <auto Kernel>
 inline int sg_clusters_at_once(sg_fit_t* known, int blocks, int threads, int per_sm) {
+  if (per_sm == 2 && (blocks == 6 || blocks == 8)) {
+    blocks /= 2;
+    per_sm = 1;
+  }
   int n = known[blocks].load(std::memory_order_relaxed);
   if (n > 0) return n * per_sm;
   cudaLaunchConfig_t cfg = {};
