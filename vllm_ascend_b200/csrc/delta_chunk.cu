@@ -10,7 +10,7 @@
 //
 // Bound: the token-serial kernel (linear_attention.cu) spends 0.7 us per token of a sequence whatever the batch.  Here a chunk of 64
 // takes 36,900 clocks (19 us) one after the other: 11,800 are the solve and 8,800 the new state and its parts (CUDA cores, bound by
-// what shared memory returns), the rest staging, products and factors.  6000 tokens in three prompts, 32 heads: 1603 -> 772 us.
+// what shared memory returns), the rest staging, products and factors.  6000 tokens in three prompts, 32 heads: 1603 -> about 780 us.
 //
 // 32 bits stay 32 bits.  q and k are bf16 as they come, so k . k and q . k are exact products summed in fp32; their norms
 // are factors of rows.  The state and u are fp32: as MMA operands they are three bf16 parts (8 + 8 + 8 bits), which times
