@@ -161,7 +161,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
   using Cfg = DecCfg<D>;
   constexpr int NH = Cfg::NH, ST = Cfg::STAGES;
   const int G = p.G;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   long long* tl = (p.timeline && blockIdx.x == 0 && lane == 0) ? p.timeline : nullptr;
   const long long tl_t0 = clock64();
 
@@ -235,7 +235,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_ptr;
+  const uint32_t tmem_base = warp_uniform(*tmem_ptr);
   const int num_items = p.num_items;
 
   if (warp == 0) {
@@ -274,7 +274,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
     auto load_q = [&](uint32_t idx, const DecItem& d) -> bool {
       const int b = idx & 1;
       if (!mbar_wait(&q_empty[b], ((idx >> 1) & 1u) ^ 1u, abort_word)) return false;
-      if (lane == 0) {
+      if (elect_one()) {
         mbar_expect_tx(&q_full[b], VAR ? NH * 128 * G : Cfg::Q_BYTES);
 #pragma unroll
         for (int hf = 0; hf < NH; hf++)
@@ -344,7 +344,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
           }
           if (nsub < 4) {
             const int blk = __shfl_sync(0xffffffffu, blk_cur, 0);
-            if (lane == 0) {
+            if (elect_one()) {
               uint8_t* dst = (kv == 0 ? Ks : Vs) + st * Cfg::TILE_BYTES;
               const CUtensorMap* tm = kv == 0 ? &tmap_k32 : &tmap_v32;
               mbar_expect_tx(fullb, nsub * NH * 32 * 128);
@@ -361,7 +361,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
           }
           for (int part = 0; part < parts; part++) {
             const int blk = __shfl_sync(0xffffffffu, blk_cur, part);
-            if (lane == 0) {
+            if (elect_one()) {
               uint8_t* dst = (kv == 0 ? Ks : Vs) + st * Cfg::TILE_BYTES;
               const CUtensorMap* tm = kv == 0 ? &tmap_k : &tmap_v;
               if (part == 0) mbar_expect_tx(fullb, Cfg::TILE_BYTES);
@@ -385,82 +385,70 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
       it++;
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    constexpr uint32_t idesc_s = make_idesc_f16(128, DEC_NQ, true, false, false);
-    constexpr uint32_t idesc_o = make_idesc_f16(D, DEC_NQ, true, true, false);   // A = V, MN-major
-    const uint32_t q_addr0 = smem_u32(Qs), k_addr = smem_u32(Ks), v_addr = smem_u32(Vs),
-                   p_addr = smem_u32(Ps);
-    uint32_t gt = 0, it = 0;
-    DecRaw raw_next = {0, 0, 0};
-    if ((int)blockIdx.x < num_items) raw_next = dec_load(p, blockIdx.x);
-    for (int item = blockIdx.x; item < num_items; item += gridDim.x) {
-      const DecItem w = dec_make(p, item, raw_next);
-      if (item + (int)gridDim.x < num_items) raw_next = dec_load(p, item + gridDim.x);
-      if (w.n <= 0) continue;
-      const int qb = it & 1;
-      const uint32_t q_addr = q_addr0 + qb * Cfg::Q_BYTES;
-      const uint32_t o_col = Cfg::O_COL + qb * DEC_NQ;
-      if (!mbar_wait(&q_full[qb], (it >> 1) & 1u, abort_word)) goto done;
-      // the accumulator of two items ago has been read out by its epilogue
-      if (!mbar_wait(&o_free[qb], ((it >> 1) & 1u) ^ 1u, abort_word)) goto done;
-      auto issue_s = [&](int j) -> bool {
-        const uint32_t g = gt + (uint32_t)j;
-        const int st = g % ST;
-        const uint32_t ph = (g / ST) & 1u;
-        const int b = g & 1;
-        if (!mbar_wait(&k_full[st], ph, abort_word)) return false;
-        DEC_STAMP(1, g, 0);
-        if (!mbar_wait(&s_free[b], ((g >> 1) & 1u) ^ 1u, abort_word)) return false;
-        tc_fence_after();
-        if (lane == 0) {
+    // ------------------------------------------------------------ MMA issuer: one thread walks the loop (see warp_uniform)
+    if (elect_one()) {
+      constexpr uint32_t idesc_s = make_idesc_f16(128, DEC_NQ, true, false, false);
+      constexpr uint32_t idesc_o = make_idesc_f16(D, DEC_NQ, true, true, false);   // A = V, MN-major
+      const uint64_t dq0 = make_smem_desc(smem_u32(Qs), 16, 1024, kLayoutSw128), dk0 = make_smem_desc(smem_u32(Ks), 16, 1024, kLayoutSw128);
+      // A of the second product: 16 keys of V^T (two 64-wide d atoms DEC_HALF apart, 8-key groups 1024 B apart)
+      const uint64_t dv0 = make_smem_desc(smem_u32(Vs), DEC_HALF, 1024, kLayoutSw128), dp0 = make_smem_desc(smem_u32(Ps), 16, 1024, kLayoutSw128);
+      uint32_t gt = 0, it = 0;
+      DecRaw raw_next = {0, 0, 0};
+      if ((int)blockIdx.x < num_items) raw_next = dec_load(p, blockIdx.x);
+      for (int item = blockIdx.x; item < num_items; item += gridDim.x) {
+        const DecItem w = dec_make(p, item, raw_next);
+        if (item + (int)gridDim.x < num_items) raw_next = dec_load(p, item + gridDim.x);
+        if (w.n <= 0) continue;
+        const int qb = it & 1;
+        const uint64_t dq = dq0 + (uint32_t)(qb * (Cfg::Q_BYTES >> 4));
+        const uint32_t o_col = Cfg::O_COL + qb * DEC_NQ;
+        if (!mbar_wait(&q_full[qb], (it >> 1) & 1u, abort_word)) goto done;
+        // the accumulator of two items ago has been read out by its epilogue
+        if (!mbar_wait(&o_free[qb], ((it >> 1) & 1u) ^ 1u, abort_word)) goto done;
+        auto issue_s = [&](int j) -> bool {
+          const uint32_t g = gt + (uint32_t)j;
+          const int st = g % ST;
+          const uint32_t ph = (g / ST) & 1u;
+          const int b = g & 1;
+          if (!mbar_wait(&k_full[st], ph, abort_word)) return false;
+          DEC_STAMP(1, g, 0);
+          if (!mbar_wait(&s_free[b], ((g >> 1) & 1u) ^ 1u, abort_word)) return false;
+          tc_fence_after();
+          const uint64_t dk = dk0 + (uint32_t)(st * (Cfg::TILE_BYTES >> 4));
 #pragma unroll
-          for (int kk = 0; kk < D / 16; kk++) {
-            const uint64_t da = make_smem_desc(
-                k_addr + st * Cfg::TILE_BYTES + (kk >> 2) * DEC_HALF + (kk & 3) * 32, 16, 1024,
-                kLayoutSw128);
-            const uint64_t db = make_smem_desc(q_addr + (kk >> 2) * DEC_QHALF + (kk & 3) * 32, 16,
-                                               1024, kLayoutSw128);
-            umma_f16_ss(tmem_base + b * DEC_NQ, da, db, idesc_s, kk > 0 ? 1u : 0u);
-          }
+          for (int kk = 0; kk < D / 16; kk++)
+            umma_f16_ss(tmem_base + b * DEC_NQ, dk + (((kk >> 2) * DEC_HALF + (kk & 3) * 32) >> 4),
+                        dq + (((kk >> 2) * DEC_QHALF + (kk & 3) * 32) >> 4), idesc_s, kk > 0 ? 1u : 0u);
           umma_commit(&k_empty[st]);
           umma_commit(&s_ready[b]);
           if (j == w.n - 1) umma_commit(&q_empty[qb]);     // last read of this item's Q
-        }
-        __syncwarp();
-        return true;
-      };
-      if (!issue_s(0)) goto done;
-      for (int j = 0; j < w.n; j++) {
-        if (j + 1 < w.n) {
-          if (!issue_s(j + 1)) goto done;
-        }
-        const uint32_t g = gt + (uint32_t)j;
-        const int st = g % ST;
-        const uint32_t ph = (g / ST) & 1u;
-        const int pb = g & 1;
-        if (!mbar_wait(&v_full[st], ph, abort_word)) goto done;
-        DEC_STAMP(1, g, 1);
-        if (!mbar_wait(&p_ready[pb], (g >> 1) & 1u, abort_word)) goto done;
-        DEC_STAMP(1, g, 2);
-        tc_fence_after();
-        if (lane == 0) {
-#pragma unroll
-          for (int kk = 0; kk < 8; kk++) {
-            // A: 16 keys of V^T (two 64-wide d atoms DEC_HALF apart, 8-key groups 1024 B apart)
-            const uint64_t da = make_smem_desc(v_addr + st * Cfg::TILE_BYTES + kk * 2048, DEC_HALF,
-                                               1024, kLayoutSw128);
-            const uint64_t db = make_smem_desc(
-                p_addr + pb * Cfg::P_BYTES + (kk >> 2) * DEC_QHALF + (kk & 3) * 32, 16, 1024,
-                kLayoutSw128);
-            umma_f16_ss(tmem_base + o_col, da, db, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
+          return true;
+        };
+        if (!issue_s(0)) goto done;
+        for (int j = 0; j < w.n; j++) {
+          if (j + 1 < w.n) {
+            if (!issue_s(j + 1)) goto done;
           }
+          const uint32_t g = gt + (uint32_t)j;
+          const int st = g % ST;
+          const uint32_t ph = (g / ST) & 1u;
+          const int pb = g & 1;
+          if (!mbar_wait(&v_full[st], ph, abort_word)) goto done;
+          DEC_STAMP(1, g, 1);
+          if (!mbar_wait(&p_ready[pb], (g >> 1) & 1u, abort_word)) goto done;
+          DEC_STAMP(1, g, 2);
+          tc_fence_after();
+          const uint64_t dv = dv0 + (uint32_t)(st * (Cfg::TILE_BYTES >> 4)), dp = dp0 + (uint32_t)(pb * (Cfg::P_BYTES >> 4));
+#pragma unroll
+          for (int kk = 0; kk < 8; kk++)
+            umma_f16_ss(tmem_base + o_col, dv + kk * 128, dp + (((kk >> 2) * DEC_QHALF + (kk & 3) * 32) >> 4), idesc_o,
+                        (j > 0 || kk > 0) ? 1u : 0u);
           umma_commit(&v_empty[st]);
           umma_commit(&pv_done[pb]);
         }
-        __syncwarp();
+        gt += (uint32_t)w.n;
+        it++;
       }
-      gt += (uint32_t)w.n;
-      it++;
     }
   } else {
     // ------------------------------------------------------------ softmax / epilogue
@@ -668,6 +656,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
     }
   }
 done:
+  __syncwarp();             // the elected threads come back to their warps
   tc_fence_before();
   __syncthreads();
   if (*abort_word != 0) {

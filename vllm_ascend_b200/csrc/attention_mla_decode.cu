@@ -135,7 +135,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   const int t0 = t_lo + split * per_split;
   const int t1 = min(t_lo + n_all, t0 + per_split);
   const int n = t1 - t0;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int dc = p.dc;
 
   if (n <= 0) {
@@ -207,7 +207,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_ptr;
+  const uint32_t tmem_base = warp_uniform(*tmem_ptr);
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
@@ -236,7 +236,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         if (!mbar_wait(&h_empty[s], ph ^ 1u, abort_word)) goto done;
         for (int part = 0; part < parts; part++) {
           const int b = __shfl_sync(0xffffffffu, blk, part);
-          if (lane == 0) {
+          if (elect_one()) {
             if (part == 0) mbar_expect_tx(&h_full[s], MLA_SLAB);
             const int off = (key_base + part * rpl) % p.block_size;
             uint8_t* dst = KVs + s * MLA_SLAB + part * rpl * 128;
@@ -248,57 +248,43 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    constexpr uint32_t idesc_s = make_idesc_f16(128, NQ, true, false, false);
-    constexpr uint32_t idesc_o = make_idesc_f16(128, NQ, true, true, false);   // A = latent^T, MN-major
-    const uint32_t q_addr = smem_u32(Qs), kv_addr = smem_u32(KVs), p_addr = smem_u32(Ps);
-    if (!mbar_wait(q_full, 0, abort_word)) goto done;
-    for (int j = 0; j < n; j++) {
-      const uint32_t ph = (uint32_t)j & 1u;
-      const int b = j & 1;
-      if (!mbar_wait(&s_free[b], (((uint32_t)j >> 1) & 1u) ^ 1u, abort_word)) goto done;
-#pragma unroll 1
-      for (int s = 0; s < slabs; s++) {
-        if (!mbar_wait(&h_full[s], ph, abort_word)) goto done;
-        tc_fence_after();
-        if (lane == 0) {
+    // ------------------------------------------------------------ MMA issuer: one thread walks the loop (see warp_uniform)
+    if (elect_one()) {
+      constexpr uint32_t idesc_s = make_idesc_f16(128, NQ, true, false, false);
+      constexpr uint32_t idesc_o = make_idesc_f16(128, NQ, true, true, false);   // A = latent^T, MN-major
+      const uint64_t dq0 = make_smem_desc(smem_u32(Qs), 16, 1024, kLayoutSw128), dk0 = make_smem_desc(smem_u32(KVs), 16, 1024, kLayoutSw128);
+      const uint64_t dv0 = make_smem_desc(smem_u32(KVs), MLA_SLAB, 1024, kLayoutSw128), dp0 = make_smem_desc(smem_u32(Ps), 16, 1024, kLayoutSw128);
+      if (!mbar_wait(q_full, 0, abort_word)) goto done;
+      for (int j = 0; j < n; j++) {
+        const uint32_t ph = (uint32_t)j & 1u;
+        const int b = j & 1;
+        if (!mbar_wait(&s_free[b], (((uint32_t)j >> 1) & 1u) ^ 1u, abort_word)) goto done;
+        for (int s = 0; s < slabs; s++) {
+          if (!mbar_wait(&h_full[s], ph, abort_word)) goto done;
+          tc_fence_after();
+          const uint64_t dk = dk0 + (uint32_t)(s * (MLA_SLAB >> 4)), dq = dq0 + (uint32_t)(s * (Cfg::Q_SLAB >> 4));
 #pragma unroll
-          for (int kk = 0; kk < 4; kk++) {
-            const uint64_t da = make_smem_desc(kv_addr + s * MLA_SLAB + kk * 32, 16, 1024, kLayoutSw128);
-            const uint64_t db = make_smem_desc(q_addr + s * Cfg::Q_SLAB + kk * 32, 16, 1024, kLayoutSw128);
-            umma_f16_ss(tmem_base + b * NQ, da, db, idesc_s, (s > 0 || kk > 0) ? 1u : 0u);
-          }
-          if (s == lat_slabs) {
-            umma_commit(&h_empty[s]);        // the rope slab is not a value operand
-            umma_commit(&s_ready[b]);
-          }
+          for (int kk = 0; kk < 4; kk++) umma_f16_ss(tmem_base + b * NQ, dk + 2 * kk, dq + 2 * kk, idesc_s, (s > 0 || kk > 0) ? 1u : 0u);
         }
-        __syncwarp();
-      }
-      if (!mbar_wait(&p_ready[b], ((uint32_t)j >> 1) & 1u, abort_word)) goto done;
-      tc_fence_after();
-      if (lane == 0) {
-#pragma unroll 1
+        umma_commit(&h_empty[lat_slabs]);        // the rope slab is not a value operand
+        umma_commit(&s_ready[b]);
+        if (!mbar_wait(&p_ready[b], ((uint32_t)j >> 1) & 1u, abort_word)) goto done;
+        tc_fence_after();
+        const uint64_t dp = dp0 + (uint32_t)(b * (Cfg::P_BYTES >> 4));
         for (int blk = 0; blk < val_blocks; blk++) {
+          // A: 16 keys of latent^T for d in [128 blk, 128 blk + 128): two 64-wide d atoms one
+          // slab apart, 8-key groups 1024 B apart.  With an odd number of latent slabs the last
+          // block's upper half reads the rope slab: those rows of O^T are never read.
+          const uint64_t dv = dv0 + (uint32_t)(2 * blk * (MLA_SLAB >> 4));
 #pragma unroll
-          for (int kk = 0; kk < 8; kk++) {
-            // A: 16 keys of latent^T for d in [128 blk, 128 blk + 128): two 64-wide d atoms one
-            // slab apart, 8-key groups 1024 B apart.  With an odd number of latent slabs the last
-            // block's upper half reads the rope slab: those rows of O^T are never read.
-            const uint64_t da = make_smem_desc(kv_addr + (2 * blk) * MLA_SLAB + kk * 2048, MLA_SLAB,
-                                               1024, kLayoutSw128);
-            const uint64_t db = make_smem_desc(
-                p_addr + b * Cfg::P_BYTES + (kk >> 2) * Cfg::P_HALF + (kk & 3) * 32, 16, 1024,
-                kLayoutSw128);
-            umma_f16_ss(tmem_base + Cfg::O_COL + blk * NQ, da, db, idesc_o,
+          for (int kk = 0; kk < 8; kk++)
+            umma_f16_ss(tmem_base + Cfg::O_COL + blk * NQ, dv + kk * 128, dp + (((kk >> 2) * Cfg::P_HALF + (kk & 3) * 32) >> 4), idesc_o,
                         (j > 0 || kk > 0) ? 1u : 0u);
-          }
           umma_commit(&h_empty[2 * blk]);
           if (2 * blk + 1 < lat_slabs) umma_commit(&h_empty[2 * blk + 1]);
         }
         umma_commit(&pv_done[b]);
       }
-      __syncwarp();
     }
   } else {
     // ------------------------------------------------------------ softmax / epilogue
@@ -459,6 +445,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     }
   }
 done:
+  __syncwarp();             // the elected threads come back to their warps
   tc_fence_before();
   __syncthreads();
   if (*abort_word != 0) {

@@ -93,7 +93,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   const int n0 = t_hi[0] - t_lo, n = max(t_hi[0], t_hi[1]) - t_lo, n1 = ntok[1] > 0 ? n : 0;    // key tiles of each query tile
   if (n <= 0) return;                        // no keys: nothing would arrive that the roles below wait for; rows stay as they are
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* Qs = smem;
@@ -137,7 +137,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_ptr;
+  const uint32_t tmem_base = warp_uniform(*tmem_ptr);
 
   if (warp == 8) {
     // ------------------------------------------------------------ producer
@@ -175,9 +175,9 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           goto done;
         }
         uint8_t* dst = kv == 0 ? Ks + st * Cfg::K_BYTES : Vs + st * PF_V_BYTES;
-        if (lane == 0) mbar_expect_tx(fullb, kv == 0 ? Cfg::K_BYTES : PF_V_BYTES);
+        if (elect_one()) mbar_expect_tx(fullb, kv == 0 ? Cfg::K_BYTES : PF_V_BYTES);
         if (LATENT) {
-          if (lane == 0) {
+          if (elect_one()) {
             for (int s = 0; s < 2; s++)
               tma_load_3d(dst + s * PF_HALF, kv == 0 ? &tmap_k : &tmap_v, fullb, s * 64, h, k_row0 + key0);
             if (kv == 0) tma_load_2d(dst + 2 * PF_HALF, &tmap_pe, fullb, 0, k_row0 + key0);
@@ -186,7 +186,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           for (int part = 0; part < parts; part++) {
             const int blk = __shfl_sync(0xffffffffu, blk_cur, part);
             const int off = (key0 + part * p.rows_per_load) % p.block_size;
-            if (lane == 0)
+            if (elect_one())
               for (int s = 0; s < 2; s++)
                 tma_load_4d(dst + s * PF_HALF + part * p.rows_per_load * 128, kv == 0 ? &tmap_k : &tmap_v, fullb, s * 64, h, off, blk);
           }
@@ -196,57 +196,49 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       blk_cur = blk_next;
     }
   } else if (warp == 9) {
-    // ------------------------------------------------------------ MMA issuer
-    constexpr uint32_t idesc_s = make_idesc_f16(128, 128, true, false, false);
-    constexpr uint32_t idesc_o = make_idesc_f16(128, 128, true, false, true);
-    auto issue_s = [&](int w, int j) {
-      if (lane == 0) {
-        const uint32_t qa = smem_u32(Qs + w * Cfg::Q_BYTES), ka = smem_u32(Ks + (j & 1) * Cfg::K_BYTES);
+    // ------------------------------------------------------------ MMA issuer: one thread walks the loop (see warp_uniform)
+    if (elect_one()) {
+      constexpr uint32_t idesc_s = make_idesc_f16(128, 128, true, false, false);
+      constexpr uint32_t idesc_o = make_idesc_f16(128, 128, true, false, true);
+      const uint64_t dq0 = make_smem_desc(smem_u32(Qs), 16, 1024, kLayoutSw128), dk0 = make_smem_desc(smem_u32(Ks), 16, 1024, kLayoutSw128);
+      const uint64_t dv0 = make_smem_desc(smem_u32(Vs), PF_HALF, 1024, kLayoutSw128);
+      auto issue_s = [&](int w, int j) {
+        const uint64_t dq = dq0 + (uint32_t)(w * (Cfg::Q_BYTES >> 4)), dk = dk0 + (uint32_t)((j & 1) * (Cfg::K_BYTES >> 4));
 #pragma unroll
         for (int kk = 0; kk < NK * 4; kk++) {
-          const uint32_t o = (kk >> 2) * PF_HALF + (kk & 3) * 32;
-          umma_f16_ss(tmem_base + w * 128, make_smem_desc(qa + o, 16, 1024, kLayoutSw128),
-                      make_smem_desc(ka + o, 16, 1024, kLayoutSw128), idesc_s, kk > 0 ? 1u : 0u);
+          const uint32_t o = ((kk >> 2) * PF_HALF + (kk & 3) * 32) >> 4;
+          umma_f16_ss(tmem_base + w * 128, dq + o, dk + o, idesc_s, kk > 0 ? 1u : 0u);
         }
         umma_commit(&s_full[w]);
-      }
-      __syncwarp();
-    };
-    if (!mbar_wait(&q_full[0], 0, abort_word)) goto done;
-    if (n1 > 0 && !mbar_wait(&q_full[1], 0, abort_word)) goto done;
-    if (!mbar_wait(&k_full[0], 0, abort_word)) goto done;
-    tc_fence_after();
-    issue_s(0, 0);
-    if (n1 > 0) issue_s(1, 0);
-    if (lane == 0) umma_commit(&k_empty[0]);
-    __syncwarp();
-    for (int j = 0; j < n; j++) {
-      const int vs = j % VST;
-      if (!mbar_wait(&v_full[vs], (uint32_t)(j / VST) & 1u, abort_word)) goto done;
-      if (j + 1 < n && !mbar_wait(&k_full[(j + 1) & 1], (uint32_t)((j + 1) >> 1) & 1u, abort_word)) goto done;
+      };
+      if (!mbar_wait(&q_full[0], 0, abort_word)) goto done;
+      if (n1 > 0 && !mbar_wait(&q_full[1], 0, abort_word)) goto done;
+      if (!mbar_wait(&k_full[0], 0, abort_word)) goto done;
+      tc_fence_after();
+      issue_s(0, 0);
+      if (n1 > 0) issue_s(1, 0);
+      umma_commit(&k_empty[0]);
+      for (int j = 0; j < n; j++) {
+        const int vs = j % VST;
+        if (!mbar_wait(&v_full[vs], (uint32_t)(j / VST) & 1u, abort_word)) goto done;
+        if (j + 1 < n && !mbar_wait(&k_full[(j + 1) & 1], (uint32_t)((j + 1) >> 1) & 1u, abort_word)) goto done;
+        const uint64_t dv = dv0 + (uint32_t)(vs * (PF_V_BYTES >> 4));
 #pragma unroll 1
-      for (int w = 0; w < 2; w++) {
-        const int nw = w == 0 ? n0 : n1;
-        if (j < nw) {
-          if (!mbar_wait(&p_full[w], (uint32_t)j & 1u, abort_word)) goto done;
-          tc_fence_after();
-          if (lane == 0) {
-            const uint32_t va = smem_u32(Vs + vs * PF_V_BYTES);
+        for (int w = 0; w < 2; w++) {
+          const int nw = w == 0 ? n0 : n1;
+          if (j < nw) {
+            if (!mbar_wait(&p_full[w], (uint32_t)j & 1u, abort_word)) goto done;
+            tc_fence_after();
 #pragma unroll
             for (int kk = 0; kk < 8; kk++)
-              umma_f16_ts(tmem_base + O_COL + w * 128, tmem_base + w * 128 + kk * 8,
-                          make_smem_desc(va + kk * 2048, PF_HALF, 1024, kLayoutSw128), idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
+              umma_f16_ts(tmem_base + O_COL + w * 128, tmem_base + w * 128 + kk * 8, dv + kk * 128, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
             if (j == nw - 1) umma_commit(&o_full[w]);
+            if (j + 1 < nw) issue_s(w, j + 1);
           }
-          __syncwarp();
-          if (j + 1 < nw) issue_s(w, j + 1);
         }
-      }
-      if (lane == 0) {
         umma_commit(&v_empty[vs]);
         if (j + 1 < n) umma_commit(&k_empty[(j + 1) & 1]);
       }
-      __syncwarp();
     }
   } else {
     // ------------------------------------------------------------ softmax / epilogue of query tile w
@@ -357,6 +349,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     }
   }
 done:
+  __syncwarp();             // the elected threads come back to their warps
   tc_fence_before();
   __syncthreads();
   if (*abort_word != 0) {

@@ -129,7 +129,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
   const int dv = VAR ? p.Dv : D;
   auto tile_no = [&](int j) { return VAR && first + j < kept ? first + j : t0 + j; };
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
 
   if (n <= 0) {  // empty split: neutral partial
@@ -193,7 +193,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_ptr;
+  const uint32_t tmem_base = warp_uniform(*tmem_ptr);
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
@@ -233,7 +233,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
         }
         for (int part = 0; part < parts; part++) {
           const int blk = __shfl_sync(0xffffffffu, blk_cur, part);
-          if (lane == 0) {
+          if (elect_one()) {
             uint8_t* dst = (kv == 0 ? Ks : Vs) + ks * Cfg::TILE_BYTES;
             const CUtensorMap* tm = kv == 0 ? &tmap_k : &tmap_v;
             if (part == 0) mbar_expect_tx(fullb, Cfg::TILE_BYTES);
@@ -248,59 +248,49 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
       blk_cur = blk_next;
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    constexpr uint32_t idesc_s = make_idesc_f16(128, 128, true, false, false);
-    constexpr uint32_t idesc_o = make_idesc_f16(128, D, true, false, true);
-    const uint32_t q_addr = smem_u32(Qs), k_addr = smem_u32(Ks), v_addr = smem_u32(Vs),
-                   p_addr = smem_u32(Ps);
-    if (!mbar_wait(q_full, 0, abort_word)) goto done;
-    auto issue_s = [&](int j) -> bool {
-      const int ks = j % KS;
-      const uint32_t ph = (uint32_t)(j / KS) & 1u;
-      const int b = j & 1;
-      if (!mbar_wait(&k_full[ks], ph, abort_word)) return false;
-      if (!mbar_wait(&s_free[b], (((uint32_t)j >> 1) & 1u) ^ 1u, abort_word)) return false;
-      tc_fence_after();
-      if (lane == 0) {
+    // ------------------------------------------------------------ MMA issuer: one thread walks the loop (see warp_uniform)
+    if (elect_one()) {
+      constexpr uint32_t idesc_s = make_idesc_f16(128, 128, true, false, false);
+      constexpr uint32_t idesc_o = make_idesc_f16(128, D, true, false, true);
+      const uint64_t dq0 = make_smem_desc(smem_u32(Qs), 16, 1024, kLayoutSw128), dk0 = make_smem_desc(smem_u32(Ks), 16, 1024, kLayoutSw128);
+      const uint64_t dp0 = make_smem_desc(smem_u32(Ps), 16, 1024, kLayoutSw128), dv0 = make_smem_desc(smem_u32(Vs), p.v_lbo, p.v_sbo, kLayoutSw128);
+      if (!mbar_wait(q_full, 0, abort_word)) goto done;
+      auto issue_s = [&](int j) -> bool {
+        const int ks = j % KS;
+        const uint32_t ph = (uint32_t)(j / KS) & 1u;
+        const int b = j & 1;
+        if (!mbar_wait(&k_full[ks], ph, abort_word)) return false;
+        if (!mbar_wait(&s_free[b], (((uint32_t)j >> 1) & 1u) ^ 1u, abort_word)) return false;
+        tc_fence_after();
+        const uint64_t dk = dk0 + (uint32_t)(ks * (Cfg::TILE_BYTES >> 4));
 #pragma unroll
         for (int kk = 0; kk < D / 16; kk++) {
-          const uint32_t o = (kk >> 2) * ATT_HALF_BYTES + (kk & 3) * 32;
-          const uint64_t da = make_smem_desc(q_addr + o, 16, 1024, kLayoutSw128);
-          const uint64_t db =
-              make_smem_desc(k_addr + ks * Cfg::TILE_BYTES + o, 16, 1024, kLayoutSw128);
-          umma_f16_ss(tmem_base + b * 128, da, db, idesc_s, kk > 0 ? 1u : 0u);
+          const uint32_t o = ((kk >> 2) * ATT_HALF_BYTES + (kk & 3) * 32) >> 4;
+          umma_f16_ss(tmem_base + b * 128, dq0 + o, dk + o, idesc_s, kk > 0 ? 1u : 0u);
         }
         umma_commit(&k_empty[ks]);
         umma_commit(&s_ready[b]);
-      }
-      __syncwarp();
-      return true;
-    };
-    if (!issue_s(0)) goto done;
-    for (int j = 0; j < n; j++) {
-      if (j + 1 < n) {
-        if (!issue_s(j + 1)) goto done;
-      }
-      const int vs = j % KS;
-      const uint32_t ph = (uint32_t)(j / KS) & 1u;
-      if (!mbar_wait(&v_full[vs], ph, abort_word)) goto done;
-      const int pb = j & 1;
-      if (!mbar_wait(&p_ready[pb], ((uint32_t)j >> 1) & 1u, abort_word)) goto done;
-      tc_fence_after();
-      if (lane == 0) {
-#pragma unroll
-        for (int kk = 0; kk < 8; kk++) {
-          const uint32_t po = (kk >> 2) * ATT_HALF_BYTES + (kk & 3) * 32;
-          const uint64_t da =
-              make_smem_desc(p_addr + pb * Cfg::P_BYTES + po, 16, 1024, kLayoutSw128);
-          const uint64_t db = make_smem_desc(v_addr + vs * Cfg::TILE_BYTES + kk * 2048, p.v_lbo,
-                                             p.v_sbo, kLayoutSw128);
-          umma_f16_ss(tmem_base + Cfg::O_COL, da, db, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
+        return true;
+      };
+      if (!issue_s(0)) goto done;
+      for (int j = 0; j < n; j++) {
+        if (j + 1 < n) {
+          if (!issue_s(j + 1)) goto done;
         }
+        const int vs = j % KS;
+        const uint32_t ph = (uint32_t)(j / KS) & 1u;
+        if (!mbar_wait(&v_full[vs], ph, abort_word)) goto done;
+        const int pb = j & 1;
+        if (!mbar_wait(&p_ready[pb], ((uint32_t)j >> 1) & 1u, abort_word)) goto done;
+        tc_fence_after();
+        const uint64_t dp = dp0 + (uint32_t)(pb * (Cfg::P_BYTES >> 4)), dv = dv0 + (uint32_t)(vs * (Cfg::TILE_BYTES >> 4));
+#pragma unroll
+        for (int kk = 0; kk < 8; kk++)
+          umma_f16_ss(tmem_base + Cfg::O_COL, dp + (((kk >> 2) * ATT_HALF_BYTES + (kk & 3) * 32) >> 4), dv + kk * 128, idesc_o,
+                      (j > 0 || kk > 0) ? 1u : 0u);
         umma_commit(&v_empty[vs]);
         umma_commit(&pv_done[pb]);
       }
-      __syncwarp();
     }
   } else {
     // ------------------------------------------------------------ softmax / epilogue
@@ -513,6 +503,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
     }
   }
 done:
+  __syncwarp();             // the elected threads come back to their warps
   tc_fence_before();
   __syncthreads();
   if (*abort_word != 0) {

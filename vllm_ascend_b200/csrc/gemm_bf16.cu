@@ -151,7 +151,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
   volatile int* abort_word = (volatile int*)(tmem_ptr + 1);
   int* grp_tiles = (int*)(tmem_ptr + 2);            // [num_groups + 1] (GROUPED only)
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int num_kb = (p.K + GEMM_BK - 1) / GEMM_BK;
   const bool swiglu = (p.mode & GEMM_SWIGLU) != 0;
@@ -207,33 +207,30 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_ptr;
+  const uint32_t tmem_base = warp_uniform(*tmem_ptr);
   const int num_tiles = (p.mode & GEMM_GROUPED) ? grp_tiles[p.num_groups] * p.tiles_n
                                                 : p.tiles_m * p.tiles_n;
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    int stage = 0;
-    uint32_t phase = 0;
-    uint32_t ag_epoch = 0;
-    if (p.mode & GEMM_AG) ag_epoch = *((volatile const uint32_t*)p.ag_epoch);
-    if ((p.mode & GEMM_WAITFLAGS) && blockIdx.x < num_tiles) {
-      // rows of A are written by peers: wait until every rank has published this call's epoch
-      if (lane == 0) {
+    if (elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      uint32_t ag_epoch = 0;
+      if (p.mode & GEMM_AG) ag_epoch = *((volatile const uint32_t*)p.ag_epoch);
+      if ((p.mode & GEMM_WAITFLAGS) && blockIdx.x < num_tiles) {
+        // rows of A are written by peers: wait until every rank has published this call's epoch
         const uint32_t e = *((volatile const uint32_t*)p.wait_epoch) + 1;
         for (int s = 0; s < p.num_ranks; s++)
           if (!wait_flag_ge(&p.wait_flags[s], e, p.status)) { *abort_word = B200_TIMEOUT; break; }
         fence_proxy_async_global();
+        if (*abort_word) goto done;
       }
-      __syncwarp();
-      if (*abort_word) goto done;
-    }
-    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
-      TileCoord c;
-      tile_coord<BN>(p, grp_tiles, t, c);
-      if (p.mode & GEMM_AG) {
-        // rows of this tile come from source ranks s0..s1: wait for their pushes
-        if (lane == 0) {
+      for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
+        TileCoord c;
+        tile_coord<BN>(p, grp_tiles, t, c);
+        if (p.mode & GEMM_AG) {
+          // rows of this tile come from source ranks s0..s1: wait for their pushes
           const int last_row = min(c.row0 + GEMM_BM, p.M) - 1;
           const int s0 = c.row0 / p.rows_per_src, s1 = last_row / p.rows_per_src;
           for (int s = s0; s <= s1; s++) {
@@ -241,59 +238,46 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
             if (!wait_flag_ge(&p.ag_flags[s], ag_epoch, p.status)) *abort_word = B200_TIMEOUT;
           }
           fence_proxy_async_global();
+          if (*abort_word) goto done;
         }
-        __syncwarp();
-        if (*abort_word) goto done;
-      }
-      for (int kb = 0; kb < num_kb; kb++) {
-        if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_word)) goto done;
-        if (lane == 0) {
+        for (int kb = 0; kb < num_kb; kb++) {
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_word)) goto done;
           uint8_t* sa = tiles + stage * Cfg::kStageBytes;
           uint8_t* sb = sa + Cfg::kABytes;
           mbar_expect_tx(&full_bar[stage], Cfg::kStageBytes);
           tma_load_2d(sa, &tmap_a, &full_bar[stage], kb * GEMM_BK, c.row0);
-          if (swiglu) {
-            // 128 gate rows then 128 up rows (the W tensor map has a 128-row box)
-            tma_load_2d(sb, &tmap_b, &full_bar[stage], kb * GEMM_BK, c.w_row0);
-            tma_load_2d(sb + Cfg::kBBytes / 2, &tmap_b, &full_bar[stage], kb * GEMM_BK,
-                        c.w_row0 + p.up_row_offset);
-          } else {
-            tma_load_2d(sb, &tmap_b, &full_bar[stage], kb * GEMM_BK, c.w_row0);
-          }
+          tma_load_2d(sb, &tmap_b, &full_bar[stage], kb * GEMM_BK, c.w_row0);
+          // with a gate 128 of its rows, then 128 rows of up (the W tensor map has a 128-row box)
+          if (swiglu) tma_load_2d(sb + Cfg::kBBytes / 2, &tmap_b, &full_bar[stage], kb * GEMM_BK, c.w_row0 + p.up_row_offset);
+          if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
         }
-        __syncwarp();
-        if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    constexpr uint32_t idesc = make_idesc_f16(GEMM_BM, BN, true, false, false);
-    int stage = 0;
-    uint32_t phase = 0;
-    int it = 0;
-    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, it++) {
-      const int acc = it & 1;
-      const uint32_t acc_phase = (it >> 1) & 1;
-      if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_word)) goto done;
-      tc_fence_after();
-      const uint32_t d_tmem = tmem_base + acc * BN;
-      for (int kb = 0; kb < num_kb; kb++) {
-        if (!mbar_wait(&full_bar[stage], phase, abort_word)) goto done;
+    // ------------------------------------------------------------ MMA issuer: one thread walks the loop (see warp_uniform)
+    if (elect_one()) {
+      constexpr uint32_t idesc = make_idesc_f16(GEMM_BM, BN, true, false, false);
+      const uint64_t da0 = make_smem_desc(smem_u32(tiles), 16, 1024, kLayoutSw128);
+      int stage = 0;
+      uint32_t phase = 0;
+      int it = 0;
+      for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, it++) {
+        const int acc = it & 1;
+        const uint32_t acc_phase = (it >> 1) & 1;
+        if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_word)) goto done;
         tc_fence_after();
-        if (lane == 0) {
-          const uint32_t sa = smem_u32(tiles + stage * Cfg::kStageBytes);
-          const uint32_t sb = sa + Cfg::kABytes;
+        const uint32_t d_tmem = tmem_base + acc * BN;
+        for (int kb = 0; kb < num_kb; kb++) {
+          if (!mbar_wait(&full_bar[stage], phase, abort_word)) goto done;
+          tc_fence_after();
+          const uint64_t da = da0 + (uint32_t)(stage * (Cfg::kStageBytes >> 4)), db = da + (Cfg::kABytes >> 4);
 #pragma unroll
-          for (int kk = 0; kk < GEMM_BK / 16; kk++) {
-            const uint64_t da = make_smem_desc(sa + kk * 32, 16, 1024, kLayoutSw128);
-            const uint64_t db = make_smem_desc(sb + kk * 32, 16, 1024, kLayoutSw128);
-            umma_f16_ss(d_tmem, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-          }
+          for (int kk = 0; kk < GEMM_BK / 16; kk++)
+            umma_f16_ss(d_tmem, da + 2 * kk, db + 2 * kk, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
           umma_commit(&empty_bar[stage]);
-          if (kb == num_kb - 1) umma_commit(&tmem_full[acc]);
+          if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
         }
-        __syncwarp();
-        if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
+        umma_commit(&tmem_full[acc]);
       }
     }
   } else {
@@ -427,6 +411,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a,
     if (p.mode & (GEMM_RS | GEMM_SCATTER | GEMM_PUB)) __threadfence_system();   // rows visible to their owners
   }
 done:
+  __syncwarp();             // the elected threads come back to their warps
   tc_fence_before();
   __syncthreads();
   if (*abort_word != 0) {

@@ -11,9 +11,10 @@
 // TMA loads are plain `cta_group::2` loads (no multicast): each CTA fetches its
 // own tiles and reports the bytes to the leader's barrier.
 //
-//   warp 0      TMA producer (both CTAs)
+//   warp 0      TMA producer of A (both CTAs)
 //   warp 1      MMA issuer (leader CTA only) + TMEM alloc/dealloc (both)
 //   warps 2..5  epilogue (both CTAs, each for its own 128 rows)
+//   warp 6      TMA producer of W (both CTAs)
 // All waits are bounded (common.cuh); the cluster barriers at start and end are
 // reached by every thread on every path.
 #include "comm.cuh"
@@ -26,7 +27,7 @@ namespace b200 {
 constexpr int G2_BM = 256;          // per CTA pair
 constexpr int G2_BN = 256;
 constexpr int G2_BK = 64;
-constexpr int G2_THREADS = 192;
+constexpr int G2_THREADS = 224;
 constexpr int G2_STAGES = 6;
 constexpr int G2_A_BYTES = 128 * G2_BK * 2;        // 16 KB: this CTA's rows of A
 constexpr int G2_B_BYTES = 128 * G2_BK * 2;        // 16 KB: this CTA's half of the W tile
@@ -94,11 +95,11 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
                : "memory");
 }
-__device__ __forceinline__ void tma_load_2d_2sm(void* dst, const CUtensorMap* map,
+__device__ __forceinline__ void tma_load_2d_2sm(uint32_t dst, const CUtensorMap* map,
                                                 uint32_t leader_bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
+      " [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
       "l"(map), "r"(leader_bar), "r"(x), "r"(y)
       : "memory");
 }
@@ -164,7 +165,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a,
   uint32_t* tmem_ptr = (uint32_t*)(tmem_empty + 2);
   volatile int* abort_word = (volatile int*)(tmem_ptr + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
@@ -197,22 +198,25 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a,
   __syncthreads();
   cluster_sync_all();       // both CTAs' barriers exist before anyone signals across
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_ptr;
+  const uint32_t tmem_base = warp_uniform(*tmem_ptr);
 
-  if (warp == 0) {
-    // ------------------------------------------------------------ producer (both CTAs)
-    int stage = 0;
-    uint32_t phase = 0;
-    uint32_t ag_epoch = 0;
-    if (p.mode & G2_AG) ag_epoch = *((volatile const uint32_t*)p.ag_epoch);
-    for (int t = cluster_id; t < num_tiles; t += num_clusters) {
-      int tm, tn;
-      tile_of(p, t, tm, tn);
-      if (p.mode & G2_AG) tm = (tm + (p.my_rank * p.rows_per_src) / G2_BM) % p.tiles_m;   // local rows first
-      const int a_row = tm * G2_BM + (int)rank * 128;
-      if (p.mode & G2_AG) {
-        // this CTA's 128 rows come from source ranks s0..s1: wait for their pushes
-        if (lane == 0 && a_row < p.M) {
+  if (warp == 0 || warp == 6) {
+    // ------------------------------------------------------------ producers (both CTAs)
+    if (elect_one()) {
+      const bool for_a = warp == 0;
+      int stage = 0;
+      uint32_t phase = 0;
+      uint32_t ag_epoch = 0;
+      if (p.mode & G2_AG) ag_epoch = *((volatile const uint32_t*)p.ag_epoch);
+      const uint32_t tiles_addr = smem_u32(tiles), lbar0 = smem_u32(full_bar) & kPeerBitMask;
+      const uint32_t tx_bytes = 2 * (G2_A_BYTES + (p.bn >> 1) * G2_BK * 2);
+      for (int t = cluster_id; t < num_tiles; t += num_clusters) {
+        int tm, tn;
+        tile_of(p, t, tm, tn);
+        if (p.mode & G2_AG) tm = (tm + (p.my_rank * p.rows_per_src) / G2_BM) % p.tiles_m;   // local rows first
+        const int a_row = tm * G2_BM + (int)rank * 128;
+        if (for_a && (p.mode & G2_AG) && a_row < p.M) {
+          // this CTA's 128 rows come from source ranks s0..s1: wait for their pushes
           const int last_row = min(a_row + 128, p.M) - 1;
           const int s0 = a_row / p.rows_per_src, s1 = last_row / p.rows_per_src;
           for (int s = s0; s <= s1; s++) {
@@ -220,48 +224,54 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a,
             if (!wait_flag_ge(&p.ag_flags[s], ag_epoch, p.status)) *abort_word = B200_TIMEOUT;
           }
           fence_proxy_async_global();
+          if (*abort_word) goto done;
         }
-        __syncwarp();
-        if (*abort_word) goto done;
-      }
-      // plain: this CTA's 128 of the tile's 256 W rows.  SwiGLU: the leader stages the 128
-      // gate rows, the peer the matching 128 up rows.
-      const int w_row = p.swiglu ? tn * 128 + (int)rank * p.up_row_offset
-                                 : tn * p.bn + (int)rank * (p.bn >> 1);
-      // Few row tiles (decode batches): every weight byte is read from DRAM once and nothing else
-      // hides that latency but the depth of the stage ring, so the boxes of later k-blocks are
-      // requested into L2 ahead of time.  One row tile asks for W, one column tile for A.
-      const bool pf_w = p.l2_prefetch > 0 && tm == 0;
-      const bool pf_a = p.l2_prefetch > 0 && p.mode == 0 && tn == 0 && a_row < p.M;
-      if (lane == 0 && (pf_w || pf_a)) {
-        for (int kb = 0; kb < p.l2_prefetch && kb < num_kb; kb++) {
-          if (pf_w) tma_prefetch_l2_2d(&tmap_b, kb * G2_BK, w_row);
-          if (pf_a) tma_prefetch_l2_2d(&tmap_a, kb * G2_BK, a_row);
-        }
-      }
-      for (int kb = 0; kb < num_kb; kb++) {
-        if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_word)) goto done;
-        if (lane == 0) {
-          const int kpf = kb + p.l2_prefetch;
-          if (kpf < num_kb) {
-            if (pf_w) tma_prefetch_l2_2d(&tmap_b, kpf * G2_BK, w_row);
-            if (pf_a) tma_prefetch_l2_2d(&tmap_a, kpf * G2_BK, a_row);
+        // plain: this CTA's 128 of the tile's 256 W rows.  SwiGLU: the leader stages the 128
+        // gate rows, the peer the matching 128 up rows.
+        const int w_row = p.swiglu ? tn * 128 + (int)rank * p.up_row_offset
+                                   : tn * p.bn + (int)rank * (p.bn >> 1);
+        // Few row tiles (decode batches): every weight byte is read from DRAM once and nothing else
+        // hides that latency but the depth of the stage ring, so the boxes of later k-blocks are
+        // requested into L2 ahead of time.  One row tile asks for W, one column tile for A.
+        const bool pf_w = !for_a && p.l2_prefetch > 0 && tm == 0;
+        const bool pf_a = for_a && p.l2_prefetch > 0 && p.mode == 0 && tn == 0 && a_row < p.M;
+        const bool ahead = pf_w || pf_a;
+        if (ahead)
+          for (int kb = 0; kb < p.l2_prefetch && kb < num_kb; kb++)
+            tma_prefetch_l2_2d(for_a ? &tmap_a : &tmap_b, kb * G2_BK, for_a ? a_row : w_row);
+        // Prefetching has a loop to itself: two branches not taken cost 145 of the 440 clocks that a k-block then took.
+        auto load = [&](int kb) {
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_word)) return false;
+          const uint32_t sa = tiles_addr + stage * G2_STAGE_BYTES, lbar = lbar0 + stage * 8;
+          if (for_a) {
+            if (leader) mbar_expect_tx(&full_bar[stage], tx_bytes);
+            tma_load_2d_2sm(sa, &tmap_a, lbar, kb * G2_BK, a_row);
+          } else {
+            tma_load_2d_2sm(sa + G2_A_BYTES, &tmap_b, lbar, kb * G2_BK, w_row);
           }
-          uint8_t* sa = tiles + stage * G2_STAGE_BYTES;
-          uint8_t* sb = sa + G2_A_BYTES;
-          const uint32_t lbar = smem_u32(&full_bar[stage]) & kPeerBitMask;
-          if (leader) mbar_expect_tx(&full_bar[stage], 2 * (G2_A_BYTES + (p.bn >> 1) * G2_BK * 2));
-          tma_load_2d_2sm(sa, &tmap_a, lbar, kb * G2_BK, a_row);
-          tma_load_2d_2sm(sb, &tmap_b, lbar, kb * G2_BK, w_row);
+          if (++stage == G2_STAGES) { stage = 0; phase ^= 1; }
+          return true;
+        };
+        if (ahead) {
+          for (int kb = 0; kb < num_kb; kb++) {
+            if (!load(kb)) goto done;
+            if (kb + p.l2_prefetch < num_kb)
+              tma_prefetch_l2_2d(for_a ? &tmap_a : &tmap_b, (kb + p.l2_prefetch) * G2_BK, for_a ? a_row : w_row);
+          }
+        } else {
+          for (int kb = 0; kb < num_kb; kb++)
+            if (!load(kb)) goto done;
         }
-        __syncwarp();
-        if (++stage == G2_STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader only)
-    if (leader) {
+    // One thread walks the whole loop and finds its descriptors by addition.  With the loop walked by the warp and one lane's
+    // branch inside it, four MMAs and their commit took 570 clocks to issue whatever the tile's width, and 256 columns
+    // need 512 on the tensor cores: 4096 x 4096 x 12288 measured 1.26 PFLOP/s in 256-wide tiles and 0.73 in 128-wide ones.
+    if (leader && elect_one()) {
       const uint32_t idesc = make_idesc_f16(G2_BM, p.bn, true, false, false);
+      const uint64_t da0 = make_smem_desc(smem_u32(tiles), 16, 1024, kLayoutSw128);
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
@@ -274,21 +284,14 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a,
         for (int kb = 0; kb < num_kb; kb++) {
           if (!mbar_wait(&full_bar[stage], phase, abort_word)) goto done;
           tc_fence_after();
-          if (lane == 0) {
-            const uint32_t sa = smem_u32(tiles + stage * G2_STAGE_BYTES);
-            const uint32_t sb = sa + G2_A_BYTES;
+          const uint64_t da = da0 + (uint32_t)(stage * (G2_STAGE_BYTES >> 4)), db = da + (G2_A_BYTES >> 4);
 #pragma unroll
-            for (int kk = 0; kk < G2_BK / 16; kk++) {
-              const uint64_t da = make_smem_desc(sa + kk * 32, 16, 1024, kLayoutSw128);
-              const uint64_t db = make_smem_desc(sb + kk * 32, 16, 1024, kLayoutSw128);
-              umma_f16_ss_2sm(d_tmem, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-            }
-            umma_commit_2sm(&empty_bar[stage]);
-            if (kb == num_kb - 1) umma_commit_2sm(&tmem_full[acc]);
-          }
-          __syncwarp();
+          for (int kk = 0; kk < G2_BK / 16; kk++)
+            umma_f16_ss_2sm(d_tmem, da + 2 * kk, db + 2 * kk, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+          umma_commit_2sm(&empty_bar[stage]);
           if (++stage == G2_STAGES) { stage = 0; phase ^= 1; }
         }
+        umma_commit_2sm(&tmem_full[acc]);
       }
     }
   } else {
@@ -440,6 +443,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a,
     if (p.mode & G2_PUB) __threadfence_system();   // partial rows visible to their owners
   }
 done:
+  __syncwarp();             // the elected threads come back to their warps
   tc_fence_before();
   __syncthreads();
   if (*abort_word != 0) {

@@ -105,7 +105,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a,
   volatile int* abort_word = (volatile int*)(tmem_ptr + 1);
   int* grp_tiles = (int*)(tmem_ptr + 2);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int num_kb = p.num_kb;
 
   if (threadIdx.x == 0) {
@@ -148,56 +148,51 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a,
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_ptr;
+  const uint32_t tmem_base = warp_uniform(*tmem_ptr);
   const int num_tiles = (p.num_groups > 0 ? grp_tiles[p.num_groups] : p.tiles_m) * p.tiles_n;
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    int stage = 0;
-    uint32_t phase = 0;
-    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
-      F8Tile c;
-      f8_tile<BN>(p, grp_tiles, t, c);
-      for (int kb = 0; kb < num_kb; kb++) {
-        if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_word)) goto done;
-        if (lane == 0) {
+    if (elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
+        F8Tile c;
+        f8_tile<BN>(p, grp_tiles, t, c);
+        for (int kb = 0; kb < num_kb; kb++) {
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_word)) goto done;
           uint8_t* sa = tiles + stage * F8_STAGE_BYTES;
           mbar_expect_tx(&full_bar[stage], F8_STAGE_BYTES);
           tma_load_2d(sa, &tmap_a, &full_bar[stage], kb * F8_BK, c.row0);
 #pragma unroll
           for (int h = 0; h < BN / 128; h++)
             tma_load_2d(sa + (1 + h) * F8_TILE_BYTES, &tmap_b, &full_bar[stage], kb * F8_BK, c.w_row0 + h * 128);
+          if (++stage == F8_STAGES) { stage = 0; phase ^= 1; }
         }
-        __syncwarp();
-        if (++stage == F8_STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    constexpr uint32_t idesc = make_idesc_e4m3(F8_BM, BN);
-    int stage = 0;
-    uint32_t phase = 0;
-    uint32_t it = 0;          // K blocks issued so far (selects the partial buffer)
-    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
-      for (int kb = 0; kb < num_kb; kb++, it++) {
-        const int b = it & 1;
-        if (!mbar_wait(&part_empty[b], ((it >> 1) & 1u) ^ 1u, abort_word)) goto done;
-        if (!mbar_wait(&full_bar[stage], phase, abort_word)) goto done;
-        tc_fence_after();
-        if (lane == 0) {
-          const uint32_t sa = smem_u32(tiles + stage * F8_STAGE_BYTES);
-          const uint32_t sb = sa + F8_TILE_BYTES;
+    // ------------------------------------------------------------ MMA issuer: one thread walks the loop (see warp_uniform)
+    if (elect_one()) {
+      constexpr uint32_t idesc = make_idesc_e4m3(F8_BM, BN);
+      const uint64_t da0 = make_smem_desc(smem_u32(tiles), 16, 1024, kLayoutSw128);
+      int stage = 0;
+      uint32_t phase = 0;
+      uint32_t it = 0;          // K blocks issued so far (selects the partial buffer)
+      for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
+        for (int kb = 0; kb < num_kb; kb++, it++) {
+          const int b = it & 1;
+          if (!mbar_wait(&part_empty[b], ((it >> 1) & 1u) ^ 1u, abort_word)) goto done;
+          if (!mbar_wait(&full_bar[stage], phase, abort_word)) goto done;
+          tc_fence_after();
+          const uint64_t da = da0 + (uint32_t)(stage * (F8_STAGE_BYTES >> 4)), db = da + (F8_TILE_BYTES >> 4);
 #pragma unroll
-          for (int kk = 0; kk < F8_BK / 32; kk++) {       // 32 e4m3 = 32 bytes per MMA
-            const uint64_t da = make_smem_desc(sa + kk * 32, 16, 1024, kLayoutSw128);
-            const uint64_t db = make_smem_desc(sb + kk * 32, 16, 1024, kLayoutSw128);
-            umma_f8_ss(tmem_base + b * BN, da, db, idesc, kk > 0 ? 1u : 0u);
-          }
+          for (int kk = 0; kk < F8_BK / 32; kk++)         // 32 e4m3 = 32 bytes per MMA
+            umma_f8_ss(tmem_base + b * BN, da + 2 * kk, db + 2 * kk, idesc, kk > 0 ? 1u : 0u);
           umma_commit(&empty_bar[stage]);
           umma_commit(&part_full[b]);
+          if (++stage == F8_STAGES) { stage = 0; phase ^= 1; }
         }
-        __syncwarp();
-        if (++stage == F8_STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else {
@@ -294,6 +289,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
   }
 done:
+  __syncwarp();             // the elected threads come back to their warps
   tc_fence_before();
   __syncthreads();
   if (*abort_word != 0) {

@@ -63,7 +63,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   uint32_t* tmem_ptr = (uint32_t*)(tmem_full + 1);
   volatile int* abort_word = (volatile int*)(tmem_ptr + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int split = blockIdx.x, tile = blockIdx.y;       // the cluster is the whole x extent of the grid
   const int num_kb = (p.K + SG_BK - 1) / SG_BK;
   const int kb0 = (int)((long)num_kb * split / p.splits), kb1 = (int)((long)num_kb * (split + 1) / p.splits);
@@ -94,46 +94,46 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_ptr;
+  const uint32_t tmem_base = warp_uniform(*tmem_ptr);
   asm volatile("griddepcontrol.wait;" ::: "memory");     // activations, residual and C belong to earlier kernels until here
 
   bool ok = true;
   if (warp == 4) {
     // ------------------------------------------------------------ producer
-    int stage = 0;
-    uint32_t phase = 0;
-    for (int kb = kb0; kb < kb1 && ok; kb++) {
-      ok = mbar_wait(&empty_bar[stage], phase ^ 1, abort_word);
-      if (ok && lane == 0) {
+    if (elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int kb = kb0; kb < kb1; kb++) {
+        if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_word)) break;
         uint8_t* sw = smem + stage * p.stage_bytes;
         mbar_expect_tx(&full_bar[stage], SG_WBYTES + p.nt * SG_BK * 2);
         tma_load_2d(sw, &tmap_w, &full_bar[stage], kb * SG_BK, w_row);
         if (p.glu) tma_load_2d(sw + SG_WBYTES / 2, &tmap_w, &full_bar[stage], kb * SG_BK, p.N + w_row);
         tma_load_2d(sw + SG_WBYTES, &tmap_a, &full_bar[stage], kb * SG_BK, 0);
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
       }
-      __syncwarp();
-      if (++stage == p.stages) { stage = 0; phase ^= 1; }
     }
+    __syncwarp();
   } else if (warp == 5) {
-    // ------------------------------------------------------------ MMA issuer
-    const uint32_t idesc = make_idesc_f16(SG_ROWS, p.nt, true, false, false);
-    int stage = 0;
-    uint32_t phase = 0;
-    for (int kb = kb0; kb < kb1 && ok; kb++) {
-      ok = mbar_wait(&full_bar[stage], phase, abort_word);
-      tc_fence_after();
-      if (ok && lane == 0) {
-        const uint32_t sw = smem_u32(smem + stage * p.stage_bytes);
+    // ------------------------------------------------------------ MMA issuer: one thread walks the loop (see warp_uniform)
+    if (elect_one()) {
+      const uint32_t idesc = make_idesc_f16(SG_ROWS, p.nt, true, false, false);
+      const uint64_t dw0 = make_smem_desc(smem_u32(smem), 16, 1024, kLayoutSw128);
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int kb = kb0; kb < kb1; kb++) {
+        ok = mbar_wait(&full_bar[stage], phase, abort_word);
+        if (!ok) break;
+        tc_fence_after();
+        const uint64_t dw = dw0 + (uint32_t)(stage * (p.stage_bytes >> 4)), da = dw + (SG_WBYTES >> 4);
 #pragma unroll
-        for (int kk = 0; kk < SG_BK / 16; kk++)
-          umma_f16_ss(tmem_base, make_smem_desc(sw + kk * 32, 16, 1024, kLayoutSw128),
-                      make_smem_desc(sw + SG_WBYTES + kk * 32, 16, 1024, kLayoutSw128), idesc, (kb > kb0 || kk > 0) ? 1u : 0u);
+        for (int kk = 0; kk < SG_BK / 16; kk++) umma_f16_ss(tmem_base, dw + 2 * kk, da + 2 * kk, idesc, (kb > kb0 || kk > 0) ? 1u : 0u);
         umma_commit(&empty_bar[stage]);
-        if (kb == kb1 - 1) umma_commit(tmem_full);
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
       }
-      __syncwarp();
-      if (++stage == p.stages) { stage = 0; phase ^= 1; }
+      if (ok) umma_commit(tmem_full);
     }
+    __syncwarp();
   } else {
     // ------------------------------------------------------------ accumulator -> shared memory, [token][weight row]
     ok = mbar_wait(tmem_full, 0, abort_word);

@@ -56,7 +56,7 @@ gemm_small_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
   uint32_t* tmem_ptr = (uint32_t*)(part_empty + NB);
   volatile int* abort_word = (volatile int*)(tmem_ptr + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int split = blockIdx.x, tile = blockIdx.y;
   const int kb0 = (int)((long)p.num_kb * split / p.splits), kb1 = (int)((long)p.num_kb * (split + 1) / p.splits);
   const int w_row = tile * SG_ROWS;
@@ -86,47 +86,47 @@ gemm_small_fp8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_ptr;
+  const uint32_t tmem_base = warp_uniform(*tmem_ptr);
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
   bool ok = true;
   if (warp == 8) {
     // ------------------------------------------------------------ producer
-    int stage = 0;
-    uint32_t phase = 0;
-    for (int kb = kb0; kb < kb1 && ok; kb++) {
-      ok = mbar_wait(&empty_bar[stage], phase ^ 1, abort_word);
-      if (ok && lane == 0) {
+    if (elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int kb = kb0; kb < kb1; kb++) {
+        if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_word)) break;
         uint8_t* sw = smem + stage * p.stage_bytes;
         mbar_expect_tx(&full_bar[stage], SF_WBYTES + NT * 128);
         tma_load_2d(sw, &tmap_w, &full_bar[stage], kb * 128, w_row);
         tma_load_2d(sw + SF_WBYTES, &tmap_a, &full_bar[stage], kb * 128, 0);
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
       }
-      __syncwarp();
-      if (++stage == p.stages) { stage = 0; phase ^= 1; }
     }
+    __syncwarp();
   } else if (warp == 9) {
-    // ------------------------------------------------------------ MMA issuer
-    constexpr uint32_t idesc = make_idesc_e4m3(SG_ROWS, NT);
-    int stage = 0;
-    uint32_t phase = 0;
-    for (int kb = kb0, it = 0; kb < kb1 && ok; kb++, it++) {
-      const int b = it % NB;
-      ok = mbar_wait(&part_empty[b], ((uint32_t)(it / NB) & 1u) ^ 1u, abort_word) &&
-           mbar_wait(&full_bar[stage], phase, abort_word);
-      tc_fence_after();
-      if (ok && lane == 0) {
-        const uint32_t sw = smem_u32(smem + stage * p.stage_bytes);
+    // ------------------------------------------------------------ MMA issuer: one thread walks the loop (see warp_uniform)
+    if (elect_one()) {
+      constexpr uint32_t idesc = make_idesc_e4m3(SG_ROWS, NT);
+      const uint64_t dw0 = make_smem_desc(smem_u32(smem), 16, 1024, kLayoutSw128);
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int kb = kb0, it = 0; kb < kb1; kb++, it++) {
+        const int b = it % NB;
+        if (!mbar_wait(&part_empty[b], ((uint32_t)(it / NB) & 1u) ^ 1u, abort_word) ||
+            !mbar_wait(&full_bar[stage], phase, abort_word))
+          break;
+        tc_fence_after();
+        const uint64_t dw = dw0 + (uint32_t)(stage * (p.stage_bytes >> 4)), da = dw + (SF_WBYTES >> 4);
 #pragma unroll
-        for (int kk = 0; kk < 4; kk++)
-          umma_f8_ss(tmem_base + b * NT, make_smem_desc(sw + kk * 32, 16, 1024, kLayoutSw128),
-                     make_smem_desc(sw + SF_WBYTES + kk * 32, 16, 1024, kLayoutSw128), idesc, kk > 0 ? 1u : 0u);
+        for (int kk = 0; kk < 4; kk++) umma_f8_ss(tmem_base + b * NT, dw + 2 * kk, da + 2 * kk, idesc, kk > 0 ? 1u : 0u);
         umma_commit(&empty_bar[stage]);
         umma_commit(&part_full[b]);
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
       }
-      __syncwarp();
-      if (++stage == p.stages) { stage = 0; phase ^= 1; }
     }
+    __syncwarp();
   } else {
     // ------------------------------------------------------------ promotion
     const int half = warp >> 2;
