@@ -46,7 +46,7 @@ struct Gemm2Params {
   __nv_bfloat16* C;
   int* status;
   int tiles_m, tiles_n;
-  int swiglu;          // W = [gate; up]: tile pairs 128 gate + 128 up columns
+  int swiglu;          // W = [gate; up]: a tile pairs bn / 2 gate and bn / 2 up columns
   float glu_alpha, glu_limit;      // alpha > 0: clamped gate instead of SiLU
   int up_row_offset;
   // ---- fused collectives (same protocol as the single-CTA kernel's AG / RS modes)
@@ -60,8 +60,8 @@ struct Gemm2Params {
   int rows_per_owner;
   int raster;                         // M-tiles per raster group (0/1: column-major order)
   int bn;                             // tile width: 128..256 in steps of 16 (32 with the reduce-scatter
-                                      // epilogue, whose staging flushes 64-column pairs; SwiGLU tiles: 256); from 64
-                                      // on with a single row of tiles, no row statistics and no peer memory
+                                      // epilogue, whose staging flushes 64-column pairs, and with a gate); from 64 on with a
+                                      // single row of tiles, no gate, no row statistics and no peer memory
   // ---- RMSNorm folded into the GEMMs around it (the norm weight lives in W of the consumer)
   // Row statistics travel as per-column-tile partial sums so that their total does not depend on
   // the order in which tiles finish: buffer [ss_parts_max][ss_stride] fp32 followed by one int32
@@ -226,9 +226,9 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a,
           fence_proxy_async_global();
           if (*abort_word) goto done;
         }
-        // plain: this CTA's 128 of the tile's 256 W rows.  SwiGLU: the leader stages the 128
-        // gate rows, the peer the matching 128 up rows.
-        const int w_row = p.swiglu ? tn * 128 + (int)rank * p.up_row_offset
+        // plain: this CTA's half of the tile's W rows.  SwiGLU: the leader stages the gate rows,
+        // the peer the matching up rows.
+        const int w_row = p.swiglu ? tn * (p.bn >> 1) + (int)rank * p.up_row_offset
                                    : tn * p.bn + (int)rank * (p.bn >> 1);
         // Few row tiles (decode batches): every weight byte is read from DRAM once and nothing else
         // hides that latency but the depth of the stage ring, so the boxes of later k-blocks are
@@ -297,7 +297,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a,
   } else {
     // ------------------------------------------------------------ epilogue (both CTAs)
     const int q = warp & 3;
-    const int out_per_tile = p.swiglu ? 128 : p.bn;
+    const int out_per_tile = p.swiglu ? p.bn >> 1 : p.bn;
     uint8_t* rs_stage = smem + G2_STAGES * G2_STAGE_BYTES + 256 + q * (32 * G2_RS_ROW_BYTES);
     int it = 0;
     for (int t = cluster_id; t < num_tiles; t += num_clusters, it++) {
@@ -339,7 +339,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a,
         tmem_ld_32x32b_x32(t_row + c0, r);
         if (p.swiglu) {
           uint32_t u[32];
-          tmem_ld_32x32b_x32(t_row + 128 + c0, u);
+          tmem_ld_32x32b_x32(t_row + (p.bn >> 1) + c0, u);
           tmem_ld_wait();
           if (p.glu_alpha > 0.f) {
 #pragma unroll
@@ -531,29 +531,30 @@ static int launch_2cta(const void* A, const void* W, Gemm2Params& p, int lda, in
   }
   const int max_clusters = num_sms() / 2;
   p.tiles_m = (p.M + G2_BM - 1) / G2_BM;
-  // Tile width.  256 columns make the best use of the tensor cores, but whole waves of tiles
-  // over the CTA pairs matter more when there are only a few tiles: a decode batch of 768 rows
-  // against N = 4096 is 48 tiles of 256 columns on 74 pairs (35% of the GPU idle), or 66 tiles
-  // of 192 columns in the same single wave.  Cost model: waves x tile width; a narrower tile
-  // must win by 8% to be taken.  M = 768, N = 4096 ends at 176 columns: 72 tiles on 74 pairs.
-  const int bn_step = (p.mode & G2_RS) ? 32 : 16;
-  if (p.swiglu) {
-    p.bn = G2_BN;
-  } else if (g_force_bn >= 128 && g_force_bn <= 256 && (g_force_bn % bn_step) == 0) {
+  // Tile width: waves of tiles over the CTA pairs, times what a tile takes.  That is about bn + 45 (its loads and MMAs, and what
+  // issuing them costs), and no less below 144 columns, where issue is all of it.  us at widths 256 / 240 / 224 / 192 / 176 / 160 / 128:
+  //   4096 x 4096 x 12288   345  323  375  332  369  350  382        6000 x 2048 x 6144   120  114  139  124  118  134  157
+  //   4096 x 1536 x 4096     61   58   55   47   45   57   55        4000 x 5120 x 2048    80   75   71   75   82   79   91
+  //   768 x 4096 x 12288     84   80   76   68   64  108  101
+  // One tile of rows: the weights are streamed once, and what counts is how many pairs stream them; down to 64 columns, or the pairs
+  // without a tile idle while the others stream all of them (256 x 6144 x 4096: 24 tiles of 256 columns 31 us, 48 of 128 23).  The row
+  // statistics have a part per 128 columns at least.  With a gate a tile holds bn / 2 columns of each half.
+  const int bn_step = (p.mode & G2_RS) || p.swiglu ? 32 : 16;
+  const long cols = p.swiglu ? 2L * p.N : p.N;
+  if (!p.swiglu && g_force_bn >= 128 && g_force_bn <= 256 && (g_force_bn % bn_step) == 0) {
     p.bn = g_force_bn;
   } else {
+    const bool streams = p.tiles_m == 1 && p.mode == 0;
     auto cost = [&](int bn) {
-      const long tiles = (long)p.tiles_m * ((p.N + bn - 1) / bn);
-      return ((tiles + max_clusters - 1) / max_clusters) * bn;
+      const long tiles = (long)p.tiles_m * ((cols + bn - 1) / bn);
+      return ((tiles + max_clusters - 1) / max_clusters) * (streams ? bn : (bn > 144 ? bn : 144) + 45);
     };
     p.bn = G2_BN;
     long best = cost(G2_BN);
-    // one tile of rows: down to 64 columns, or the pairs without a tile idle while the others stream all of the weights
-    // (256 x 6144 x 4096: 24 tiles of 256 columns 34 us); the row statistics have a part per 128 columns at least
-    const int bn_min = p.tiles_m == 1 && !p.row_ss_out && p.mode == 0 ? 64 : 128;
+    const int bn_min = streams && !p.row_ss_out && !p.swiglu ? 64 : 128;
     for (int bn = G2_BN - bn_step; bn >= bn_min; bn -= bn_step) {
       const long c = cost(bn);
-      if (c * 100 < best * 92) {
+      if (c * 100 < best * (streams ? 92 : 98)) {
         best = c;
         p.bn = bn;
       }
@@ -563,10 +564,10 @@ static int launch_2cta(const void* A, const void* W, Gemm2Params& p, int lda, in
   int rc = get_tmap_128x64(&ta, A, (uint64_t)a_rows, (uint64_t)p.K, (uint64_t)lda);
   if (rc) return rc;
   rc = get_tmap_128x64(&tb, W, (uint64_t)(p.swiglu ? 2L * p.N : p.N), (uint64_t)p.K, (uint64_t)ldw,
-                       p.swiglu ? 128u : (uint32_t)(p.bn >> 1));
+                       (uint32_t)(p.bn >> 1));
   if (rc) return rc;
   p.up_row_offset = p.N;
-  const int out_per_tile = p.swiglu ? 128 : p.bn;
+  const int out_per_tile = p.swiglu ? p.bn >> 1 : p.bn;
   p.tiles_n = (p.N + out_per_tile - 1) / out_per_tile;
   int clusters = p.tiles_m * p.tiles_n;
   if (clusters > max_clusters) clusters = max_clusters;
