@@ -10,16 +10,18 @@
 //
 // What does not need S0 is done for all chunks at once: T = (I + A)^-1 and P T, P the matrix of the read-outs, are 64 x 64 triangles
 // per chunk and head (delta_prep_kernel, fp32 on CUDA cores).  What is left of a chunk is a chain of three products,
-//     [K; Q] S0   ->   r   ->   [T; P T] r = [u; o - read-out of S0]   ->   S = e^{gamma_C} S0 + K^T u
+//     [K; Q] S0   ->   r   ->   [T - 1; P T] r = [u - r; o - read-out of S0]   ->   S = e^{gamma_C} S0 + K^T u
 // with rows turned into operands in between (delta_chain_kernel).  A block has one sequence, one head and 64 value columns, and two blocks
 // fit an SM.  Bound: the chain, chunk after chunk of a sequence: 8,100 clocks a chunk, 10,200 with a second block on the SM, of which the
 // three products are 3,400 (60 MMAs of 64 columns: 55 clocks each, 40 with an operand in tensor memory).  Preparing takes 0.047 us a chunk and
-// head, three blocks on an SM, issue and shared-memory latency.  6000 tokens in three prompts, 32 heads, us: both together 333 (chain 180,
+// head, three blocks on an SM, issue and shared-memory latency.  6000 tokens in three prompts, 32 heads, us: both together 350 (chain 200,
 // preparation 150); the solve, the state's products and their conversions one after the other in one block per head 785; token by token 1603.
 //
 // 32 bits stay 32 bits.  q and k are bf16 as they come, so k . k and q . k are exact products summed in fp32; their norms
 // are factors of rows.  The state, u, r and T are fp32: as MMA operands they are three bf16 parts (8 + 8 + 8 bits), which times an exact
-// bf16 operand is the fp32 product, and of two such operands the six products above 2^-24.  gamma is summed in fp64 and kept in two floats.
+// bf16 operand is the fp32 product, and of two such operands the six products above 2^-24.  T's diagonal of ones stays out of that product, and
+// r is added by itself: the tensor cores' sums truncate, which with the diagonal made the state's error 1.2 times that of a solve in fp32
+// where decays are strong.  gamma is summed in fp64 and kept in two floats.
 //
 // A matrix product would carry a NaN or infinity of r to earlier tokens (zero times NaN).  A chunk whose r has one takes that product
 // row by row on CUDA cores, without the zeros.
@@ -74,15 +76,16 @@ __device__ __forceinline__ long dc_place(const DeltaChunkArgs& p, int b, int c, 
   return p.per_seq ? (long)b * p.per_seq + (c - p.c0) : (long)(t0 / DC_C + b) + c;
 }
 
-// A pair of fp32 values as three pairs of bf16 that sum to it: what a truncation leaves of 24 bits fits the next parts.  Full-rate
-// instructions, where rounding conversions are not.
+// A pair of fp32 values as three pairs of bf16 that sum to it: the parts are rounded (half up) by integer additions, which are full-rate
+// where conversions are not, and what is left of 24 bits after two of them fits the third.  A NaN is one in the last part.
 __device__ __forceinline__ void dc_split2(float a, float b, uint32_t* part) {
-  part[0] = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
-  a -= __uint_as_float(__float_as_uint(a) & 0xffff0000u);
-  b -= __uint_as_float(__float_as_uint(b) & 0xffff0000u);
-  part[1] = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
-  a -= __uint_as_float(__float_as_uint(a) & 0xffff0000u);
-  b -= __uint_as_float(__float_as_uint(b) & 0xffff0000u);
+#pragma unroll
+  for (int p = 0; p < 2; p++) {
+    const uint32_t u = __float_as_uint(a) + 0x8000u, v = __float_as_uint(b) + 0x8000u;
+    part[p] = __byte_perm(u, v, 0x7632);
+    a -= __uint_as_float(u & 0xffff0000u);
+    b -= __uint_as_float(v & 0xffff0000u);
+  }
   part[2] = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
 }
 // eight fp32 values as three rows of eight bf16, part p at dst + p * stride
@@ -368,10 +371,16 @@ __global__ void __launch_bounds__(DC_THREADS, 3) delta_prep_kernel(const DeltaCh
     if (tid < 128) store_vec<float, 4>(us + ((tid >> 6) * 32 + ((tid >> 2) & 15)) * UP + (tid >> 6) * 32 + 16 + (tid & 3) * 4, zero);
   }
   __syncthreads();
-  // ---- T and the factors of rows
+  // ---- T without its diagonal of ones, and the factors of rows
   for (int e = tid; e < DC_C * 16; e += DC_THREADS) {
     const int g = e >> 6, j = e & 63;
-    if (g >> 2 <= j >> 4) *reinterpret_cast<float4*>(ws + dc_tri(g, j)) = *reinterpret_cast<const float4*>(us + j * UP + 4 * g);
+    if (g >> 2 <= j >> 4) {
+      float x[4];
+      load_vec<float, 4>(us + j * UP + 4 * g, x);
+#pragma unroll
+      for (int i = 0; i < 4; i++) if (4 * g + i == j) x[i] = 0.f;
+      store_vec<float, 4>(ws + dc_tri(g, j), x);
+    }
   }
   const float2 ge = sc->gam[DC_C - 1], zero2 = make_float2(0.f, 0.f);
   if (tid < DC_C) {
@@ -608,14 +617,17 @@ __global__ void __launch_bounds__(DC_CHAIN_THREADS, 2) delta_chain_kernel(const 
     tc_fence_after();
     // ---- r = beta (v - e^gamma S0^T k) -> parts, its accumulator cleared; e^gamma S0^T q stays in the accumulator
     int odd = 0;
+    float x[32];                                           // r, then u (0, then o)
     {
       uint32_t d[32];
       tmem_ld_32x32b_x32(t_lane + Cfg::D_COL + col0, d);
       tmem_ld_wait();
-      float x[32];
       if (is_q) {
 #pragma unroll
-        for (int i = 0; i < 32; i++) d[i] = __float_as_uint(__uint_as_float(d[i]) * fac.y);
+        for (int i = 0; i < 32; i++) {
+          d[i] = __float_as_uint(__uint_as_float(d[i]) * fac.y);
+          x[i] = 0.f;
+        }
       } else {
 #pragma unroll
         for (int i = 0; i < 4; i++) {
@@ -655,16 +667,20 @@ __global__ void __launch_bounds__(DC_CHAIN_THREADS, 2) delta_chain_kernel(const 
       tmem_st_32x32b_x32(t_lane + Cfg::S_COL + col0, s);
     }
     tmem_st_wait();
-    float x[32];
     if (!odd) {
       mbar_wait(&bars[1], ph_r, abort_word);
       ph_r ^= 1;
       tc_fence_after();
-      tmem_ld_32x32b_x32(t_lane + Cfg::D_COL + col0, reinterpret_cast<uint32_t*>(x));
+    }
+#pragma unroll
+    for (int h = 0; h < 32; h += 16) {
+      uint32_t d[16];
+      tmem_ld_32x32b_x16(t_lane + Cfg::D_COL + col0 + h, d);
       tmem_ld_wait();
-    } else {
-      tmem_ld_32x32b_x32(t_lane + Cfg::D_COL + col0, reinterpret_cast<uint32_t*>(x));
-      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 16; i++) x[h + i] += __uint_as_float(d[i]);
+    }
+    if (odd) {
 #pragma unroll 1
       for (int m = 0; m <= j; m++) {
         const float a = tri[dc_tri(m >> 2, j) + (m & 3)];

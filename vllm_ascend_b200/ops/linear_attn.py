@@ -204,7 +204,7 @@ def gated_delta_rule_chunked(q, k, v, g, beta, state, cu_cpu, slots, has_init, s
 def _chunk_min(on_cuda: bool = False) -> int:
     """Fewest new tokens of a sequence that take the chunk-parallel form built from fp32 matrix products; 0 = never.
     Unset, the form serves host tensors only: on a B200 it takes 10.3 ms for 4 x 2048 tokens of 32 heads, the kernels 1.3 ms token
-    by token (three prompts of 2000 tokens: 1.6 ms, and 0.33 ms in chunks: ``_portions``)."""
+    by token (three prompts of 2000 tokens: 1.6 ms, and 0.35 ms in chunks: ``_portions``)."""
     from .. import envs
     if "VLLM_B200_GDN_CHUNK_MIN" not in os.environ and on_cuda:
         return 0
@@ -218,7 +218,7 @@ def _kernel_times(lens: np.ndarray, Hv: int, DV: int, sms: int, least: int) -> f
     per chunk, full or not (4.4 us alone on their SM).  A block of the token-serial kernel, of which three share an SM, takes 0.42 us per token
     alone and 0.79 us among others.  Blocks run in waves, or packed one behind the other where they differ, whichever is shorter.  32 heads,
     token by token and in chunks: 16 portions of 32 tokens 75 and 77 us (estimates 89 and 76), 12 of 64 117 and 65 (116 and 66), 64 of 65 517 and 415
-    (563 and 470), one of 128 60 and 30 (68 and 28), three of 2000 - and 333 (- and 332)."""
+    (563 and 470), one of 128 60 and 30 (68 and 28), three of 2000 - and 350 (- and 332)."""
     def packed(each, blocks, slots):
         n = len(each) * blocks
         longest = float(each.max())
