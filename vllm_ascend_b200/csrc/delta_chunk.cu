@@ -48,7 +48,7 @@ struct DcPrepSmem {
 static_assert(3 * (DcPrepSmem::BYTES + 1024) <= 228 * 1024, "three blocks per SM");
 struct DcChainSmem {
   static constexpr int S_PART = DC_K * 128, R_PART = DC_C * 128;     // bytes of one bf16 part of S, of r and u
-  static constexpr int KQ_BYTES = 32768;                             // K and Q of a chunk, of two chunks; Q's place holds the next chunk's v
+  static constexpr int KQ_BYTES = 32768;                             // K and Q of a chunk, of two chunks; Q's place holds the next chunk's v and outputs
   static constexpr int S_OFF = 2 * KQ_BYTES;                         // parts of S; from product to product of r, then of u
   static constexpr int SC_OFF = S_OFF + 3 * S_PART;
   static constexpr int BYTES = SC_OFF + 64;
@@ -446,7 +446,6 @@ __global__ void __launch_bounds__(DC_CHAIN_THREADS, 2) delta_chain_kernel(const 
   uint8_t* smem = dc_smem;
   uint8_t* s_parts = smem + Cfg::S_OFF;
   uint8_t* r_parts = s_parts;
-  uint8_t* o_tile = s_parts + 3 * Cfg::R_PART;             // a chunk's outputs, on their way to whole rows
   uint64_t* bars = (uint64_t*)(smem + Cfg::SC_OFF);        // [K; Q] S0, [T; P T] r, K^T u
   uint32_t* tmem_ptr = (uint32_t*)(bars + 3);
   volatile int* abort_word = (volatile int*)(tmem_ptr + 1);
@@ -584,6 +583,9 @@ __global__ void __launch_bounds__(DC_CHAIN_THREADS, 2) delta_chain_kernel(const 
   uint32_t ph = 0, ph_r = 0;
   for (int c = p.c0; c < c_end; c++, ph ^= 1) {
     const int tc = t0 + c * DC_C;
+    // the chunk's outputs, on their way to whole rows: the half of Q's place that v leaves, free until Q of the chunk after the next.  (Not
+    // beside u: a thread ahead of others writes parts of S there.)
+    uint8_t* o_tile = smem + ((c - p.c0) & 1) * Cfg::KQ_BYTES + 24576;
     const float* ws = p.ws + (dc_place(p, b, c, t0) * p.Hv + hv) * DC_WS;
     asm volatile("cp.async.wait_all;" ::: "memory");
     fence_proxy_async_smem();
