@@ -157,16 +157,25 @@ __global__ void penalties_kernel(float* logits, long ld, int V, const long* prom
 //   * bins are integers (mass in units of 2^-40: shared memory adds 64-bit integers by itself, floats in a loop, and the
 //     sum has no order), added and searched in parallel;
 //   * where the cut leaves at most 2048 elements (top-k, peaked top-p), one block sorts them and ends the row by itself;
+//   * rows with a small top-k need neither exponentials nor cuts of the whole row: the k-th largest of the threads' own maxima is a
+//     bound that k elements of the block's slice reach, so no smaller one is among the row's k largest.  What reaches it, little more than
+//     k a block, is all that the rest looks at;
+//   * a slice comes in by bulk copies, all of it in flight at once;
 //   * random numbers are drawn only for groups of four that hold a kept element;
 //   * what the other blocks of the cluster say is read once per block: read by every thread, 192 x 32000 without top-k and top-p
 //     took 115 us of which 88 reads per thread were most, 56 us so (37 us with two blocks a row, 66 us one block with the row in L2).
-// 192 rows of 151936, top-k 50: one block per row with thread-serial bins 849 us, 131 us so.
+//   * top-p without top-k: one histogram of fine bins between the cut and the maximum, and the elements of the bin in question to rank 0.
+// 192 rows of 151936, cold, us: greedy 44 (58 with plain loads), top-k 50 78 (135 with exponentials and cuts of the whole row, 849 with one block
+// per row and thread-serial bins), top-p 0.8 144 (172), 0.95 at temperature 0.8 233 (278) and 1 272 (366; three digits and remote additions
+// per warp), nothing cut 122 (135).
 constexpr int SAMP_T = 512;
 constexpr int SAMP_BINS = 2048;
 constexpr int SAMP_MAX_SLICE = 50 * 1024;        // elements of a row that a block keeps in shared memory
 constexpr int SAMP_PAIR_SLICE = 23000;           // ... while an SM holds two such blocks
 constexpr int SAMP_TWO_HIST_SLICE = 47000;       // ... beside a second histogram (256 flat rows of 262144, top-p: 4294 -> 2960 us)
 constexpr int SAMP_CUTS = 5;
+constexpr int SAMP_SMALL_K = 1024;               // blocks of a row (four or more) times k, up to which top-k takes what threads' maxima bound
+constexpr int SAMP_BULK = 4;                     // bulk copies of a slice
 using samp_n = unsigned long long;     // elements, or mass in units of 2^-40 (e <= 1, so a row's mass fits)
 constexpr float SAMP_UNIT = 1099511627776.f;
 
@@ -176,7 +185,8 @@ struct SampXch { float v[1 + SAMP_CUTS]; uint32_t n[SAMP_CUTS]; int i; };
 template <int C, int K>
 struct SampSmem {
   samp_n hist[K * SAMP_BINS];
-  samp_n own[C > 1 ? SAMP_BINS / C : 1];       // this block's bins, summed over the cluster
+  static constexpr int OWN = C > 1 ? SAMP_BINS / C : 512;
+  samp_n own[OWN];                     // this block's bins, summed over the cluster; top-k: its candidates (logit, index)
   samp_n tot[6];                       // sum of `own`, one slot per select pass
   samp_n remaining;
   SampXch xch[4];                      // what a block tells the others: one slot per meeting
@@ -185,8 +195,11 @@ struct SampSmem {
   float sv[32];
   int si[32];
   samp_n sn[SAMP_T / 32];
+  uint64_t bar[SAMP_BULK];
   uint32_t prefix;
   uint32_t listed;                     // candidates in hist (rank 0)
+  uint32_t found, odd;                 // top-k: candidates in `own`, whether one is a NaN
+  int abort;
 };
 
 template <int C>
@@ -230,16 +243,24 @@ __device__ __forceinline__ samp_n samp_warp_sum(samp_n v) {
 __device__ __forceinline__ void samp_better(float& v, int& i, float ov, int oi) {
   if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
 }
-// argmax over the cluster, lowest index on ties
+// argmax over the cluster, lowest index on ties; `found`: all blocks' numbers of candidates (SAMP_NONE: one has none to offer), in
+// all[slot].n[0] the sum and in n[1] what blocks before this one have
+constexpr uint32_t SAMP_NONE = 1u << 20;
 template <int C, int K>
-__device__ void samp_cluster_argmax(float& v, int& idx, SampSmem<C, K>* s, int slot) {
+__device__ void samp_cluster_argmax(float& v, int& idx, SampSmem<C, K>* s, int slot, uint32_t found = 0, int rank = 0) {
   block_argmax(v, idx, s->sv, s->si);
-  if constexpr (C > 1) {
-    if (threadIdx.x == 0) { s->xch[slot].v[0] = v; s->xch[slot].i = idx; }
+  if constexpr (C == 1) {
+    if (threadIdx.x == 0) { s->all[slot].n[0] = found; s->all[slot].n[1] = 0; }
+    __syncthreads();
+  } else {
+    if (threadIdx.x == 0) { s->xch[slot].v[0] = v; s->xch[slot].i = idx; s->xch[slot].n[0] = found; }
     samp_meet<C>();
     if (threadIdx.x < 32) {
       v = samp_peek<C>(&s->xch[slot].v[0], threadIdx.x % C);
       idx = samp_peek<C>(&s->xch[slot].i, threadIdx.x % C);
+      const uint32_t f = threadIdx.x < C ? samp_peek<C>(&s->xch[slot].n[0], threadIdx.x) : 0;
+      const uint32_t sum = __reduce_add_sync(0xffffffffu, f), before = __reduce_add_sync(0xffffffffu, (int)threadIdx.x < rank ? f : 0);
+      if (threadIdx.x == 0) { s->all[slot].n[0] = sum; s->all[slot].n[1] = before; }
 #pragma unroll
       for (int o = C / 2; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, v, o);
@@ -254,11 +275,12 @@ __device__ void samp_cluster_argmax(float& v, int& idx, SampSmem<C, K>* s, int s
   }
 }
 
-// One digit of the select: histogram (elements or their mass) of the `bits`-wide digit at `shift` over the elements whose
-// higher bits equal the prefix and whose key reaches floor_key, then the bin, walking down from the top, at which the
+// One digit of the select: histogram (elements or their mass) of the `bits`-wide digit at `shift` of the key less `base` over the
+// elements whose higher bits equal the prefix and whose key reaches floor_key, then the bin, walking down from the top, at which the
 // running sum reaches `remaining`.  Every block of the cluster ends with the same prefix and remaining.
 template <bool MASS, int C, int K>
-__device__ void samp_pass(const float* e, int n, SampSmem<C, K>* s, int pass, int shift, int bits, uint32_t hi_mask, uint32_t floor_key, int rank) {
+__device__ void samp_pass(const float* e, int n, SampSmem<C, K>* s, int pass, int shift, int bits, uint32_t hi_mask, uint32_t floor_key, int rank,
+                          uint32_t base = 0) {
   const int nb = 1 << bits;
   for (int i = threadIdx.x; i < K * nb; i += SAMP_T) s->hist[i] = 0;
   samp_n* hist = s->hist + (threadIdx.x & (K - 1)) * nb;
@@ -269,7 +291,7 @@ __device__ void samp_pass(const float* e, int n, SampSmem<C, K>* s, int pass, in
     const float v = e[i];
     const uint32_t k = __float_as_uint(v);
     if (k < floor_key || (k & hi_mask) != prefix) continue;
-    atomicAdd(&hist[(k >> shift) & (nb - 1)], MASS ? __float2ull_rn(v * SAMP_UNIT) : 1ull);
+    atomicAdd(&hist[((k - base) >> shift) & (nb - 1)], MASS ? __float2ull_rn(v * SAMP_UNIT) : 1ull);
   }
   samp_meet<C>();
   if constexpr (C == 1) {
@@ -371,33 +393,62 @@ __device__ void samp_pass(const float* e, int n, SampSmem<C, K>* s, int pass, in
   __syncthreads();
 }
 
-// Elements above the cut, gathered from the whole cluster into rank 0's `hist` as (key, inverted index): value descending, index
-// ascending is then one 64-bit order.
+// Elements above the cut (and no higher than `top`), gathered from the whole cluster into rank 0's `hist` as (key, inverted index): value
+// descending, index ascending is then one 64-bit order.  A block counts before it writes, so that it asks rank 0 for room once: with a
+// remote addition per warp and hit, 2000 candidates of a row took 10 us, one after the other.
 template <int C, int K>
-__device__ void samp_gather(const float* e, int n, int first, uint32_t cut, SampSmem<C, K>* s) {
+__device__ void samp_gather(const float* e, int n, int first, uint32_t cut, SampSmem<C, K>* s, uint32_t top = 0xffffffffu) {
   uint32_t list, count;
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(list) : "r"(smem_u32(s->hist)));
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(count) : "r"(smem_u32(&s->listed)));
-  const int lane = threadIdx.x & 31;
-  for (int i0 = threadIdx.x - lane; i0 < n; i0 += SAMP_T) {
-    const int i = i0 + lane;
-    const uint32_t k = i < n ? __float_as_uint(e[i]) : 0;
-    const uint32_t on = __ballot_sync(0xffffffffu, i < n && k >= cut);
-    if (on == 0) continue;
-    uint32_t at = 0;
-    if (lane == 0) asm volatile("atom.relaxed.cluster.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(at) : "r"(count), "r"(__popc(on)) : "memory");
-    at = __shfl_sync(0xffffffffu, at, 0) + __popc(on & ((1u << lane) - 1));
-    if ((on >> lane & 1) && at < SAMP_BINS) {
-      const samp_n v = (samp_n)k << 32 | (uint32_t)~(first + i);
-      asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(list + at * 8), "l"(v) : "memory");
+  const bool whole = (reinterpret_cast<uintptr_t>(e) & 15) == 0;
+  const int nv = whole ? n >> 2 : 0, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto in = [&](float v) { const uint32_t k = __float_as_uint(v); return k >= cut && k <= top; };
+  auto each = [&](auto f) {
+    for (int c = threadIdx.x; c < nv; c += SAMP_T) {
+      const float4 q = reinterpret_cast<const float4*>(e)[c];
+      if (in(q.x)) f(q.x, 4 * c);
+      if (in(q.y)) f(q.y, 4 * c + 1);
+      if (in(q.z)) f(q.z, 4 * c + 2);
+      if (in(q.w)) f(q.w, 4 * c + 3);
     }
+    for (int i = 4 * nv + threadIdx.x; i < n; i += SAMP_T)
+      if (in(e[i])) f(e[i], i);
+  };
+  uint32_t mine = 0;
+  each([&](float, int) { mine++; });
+  uint32_t upto = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, upto, o);
+    if (lane >= o) upto += t;
   }
+  __syncthreads();
+  if (lane == 31) s->sn[warp] = upto;
+  __syncthreads();
+  uint32_t before = 0, all = 0;
+  for (int w = 0; w < SAMP_T / 32; w++) {
+    if (w < warp) before += (uint32_t)s->sn[w];
+    all += (uint32_t)s->sn[w];
+  }
+  if (threadIdx.x == 0) {
+    uint32_t at = 0;
+    if (all) asm volatile("atom.relaxed.cluster.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(at) : "r"(count), "r"(all) : "memory");
+    s->found = at;
+  }
+  __syncthreads();
+  uint32_t at = s->found + before + upto - mine;
+  if (mine)
+    each([&](float v, int i) {
+      const samp_n w = (samp_n)__float_as_uint(v) << 32 | (uint32_t)~(first + i);
+      if (at < SAMP_BINS) asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(list + at * 8), "l"(w) : "memory");
+      at++;
+    });
 }
 
-// Rank 0 alone: orders the n gathered candidates, cuts them by rank and by mass, and runs the race.  `mass` is what top-p is a
-// share of where top-k is off.
+// Rank 0 alone: the n gathered candidates in descending order
 template <int C, int K>
-__device__ int samp_finish(SampSmem<C, K>* s, int n, int k, float pth, float mp, float mass, uint2 key, long offset, int fallback) {
+__device__ void samp_sort(SampSmem<C, K>* s, int n) {
   samp_n* c = s->hist;
   int size = 32;
   while (size < n) size *= 2;
@@ -412,41 +463,59 @@ __device__ int samp_finish(SampSmem<C, K>* s, int n, int k, float pth, float mp,
       }
       __syncthreads();
     }
+}
+// Rank 0 alone: running mass over the n sorted candidates that reach thr, in units of 2^-40 (a thread sums its run of neighbours, then
+// their sums are scanned); s->prefix becomes the value of the first at which it reaches want(total).  Returns want.
+template <int C, int K, typename F>
+__device__ samp_n samp_reach(SampSmem<C, K>* s, int n, uint32_t thr, F want_of) {
+  const samp_n* c = s->hist;
+  auto value = [&](int i) { return (uint32_t)(c[i] >> 32); };
+  constexpr int PER = SAMP_BINS / SAMP_T;
+  samp_n run[PER], sum = 0;
+#pragma unroll
+  for (int j = 0; j < PER; j++) {
+    const int i = threadIdx.x * PER + j;
+    if (i < n && value(i) >= thr) sum += __float2ull_rn(__uint_as_float(value(i)) * SAMP_UNIT);
+    run[j] = sum;
+  }
+  samp_n upto = sum;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const samp_n t = __shfl_up_sync(0xffffffffu, upto, o);
+    if (lane >= o) upto += t;
+  }
+  if (lane == 31) s->sn[warp] = upto;
+  if (threadIdx.x == 0) s->prefix = 0;
+  __syncthreads();
+  samp_n before = upto - sum, all = 0;
+  for (int w = 0; w < SAMP_T / 32; w++) {
+    if (w < warp) before += s->sn[w];
+    all += s->sn[w];
+  }
+  const samp_n want = want_of(all);
+#pragma unroll
+  for (int j = 0; j < PER; j++) {                        // the first element at which the sum reaches what is wanted
+    const int i = threadIdx.x * PER + j;
+    const samp_n prev = before + (j ? run[j - 1] : 0);
+    if (i < n && before + run[j] >= want && (prev < want || i == 0)) s->prefix = value(i);
+  }
+  __syncthreads();
+  return want;
+}
+
+// Rank 0 alone: orders the n gathered candidates, cuts them by rank and by mass, and runs the race.  `mass` is what top-p is a
+// share of where top-k is off.
+template <int C, int K>
+__device__ int samp_finish(SampSmem<C, K>* s, int n, int k, float pth, float mp, float mass, uint2 key, long offset, int fallback) {
+  samp_n* c = s->hist;
+  samp_sort(s, n);
   auto value = [&](int i) { return (uint32_t)(c[i] >> 32); };
   uint32_t thr = k > 0 ? value(k - 1) : 0;
   if (pth < 1.f && value(0) <= 0x7F800000u) {              // a row with a NaN has no mass to take a share of
-    // running mass in units of 2^-40: a thread sums its run of neighbours, then their sums are scanned
-    constexpr int PER = SAMP_BINS / SAMP_T;
-    samp_n run[PER], sum = 0;
-#pragma unroll
-    for (int j = 0; j < PER; j++) {
-      const int i = threadIdx.x * PER + j;
-      if (i < n && value(i) >= thr) sum += __float2ull_rn(__uint_as_float(value(i)) * SAMP_UNIT);
-      run[j] = sum;
-    }
-    samp_n upto = sum;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const samp_n t = __shfl_up_sync(0xffffffffu, upto, o);
-      if (lane >= o) upto += t;
-    }
-    if (lane == 31) s->sn[warp] = upto;
-    if (threadIdx.x == 0) s->prefix = 0;
-    __syncthreads();
-    samp_n before = upto - sum, all = 0;
-    for (int w = 0; w < SAMP_T / 32; w++) {
-      if (w < warp) before += s->sn[w];
-      all += s->sn[w];
-    }
-    const samp_n want = __float2ull_rn(pth * (k > 0 ? (float)all / SAMP_UNIT : mass) * SAMP_UNIT);
-#pragma unroll
-    for (int j = 0; j < PER; j++) {                        // the first element at which the sum reaches what is wanted
-      const int i = threadIdx.x * PER + j;
-      const samp_n prev = before + (j ? run[j - 1] : 0);
-      if (i < n && before + run[j] >= want && (prev < want || i == 0)) s->prefix = value(i);
-    }
-    __syncthreads();
+    const samp_n want = samp_reach(s, n, thr, [&](samp_n all) {
+      return __float2ull_rn(pth * (k > 0 ? (float)all / SAMP_UNIT : mass) * SAMP_UNIT);
+    });
     if (want == 0) thr = 0xffffffffu;                      // a share of nothing: the largest element
     else if (s->prefix > thr) thr = s->prefix;
   }
@@ -491,16 +560,46 @@ sample_kernel(float* logits, long ld, int V, int slice, int resident, const floa
   int bi = 0x7fffffff;
   const bool keep = resident && !greedy;
   int done = 0;
+  auto look = [&](const float4& q, int c) {
+    if (q.x > best) { best = q.x; bi = first + 4 * c; }
+    if (q.y > best) { best = q.y; bi = first + 4 * c + 1; }
+    if (q.z > best) { best = q.z; bi = first + 4 * c + 2; }
+    if (q.w > best) { best = q.w; bi = first + 4 * c + 3; }
+  };
+  if (threadIdx.x == 0) { s.listed = 0; s.found = 0; s.odd = 0; s.abort = 0; }
   if ((reinterpret_cast<uintptr_t>(row) & 15) == 0) {
     const int nv = n >> 2;
+    bool here = false;                   // the slice is in shared memory
+    if (resident) {
+      if (threadIdx.x == 0) {
+        for (int i = 0; i < SAMP_BULK; i++) mbar_init(&s.bar[i], 1);
+        mbar_fence_init();
+        for (int i = 0; i < SAMP_BULK; i++) {
+          const int c0 = nv * i / SAMP_BULK, bytes = (nv * (i + 1) / SAMP_BULK - c0) * 16;
+          mbar_expect_tx(&s.bar[i], bytes);
+          if (bytes)
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                             smem_u32(e + 4 * c0)), "l"(row + 4 * c0), "r"(bytes), "r"(smem_u32(&s.bar[i])) : "memory");
+        }
+      }
+      __syncthreads();
+      here = true;
+      for (int i = 0; i < SAMP_BULK && here; i++) {
+        here = mbar_wait(&s.bar[i], 0, &s.abort);
+        const int c1 = nv * (i + 1) / SAMP_BULK;
+        if (here)
 #pragma unroll 4
-    for (int c = threadIdx.x; c < nv; c += SAMP_T) {
-      const float4 q = reinterpret_cast<const float4*>(row)[c];
-      if (keep) reinterpret_cast<float4*>(e)[c] = q;
-      if (q.x > best) { best = q.x; bi = first + 4 * c; }
-      if (q.y > best) { best = q.y; bi = first + 4 * c + 1; }
-      if (q.z > best) { best = q.z; bi = first + 4 * c + 2; }
-      if (q.w > best) { best = q.w; bi = first + 4 * c + 3; }
+          for (int c = nv * i / SAMP_BULK + threadIdx.x; c < c1; c += SAMP_T) look(reinterpret_cast<const float4*>(e)[c], c);
+      }
+      here = __syncthreads_and(here);
+    }
+    if (!here) {                         // not resident, or a copy that did not arrive
+#pragma unroll 4
+      for (int c = threadIdx.x; c < nv; c += SAMP_T) {
+        const float4 q = reinterpret_cast<const float4*>(row)[c];
+        if (keep) reinterpret_cast<float4*>(e)[c] = q;
+        look(q, c);
+      }
     }
     done = 4 * nv;
   }
@@ -510,16 +609,61 @@ sample_kernel(float* logits, long ld, int V, int slice, int resident, const floa
     if (keep) e[i] = v;
     if (v > best) { best = v; bi = first + i; }
   }
-  if (threadIdx.x == 0) s.listed = 0;
-  samp_cluster_argmax(best, bi, &s, 0);
+  // ---- a small top-k: what reaches the k-th largest of the threads' maxima (its upper sixteen bits, in an order of integers)
+  uint32_t found = SAMP_NONE;
+  if (by_rank && keep && k <= SAMP_SMALL_K / (C > 4 ? C : 4)) {
+    uint32_t key = __float_as_uint(best);
+    key ^= (uint32_t)((int)key >> 31) | 0x80000000u;
+    uint32_t t = 0;
+#pragma unroll 1
+    for (int bit = 31; bit >= 16; bit--)
+      if (__syncthreads_count(key >= (t | 1u << bit)) >= k) t |= 1u << bit;
+    const float bound = __uint_as_float(t & 0x80000000u ? t ^ 0x80000000u : ~t);
+    auto offer = [&](float v, int i) {
+      if (v < bound) return;             // a NaN is offered, and told
+      if (v != v) s.odd = 1;
+      const uint32_t at = atomicAdd(&s.found, 1u);
+      if (at < s.OWN) s.own[at] = (samp_n)__float_as_uint(v) << 32 | (uint32_t)i;
+    };
+    for (int c = threadIdx.x; c < n >> 2; c += SAMP_T) {
+      const float4 q = reinterpret_cast<const float4*>(e)[c];
+      if (q.x < bound && q.y < bound && q.z < bound && q.w < bound) continue;
+      offer(q.x, 4 * c); offer(q.y, 4 * c + 1); offer(q.z, 4 * c + 2); offer(q.w, 4 * c + 3);
+    }
+    for (int i = (n & ~3) + threadIdx.x; i < n; i += SAMP_T) offer(e[i], i);
+    __syncthreads();
+    if (!s.odd && s.found <= s.OWN) found = s.found;
+  }
+  samp_cluster_argmax(best, bi, &s, 0, found, rank);
   if (greedy) {
     if (rank == 0 && threadIdx.x == 0) out[b] = bi;
     samp_meet<C>();                    // nobody leaves while another reads its memory
     return;
   }
+  const float invT = 1.f / temp;
+  const unsigned long long seed = seeds ? seeds[b] : 0ull;
+  const long offset = offsets ? offsets[b] : 0;
+  const uint2 key = make_uint2((uint32_t)seed, (uint32_t)(seed >> 32));
+  const uint32_t offered = s.all[0].n[0];
+  if (offered < SAMP_NONE && fabsf(best) < INFINITY) {               // every block has offered: the same in all of them
+    uint32_t list;
+    if constexpr (C > 1) asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(list) : "r"(smem_u32(s.hist)));
+    else list = smem_u32(s.hist);
+    list += s.all[0].n[1] * 8;
+    for (uint32_t i = threadIdx.x; i < found; i += SAMP_T) {
+      const float v = __uint_as_float((uint32_t)(s.own[i] >> 32));
+      const samp_n w = (samp_n)__float_as_uint(__expf((v - best) * invT)) << 32 | (uint32_t)~(first + (uint32_t)s.own[i]);
+      if constexpr (C > 1) asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(list + i * 8), "l"(w) : "memory");
+      else s.hist[i] = w;
+    }
+    samp_meet<C>();
+    if (rank != 0) return;
+    const int win = samp_finish(&s, (int)offered, k, pth, mp, 0.f, key, offset, bi);
+    if (threadIdx.x == 0) out[b] = win;
+    return;
+  }
   // ---- e = exp((x - max)/T); where something is cut by rank or mass, their sum and how much lies above each cut
   const uint32_t cuts[SAMP_CUTS] = {0x3C800000u, 0x3A800000u, 0x38800000u, 0x36800000u, 0x33800000u};   // 2^-6, -10, -14, -18, -24
-  const float invT = 1.f / temp;
   float z = 0.f, zc[SAMP_CUTS];
   uint32_t nc[SAMP_CUTS];
   if (by_rank || pth < 1.f) {
@@ -571,9 +715,6 @@ sample_kernel(float* logits, long ld, int V, int slice, int resident, const floa
   float mass = z;
   uint32_t thr_key = 0;                // keep elements with key >= thr_key
 
-  const unsigned long long seed = seeds ? seeds[b] : 0ull;
-  const long offset = offsets ? offsets[b] : 0;
-  const uint2 key = make_uint2((uint32_t)seed, (uint32_t)(seed >> 32));
   uint32_t cut = 0, above = 0;         // the highest cut that holds enough, and how many elements reach it
 #pragma unroll
   for (int j = SAMP_CUTS - 1; j >= 0; j--)
@@ -618,10 +759,44 @@ sample_kernel(float* logits, long ld, int V, int slice, int resident, const floa
     if (thr_key > cut) cut = thr_key;
     if (threadIdx.x == 0) { s.prefix = 0; s.remaining = __float2ull_rn(pth * mass * SAMP_UNIT); }
     __syncthreads();
-    samp_pass<true, C, K>(e, n, &s, 3, 21, 11, 0x00000000u, cut, rank);
-    samp_pass<true, C, K>(e, n, &s, 4, 10, 11, 0xFFE00000u, cut, rank);
-    samp_pass<true, C, K>(e, n, &s, 5, 0, 10, 0xFFFFFC00u, cut, rank);
-    if (s.prefix > thr_key) thr_key = s.prefix;
+    bool found_it = false;
+    if (cut != 0) {
+      // between the cut and the maximum there are few enough values for bins of 64 or more to a factor of two: the one in question
+      // holds so little that rank 0 sorts it
+      constexpr uint32_t ONE = 0x3F800000u;
+      int shift = 0;
+      while ((ONE - cut) >> shift >= SAMP_BINS) shift++;
+      samp_pass<true, C, K>(e, n, &s, 3, shift, 11, 0x00000000u, cut, rank, cut);
+      const uint32_t low = cut + s.prefix;
+      const samp_n rem = s.remaining;
+      samp_gather(e, n, first, low, &s, low + (1u << shift) - 1);      // over rank 0's bins, which nobody reads any more
+      samp_meet<C>();
+      if (threadIdx.x == 0) s.all[3].n[0] = samp_peek<C>(&s.listed, 0);
+      __syncthreads();
+      const int listed = (int)s.all[3].n[0];
+      if (listed > 0 && listed <= SAMP_BINS) {
+        if (rank == 0) {
+          samp_sort(&s, listed);
+          samp_reach(&s, listed, 0u, [&](samp_n) { return rem; });
+          // rounding can leave the bin's sum below what remains: its lowest element
+          if (threadIdx.x == 0 && s.prefix == 0) s.prefix = (uint32_t)(s.hist[listed - 1] >> 32);
+        }
+        samp_meet<C>();
+        if (threadIdx.x == 0) s.all[3].n[1] = samp_peek<C>(&s.prefix, 0);
+        __syncthreads();
+        if (s.all[3].n[1] > thr_key) thr_key = s.all[3].n[1];
+        found_it = true;
+      } else {
+        if (threadIdx.x == 0) { s.prefix = 0; s.remaining = __float2ull_rn(pth * mass * SAMP_UNIT); }
+        samp_meet<C>();                  // the number has been read
+      }
+    }
+    if (!found_it) {
+      samp_pass<true, C, K>(e, n, &s, 3, 21, 11, 0x00000000u, cut, rank);
+      samp_pass<true, C, K>(e, n, &s, 4, 10, 11, 0xFFE00000u, cut, rank);
+      samp_pass<true, C, K>(e, n, &s, 5, 0, 10, 0xFFFFFC00u, cut, rank);
+      if (s.prefix > thr_key) thr_key = s.prefix;
+    }
   }
   if (mp > 0.f) {
     const uint32_t tm = __float_as_uint(mp);  // max e is exactly 1
@@ -692,7 +867,7 @@ B200_API int b200_argmax(const void* logits, int dtype, long ld, int B, int V, v
 B200_API int b200_cast_bf16_f32(const void* in, long ld_in, void* out, long ld_out, int B, int V,
                                 cudaStream_t stream) {
   if (B <= 0 || V <= 0) return 0;
-  const unsigned blocks = (unsigned)((V + 16383) / 16384);           // 64 elements a thread
+  const unsigned blocks = (unsigned)((V + 8191) / 8192);             // 32 elements a thread
   for (int b0 = 0; b0 < B; b0 += 65535)                              // rows are the grid's y
     cast_bf16_to_f32_kernel<<<dim3(blocks, (unsigned)(B - b0 < 65535 ? B - b0 : 65535)), 256, 0, stream>>>(
         (const __nv_bfloat16*)in + (long)b0 * ld_in, ld_in, (float*)out + (long)b0 * ld_out, ld_out, V);
