@@ -14,6 +14,7 @@
 //               fp32 accumulators held in registers; store bf16 at the end.  A warpgroup per 64
 //               columns of the tile (64 accumulators per thread): the promotion of a block has to keep up
 //               with its MMA, which four warps with 128 accumulators each did not
+//   last two    multiply the scales of rows and columns and put them into shared memory, eight K blocks ahead
 // Tiles are 128 x 256 where they fill the GPU as well as 128 x 128 do: a K block of the small tile brings 32 KB for
 // 4.2 MFLOP, and at 1.3 PFLOP/s that is 10 TB/s out of L2, which bounds it (four warpgroups and four buffers for the
 // small tile changed nothing); the wide one brings 24 KB for the same.
@@ -31,13 +32,17 @@ constexpr int F8_BLOCK = 128;              // rows of W that share a scale
 constexpr int F8_COLS = 64;                // columns per promotion warpgroup
 constexpr int F8_TILE_BYTES = 128 * 128;                 // 16 KB per 128 operand rows
 constexpr int F8_MAX_GROUPS = 512;
+// K blocks whose scales (row times block of columns) lie in shared memory together, twice: loads of a scale per row and block by the
+// promotion itself, a line of memory per lane, took 210 of the 1140 clocks of a block
+constexpr int F8_SCALE_KB = 8;
 
 template <int BN>
 struct F8Cfg {
-  static constexpr int kThreads = 64 + 2 * BN;           // producer, MMA issuer, BN / 64 promotion warpgroups
+  static constexpr int kThreads = 128 + 2 * BN;          // producer, MMA issuer, BN / 64 promotion warpgroups, two warps for scales
   static constexpr int kStages = BN == 256 ? 4 : 6;
   static constexpr int kStageBytes = F8_TILE_BYTES * (1 + BN / 128);
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256 + (F8_MAX_GROUPS + 1) * 4;
+  static constexpr int kScaleBytes = 2 * F8_SCALE_KB * (BN / 128) * F8_BM * 4;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kScaleBytes + 1024 + 256 + (F8_MAX_GROUPS + 1) * 4;
 };
 
 struct Fp8Params {
@@ -97,11 +102,15 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a,
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* tiles = smem;
-  uint64_t* full_bar = (uint64_t*)(smem + F8_STAGES * F8_STAGE_BYTES);
+  constexpr int NB = BN / 128;                    // scale blocks of a tile's columns
+  float* scales = (float*)(smem + F8_STAGES * F8_STAGE_BYTES);        // [2][F8_SCALE_KB][NB][rows]
+  uint64_t* full_bar = (uint64_t*)(smem + F8_STAGES * F8_STAGE_BYTES + F8Cfg<BN>::kScaleBytes);
   uint64_t* empty_bar = full_bar + F8_STAGES;
   uint64_t* part_full = empty_bar + F8_STAGES;    // [2]
   uint64_t* part_empty = part_full + 2;           // [2]
-  uint32_t* tmem_ptr = (uint32_t*)(part_empty + 2);
+  uint64_t* sc_full = part_empty + 2;             // [2]
+  uint64_t* sc_empty = sc_full + 2;               // [2]
+  uint32_t* tmem_ptr = (uint32_t*)(sc_empty + 2);
   volatile int* abort_word = (volatile int*)(tmem_ptr + 1);
   int* grp_tiles = (int*)(tmem_ptr + 2);
 
@@ -116,6 +125,8 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a,
     for (int b = 0; b < 2; b++) {
       mbar_init(&part_full[b], 1);
       mbar_init(&part_empty[b], 4 * (BN / F8_COLS));
+      mbar_init(&sc_full[b], 2);
+      mbar_init(&sc_empty[b], 4 * (BN / F8_COLS));
     }
     *abort_word = 0;
     mbar_fence_init();
@@ -195,12 +206,52 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a,
         }
       }
     }
+  } else if (warp >= 2 + BN / 16) {
+    // ------------------------------------------------------------ scales (two warps, two rows per thread)
+    if (p.row_scale == nullptr) {
+      const int t64 = threadIdx.x - (64 + 2 * BN), kblocks = p.K / F8_BK, n_blocks = (p.N + F8_BLOCK - 1) / F8_BLOCK;
+      uint32_t grp = 0;
+      for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
+        F8Tile c;
+        f8_tile<BN>(p, grp_tiles, t, c);
+        const float* ws[NB];
+#pragma unroll
+        for (int h = 0; h < NB; h++)                       // columns beyond N have no scale
+          ws[h] = p.w_scale + ((size_t)c.group * n_blocks + min(c.tn * NB + h, n_blocks - 1)) * kblocks;
+        for (int k0 = 0; k0 < num_kb; k0 += F8_SCALE_KB, grp++) {
+          const int b = grp & 1, n = min(F8_SCALE_KB, num_kb - k0);
+          if (!mbar_wait(&sc_empty[b], ((grp >> 1) & 1u) ^ 1u, abort_word)) goto done;
+#pragma unroll
+          for (int i = 0; i < 2; i++) {
+            const int r = t64 + 64 * i, row = c.row0 + r;
+            const float* as = p.a_scale + (size_t)(row < c.row_end ? row : c.row0) * kblocks + k0;
+            float a[F8_SCALE_KB];
+            if ((kblocks & 3) == 0 && (reinterpret_cast<uintptr_t>(p.a_scale) & 15) == 0 && n == F8_SCALE_KB) {
+#pragma unroll
+              for (int k = 0; k < F8_SCALE_KB; k += 4) {
+                const float4 v = *reinterpret_cast<const float4*>(as + k);
+                a[k] = v.x; a[k + 1] = v.y; a[k + 2] = v.z; a[k + 3] = v.w;
+              }
+            } else {
+#pragma unroll
+              for (int k = 0; k < F8_SCALE_KB; k++) a[k] = k < n ? as[k] : 0.f;
+            }
+#pragma unroll
+            for (int k = 0; k < F8_SCALE_KB; k++)
+#pragma unroll
+              for (int h = 0; h < NB; h++)
+                if (k < n) scales[((b * F8_SCALE_KB + k) * NB + h) * F8_BM + r] = a[k] * ws[h][k0 + k];
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sc_full[b]);
+        }
+      }
+    }
   } else {
     // ------------------------------------------------------------ promotion + epilogue
     const int q = warp & 3;                              // TMEM lane quarter this warp may read
     const int wg = (warp - 2) >> 2;                      // which 64 columns of the tile
-    const int kblocks = p.K / F8_BK;                     // columns of the scale matrices
-    const int n_blocks = (p.N + F8_BLOCK - 1) / F8_BLOCK;
+    uint32_t grp = 0;                                    // groups of scales so far
     uint32_t it = 0;
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
       F8Tile c;
@@ -208,17 +259,22 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const int row = c.row0 + q * 32 + lane;
       const bool row_ok = row < c.row_end;
       const bool per_channel = p.row_scale != nullptr;
-      const float* as_row = per_channel ? nullptr : p.a_scale + (size_t)(row_ok ? row : 0) * kblocks;
-      const int blk = min(c.tn * (BN / F8_BLOCK) + wg * F8_COLS / F8_BLOCK, n_blocks - 1);     // columns beyond N have no scale
-      const float* ws_row = per_channel ? nullptr : p.w_scale + ((size_t)c.group * n_blocks + blk) * kblocks;
       float acc[F8_COLS];
 #pragma unroll
       for (int i = 0; i < F8_COLS; i++) acc[i] = 0.f;
-      float sc_next = per_channel ? 1.f : as_row[0] * ws_row[0];
       for (int kb = 0; kb < num_kb; kb++, it++) {
         const int b = it & 1;
-        const float sc = sc_next;
-        if (!per_channel && kb + 1 < num_kb) sc_next = as_row[kb + 1] * ws_row[kb + 1];
+        float sc = 1.f;
+        if (!per_channel) {
+          const int k = kb % F8_SCALE_KB, sb = grp & 1;
+          if (k == 0 && !mbar_wait(&sc_full[sb], (grp >> 1) & 1u, abort_word)) goto done;
+          sc = scales[((sb * F8_SCALE_KB + k) * NB + wg * F8_COLS / F8_BLOCK) * F8_BM + q * 32 + lane];
+          if (k == F8_SCALE_KB - 1 || kb + 1 == num_kb) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sc_empty[sb]);
+            grp++;
+          }
+        }
         if (!mbar_wait(&part_full[b], (it >> 1) & 1u, abort_word)) goto done;
         tc_fence_after();
         const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + b * BN + wg * F8_COLS;
@@ -236,19 +292,21 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a,
 #pragma unroll
           for (int i = 0; i < 32; i++) acc[32 + i] = fmaf(__uint_as_float(r1[i]), sc, acc[32 + i]);
         } else {
-          // 576 threads: 16 columns at a time keep the accumulators in registers
+          // 640 threads have 96 registers: eight columns at a time leave the accumulators and the loop their own.  With sixteen, what was
+          // spilled around the loop cost as much as the loads (2048 x 57344 x 8192 with loads of scales 1010 us, with scales from shared
+          // memory 1100, and 940 so)
 #pragma unroll
-          for (int c0 = 0; c0 < F8_COLS; c0 += 16) {
-            uint32_t r[16];
-            tmem_ld_32x32b_x16(t_row + c0, r);
+          for (int c0 = 0; c0 < F8_COLS; c0 += 8) {
+            uint32_t r[8];
+            tmem_ld_32x32b_x8(t_row + c0, r);
             tmem_ld_wait();
-            if (c0 + 16 == F8_COLS) {
+            if (c0 + 8 == F8_COLS) {
               tc_fence_before();
               __syncwarp();
               if (lane == 0) mbar_arrive(&part_empty[b]);
             }
 #pragma unroll
-            for (int i = 0; i < 16; i++) acc[c0 + i] = fmaf(__uint_as_float(r[i]), sc, acc[c0 + i]);
+            for (int i = 0; i < 8; i++) acc[c0 + i] = fmaf(__uint_as_float(r[i]), sc, acc[c0 + i]);
           }
         }
       }
