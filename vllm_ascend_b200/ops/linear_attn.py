@@ -5,7 +5,6 @@ csrc/attention/recurrent_gated_delta_rule*)."""
 from __future__ import annotations
 
 import functools
-import math
 import os
 from ctypes import c_float, c_int, c_long, c_void_p
 
@@ -215,10 +214,10 @@ def _kernel_times(lens: np.ndarray, Hv: int, DV: int, sms: int, least: int) -> f
     """Estimated us of a step whose sequences of ``least`` tokens and more run in chunks of 64 and the others token by token.
 
     In chunks: a block of every head prepares a chunk, 0.047 us of the GPU each, and blocks of 64 value columns, two to an SM, take 8 us and 5.4 us
-    per chunk, full or not (4.4 us alone on their SM).  A block of the token-serial kernel, of which three share an SM, takes 0.42 us per token
-    alone and 0.79 us among others.  Blocks run in waves, or packed one behind the other where they differ, whichever is shorter.  32 heads,
-    token by token and in chunks: 16 portions of 32 tokens 75 and 77 us (estimates 89 and 76), 12 of 64 117 and 65 (116 and 66), 64 of 65 517 and 415
-    (563 and 470), one of 128 60 and 30 (68 and 28), three of 2000 - and 350 (- and 332)."""
+    per chunk, full or not (4.4 us alone on their SM); counted 1.3 times, so that portions run in chunks where that is clearly the shorter way.  A
+    block of the token-serial kernel, of which three share an SM, takes 0.42 us per token alone and 0.79 us among others.  Blocks run in waves,
+    or packed one behind the other where they differ, whichever is shorter.  32 heads, token by token and in chunks: 16 portions of 32
+    tokens 75 and 77 us, 12 of 64 117 and 65, 64 of 65 517 and 415, one of 128 60 and 30, three of 2000 1600 and 350."""
     def packed(each, blocks, slots):
         n = len(each) * blocks
         longest = float(each.max())
@@ -227,7 +226,8 @@ def _kernel_times(lens: np.ndarray, Hv: int, DV: int, sms: int, least: int) -> f
     us, halves = 0.0, Hv * -(-DV // 64)
     if len(far):
         chunks = -(-far // 64)
-        us += 8 + 0.047 * Hv * float(chunks.sum()) + packed(8 + (4.4 if len(far) * halves <= sms else 5.4) * chunks, halves, 2 * sms)
+        us += 1.3 * (6 + 0.047 * Hv * float(chunks.sum())
+                     + packed(8 + (4.4 if len(far) * halves <= sms else 5.4) * chunks, halves, 2 * sms))
     if len(near):
         us += packed(14 + 0.42 * near, halves, sms) if len(near) * halves <= sms else packed(6.5 + 0.79 * near, halves, 3 * sms)
     return us
@@ -236,17 +236,11 @@ def _kernel_times(lens: np.ndarray, Hv: int, DV: int, sms: int, least: int) -> f
 @functools.lru_cache(maxsize=256)
 def _portions(cu: bytes, Hv: int, DV: int, sms: int) -> tuple[int, int]:
     """(new tokens from which sequences run in chunks of 64, or 0; 1 where there are shorter ones) for int32 token offsets ``cu``: the share-out
-    that is estimated to take the least time.  Where long portions run in chunks anyway, shorter ones join them only where that
-    is estimated to save a sixth: estimates of mixed steps are that rough.  A step's layers ask the same, and the host has no time for it in
-    each."""
+    that is estimated to take the least time.  A step's layers ask the same, and the host has no time for it in each."""
     lens = np.diff(np.frombuffer(cu, dtype=np.int32))
-    least, best = 0, math.inf
-    for n in (75, 40, 32):
-        if (lens >= n).any():
-            us = _kernel_times(lens, Hv, DV, sms, n)
-            if us < best * 5 / 6:
-                least, best = n, us
-    if not least or _kernel_times(lens, Hv, DV, sms, 1 << 30) < best:
+    marks = [n for n in (32, 40, 75) if (lens >= n).any()]
+    least = min(marks + [1 << 30], key=lambda n: _kernel_times(lens, Hv, DV, sms, n)) if marks else 1 << 30
+    if least == 1 << 30:
         return 0, 0
     return least, int(((lens > 0) & (lens < least)).any())
 
