@@ -21,6 +21,9 @@ from __future__ import annotations
 
 import os
 
+from . import envs
+
+_flag = envs.raw("VLLM_B200_BATCH_INVARIANT")
 _enabled = False
 _training_consistent = False
 
@@ -41,7 +44,7 @@ def is_training_consistent() -> bool:
 
 
 def is_batch_invariant() -> bool:
-    return _enabled or os.environ.get("VLLM_B200_BATCH_INVARIANT") == "1"
+    return _enabled or _flag() == b"1"
 
 
 def enable_batch_invariant_mode() -> None:

@@ -6,20 +6,47 @@ monkeypatch ``os.environ``.  Parity: vllm_ascend/envs.py:30-108 (same lazy
 """
 from __future__ import annotations
 
+import functools
 import os
 from typing import Any, Callable
 
 
+def raw(name: str) -> Callable[[], bytes | None]:
+    """Reader of a variable's bytes as ``os.environ`` holds them now.  ``os.environ.get`` encodes the name and decodes the value each
+    time, 1.5 us; an op asks two or three variables, and a step of a few hundred tokens takes as long as the host needs for it."""
+    key = os.fsencode(name)
+    return lambda: os.environ._data.get(key)
+
+
+_text = functools.lru_cache(maxsize=256)(os.fsdecode)
+_number = functools.lru_cache(maxsize=256)(int)
+
+
 def _bool(name: str, default: str = "0") -> Callable[[], bool]:
-    return lambda: os.getenv(name, default).strip().lower() in ("1", "true", "yes", "on")
+    get, fallback = raw(name), default.encode()
+
+    def read() -> bool:
+        v = get()
+        return (fallback if v is None else v).strip().lower() in (b"1", b"true", b"yes", b"on")
+    return read
 
 
 def _int(name: str, default: int) -> Callable[[], int]:
-    return lambda: int(os.getenv(name, str(default)))
+    get = raw(name)
+
+    def read() -> int:
+        v = get()
+        return default if v is None else _number(v)
+    return read
 
 
 def _str(name: str, default: str | None = None) -> Callable[[], str | None]:
-    return lambda: os.getenv(name, default)
+    get = raw(name)
+
+    def read() -> str | None:
+        v = get()
+        return default if v is None else _text(v)
+    return read
 
 
 env_variables: dict[str, Callable[[], Any]] = {
@@ -83,8 +110,9 @@ env_variables: dict[str, Callable[[], Any]] = {
 
 
 def __getattr__(name: str) -> Any:
-    if name in env_variables:
-        return env_variables[name]()
+    read = env_variables.get(name)
+    if read is not None:
+        return read()
     raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 

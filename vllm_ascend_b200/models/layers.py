@@ -8,6 +8,7 @@ all-reduce or reduce-scatter, chosen by the layer's ``TPComm``.
 """
 from __future__ import annotations
 
+import functools
 import hashlib
 import math
 from typing import Optional
@@ -295,9 +296,14 @@ def get_cos_sin_cache(rot_dim: int, max_pos: int, theta: float, scaling, device)
 
 
 # ---------------------------------------------------------------- attention + MLP
+@functools.lru_cache(maxsize=None)
+def _fusion():
+    from ..compilation import fusion
+    return fusion
+
+
 def _plan():
-    from ..compilation.fusion import get_plan
-    return get_plan()
+    return _fusion().get_plan()
 
 
 class GQAAttention:
@@ -402,7 +408,6 @@ class GQAAttention:
         k_cache, v_cache = kv_cache
         T = qkv.shape[0]
         q = qkv[:, :self.Hq * self.D].view(T, self.Hq, self.D)
-        from ..parallel import state as pstate
         dcp = pstate.get_dcp_group()
         if dcp.world_size > 1:
             # the KV cache holds this rank's share of every sequence

@@ -12,14 +12,13 @@ The op set corresponds to the reference's OOT custom-op table
 from __future__ import annotations
 
 import functools
-import os
 from typing import Optional
 
 import numpy as np
 import torch
 
 from .. import _native, envs
-from ..batch_invariant import fixed_sums
+from ..batch_invariant import fixed_sums, is_batch_invariant, is_training_consistent
 from . import reference as ref
 
 _BF16 = torch.bfloat16
@@ -64,10 +63,12 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float,
     if not _use_native(x):
         return ref.rms_norm(x, weight, eps, residual, gemma)
     H = x.shape[-1]
-    x2 = x.reshape(-1, H) if x.stride(-1) == 1 else x.contiguous().view(-1, H)
+    if x.stride(-1) != 1:
+        x = x.contiguous()
+    x2 = x if x.dim() == 2 else x.reshape(-1, H)
     T = x2.shape[0]
     if out is None:
-        out = torch.empty((T, H), dtype=x.dtype, device=x.device)
+        out = x2.new_empty((T, H))
     if residual is not None:
         assert residual.is_contiguous()
     rc = _native.lib().b200_rms_norm(x2.data_ptr(), _native.ptr(residual), weight.data_ptr(),
@@ -75,7 +76,7 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float,
                                      out.stride(0), _native.stream_ptr())
     _native.check(rc, "rms_norm")
     launch_counter[0] += 1
-    return out.view(x.shape), residual
+    return out if x2 is x else out.view(x.shape), residual
 
 
 def layer_norm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], eps: float) -> torch.Tensor:
@@ -169,6 +170,12 @@ def qknorm_rope_kvwrite(qkv: torch.Tensor, positions: torch.Tensor, cos_sin: tor
 
 
 # ---------------------------------------------------------------- GEMM
+def _dense_rows(x: torch.Tensor, K: int) -> torch.Tensor:
+    """x as [rows, K] with adjacent columns and rows on 16-byte boundaries apart, as the GEMM kernels take it."""
+    x2 = x if x.dim() == 2 else x.reshape(-1, K)
+    return x2 if x2.stride(1) == 1 and x2.stride(0) % 8 == 0 else x2.contiguous()
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
            residual: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
            bn: int = 0) -> torch.Tensor:
@@ -180,17 +187,15 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         if residual is not None:
             y = y + residual
         return y
-    x2 = x.reshape(-1, K)
-    if x2.stride(-1) != 1 or (x2.stride(0) % 8) != 0:
-        x2 = x2.contiguous()
+    x2 = _dense_rows(x, K)
     M = x2.shape[0]
-    if envs.VLLM_B200_GEMM == "cublas" or (K % 8) or (N % 8):
+    if (K % 8) or (N % 8) or envs.VLLM_B200_GEMM == "cublas":
         y = torch.nn.functional.linear(x2, weight, bias)
         if residual is not None:
             y = y + residual.view(M, N)
         return y.view(*x.shape[:-1], N)
     if out is None:
-        out = torch.empty((M, N), dtype=x.dtype, device=x.device)
+        out = x2.new_empty((M, N))
     if M == 0:
         return out.view(*x.shape[:-1], N)
     res2 = None
@@ -211,7 +216,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
             _native.status_word(x.device).data_ptr(), 0, _native.stream_ptr())
     _native.check(rc, "gemm_bf16")
     launch_counter[0] += 1
-    return out.view(*x.shape[:-1], N)
+    return out if x.dim() == 2 else out.view(*x.shape[:-1], N)
 
 
 def linear_fp32(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
@@ -296,12 +301,10 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Ten
         y = linear(x, weight)
         return silu_and_mul(y) if limit is None else activation(y.contiguous(), "swiglu_oai", True, CLAMPED_GATE_ALPHA, limit)
     alpha, limit = (0.0, 0.0) if limit is None else (CLAMPED_GATE_ALPHA, float(limit))
-    x2 = x.reshape(-1, K)
-    if x2.stride(-1) != 1 or (x2.stride(0) % 8) != 0:
-        x2 = x2.contiguous()
+    x2 = _dense_rows(x, K)
     M = x2.shape[0]
     if out is None:
-        out = torch.empty((M, I), dtype=x.dtype, device=x.device)
+        out = x2.new_empty((M, I))
     min2 = envs.VLLM_B200_GEMM_2CTA_MIN_M
     if M > 0 and I % 128 == 0 and (two_cta or (min2 > 0 and M >= min2)):
         rc = _native.lib().b200_gemm_glu_bf16_2cta(
@@ -315,7 +318,7 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Ten
             alpha, limit, _native.status_word(x.device).data_ptr(), _native.stream_ptr())
         _native.check(rc, "gemm_swiglu")
         launch_counter[0] += 1
-    return out.view(*x.shape[:-1], I)
+    return out if x.dim() == 2 else out.view(*x.shape[:-1], I)
 
 
 #: most rows of the few-row GEMM
@@ -358,7 +361,7 @@ def _few_rows_faster(M: int, N: int, K: int, glu: bool) -> bool:
 def _few_rows(M: int, N: int, K: int, glu: bool = False) -> bool:
     """Whether a step's product (N columns; ``glu``: of gate and up together twice as many) runs in the kernel that splits K over
     blocks.  Its rows may differ in the last bit from those of a larger batch, so modes that fix the order of sums never take it."""
-    if M > _FEW_ROWS or K % 8 or N % 8 or os.environ.get("VLLM_B200_GEMM") == "cublas":
+    if M > _FEW_ROWS or K % 8 or N % 8 or envs.VLLM_B200_GEMM == "cublas":
         return False
     return not fixed_sums() and _few_rows_faster(M, N, K, glu)
 
@@ -394,16 +397,14 @@ def linear_step(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
     M = x.numel() // K if K else 0
     if M == 0 or not _use_native(x) or weight.dtype != _BF16 or not _few_rows(M, N, K):
         return linear(x, weight, bias, residual, bn=512 if x.is_cuda and _pair_rows(M, N, K) else 0)
-    x2 = x.reshape(-1, K)
-    if x2.stride(-1) != 1 or (x2.stride(0) % 8) != 0:
-        x2 = x2.contiguous()
-    out = torch.empty((M, N), dtype=x.dtype, device=x.device)
+    x2 = _dense_rows(x, K)
+    out = x2.new_empty((M, N))
     res2 = None
     if residual is not None:
         res2 = residual.view(M, N)
         assert res2.stride(0) == out.stride(0) and res2.stride(1) == 1
     _gemm_small(x2, weight, out, bias, res2, N, False)
-    return out.view(*x.shape[:-1], N)
+    return out if x.dim() == 2 else out.view(*x.shape[:-1], N)
 
 
 def linear_swiglu_step(x: torch.Tensor, weight: torch.Tensor, limit: Optional[float] = None) -> torch.Tensor:
@@ -412,12 +413,10 @@ def linear_swiglu_step(x: torch.Tensor, weight: torch.Tensor, limit: Optional[fl
     M = x.numel() // K if K else 0
     if M == 0 or not _use_native(x) or weight.dtype != _BF16 or not _few_rows(M, I, K, True):
         return linear_swiglu(x, weight, limit=limit, two_cta=x.is_cuda and _pair_rows(M, I, K, True))
-    x2 = x.reshape(-1, K)
-    if x2.stride(-1) != 1 or (x2.stride(0) % 8) != 0:
-        x2 = x2.contiguous()
-    out = torch.empty((M, I), dtype=x.dtype, device=x.device)
+    x2 = _dense_rows(x, K)
+    out = x2.new_empty((M, I))
     _gemm_small(x2, weight, out, None, None, I, True, *((0.0, 0.0) if limit is None else (CLAMPED_GATE_ALPHA, float(limit))))
-    return out.view(*x.shape[:-1], I)
+    return out if x.dim() == 2 else out.view(*x.shape[:-1], I)
 
 
 # ---------------------------------------------------------------- attention
@@ -615,7 +614,6 @@ def choose_num_splits(num_seqs: int, Hkv: int, max_seq_len: int, sm_count: int =
                       tile: int = 128) -> int:
     """Split-KV factor: enough CTAs to fill the GPU, never more splits than KV tiles.  In
     batch-invariant mode the factor is 1: the merge order must not depend on the batch."""
-    from ..batch_invariant import is_batch_invariant
     if is_batch_invariant():
         return 1
     ctas = max(1, num_seqs * Hkv)
@@ -660,8 +658,7 @@ def paged_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
     T, Hq, D = q.shape
     if out is None:
         out = torch.empty((T, Hq, v_cache.shape[-1]), dtype=q.dtype, device=q.device)
-    from ..attention.backend import training_consistent_attention
-    if training_consistent_attention() and causal and window == 0:
+    if is_training_consistent() and causal and window == 0:
         return paged_attention_consistent(q, k_cache, v_cache, meta, scale, out)
     if not _use_native(q):
         return ref.paged_attention(q, k_cache, v_cache, meta.query_start_loc_cpu,

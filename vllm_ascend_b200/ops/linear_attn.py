@@ -5,15 +5,16 @@ csrc/attention/recurrent_gated_delta_rule*)."""
 from __future__ import annotations
 
 import functools
-import os
 from ctypes import c_float, c_int, c_long, c_void_p
 
 import numpy as np
 import torch
 import torch.nn.functional as F
 
-from .. import _native
+from .. import _native, envs
+from ..batch_invariant import fixed_sums
 
+_chunk_flag = envs.raw("VLLM_B200_GDN_CHUNK_MIN")
 P, I, L, Fl = c_void_p, c_int, c_long, c_float
 _native.register_signature("b200_causal_conv1d", [P, L, P, P, P, P, P, P, P, L, L, I, I, I, I, I, L, I, P, L, P, P, I, P, P,
                                                   P, P])
@@ -204,8 +205,7 @@ def _chunk_min(on_cuda: bool = False) -> int:
     """Fewest new tokens of a sequence that take the chunk-parallel form built from fp32 matrix products; 0 = never.
     Unset, the form serves host tensors only: on a B200 it takes 10.3 ms for 4 x 2048 tokens of 32 heads, the kernels 1.3 ms token
     by token (three prompts of 2000 tokens: 1.6 ms, and 0.35 ms in chunks: ``_portions``)."""
-    from .. import envs
-    if "VLLM_B200_GDN_CHUNK_MIN" not in os.environ and on_cuda:
+    if on_cuda and _chunk_flag() is None:
         return 0
     return int(envs.VLLM_B200_GDN_CHUNK_MIN)
 
@@ -248,8 +248,7 @@ def _portions(cu: bytes, Hv: int, DV: int, sms: int) -> tuple[int, int]:
 def _token_by_token() -> bool:
     """No chunks on the GPU: asked for with VLLM_B200_GDN_CHUNK_MIN=0, or a mode that fixes the order of sums (a portion's split
     into chunks must not show)."""
-    from ..batch_invariant import fixed_sums
-    return fixed_sums() or os.environ.get("VLLM_B200_GDN_CHUNK_MIN") == "0"
+    return fixed_sums() or _chunk_flag() == b"0"
 
 
 #: bytes that a chunk of 64 tokens leaves per head in the workspace, and the most that a workspace takes (a longer step goes in slices)
@@ -324,11 +323,16 @@ def gated_delta_rule(q, k, v, g, beta, state, cu, slots, has_init, scale, l2norm
     return out.view(T, Hv * DV) if z is not None else _gate(out, gate)
 
 
+@functools.lru_cache(maxsize=None)
+def _stream():
+    from . import stream
+    return stream
+
+
 def _gate(out, gate):
     if gate is None:
         return out
-    from .stream import gated_head_norm
-    return gated_head_norm(out, *gate)
+    return _stream().gated_head_norm(out, *gate)
 
 
 # ---------------------------------------------------------------------------- lightning attention
