@@ -47,14 +47,14 @@ def _best_splits(sms: int, ctas: int, tiles: int) -> int:
 
 
 def _num_splits(dev, ctas: int, max_keys: int) -> int:
-    """Splits of the key range: at most one per 128-key tile and two CTAs per SM.  A CTA has an SM to itself, so what a split
-    count costs is its waves times the tiles that a CTA walks one after the other, and two more for its start and end (32 sequences
-    of 2500 to 5700 tokens, 32 heads: ten splits in three waves 137 us)."""
+    """Most splits of a key range: at most one per 128-key tile and two CTAs per SM; one where whole sequences fill the SMs as
+    well.  The kernel sets the tiles of a split from the lengths that it finds, so a short sequence uses fewer of them."""
     from ..batch_invariant import is_batch_invariant
     if is_batch_invariant():
         return 1
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
-    return _best_splits(sms, max(ctas, 1), max(1, (max_keys + 127) // 128))
+    ctas, tiles = max(ctas, 1), max(1, (max_keys + 127) // 128)
+    return 1 if _best_splits(sms, ctas, tiles) == 1 else min(tiles, _most_splits(sms, ctas))
 
 
 def _tc_sizes_ok(q_lat: torch.Tensor, q_pe: torch.Tensor, lat_cache: torch.Tensor) -> bool:

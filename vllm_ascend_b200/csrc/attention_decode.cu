@@ -148,7 +148,11 @@ paged_decode_kernel(const __nv_bfloat16* __restrict__ q, long q_stride,
 }
 
 // out[t, hq, :] = sum_s softmax_s(lse)[s] * partial_o[t, hq, s, :]
-template <typename TO>
+// Bound by the latency of its loads (few bytes, one pass): the lanes of a warp load 32 splits' sums of exponentials at once,
+// and with VEC = 4 a thread has four neighbouring elements, so that a row of 512 is one pass of a block.  Splits behind
+// the last one with a key are not read (32 rows x 32 heads of 512, ten splits of which three to six have keys: 7.5 us with
+// one element a thread, now 5.0).
+template <typename TO, int VEC>
 __global__ void merge_splits_kernel(const float* __restrict__ partial_o,
                                     const float* __restrict__ partial_lse, int num_splits, int D,
                                     int Hq, TO* __restrict__ out, long out_stride,
@@ -156,27 +160,54 @@ __global__ void merge_splits_kernel(const float* __restrict__ partial_o,
                                     const float* __restrict__ sink,
                                     const __nv_bfloat16* __restrict__ gate, long gate_stride, float out_scale) {
   const long t = blockIdx.x;
-  const int hq = blockIdx.y;
+  const int hq = blockIdx.y, lane = threadIdx.x & 31;
   const long base = (t * Hq + hq) * num_splits;
   float M = sink ? sink[hq] : -INFINITY;
-  for (int s = 0; s < num_splits; s++) M = fmaxf(M, partial_lse[base + s]);
+  int used = 0;
+  for (int s0 = 0; s0 < num_splits; s0 += 32) {
+    const float v = s0 + lane < num_splits ? partial_lse[base + s0 + lane] : -INFINITY;
+    const unsigned has = __ballot_sync(0xffffffffu, v != -INFINITY);
+    if (has) used = s0 + 32 - __clz(has);
+    M = fmaxf(M, v);
+  }
+  for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
   if (lse_out && threadIdx.x == 0) {
     float L = 0.f;
     if (M != -INFINITY)
-      for (int s = 0; s < num_splits; s++) L += __expf(partial_lse[base + s] - M);
+      for (int s = 0; s < used; s++) L += __expf(partial_lse[base + s] - M);
     lse_out[t * Hq + hq] = L > 0.f ? M + logf(L) : -INFINITY;
   }
   const float g = out_scale * (gate ? 1.f / (1.f + __expf(-__bfloat162float(gate[t * gate_stride + hq]))) : 1.f);
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float acc = 0.f, L = sink ? __expf(sink[hq] - M) : 0.f;
-    if (M != -INFINITY) {
-      for (int s = 0; s < num_splits; s++) {
-        const float w = __expf(partial_lse[base + s] - M);
+  // all lanes of a warp walk the loop, those past the end of the row without loads
+  for (int d0 = (int)(threadIdx.x & ~31u) * VEC; d0 < D; d0 += blockDim.x * VEC) {
+    const int d = d0 + lane * VEC;
+    float acc[VEC] = {}, L = sink ? __expf(sink[hq] - M) : 0.f;
+    for (int s0 = 0; s0 < used; s0 += 32) {
+      const int cnt = min(32, used - s0);
+      const float wl = lane < cnt ? __expf(partial_lse[base + s0 + lane] - M) : 0.f;
+#pragma unroll 4
+      for (int k = 0; k < cnt; k++) {
+        const float w = __shfl_sync(0xffffffffu, wl, k);
         L += w;
-        acc += w * partial_o[(base + s) * D + d];
+        if (d < D) {
+          const float* from = partial_o + (base + s0 + k) * D + d;
+          if constexpr (VEC == 4) {
+            const float4 v = *reinterpret_cast<const float4*>(from);
+            acc[0] += w * v.x;
+            acc[1] += w * v.y;
+            acc[2] += w * v.z;
+            acc[3] += w * v.w;
+          } else {
+            acc[0] += w * *from;
+          }
+        }
       }
     }
-    out[t * out_stride + hq * out_head + d] = from_f<TO>(L > 0.f ? g * acc / L : 0.f);
+    if (d < D) {
+#pragma unroll
+      for (int i = 0; i < VEC; i++)
+        out[t * out_stride + hq * out_head + d + i] = from_f<TO>(L > 0.f ? g * acc[i] / L : 0.f);
+    }
   }
 }
 
@@ -186,14 +217,19 @@ int launch_merge_splits(const float* partial_o, const float* partial_lse, long T
                         bool out_f32, float out_scale) {
   if (T <= 0) return 0;
   dim3 grid((unsigned)T, (unsigned)Hq);
-  if (out_f32)
-    merge_splits_kernel<float><<<grid, D > 64 ? 128 : 64, 0, stream>>>(
-        partial_o, partial_lse, num_splits, D, Hq, (float*)out, out_stride, out_head ? out_head : D, lse_out,
-        sink, (const __nv_bfloat16*)gate, gate_stride, out_scale);
-  else
-    merge_splits_kernel<__nv_bfloat16><<<grid, D > 64 ? 128 : 64, 0, stream>>>(
-        partial_o, partial_lse, num_splits, D, Hq, (__nv_bfloat16*)out, out_stride, out_head ? out_head : D, lse_out,
-        sink, (const __nv_bfloat16*)gate, gate_stride, out_scale);
+  const __nv_bfloat16* g = (const __nv_bfloat16*)gate;
+  const long head = out_head ? out_head : D;
+  const bool vec = D % 4 == 0 && ((uintptr_t)partial_o & 15) == 0;
+  const int per = vec ? 4 : 1, threads = D > 64 * per ? 128 : (D > 32 * per ? 64 : 32);
+#define MERGE(TO, VEC)                                                                                             \
+  merge_splits_kernel<TO, VEC><<<grid, threads, 0, stream>>>(partial_o, partial_lse, num_splits, D, Hq, (TO*)out,  \
+                                                             out_stride, head, lse_out, sink, g, gate_stride, out_scale)
+  if (out_f32) {
+    if (vec) MERGE(float, 4); else MERGE(float, 1);
+  } else {
+    if (vec) MERGE(__nv_bfloat16, 4); else MERGE(__nv_bfloat16, 1);
+  }
+#undef MERGE
   return B200_CHECK_LAUNCH();
 }
 

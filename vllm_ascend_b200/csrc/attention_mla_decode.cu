@@ -54,6 +54,7 @@ struct MlaParams {
   const float* sink;        // [H] or null
   float scale_log2;
   int num_splits;
+  int rows, slots;          // R; CTAs of a head block that run at once, 0: every sequence in num_splits even parts
   __nv_bfloat16* out;       // [R, H, dc]
   long out_stride, out_head;     // elements between rows / heads
   float* partial_o;
@@ -90,6 +91,52 @@ __device__ __forceinline__ void mla_tmem_ld(uint32_t addr, uint32_t* r) {
 template <int NQ>
 __device__ __forceinline__ void mla_tmem_st(uint32_t addr, const uint32_t* r) {
   if constexpr (NQ == 16) tmem_st_32x32b_x16(addr, r); else tmem_st_32x32b_x32(addr, r);
+}
+
+// Tiles that every KV split takes, the same for all sequences of the batch, so that short and long ones finish
+// together.  Splitting each sequence into the same number of parts instead makes the longest sequence's part the
+// time of the kernel (32 sequences of 2500 to 5700 keys, 32 heads: four parts of up to 12 tiles 71 us a call,
+// common parts of 8 tiles 56).  The lengths are read here and not on the host, which may have
+// captured the launch for other lengths.  Of the counts that fill the SMs once or twice the shorter walk wins: its tiles,
+// and two more for a CTA's start and end.  No split count above num_splits is asked of the longest sequence.
+// A warp's lanes take the sequences side by side; every warp finds the same number.
+__device__ __forceinline__ int mla_common_tiles(const MlaParams& p) {
+  const int lane = threadIdx.x & 31;
+  const bool list = p.cu == nullptr, pack = !list && !p.uniform;
+  const int units = pack ? p.B : p.rows;
+  auto tiles_of = [&](int u) {
+    const int kv = max(0, list ? p.row_kv_len[u] : p.seq_lens[u]);
+    const int lo = p.window > 0 ? max(0, kv - p.window - (p.TOK - 1)) >> 7 : 0;
+    return ((kv + 127) >> 7) - lo;
+  };
+  auto ctas_of = [&](int u) { return pack ? (p.cu[u + 1] - p.cu[u] + p.TOK - 1) / p.TOK : 1; };
+  int total = 0, most = 0;
+  for (int u = lane; u < units; u += 32) {
+    const int n = tiles_of(u);
+    total += n * ctas_of(u);
+    most = max(most, n);
+  }
+  total = __reduce_add_sync(0xffffffffu, total);
+  most = max(1, __reduce_max_sync(0xffffffffu, most));
+  const int least = (most + p.num_splits - 1) / p.num_splits;
+  int best = most, best_cost = 0x7fffffff;
+  for (int waves = 1; waves <= 2; waves++) {
+    const int room = waves * p.slots;
+    int t = min(most, max(least, (total + room - 1) / room)), used;
+    while (true) {
+      used = 0;
+      for (int u = lane; u < units; u += 32) used += (tiles_of(u) + t - 1) / t * ctas_of(u);
+      used = __reduce_add_sync(0xffffffffu, used);
+      if (used <= room || t >= most) break;
+      t = min(most, t + 1 + (t >> 4));
+    }
+    const int cost = (used + p.slots - 1) / p.slots * (t + 2);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = t;
+    }
+  }
+  return best;
 }
 
 template <int NQ>
@@ -131,7 +178,8 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   const int kv_len = kv0 + ntok - 1;                // keys the last row sees
   const int t_lo = p.window > 0 ? max(0, kv0 - p.window) >> 7 : 0;
   const int n_all = ((kv_len + 127) >> 7) - t_lo;
-  const int per_split = (n_all + p.num_splits - 1) / p.num_splits;
+  int per_split = (n_all + p.num_splits - 1) / p.num_splits;
+  if (p.slots > 0) per_split = max(per_split, mla_common_tiles(p));
   const int t0 = t_lo + split * per_split;
   const int t1 = min(t_lo + n_all, t0 + per_split);
   const int n = t1 - t0;
@@ -139,16 +187,14 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   const int dc = p.dc;
 
   if (n <= 0) {
-    for (int i = threadIdx.x; i < ntok * p.HC * dc; i += blockDim.x) {
+    const int step = p.num_splits > 1 ? dc : 1;       // the merge reads no sums of an empty split
+    for (int i = threadIdx.x * step; i < ntok * p.HC * dc; i += blockDim.x * step) {
       const int c = i / dc, d = i - c * dc, tok = c / p.HC, head = hb * p.HC + c % p.HC;
       if (head >= p.H) continue;
-      if (p.num_splits > 1) {
-        const long pidx = ((long)(row + tok) * p.H + head) * p.num_splits + split;
-        p.partial_o[pidx * dc + d] = 0.f;
-        if (d == 0) p.partial_lse[pidx] = -INFINITY;
-      } else {
+      if (p.num_splits > 1)
+        p.partial_lse[((long)(row + tok) * p.H + head) * p.num_splits + split] = -INFINITY;
+      else
         p.out[(long)(row + tok) * p.out_stride + head * p.out_head + d] = __float2bfloat16(0.f);
-      }
     }
     return;
   }
@@ -220,6 +266,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         tma_load_3d(Qs + s * Cfg::Q_SLAB, &tmap_q, q_full, s * 64, hb * p.HC, row);
       tma_load_3d(Qs + lat_slabs * Cfg::Q_SLAB, &tmap_qpe, q_full, 0, hb * p.HC, row);
     }
+#pragma unroll 1
     for (int j = 0; j < n; j++) {
       const uint32_t ph = (uint32_t)j & 1u;
       const int key_base = (t0 + j) << 7;
@@ -234,6 +281,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 #pragma unroll 1
       for (int s = 0; s < slabs; s++) {
         if (!mbar_wait(&h_empty[s], ph ^ 1u, abort_word)) goto done;
+#pragma unroll 1
         for (int part = 0; part < parts; part++) {
           const int b = __shfl_sync(0xffffffffu, blk, part);
           if (elect_one()) {
@@ -255,10 +303,12 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       const uint64_t dq0 = make_smem_desc(smem_u32(Qs), 16, 1024, kLayoutSw128), dk0 = make_smem_desc(smem_u32(KVs), 16, 1024, kLayoutSw128);
       const uint64_t dv0 = make_smem_desc(smem_u32(KVs), MLA_SLAB, 1024, kLayoutSw128), dp0 = make_smem_desc(smem_u32(Ps), 16, 1024, kLayoutSw128);
       if (!mbar_wait(q_full, 0, abort_word)) goto done;
+#pragma unroll 1
       for (int j = 0; j < n; j++) {
         const uint32_t ph = (uint32_t)j & 1u;
         const int b = j & 1;
         if (!mbar_wait(&s_free[b], (((uint32_t)j >> 1) & 1u) ^ 1u, abort_word)) goto done;
+#pragma unroll 1
         for (int s = 0; s < slabs; s++) {
           if (!mbar_wait(&h_full[s], ph, abort_word)) goto done;
           tc_fence_after();
@@ -271,6 +321,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         if (!mbar_wait(&p_ready[b], ((uint32_t)j >> 1) & 1u, abort_word)) goto done;
         tc_fence_after();
         const uint64_t dp = dp0 + (uint32_t)(b * (Cfg::P_BYTES >> 4));
+#pragma unroll 1
         for (int blk = 0; blk < val_blocks; blk++) {
           // A: 16 keys of latent^T for d in [128 blk, 128 blk + 128): two 64-wide d atoms one
           // slab apart, 8-key groups 1024 B apart.  With an odd number of latent slabs the last
@@ -301,6 +352,7 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     float m = -INFINITY, lsum[NQ];
 #pragma unroll
     for (int c = 0; c < NQ; c++) lsum[c] = 0.f;
+#pragma unroll 1
     for (int j = 0; j < n; j++) {
       const int b = j & 1;
       if (!mbar_wait(&s_ready[b], ((uint32_t)j >> 1) & 1u, abort_word)) goto done;
@@ -316,6 +368,10 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       if (((t0 + j + 1) << 7) <= kv0 && p.window <= 0) {       // every row sees the whole tile
 #pragma unroll
         for (int c = 0; c < NQ; c++) s[c] = __uint_as_float(r[c]);
+      } else if (p.TOK == 1) {
+        const bool visible = key < kv0 && (p.window <= 0 || key >= kv0 - p.window);
+#pragma unroll
+        for (int c = 0; c < NQ; c++) s[c] = visible ? __uint_as_float(r[c]) : -INFINITY;
       } else {
         int tok = 0, left = p.HC;                     // column c = (token c / HC, head c % HC)
 #pragma unroll
@@ -389,22 +445,27 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     // ---- epilogue
     if (!mbar_wait(&pv_done[(n - 1) & 1], (((uint32_t)n - 1) >> 1) & 1u, abort_word)) goto done;
     tc_fence_after();
-    col_max[col] = m * sl2;
-    mla_softmax_bar();
+    // A CTA runs this once and its instructions come from memory, so they are few (with the loops around the waits left to
+    // the compiler to unroll and 32 columns' sink, logarithm and 64-bit indexes spelled out a CTA of one tile took 55 us, now 16): the sums are transposed instead of reduced one by one, a lane
+    // finishes its own column, and the columns that are stored lie a constant step apart (one token, or all heads of several).
 #pragma unroll
-    for (int c = 0; c < NQ; c++) {
-      const float w = warp_reduce_sum(lsum[c]);
-      if (lane == 0) redf[qd * NQ + c] = w;
+    for (int o = NQ / 2; o > 0; o >>= 1) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int c = 0; c < o; c++) {
+        const float give = up ? lsum[c] : lsum[c + o];
+        lsum[c] = (up ? lsum[c + o] : lsum[c]) + __shfl_xor_sync(0xffffffffu, give, o);
+      }
     }
+    if constexpr (NQ == 16) lsum[0] += __shfl_xor_sync(0xffffffffu, lsum[0], 16);
+    redf[qd * NQ + col] = lsum[0];
     mla_softmax_bar();
-    float inv[NQ], lse[NQ];
-    int hd = 0;
-#pragma unroll
-    for (int c = 0; c < NQ; c++) {
-      float l = redf[c] + redf[NQ + c] + redf[2 * NQ + c] + redf[3 * NQ + c];
-      float m2 = col_max[c], f = 1.f;                 // row maximum in log2 units
-      if (p.sink != nullptr && split == 0 && hb * p.HC + hd < p.H) {      // counted once, keys or not
-        const float sk = p.sink[hb * p.HC + hd] * 1.4426950408889634f;
+    const int cols = p.TOK > 1 ? ntok * p.HC : min(p.HC, p.H - hb * p.HC);
+    {
+      float l = redf[col] + redf[NQ + col] + redf[2 * NQ + col] + redf[3 * NQ + col];
+      float m2 = m * sl2, f = 1.f;                    // row maximum in log2 units
+      if (p.sink != nullptr && split == 0 && col < cols) {      // counted once, keys or not
+        const float sk = p.sink[hb * p.HC + col % p.HC] * 1.4426950408889634f;
         if (sk > m2) {
           f = mla_exp2(m2 - sk);
           l = l * f + 1.f;
@@ -413,32 +474,38 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           l += mla_exp2(sk - m2);
         }
       }
-      if (++hd == p.HC) hd = 0;
-      inv[c] = l > 0.f ? f / l : 0.f;
-      lse[c] = l > 0.f ? (m2 * 0.6931471805599453f + logf(l)) : -INFINITY;
+      col_max[col] = l > 0.f ? f / l : 0.f;
+      if (p.num_splits > 1 && qd == 0 && lane < min(cols, NQ))
+        p.partial_lse[((long)row * p.H + hb * p.HC + col) * p.num_splits + split] =
+            l > 0.f ? (m2 * 0.6931471805599453f + logf(l)) : -INFINITY;
+      __syncwarp();
     }
+    const long step = (long)p.num_splits * dc;
 #pragma unroll 1
     for (int blk = 0; blk < val_blocks; blk++) {
       uint32_t o[NQ];
       mla_tmem_ld<NQ>(t_lane + Cfg::O_COL + blk * NQ, o);
       tmem_ld_wait();
       const int d = blk * 128 + tid;
-      if (d < dc) {
-        int tok = 0, h = 0;
+      alignas(16) float inv[4];
+      if (d < dc && p.num_splits > 1) {
+        float* to = p.partial_o + (((long)row * p.H + hb * p.HC) * p.num_splits + split) * dc + d;
 #pragma unroll
-        for (int c = 0; c < NQ; c++) {
-          const int head = hb * p.HC + h;
-          if (tok < ntok && head < p.H) {
-            const float val = __uint_as_float(o[c]) * inv[c];
-            if (p.num_splits == 1) {
-              p.out[(long)(row + tok) * p.out_stride + head * p.out_head + d] = __float2bfloat16(val);
-            } else {
-              const long pidx = ((long)(row + tok) * p.H + head) * p.num_splits + split;
-              p.partial_o[pidx * dc + d] = val;
-              if (d == 0) p.partial_lse[pidx] = lse[c];
-            }
+        for (int c = 0; c < NQ; c++, to += step) {
+          if ((c & 3) == 0) *reinterpret_cast<float4*>(inv) = *reinterpret_cast<const float4*>(col_max + c);
+          if (c < cols) *to = __uint_as_float(o[c]) * inv[c & 3];
+        }
+      } else if (d < dc) {
+        __nv_bfloat16* to = p.out + row * p.out_stride + hb * p.HC * p.out_head + d;
+        int left = p.HC;
+#pragma unroll
+        for (int c = 0; c < NQ; c++, to += p.out_head) {
+          if ((c & 3) == 0) *reinterpret_cast<float4*>(inv) = *reinterpret_cast<const float4*>(col_max + c);
+          if (left-- == 0) {
+            to += p.out_stride - p.HC * p.out_head;
+            left = p.HC - 1;
           }
-          if (++h == p.HC) { h = 0; tok++; }
+          if (c < cols) *to = __float2bfloat16(__uint_as_float(o[c]) * inv[c & 3]);
         }
       }
       __syncwarp();
@@ -589,6 +656,9 @@ B200_API int b200_mla_attention(const void* q_lat, long ql_row, long ql_head, co
   p.sink = (const float*)sink;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.num_splits = num_splits;
+  p.rows = (int)R;
+  // a long list of sequences fills the SMs as it is, and every CTA would read all of its lengths
+  p.slots = num_splits > 1 && (pack ? (long)B : R) <= 1024 ? (num_sms() > head_blocks ? num_sms() / head_blocks : 1) : 0;
   p.out = (__nv_bfloat16*)out;
   p.out_stride = out_stride;
   p.out_head = out_head;
