@@ -284,6 +284,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
       return true;
     };
     bool q_ahead = false;                // the next non-empty item's Q load was already issued
+#pragma unroll 1
     for (int item = blockIdx.x; item < num_items; item += gridDim.x) {
       const DecItem w = w_next;
       const int hk = VAR ? w.h * p.key_heads / p.Hkv : w.h;
@@ -305,6 +306,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
         const int key0 = (dec_tile<VAR>(w, j) << 7) + lane * rpl;
         return bt[min(key0, w.seq_len - 1) / p.block_size];
       };
+#pragma unroll 1
       for (int j = 0; j < w.n; j++, gt++) {
         const int st = gt % ST;
         const uint32_t ph = (gt / ST) & 1u;
@@ -349,6 +351,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
               const CUtensorMap* tm = kv == 0 ? &tmap_k32 : &tmap_v32;
               mbar_expect_tx(fullb, nsub * NH * 32 * 128);
               const int off = key_base % p.block_size;
+#pragma unroll 1
               for (int sub = 0; sub < nsub; sub++) {
 #pragma unroll
                 for (int hf = 0; hf < NH; hf++)
@@ -359,6 +362,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
             __syncwarp();
             continue;
           }
+#pragma unroll 1
           for (int part = 0; part < parts; part++) {
             const int blk = __shfl_sync(0xffffffffu, blk_cur, part);
             if (elect_one()) {
@@ -395,6 +399,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
       uint32_t gt = 0, it = 0;
       DecRaw raw_next = {0, 0, 0};
       if ((int)blockIdx.x < num_items) raw_next = dec_load(p, blockIdx.x);
+#pragma unroll 1
       for (int item = blockIdx.x; item < num_items; item += gridDim.x) {
         const DecItem w = dec_make(p, item, raw_next);
         if (item + (int)gridDim.x < num_items) raw_next = dec_load(p, item + gridDim.x);
@@ -425,6 +430,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
           return true;
         };
         if (!issue_s(0)) goto done;
+#pragma unroll 1
         for (int j = 0; j < w.n; j++) {
           if (j + 1 < w.n) {
             if (!issue_s(j + 1)) goto done;
@@ -461,9 +467,11 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
     const int dv = VAR ? p.Dv : D;
     const SoftCap cap(VAR ? p.scale : 1.f, VAR && p.softcap > 0.f ? p.softcap : 1.f);
     int* redi = reinterpret_cast<int*>(red);        // [2 tiles][4 warps][16]
+    const int col = lane & (NVT - 1), col_tok = col / G, col_head = col - col_tok * G;      // the column this lane finishes
     uint32_t gt = 0, it = 0;
     DecRaw raw_next = {0, 0, 0};
     if ((int)blockIdx.x < num_items) raw_next = dec_load(p, blockIdx.x);
+#pragma unroll 1
     for (int item = blockIdx.x; item < num_items; item += gridDim.x) {
       const DecItem w = dec_make(p, item, raw_next);
       if (item + (int)gridDim.x < num_items) raw_next = dec_load(p, item + gridDim.x);
@@ -473,8 +481,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
           for (int c = tid; c < nv; c += 128) {
             const long pidx =
                 ((long)(w.q_start + c / G) * p.Hq + (w.h * G + c % G)) * p.num_splits + w.split;
-            p.partial_lse[pidx] = -INFINITY;
-            for (int d = 0; d < dv; d++) p.partial_o[pidx * dv + d] = 0.f;
+            p.partial_lse[pidx] = -INFINITY;        // the merge reads no sums behind the last split with keys
           }
         } else if (p.num_splits == 1 && p.lse_out && w.q_len > 0) {
           // a caller that merges partial results of several ranks needs a defined (zero-weight)
@@ -503,6 +510,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
         lo_max = max(lo_max, lo[c]);
       }
 
+#pragma unroll 1
       for (int j = 0; j < w.n; j++) {
         const uint32_t g = gt + (uint32_t)j;
         const int b = g & 1;
@@ -606,49 +614,56 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
         if (!mbar_wait(&pv_done[gl & 1], (gl >> 1) & 1u, abort_word)) goto done;
       }
       tc_fence_after();
+      // The sums are transposed (lane c mod NVT ends with column c's) and a lane finishes its own column: spelled out
+      // for all columns, logarithms, divisions and 64-bit indexes were code that is fetched from memory for one pass: 48 ragged
+      // sequences of 1024 keys, 4 KV heads of 8 queries, 39 -> 30 us; 33 of 2300 keys, 8 KV heads, 72 -> 63.
 #pragma unroll
-      for (int c = 0; c < NVT; c++) {
-        const float ws = warp_reduce_sum(lsum[c]);
-        if (lane == 0) red_sum[qd * DEC_NQ + c] = ws;
+      for (int o = NVT / 2; o > 0; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int c = 0; c < o; c++) {
+          const float give = up ? lsum[c] : lsum[c + o];
+          lsum[c] = (up ? lsum[c + o] : lsum[c]) + __shfl_xor_sync(0xffffffffu, give, o);
+        }
       }
+#pragma unroll
+      for (int o = NVT; o < 32; o <<= 1) lsum[0] += __shfl_xor_sync(0xffffffffu, lsum[0], o);
+      red_sum[qd * DEC_NQ + col] = lsum[0];
       uint32_t o[16];
       tmem_ld_32x32b_x16(t_lane + o_col, o);
       tmem_ld_wait();
       tc_fence_before();
       softmax_bar();            // row sums visible; every thread holds its O^T row
       if (lane == 0) mbar_arrive(&o_free[it & 1]);
-      if (tid < dv) {
+      const float l = red_sum[col] + red_sum[DEC_NQ + col] + red_sum[2 * DEC_NQ + col] + red_sum[3 * DEC_NQ + col];
+      float mc = m[0];
 #pragma unroll
-        for (int c = 0; c < NVT; c++) {
-          if (c < nv) {
-            const float l = red_sum[c] + red_sum[DEC_NQ + c] + red_sum[2 * DEC_NQ + c] +
-                            red_sum[3 * DEC_NQ + c];
-            float inv = l > 0.f ? 1.f / l : 0.f;
-            const long tok = w.q_start + c / G;
-            const int hq = w.h * G + c % G;
-            if constexpr (VAR) {
-              if (p.num_splits == 1) {            // with splits the merge does both
-                if (p.sink && l > 0.f) inv = 1.f / (l + score_exp2(p.sink[hq] * kLog2e - m[c] * sl2));
-                if (p.gate) inv *= sigmoid_f(__bfloat162float(p.gate[tok * p.gate_stride + hq]));
-                inv *= p.out_scale;
-              }
-            }
-            const float val = __uint_as_float(o[c]) * inv;
-            if (VAR && p.num_splits == 1 && p.out_f32) {
-              ((float*)p.out)[tok * p.out_stride + (long)hq * dv + tid] = val;
-            } else if (p.num_splits == 1) {
-              p.out[tok * p.out_stride + (long)hq * dv + tid] = __float2bfloat16(val);
-              if (tid == 0 && p.lse_out)
-                p.lse_out[tok * p.Hq + hq] =
-                    (l > 0.f) ? (m[c] * sl2 * 0.6931471805599453f + logf(l)) : -INFINITY;
-            } else {
-              const long pidx = (tok * p.Hq + hq) * p.num_splits + w.split;
-              p.partial_o[pidx * dv + tid] = val;
-              if (tid == 0)
-                p.partial_lse[pidx] =
-                    (l > 0.f) ? (m[c] * sl2 * 0.6931471805599453f + logf(l)) : -INFINITY;
-            }
-          }
+      for (int c = 1; c < NVT; c++) mc = col == c ? m[c] : mc;
+      float inv = l > 0.f ? 1.f / l : 0.f;
+      const long tok = w.q_start + col_tok;
+      const int hq = w.h * G + col_head;
+      if constexpr (VAR) {
+        if (p.num_splits == 1 && col < nv) {            // with splits the merge does both
+          if (p.sink && l > 0.f) inv = 1.f / (l + score_exp2(p.sink[hq] * kLog2e - mc * sl2));
+          if (p.gate) inv *= sigmoid_f(__bfloat162float(p.gate[tok * p.gate_stride + hq]));
+          inv *= p.out_scale;
+        }
+      }
+      const long pidx = (tok * p.Hq + hq) * p.num_splits + w.split;
+      float* lse_to = p.num_splits > 1 ? p.partial_lse : (VAR && p.out_f32 ? nullptr : p.lse_out);
+      if (qd == 0 && lane < nv && lane < NVT && lse_to)
+        lse_to[pidx] = (l > 0.f) ? (mc * sl2 * 0.6931471805599453f + logf(l)) : -INFINITY;
+      const long at = (p.num_splits > 1 ? pidx * dv : tok * p.out_stride + (long)hq * dv) + tid;
+      const int at_lo = (int)(uint32_t)at, at_hi = (int)(at >> 32);
+#pragma unroll
+      for (int c = 0; c < NVT; c++) {
+        const float val = __uint_as_float(o[c]) * __shfl_sync(0xffffffffu, inv, c);
+        // lane c's index, with this lane's element instead of that one's
+        const long to = (((long)__shfl_sync(0xffffffffu, at_hi, c) << 32) | (uint32_t)__shfl_sync(0xffffffffu, at_lo, c)) + (lane - c);
+        if (c < nv && tid < dv) {
+          if (p.num_splits > 1) p.partial_o[to] = val;
+          else if (VAR && p.out_f32) ((float*)p.out)[to] = val;
+          else p.out[to] = __float2bfloat16(val);
         }
       }
       // the next item's epilogue overwrites red_sum only after a softmax_bar of its tile loop
