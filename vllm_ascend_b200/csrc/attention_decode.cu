@@ -185,7 +185,7 @@ __global__ void merge_splits_kernel(const float* __restrict__ partial_o,
     for (int s0 = 0; s0 < used; s0 += 32) {
       const int cnt = min(32, used - s0);
       const float wl = lane < cnt ? __expf(partial_lse[base + s0 + lane] - M) : 0.f;
-#pragma unroll 4
+#pragma unroll 8
       for (int k = 0; k < cnt; k++) {
         const float w = __shfl_sync(0xffffffffu, wl, k);
         L += w;
