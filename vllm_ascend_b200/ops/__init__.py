@@ -327,18 +327,20 @@ _FEW_ROWS = 256
 
 @functools.lru_cache(maxsize=8192)
 def _few_rows_faster(M: int, N: int, K: int, glu: bool) -> bool:
-    """Where the few-row kernel beats the general ones.  us per product in a captured chain of norms and products with cold weights on a
-    B200, general -> few-row:
+    """Where the few-row kernel beats the general ones.  us per product, products with cold weights one after the other in a captured graph
+    on a B200, general -> few-row:
 
-    up to 32 rows     wherever weights are streamed: 4096 x 4096 28 -> 16, 24576 x 4096 62 -> 43, 151936 x 2048 150 -> 100, 2048 x 512 11 -> 9
-    33..64 rows       K unsplit (below 2048) costs its serial sums: 64 rows of 4096 x 1536 16 -> 18.  Three splits: 4096 x 2048 19 -> 13,
-                      10240 x 2048 20.5 -> 20.3.  Fewer: 14336 x 2048 22 -> 23, x 4096 33 -> 32; wider than the GPU in one go 24576 x 2048 34 -> 29
-    65..256 rows      stages carry as many or twice as many activations as weights: four splits, 128 rows of 8192 x 2048 20.0 -> 19.4, 256 of
-                      4096 x 2048 20 -> 18; three, 128 rows of 10240 x 2048 21 -> 23, x 4096 32 -> 30; fewer, 128 rows of 14336 x 4096 34 -> 36, 256
-                      of 6144 x 4096 32 -> 32.  Up to 128 rows of more tiles than SMs but no more than two per SM (one wave here, two in the
-                      general kernel) 24576 x 4096 58 -> 51, 32000 x 4096 60 -> 60
-    gate and up       nearly everywhere: 64 rows of 2 x 12288 x 4096 65 -> 47.  Level or behind: from 113 rows on with more tiles than run at
-                      once (128 rows of 2 x 28672 x 2048 29 -> 31), from 193 rows on with K unsplit (256 of 2 x 768 x 1024 24 -> 26)
+    up to 32 rows     wherever weights are streamed: 32 rows of 4096 x 4096 20 -> 10, 32000 x 4096 49 -> 44, 12288 x 2048 15.0 -> 14.2
+    33..64 rows       K unsplit (below 2048) costs its serial sums: 64 rows of 6144 x 1536 11 -> 13.  Three splits or more: 5120 x 2048 12.5 ->
+                      10.4, 6144 x 4096 20 -> 14.  Two: 12288 x 2048 15 -> 17; wider than the GPU in one go 32000 x 2048 27.5 -> 25
+    65..256 rows      stages carry as many or twice as many activations as weights: eight splits, 128 rows of 4096 x 4096 19 -> 15, 256 of
+                      2048 x 4096 18.2 -> 18.1; four, 256 of 4096 x 12288 44 -> 35; three, 256 of 5120 x 2048 13 -> 22; two, 256 of 6144 x 4096
+                      20 -> 33.  Up to 128 rows of more tiles than SMs but no more than two per SM (one wave here, two in the general kernel)
+                      32000 x 4096 52 -> 51
+    gate and up       up to 128 rows: 64 rows of 2 x 12288 x 4096 47 -> 40, 128 of it 48 -> 45, of 2 x 6144 x 2048 level.  From 129 rows on a
+                      block has an SM to itself: one wave of blocks on at least three quarters of the SMs 192 rows of 2 x 9216 x 4096 42 -> 37,
+                      of 2 x 8192 x 2048 27 -> 24; on three fifths 129 rows of 2 x 6144 x 2048 23 -> 19, 160 22.6 -> 21.5, 176 level; two waves
+                      are behind (137 rows of 2 x 12288 x 4096 51 -> 57), few blocks level (137 rows of 2 x 4096 x 2048 18.1 -> 18.6)
     """
     splits = _native.lib().b200_gemm_small_splits(M, N, K, int(glu))
     sms = _native.sm_count(torch.cuda.current_device())
@@ -347,6 +349,9 @@ def _few_rows_faster(M: int, N: int, K: int, glu: bool) -> bool:
     if glu:
         if M <= 128:
             return M <= 112 or (N + 63) // 64 <= 2 * sms
+        tiles = (N + 63) // 64
+        if K >= 2048 and tiles <= sms and tiles * 5 >= sms * 3:
+            return M <= (192 if tiles * 4 >= sms * 3 else 160)
         return 2 * N <= 5120 and (M <= 192 or K >= 2048)
     if M <= 32:
         return True
@@ -368,9 +373,9 @@ def _few_rows(M: int, N: int, K: int, glu: bool = False) -> bool:
 
 def _pair_rows(M: int, N: int, K: int, glu: bool = False) -> bool:
     """129 to 255 rows, which fill more than half of a paired tile of 256: N columns that keep the GPU busy for more than one wave of
-    128 x 128 tiles read their weights once there and twice in those tiles (137 rows of 24576 x 4096: 87 us in two tiles, 77 us in
-    one; 144 rows of 10240 x 1024 20 -> 17 us).  Narrower ones leave half of the pairs without a tile (144 rows of 8192 x 4096 32 -> 34 us), and
-    K below 1024 is all prologue (of 16384 x 512 15 -> 17 us).  Gate and up: K from 2048 on (2 x 4096 x 4096 57 -> 55 us, x 1024 38 -> 39).  The
+    128 x 128 tiles read their weights once there and twice in those tiles (137 rows of 32000 x 4096: 65 us in two tiles, 57 us in
+    one; 12288 x 2048 21 -> 18 us).  Narrower ones leave half of the pairs without a tile (6144 x 1536 11.5 -> 11.8 us), and
+    K below 1024 is all prologue.  Gate and up: K from 2048 on (2 x 12288 x 4096 66 -> 51 us, 2 x 6144 x 2048 27 -> 23).  The
     same bits.  A user's larger VLLM_B200_GEMM_2CTA_MIN_M holds."""
     if not 128 < M <= 256 or K < (2048 if glu else 1024):
         return False

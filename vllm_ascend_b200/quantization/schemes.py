@@ -132,14 +132,14 @@ _FP8_FEW_ROWS = 128
 
 @functools.lru_cache(maxsize=8192)
 def _fp8_few_rows_faster(M: int, N: int, K: int) -> bool:
-    """Where the few-row kernel beats the general one.  us per quantisation and product in a captured chain with cold weights on a B200,
-    general -> few-row:
+    """Where the few-row kernel beats the general one.  us per product, products with cold weights one after the other in a captured graph on
+    a B200, general -> few-row:
 
-    up to 32 rows   K of 1024 and more: 8192 x 2048 14 -> 12, 57344 x 8192 99 -> 84; 8192 x 512 8 -> 8, x 256 7 -> 8
-    33..64 rows     64 rows of 4096 x 4096 20 -> 16, 10240 x 4096 22 -> 21 (three splits), 14336 x 4096 22 -> 24 and x 8192 37 -> 33 (two); of K = 2048
-                    6144 columns 14.8 -> 14.1, 8192 columns 14.6 -> 15
-    65..128 rows    one block per SM, and its promotion takes as long as the general kernel's: 128 rows of 4096 x 4096 22 -> 18 (four), 8192 x 4096
-                    23 -> 23 and x 8192 37 -> 32 (two), 28672 x 8192 55 -> 95 (one)
+    up to 32 rows   K of 1024 and more: 32 rows of 8192 x 2048 11 -> 8, 57344 x 8192 89 -> 78
+    33..64 rows     64 rows of 4096 x 4096 14 -> 12, 10240 x 4096 15.4 -> 16.0 (three splits) and x 8192 25 -> 23, 14336 x 4096 16 -> 19 and x 8192
+                    26 -> 28 (two); of K = 2048 2048 columns 9.0 -> 7.2, 6144 10.1 -> 10.5, 8192 10 -> 11
+    65..128 rows    one block per SM, and its promotion takes as long as the general kernel's: 128 rows of 4096 x 4096 15.6 -> 13.8 (four), 8192 x 4096
+                    16 -> 18, x 8192 25.6 -> 26.6 and x 28672 73 -> 82 (two), 28672 x 8192 50 -> 91 (one)
     """
     splits = _native.lib().b200_gemm_small_fp8_splits(M, N, K)
     if splits < 1:
@@ -148,7 +148,7 @@ def _fp8_few_rows_faster(M: int, N: int, K: int) -> bool:
         return K >= 1024
     if M <= 64:
         return K >= 8192 or (K >= 4096 and splits >= 3) or (K >= 2048 and N <= 6144)
-    return (K >= 4096 and splits >= 3) or (K >= 8192 and splits >= 2)
+    return K >= 4096 and splits >= 3
 
 
 def fp8_block_linear(x: Optional[torch.Tensor], w8: torch.Tensor, w_scale: torch.Tensor,
