@@ -576,8 +576,8 @@ static int launch_2cta(const void* A, const void* W, Gemm2Params& p, int lda, in
   if (clusters > max_clusters) clusters = max_clusters;
   p.raster = g_raster;
   // L2 prefetch of the streamed operands ahead of the staged loads: measured neutral to slightly
-  // negative on decode-sized problems (768 x 4096 x 12288: 0.0799 ms off, 0.0799 / 0.0810 / 0.0819 ms
-  // at 8 / 16 / 32 k-blocks), so it is off unless asked for
+  // negative on decode-sized problems (768 x 4096 x 12288, when it took 0.0799 ms without: 0.0799 / 0.0810 / 0.0819 ms
+  // at 8 / 16 / 32 k-blocks; now 0.0646 without), so it is off unless asked for
   p.l2_prefetch = g_l2_prefetch > 0 ? g_l2_prefetch : 0;
   gemm_bf16_2cta_kernel<<<2 * clusters, G2_THREADS, G2_SMEM_BYTES, stream>>>(ta, tb, p);
   return B200_CHECK_LAUNCH();

@@ -12,8 +12,8 @@
 //     one block's prologue and reduction hide behind the other's loads;
 //   * launched as a programmatic dependent: barriers, TMEM and an L2 prefetch of the block's own weights (L2 is the point
 //     of coherence, so the prefetch reads nothing early) are under way while the previous kernel finishes.
-// One row, us with cold caches, general kernel -> this one: 4096 x 4096 32 -> 17, 4096 x 12288 71 -> 32, 24576 x 4096
-// (gate / up) 80 -> 53, 151936 x 4096 282 -> 204 (6.1 TB/s).
+// One row, us with cold weights in a captured chain, general kernel -> this one: 4096 x 4096 25 -> 9, 4096 x 12288 62 -> 17,
+// 24576 x 4096 (gate / up) 58 -> 36, 32000 x 4096 71 -> 43 (6.2 TB/s).
 // Roles: warps 0..3 read the accumulator (one TMEM lane quarter each), warp 4 issues TMA, warp 5 issues
 // tcgen05.mma (cta_group::1, M = 128, N = tokens, K = 16, f32 in TMEM); all six reduce and store.
 #include "cluster_sum.cuh"
