@@ -18,12 +18,8 @@ struct DeltaChunkArgs {
   long num_slots;
   int min_len;                         // sequences with fewer tokens are left alone
   int* status;
-  int B;
-  float* ws;                           // workspace
-  int c0, per_seq;                     // slices: chunks c0 .. c0 + per_seq - 1 of every sequence; per_seq 0: all chunks
 };
 
-long delta_chunk_place_bytes();
-bool launch_delta_chunk(DeltaChunkArgs p, long tokens, int max_len, long ws_bytes, int DK, cudaStream_t stream, int* rc);
+bool launch_delta_chunk(const DeltaChunkArgs& p, int B, int DK, cudaStream_t stream, int* rc);
 
 }  // namespace b200

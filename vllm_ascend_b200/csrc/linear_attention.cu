@@ -640,16 +640,15 @@ B200_API int b200_causal_conv1d(const void* x, long x_stride, const void* w, con
 }
 
 // chunk_min > 0: sequences of at least that many tokens run in chunks where the sizes allow it (delta_chunk.cu); any_short:
-// there are shorter ones; tokens: of the step, max_len: of its longest sequence; ws: a workspace of ws_bytes
-// (delta_chunk_place_bytes() a head for every 64 tokens and every sequence; less is taken in slices).  uniform: every sequence of the step has exactly one token.  z (optional, with norm_w [DV] and eps, uniform
+// there are shorter ones.  uniform: every sequence of the step has exactly one token.  z (optional, with norm_w [DV] and eps, uniform
 // steps only): the output is the gated RMS norm of the read-out; returns -1 when the sizes do not allow that.
 B200_API int b200_gated_delta_rule(const void* q, const void* k, const void* v, long qk_stride,
                                    long v_stride, const void* g, const void* beta, void* state,
                                    const void* cu, const void* slots, const void* has_init, void* out,
                                    long out_stride, int B, int Hk, int Hv, int DK, int DV, float scale,
                                    int l2norm, long num_slots, int dtype, int uniform, const void* z, long z_stride,
-                                   const void* norm_w, float eps, int chunk_min, int any_short, long tokens, int max_len,
-                                   void* ws, long ws_bytes, int* status, cudaStream_t stream) {
+                                   const void* norm_w, float eps, int chunk_min, int any_short, int* status,
+                                   cudaStream_t stream) {
   if (B <= 0) return 0;
   if (Hk <= 0 || Hv % Hk || Hv > 65535) return 9801;
   DeltaParams p{q, k, v, qk_stride, v_stride, (const float*)g, (const float*)beta, (float*)state, (const int*)cu,
@@ -666,9 +665,9 @@ B200_API int b200_gated_delta_rule(const void* q, const void* k, const void* v, 
   if (chunk_min > 0 && dtype == 0) {
     const DeltaChunkArgs a{q, k, v, qk_stride, v_stride, (const float*)g, (const float*)beta, (float*)state, (const int*)cu,
                            (const int*)slots, (const int*)has_init, out, out_stride, Hk, Hv, DV, scale, l2norm, num_slots,
-                           chunk_min, status, B, (float*)ws, 0, 0};
+                           chunk_min, status};
     int rc = 0;
-    if (launch_delta_chunk(a, tokens, max_len, ws_bytes, DK, stream, &rc)) {
+    if (launch_delta_chunk(a, B, DK, stream, &rc)) {
       if (rc || !any_short) return rc;
       p.max_len = chunk_min;
     }

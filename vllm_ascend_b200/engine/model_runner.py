@@ -262,17 +262,13 @@ class ModelRunner:
         return int(1.3 * (T * per_tok + logits)) + (1 << 30) + self._prompt_workspace_bytes()
 
     def _prompt_workspace_bytes(self) -> int:
-        """Latent attention's workspace for prompts, by the keys that a step can look at, or the delta rule's for chunks of tokens."""
-        from ..models.gdn import GatedDeltaNet
-        from ..ops.linear_attn import chunk_workspace_bytes
-        layers = [L.self_attn for L in self.model.layers]
-        chunks = max((chunk_workspace_bytes(self.max_tokens, self.max_seqs, a.Hv) for a in layers if isinstance(a, GatedDeltaNet)), default=0)
+        """Latent attention's workspace for prompts: by the keys that a step can look at."""
         if self.dcp_size > 1:
-            return chunks
+            return 0
         from ..attention.mla import expanded_workspace
         keys = self.max_seqs * self.max_blocks_per_seq * self.block_size
-        return max((expanded_workspace(a.H, a.dn, a.dr, a.dv, a.dc, keys) for a in layers
-                    if hasattr(a, "kv_b_proj") and not (a.window or a.sink is not None or a.index_topk)), default=chunks)
+        return max((expanded_workspace(a.H, a.dn, a.dr, a.dv, a.dc, keys) for a in (L.self_attn for L in self.model.layers)
+                    if hasattr(a, "kv_b_proj") and not (a.window or a.sink is not None or a.index_topk)), default=0)
 
     def determine_num_blocks(self) -> int:
         cc = self.cfg.cache

@@ -19,7 +19,7 @@ P, I, L, Fl = c_void_p, c_int, c_long, c_float
 _native.register_signature("b200_causal_conv1d", [P, L, P, P, P, P, P, P, P, L, L, I, I, I, I, I, L, I, P, L, P, P, I, P, P,
                                                   P, P])
 _native.register_signature("b200_gated_delta_rule", [P, P, P, L, L, P, P, P, P, P, P, P, L, I, I, I, I, I, Fl, I,
-                                                     L, I, I, P, L, P, Fl, I, I, L, I, P, L, P, P])
+                                                     L, I, I, P, L, P, Fl, I, I, P, P])
 _DTYPES = {torch.bfloat16: 0, torch.float32: 1}
 
 
@@ -204,7 +204,7 @@ def gated_delta_rule_chunked(q, k, v, g, beta, state, cu_cpu, slots, has_init, s
 def _chunk_min(on_cuda: bool = False) -> int:
     """Fewest new tokens of a sequence that take the chunk-parallel form built from fp32 matrix products; 0 = never.
     Unset, the form serves host tensors only: on a B200 it takes 10.3 ms for 4 x 2048 tokens of 32 heads, the kernels 1.3 ms token
-    by token (three prompts of 2000 tokens: 1.6 ms, and 0.35 ms in chunks: ``_portions``)."""
+    by token (three prompts of 2000 tokens: 1.6 ms, and 0.8 ms in chunks: ``_portions``)."""
     if on_cuda and _chunk_flag() is None:
         return 0
     return int(envs.VLLM_B200_GDN_CHUNK_MIN)
@@ -213,11 +213,10 @@ def _chunk_min(on_cuda: bool = False) -> int:
 def _kernel_times(lens: np.ndarray, Hv: int, DV: int, sms: int, least: int) -> float:
     """Estimated us of a step whose sequences of ``least`` tokens and more run in chunks of 64 and the others token by token.
 
-    In chunks: a block of every head prepares a chunk, 0.047 us of the GPU each, and blocks of 64 value columns, two to an SM, take 8 us and 5.4 us
-    per chunk, full or not (4.4 us alone on their SM); counted 1.3 times, so that portions run in chunks where that is clearly the shorter way.  A
-    block of the token-serial kernel, of which three share an SM, takes 0.42 us per token alone and 0.79 us among others.  Blocks run in waves,
-    or packed one behind the other where they differ, whichever is shorter.  32 heads, token by token and in chunks: 16 portions of 32
-    tokens 75 and 77 us, 12 of 64 117 and 65, 64 of 65 517 and 415, one of 128 60 and 30, three of 2000 1600 and 350."""
+    A block of the chunked kernel keeps an SM to itself and takes 18.5 us per chunk, full or not (14.3 us where every block of 64 value columns has
+    its own SM); one of the token-serial kernel, of which three share an SM, takes 0.42 us per token alone and 0.79 us among others.  Blocks
+    run in waves, or packed one behind the other where they differ, whichever is shorter.  16 portions of 32 tokens, 32 heads: 88 us token by
+    token, 104 us in chunks (estimates 89 and 106); 64 of 65 tokens 555 and 608 (563 and 618); one of 128 tokens 68 and 41 (68 and 35)."""
     def packed(each, blocks, slots):
         n = len(each) * blocks
         longest = float(each.max())
@@ -226,8 +225,8 @@ def _kernel_times(lens: np.ndarray, Hv: int, DV: int, sms: int, least: int) -> f
     us, halves = 0.0, Hv * -(-DV // 64)
     if len(far):
         chunks = -(-far // 64)
-        us += 1.3 * (6 + 0.047 * Hv * float(chunks.sum())
-                     + packed(8 + (4.4 if len(far) * halves <= sms else 5.4) * chunks, halves, 2 * sms))
+        us += 6 + (packed(14.3 * chunks, halves, sms) if DV % 128 or len(lens) * halves <= sms
+                   else packed(6.7 + 18.5 * chunks, Hv * (DV // 128), sms))
     if len(near):
         us += packed(14 + 0.42 * near, halves, sms) if len(near) * halves <= sms else packed(6.5 + 0.79 * near, halves, 3 * sms)
     return us
@@ -251,13 +250,8 @@ def _token_by_token() -> bool:
     return fixed_sums() or _chunk_flag() == b"0"
 
 
-#: bytes that a chunk of 64 tokens leaves per head in the workspace, and the most that a workspace takes (a longer step goes in slices)
-_CHUNK_PLACE, _CHUNK_WORKSPACE = 4 * (2 * 2560 + 4 * 64 + 16), 128 << 20
-
-
-def chunk_workspace_bytes(tokens: int, seqs: int, Hv: int) -> int:
-    """Workspace of a step's chunks: a place per head for every 64 tokens and for every sequence, or at least the last."""
-    return max(min((tokens // 64 + seqs) * Hv * _CHUNK_PLACE, _CHUNK_WORKSPACE), seqs * Hv * _CHUNK_PLACE)
+#: bytes of workspace that a chunk of 64 tokens takes per head, and the most that a step takes: the kernel keeps its chunk in shared memory
+_CHUNK_PLACE = _CHUNK_WORKSPACE = 0
 
 
 def gated_delta_rule(q, k, v, g, beta, state, cu, slots, has_init, scale, l2norm=True, cu_cpu=None, uniform=False,
@@ -304,18 +298,14 @@ def gated_delta_rule(q, k, v, g, beta, state, cu, slots, has_init, scale, l2norm
     if cu_cpu is not None and not uniform and not _token_by_token():
         chunk_min, any_short = _portions(np.ascontiguousarray(cu_cpu, dtype=np.int32)[:cu.numel()].tobytes(), Hv, DV,
                                          _native.sm_count(q.device))
-    B, max_len, ws = cu.numel() - 1, 0, None
-    if chunk_min > 0 and DK == 128 and q.dtype == torch.bfloat16:
-        max_len = int(np.diff(np.asarray(cu_cpu)[:B + 1]).max())
-        ws = torch.empty(chunk_workspace_bytes(T, B, Hv), dtype=torch.uint8, device=q.device)
     for z in ((gate[0], None) if fused else (None,)):
         rc = _native.lib().b200_gated_delta_rule(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), v.stride(0), g.data_ptr(), beta.data_ptr(),
             state.data_ptr(), cu.data_ptr(), slots.data_ptr(), has_init.data_ptr(), out.data_ptr(), out.stride(0),
-            B, Hk, Hv, DK, DV, scale, int(l2norm), state.shape[0], _DTYPES[q.dtype], int(uniform),
+            cu.numel() - 1, Hk, Hv, DK, DV, scale, int(l2norm), state.shape[0], _DTYPES[q.dtype], int(uniform),
             _native.ptr(z), 0 if z is None else z.stride(0), None if z is None else gate[1].data_ptr(),
-            0.0 if z is None else float(gate[2]), chunk_min, any_short, T, max_len, _native.ptr(ws), 0 if ws is None else ws.numel(),
-            _native.status_word(q.device).data_ptr(), _native.stream_ptr())
+            0.0 if z is None else float(gate[2]), chunk_min, any_short, _native.status_word(q.device).data_ptr(),
+            _native.stream_ptr())
         if rc != -1:                  # -1: these sizes have no fused form, nothing was launched
             break
     _native.check(rc, "gated_delta_rule")
