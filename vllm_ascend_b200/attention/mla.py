@@ -19,22 +19,19 @@ from ctypes import c_float, c_int, c_long, c_void_p
 
 from .. import _native
 from ..ops import reference as ref
+from ..ops.scratch import Scratch
 
 _P, _I, _L, _F = c_void_p, c_int, c_long, c_float
 _native.register_signature("b200_mla_attention", [_P, _L, _L, _P, _L, _L, _L, _I, _I, _I, _P, _P, _L, _I, _P, _P, _P, _P,
                                                   _I, _I, _P, _I, _P, _I, _F, _I, _P, _L, _L, _P, _P, _P, _P])
 _native.register_signature("b200_latent_attention", [_P, _L, _L, _P, _L, _L, _L, _I, _I, _I, _P, _P, _L, _I, _P, _P, _P,
                                                      _I, _P, _F, _I, _P, _L, _L, _I, _P, _P])
-_scratch: dict = {}
+_scratch = Scratch(torch.float32)
 _MAX_SPLITS = 32
 
 
 def _split_scratch(dev, numel: int) -> torch.Tensor:
-    buf = _scratch.get(dev.index)
-    if buf is None or buf.numel() < numel:
-        buf = torch.empty(max(numel, 1 << 20), dtype=torch.float32, device=dev)
-        _scratch[dev.index] = buf
-    return buf
+    return _scratch.get(dev, numel)
 
 
 def _most_splits(sms: int, ctas: int) -> int:

@@ -380,7 +380,8 @@ def variant_attention_decode(q, k_cache, v_cache, meta, o: AttnOptions, gate=Non
     a.num_seqs = num_seqs
     a.num_splits = num_splits or decode_splits(num_seqs, a.kv_heads, o, meta.block_table.shape[1] * a.block_size, q.device)
     if a.num_splits > 1:
-        a.scratch = ops._get_scratch(q.device, num_seqs * a.heads * a.num_splits * (a.vdim + 1) * 4).data_ptr()
+        scratch = ops._get_scratch(q.device, num_seqs * a.heads * a.num_splits * (a.vdim + 1) * 4)      # held until the launch
+        a.scratch = scratch.data_ptr()
     _launch("b200_attention_variant_decode", a, q.device, 2 if a.num_splits > 1 else 1)
     return out
 
@@ -395,7 +396,8 @@ def wide_attention_decode(q, k_cache, v_cache, meta, o: AttnOptions, out=None, n
     a.num_seqs = num_seqs
     a.num_splits = num_splits or decode_splits(num_seqs, a.key_heads, o, meta.block_table.shape[1] * a.block_size, q.device)
     if a.num_splits > 1:
-        a.scratch = ops._get_scratch(q.device, num_seqs * a.heads * a.num_splits * (a.vdim + 1) * 4).data_ptr()
+        scratch = ops._get_scratch(q.device, num_seqs * a.heads * a.num_splits * (a.vdim + 1) * 4)      # held until the launch
+        a.scratch = scratch.data_ptr()
     _launch("b200_attention_wide_decode", a, q.device, 2 if a.num_splits > 1 else 1)
     return out
 

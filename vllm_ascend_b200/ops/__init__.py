@@ -20,6 +20,7 @@ import torch
 from .. import _native, envs
 from ..batch_invariant import fixed_sums, is_batch_invariant, is_training_consistent
 from . import reference as ref
+from .scratch import Scratch
 
 _BF16 = torch.bfloat16
 
@@ -425,17 +426,12 @@ def linear_swiglu_step(x: torch.Tensor, weight: torch.Tensor, limit: Optional[fl
 
 
 # ---------------------------------------------------------------- attention
-_scratch: dict = {}
+_scratch = Scratch(torch.uint8)
 
 
 def _get_scratch(device, nbytes: int) -> torch.Tensor:
-    """Grow-only per-device scratch (split-KV partials)."""
-    key = (device.type, device.index)
-    buf = _scratch.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _scratch[key] = buf
-    return buf
+    """Per-device scratch (split-KV partials)."""
+    return _scratch.get(device, nbytes)
 
 
 def reserve_attention_scratch(device, nbytes: int) -> None:
