@@ -18,12 +18,13 @@ import torch
 from ctypes import c_float, c_int, c_long, c_void_p
 
 from .. import _native
+from ..batch_invariant import fixed_sums
 from ..ops import reference as ref
 from ..ops.scratch import Scratch
 
 _P, _I, _L, _F = c_void_p, c_int, c_long, c_float
 _native.register_signature("b200_mla_attention", [_P, _L, _L, _P, _L, _L, _L, _I, _I, _I, _P, _P, _L, _I, _P, _P, _P, _P,
-                                                  _I, _I, _P, _I, _P, _I, _F, _I, _P, _L, _L, _P, _P, _P, _P])
+                                                  _I, _I, _P, _I, _P, _I, _F, _I, _I, _P, _L, _L, _P, _P, _P, _P])
 _native.register_signature("b200_latent_attention", [_P, _L, _L, _P, _L, _L, _L, _I, _I, _I, _P, _P, _L, _I, _P, _P, _P,
                                                      _I, _P, _F, _I, _P, _L, _L, _I, _P, _P])
 _scratch = Scratch(torch.float32)
@@ -45,9 +46,9 @@ def _best_splits(sms: int, ctas: int, tiles: int) -> int:
 
 def _num_splits(dev, ctas: int, max_keys: int) -> int:
     """Most splits of a key range: at most one per 128-key tile and two CTAs per SM; one where whole sequences fill the SMs as
-    well.  The kernel sets the tiles of a split from the lengths that it finds, so a short sequence uses fewer of them."""
-    from ..batch_invariant import is_batch_invariant
-    if is_batch_invariant():
+    well, and in modes that fix the order of sums.  The kernel sets the tiles of a split from the lengths that it finds, so a short sequence
+    uses fewer of them."""
+    if fixed_sums():
         return 1
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
     ctas, tiles = max(ctas, 1), max(1, (max_keys + 127) // 128)
@@ -100,7 +101,7 @@ def latent_attention_tc(q_lat: torch.Tensor, q_pe: torch.Tensor, lat_cache: torc
         q_pe.shape[2], lat_cache.data_ptr(), pe_cache.data_ptr(), lat_cache.shape[0], lat_cache.shape[1],
         _native.ptr(row_seq), _native.ptr(row_kv_len), _native.ptr(cu), _native.ptr(seq_lens), B, int(uniform),
         block_table.data_ptr(), block_table.stride(0), _native.ptr(sink), int(window), scale, num_splits,
-        out.data_ptr(), out.stride(0), out.stride(1), _native.ptr(scratch), _native.ptr(lse_out),
+        int(fixed_sums()), out.data_ptr(), out.stride(0), out.stride(1), _native.ptr(scratch), _native.ptr(lse_out),
         _native.status_word(dev).data_ptr(), _native.stream_ptr())
     _native.check(rc, "mla_attention")
     _native.count_launch(2 if num_splits > 1 else 1)
@@ -259,7 +260,6 @@ def expanded_prompts(meta, heads: int, dn: int, dr: int, dv: int, q: torch.Tenso
     place (decode steps, few new tokens behind long contexts) or the only one (captured steps, modes that fix the order of sums)."""
     import numpy as np
     from .. import envs
-    from ..batch_invariant import fixed_sums
     if not (q.is_cuda and q.dtype == lat_cache.dtype == torch.bfloat16 and meta.max_query_len > 1
             and envs.VLLM_B200_MLA_ATTN == "tcgen05") or fixed_sums() or torch.cuda.is_current_stream_capturing():
         return None

@@ -18,6 +18,7 @@ from typing import Optional
 import torch
 
 from .. import _native
+from ..batch_invariant import fixed_sums
 from ..ops import linear_attn as la
 from ..ops import reference as ref
 
@@ -38,7 +39,7 @@ class _AttnArgs(ctypes.Structure):
         pointers="q k_cache v_cache out cu seq_lens block_table row_seq row_kv_len bias sink gate scratch",
         longs="q_stride out_stride gate_stride num_blocks tokens k_block k_tok k_head v_block v_tok v_head",
         ints="num_seqs max_blocks block_size heads kv_heads dim vdim window keep_first bias_len num_splits dtype key_heads "
-             "out_f32", floats="scale softcap out_scale")
+             "out_f32 even_parts", floats="scale softcap out_scale")
 
 
 _ENTRY = [c_void_p, c_void_p, c_void_p]
@@ -294,7 +295,7 @@ def _args(q, k_cache, v_cache, meta, o: AttnOptions, gate, out) -> _AttnArgs:
         dim=q.shape[2], vdim=v_cache.shape[3], window=o.window, keep_first=o.keep_first if o.window else 0,
         bias_len=0 if o.bias is None else o.bias.shape[1], num_splits=1, dtype=int(q.dtype == torch.float32),
         scale=o.scale, softcap=o.softcap, key_heads=k_cache.shape[2], out_f32=int(out.dtype == torch.float32),
-        out_scale=o.out_scale)
+        even_parts=int(fixed_sums()), out_scale=o.out_scale)
     a.hold = gate                    # alive until the launch
     return a
 
@@ -347,9 +348,8 @@ def _kernels(q, k_cache, v_cache, out, o: AttnOptions, gate=None) -> tuple[Optio
 
 def decode_splits(num_seqs: int, kv_heads: int, o: AttnOptions, max_keys: int, device) -> int:
     """Splits of the key range of a decode batch: about one work item per SM, none below two tiles.  Depends on
-    the batch size and the capacity only, so that a captured graph and an eager step agree."""
-    from ..batch_invariant import is_batch_invariant
-    if is_batch_invariant():
+    the batch size and the capacity only, so that a captured graph and an eager step agree; one in modes that fix the order of sums."""
+    if fixed_sums():
         return 1
     keys = min(max_keys, o.window + 127 + ((o.keep_first + 127) // 128) * 128) if o.window else max_keys
     tiles = (keys + 127) // 128

@@ -819,15 +819,15 @@ static int launch_decode_nv(const CUtensorMap& tq, const CUtensorMap& tk, const 
   return B200_CHECK_LAUNCH();
 }
 
-// fills in the item count; ncols: columns that can be valid
+// fills in the item count; ncols: columns that can be valid; even_parts: no stretches, whose cuts depend on all lengths of the batch
 template <bool VAR>
 static int launch_decode(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tk32,
-                         const CUtensorMap& tv32, DecParams& p, int ncols, cudaStream_t stream) {
+                         const CUtensorMap& tv32, DecParams& p, int ncols, bool even_parts, cudaStream_t stream) {
   const long items = (long)p.Hkv * p.num_seqs * p.num_splits;
   if (items > 0x7fffffffL) return 9125;
   if (ncols > DEC_NQ) return 9126;
   p.num_items = (int)items;
-  p.stretches = p.num_splits > 1 && p.num_seqs >= DEC_STRETCH_SEQS;
+  p.stretches = p.num_splits > 1 && !even_parts && p.num_seqs >= DEC_STRETCH_SEQS;
   static int sm_count[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 9127;
@@ -858,13 +858,14 @@ B200_API int b200_attn_decode_set_l2_prefetch(int tiles) {
 // scratch needs b200_attn_scratch_bytes(T, Hq, D, num_splits) bytes when num_splits > 1.
 // lse_out (optional, fp32 [T, Hq]): log-sum-exp of every (token, head) over the keys this call saw,
 // for callers that merge the results of several calls (context-parallel ranks).
+// even_parts: the splits are even parts of every sequence by itself, whatever the others' lengths.
 B200_API int b200_attn_decode_tc_lse(const void* q, long q_stride, long T, const void* k_cache,
                                      const void* v_cache, long num_blocks, int block_size,
                                      const void* query_start_loc, const void* seq_lens,
                                      const void* block_table, int max_blocks, int num_seqs, int Hq,
                                      int Hkv, int D, float scale, int window, int num_splits,
                                      int max_q_len, void* out, long out_stride, void* scratch,
-                                     int kv_layout, void* lse_out,
+                                     int kv_layout, void* lse_out, int even_parts,
                                      int* status, void* timeline, cudaStream_t stream) {
   using namespace b200;
   if (num_seqs <= 0 || T <= 0) return 0;
@@ -936,7 +937,7 @@ B200_API int b200_attn_decode_tc_lse(const void* q, long q_stride, long T, const
   p.l2_prefetch = g_dec_l2_prefetch;
   p.keep_first = 0;
   {
-    const int lrc = launch_decode<false>(tq, tk, tv, tk32, tv32, p, max_q_len * G, stream);
+    const int lrc = launch_decode<false>(tq, tk, tv, tk32, tv32, p, max_q_len * G, even_parts != 0, stream);
     if (lrc) return lrc;
   }
   if (num_splits > 1)
@@ -956,7 +957,7 @@ B200_API int b200_attn_decode_tc(const void* q, long q_stride, long T, const voi
   return b200_attn_decode_tc_lse(q, q_stride, T, k_cache, v_cache, num_blocks, block_size,
                                  query_start_loc, seq_lens, block_table, max_blocks, num_seqs, Hq,
                                  Hkv, D, scale, window, num_splits, max_q_len, out, out_stride,
-                                 scratch, kv_layout, nullptr, status, timeline, stream);
+                                 scratch, kv_layout, nullptr, 0, status, timeline, stream);
 }
 
 // Options as in AttnVariantArgs; one query token per sequence (row b of q belongs to sequence b), bf16, D and Dv
@@ -1019,7 +1020,7 @@ B200_API int b200_attention_variant_decode(const b200::AttnVariantArgs* a, int* 
   p.bias = a->bias; p.sink = a->sink;
   p.gate = (const __nv_bfloat16*)a->gate;
   p.gate_stride = a->gate_stride;
-  int rc = launch_decode<true>(tq, tkv[0], tkv[1], tkv32[0], tkv32[1], p, G, stream);
+  int rc = launch_decode<true>(tq, tkv[0], tkv[1], tkv32[0], tkv32[1], p, G, a->even_parts != 0, stream);
   if (rc) return rc;
   if (a->num_splits > 1)
     return launch_merge_splits(p.partial_o, p.partial_lse, a->num_seqs, a->Hq, a->num_splits, a->Dv, a->out,

@@ -582,13 +582,14 @@ static int launch_mla(const CUtensorMap& tq, const CUtensorMap& tqp, const CUten
 // out: [R, H, dc] with row / head strides.  scratch: R * H * num_splits * (dc + 1) floats when num_splits > 1.
 // lse_out (optional, fp32 [R, H]): log-sum-exp of every (row, head) over the keys the row saw, for
 // callers that merge the results of several calls (context-parallel ranks).  It is produced by the
-// split merge, so a call that wants it runs with at least two KV splits.
+// split merge, so a call that wants it runs with at least two KV splits.  even_parts: the splits are even parts of every sequence by itself,
+// so that where a row's keys are cut does not depend on its neighbours; otherwise they take a common number of tiles.
 B200_API int b200_mla_attention(const void* q_lat, long ql_row, long ql_head, const void* q_pe, long qp_row,
                                 long qp_head, long R, int H, int dc, int dr, const void* lat_cache,
                                 const void* pe_cache, long num_blocks, int block_size, const void* row_seq,
                                 const void* row_kv_len, const void* cu, const void* seq_lens, int B, int uniform,
                                 const void* block_table, int max_blocks, const void* sink, int window, float scale,
-                                int num_splits, void* out, long out_stride, long out_head, void* scratch,
+                                int num_splits, int even_parts, void* out, long out_stride, long out_head, void* scratch,
                                 void* lse_out, int* status, cudaStream_t stream) {
   using namespace b200;
   if (R <= 0) return 0;
@@ -658,7 +659,7 @@ B200_API int b200_mla_attention(const void* q_lat, long ql_row, long ql_head, co
   p.num_splits = num_splits;
   p.rows = (int)R;
   // a long list of sequences fills the SMs as it is, and every CTA would read all of its lengths
-  p.slots = num_splits > 1 && (pack ? (long)B : R) <= 1024 ? (num_sms() > head_blocks ? num_sms() / head_blocks : 1) : 0;
+  p.slots = num_splits > 1 && !even_parts && (pack ? (long)B : R) <= 1024 ? (num_sms() > head_blocks ? num_sms() / head_blocks : 1) : 0;
   p.out = (__nv_bfloat16*)out;
   p.out_stride = out_stride;
   p.out_head = out_head;

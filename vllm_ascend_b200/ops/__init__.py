@@ -18,7 +18,7 @@ import numpy as np
 import torch
 
 from .. import _native, envs
-from ..batch_invariant import fixed_sums, is_batch_invariant, is_training_consistent
+from ..batch_invariant import fixed_sums, is_training_consistent
 from . import reference as ref
 from .scratch import Scratch
 
@@ -552,7 +552,7 @@ def paged_attention_decode_tc(q: torch.Tensor, k_cache: torch.Tensor, v_cache: t
         meta.block_table.stride(0), num_seqs, Hq, Hkv, D, scale, int(window), num_splits,
         max_q_len if max_q_len else min(meta.max_query_len, 16 // (Hq // Hkv)), out.data_ptr(),
         out.stride(0), _native.ptr(scratch), kv_layout(k_cache), _native.ptr(lse_out),
-        _native.status_word(q.device).data_ptr(), _native.ptr(timeline), _native.stream_ptr())
+        int(fixed_sums()), _native.status_word(q.device).data_ptr(), _native.ptr(timeline), _native.stream_ptr())
     _native.check(rc, "attn_decode_tc")
     launch_counter[0] += 1 + (1 if num_splits > 1 else 0)
     return out
@@ -614,8 +614,8 @@ def paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
 def choose_num_splits(num_seqs: int, Hkv: int, max_seq_len: int, sm_count: int = 148,
                       tile: int = 128) -> int:
     """Split-KV factor: enough CTAs to fill the GPU, never more splits than KV tiles.  In
-    batch-invariant mode the factor is 1: the merge order must not depend on the batch."""
-    if is_batch_invariant():
+    modes that fix the order of sums the factor is 1: the merge order must not depend on the batch."""
+    if fixed_sums():
         return 1
     ctas = max(1, num_seqs * Hkv)
     if ctas >= 2 * sm_count:
