@@ -39,7 +39,7 @@ class _AttnArgs(ctypes.Structure):
         pointers="q k_cache v_cache out cu seq_lens block_table row_seq row_kv_len bias sink gate scratch",
         longs="q_stride out_stride gate_stride num_blocks tokens k_block k_tok k_head v_block v_tok v_head",
         ints="num_seqs max_blocks block_size heads kv_heads dim vdim window keep_first bias_len num_splits dtype key_heads "
-             "out_f32 even_parts", floats="scale softcap out_scale")
+             "out_f32", floats="scale softcap out_scale")
 
 
 _ENTRY = [c_void_p, c_void_p, c_void_p]
@@ -295,7 +295,7 @@ def _args(q, k_cache, v_cache, meta, o: AttnOptions, gate, out) -> _AttnArgs:
         dim=q.shape[2], vdim=v_cache.shape[3], window=o.window, keep_first=o.keep_first if o.window else 0,
         bias_len=0 if o.bias is None else o.bias.shape[1], num_splits=1, dtype=int(q.dtype == torch.float32),
         scale=o.scale, softcap=o.softcap, key_heads=k_cache.shape[2], out_f32=int(out.dtype == torch.float32),
-        even_parts=int(fixed_sums()), out_scale=o.out_scale)
+        out_scale=o.out_scale)
     a.hold = gate                    # alive until the launch
     return a
 

@@ -4,8 +4,8 @@ What changes a result with the batch composition here is the reduction order.  T
 choose it from the batch, and what the mode does there:
 
 * the split-KV factor of decode attention (grouped, latent, variants): 1.  Where a context-parallel rank needs the log-sum-exp
-  of latent attention, which two splits give, or a caller names a factor, the splits are even parts of each sequence by itself;
-  in other modes they are cut by the lengths of all sequences of the step;
+  of latent attention, which two splits give, or a caller names a factor, the splits are even parts of each sequence by itself
+  (latent attention cuts by the lengths of all sequences of the step in other modes);
 * the collective algorithm: a fixed one;
 * products of few rows, which split K over the blocks of a cluster (bf16 and block-scaled fp8): not
   taken.  The other GEMM kernels accumulate every output element over K in one fixed order whatever

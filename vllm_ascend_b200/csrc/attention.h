@@ -32,7 +32,7 @@ struct AttnVariantArgs {
   long q_stride, out_stride, gate_stride, num_blocks, tokens;
   long k_block, k_tok, k_head, v_block, v_tok, v_head;      // cache strides in elements
   int num_seqs, max_blocks, block_size, Hq, Hkv, D, Dv;
-  int window, keep_first, bias_len, num_splits, dtype, key_heads, out_f32, even_parts;
+  int window, keep_first, bias_len, num_splits, dtype, key_heads, out_f32;
   float scale, softcap, out_scale;
 };
 

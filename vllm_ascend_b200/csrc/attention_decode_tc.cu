@@ -34,7 +34,6 @@ constexpr int DEC_NQ = 16;                 // MMA N: query rows per CTA
 constexpr int DEC_HALF = 128 * 128;        // 128 keys x 64 bf16
 constexpr int DEC_QHALF = DEC_NQ * 128;    // 16 rows x 64 bf16
 constexpr float kRescaleLog2 = 8.f;
-constexpr int DEC_STRETCH_SEQS = 8;    // see DecWalk
 
 struct DecParams {
   const int* query_start_loc;
@@ -51,7 +50,6 @@ struct DecParams {
   float* lse_out;            // optional [T, Hq] natural-log sum-exp of the scaled scores (-inf: no key)
   long num_blocks_total;
   int num_seqs, num_items;   // items = Hkv x sequences x splits
-  int stretches;             // 1: the splits are stretches of the batch's tiles (DecWalk)
   int tail_loads;            // 1: the last tile of a sequence is loaded in 32-key pieces (pages >= 128 keys)
   int l2_prefetch;           // tiles the L2 prefetch of K / V runs ahead of the staged loads (0 = off)
   int* status;
@@ -94,8 +92,8 @@ __device__ __forceinline__ float fast_exp2(float x) {
 
 __device__ __forceinline__ void softmax_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
-// One work item = (KV head, sequence, KV split).  The kernel is persistent: a CTA serves items one
-// after the other (DecWalk) and the three roles keep running tile / item counters, so barrier
+// One work item = (KV head, sequence, KV split).  The kernel is persistent: CTA b serves items
+// b, b + gridDim.x, ... and the three roles keep running tile / item counters, so barrier
 // initialisation, the TMEM allocation and the pipeline fill are paid once per CTA, the K/V
 // stream of the next item is already in flight while the current item's epilogue runs, and
 // a short item (a few tiles) costs no more than its bytes.
@@ -103,7 +101,6 @@ struct DecItem {
   int h, seq, split;
   int q_start, q_len, seq_len, ctx, t0, n;
   int first, kept;             // place in the sequence's tile list; its tiles before the window
-  int unused_end;              // the pair's splits without keys that this item marks: from its own (the next, if it has keys) to here
 };
 
 // tile number of the item's j-th tile: kept first tokens, then the window
@@ -113,13 +110,14 @@ __device__ __forceinline__ int dec_tile(const DecItem& w, int j) {
 }
 
 // The three words of an item that live in global memory.  They are loaded one item ahead
-// (dec_load) and turned into a DecItem (dec_fill, arithmetic only) when the item starts, so no
+// (dec_load) and turned into a DecItem (dec_make, arithmetic only) when the item starts, so no
 // role waits for a dependent global load at an item boundary.
 struct DecRaw {
   int q0, q1, seq_len;
 };
 
-__device__ __forceinline__ DecRaw dec_load(const DecParams& p, int seq) {
+__device__ __forceinline__ DecRaw dec_load(const DecParams& p, int item) {
+  const int seq = (item / p.Hkv) % p.num_seqs;
   DecRaw r;
   r.q0 = p.query_start_loc[seq];
   r.q1 = p.query_start_loc[seq + 1];
@@ -127,8 +125,12 @@ __device__ __forceinline__ DecRaw dec_load(const DecParams& p, int seq) {
   return r;
 }
 
-// Fills in what w.seq's words say; returns the tiles of one of its KV heads.
-__device__ __forceinline__ int dec_fill(const DecParams& p, DecItem& w, const DecRaw& r) {
+__device__ __forceinline__ DecItem dec_make(const DecParams& p, int item, const DecRaw& r) {
+  DecItem w;
+  w.h = item % p.Hkv;
+  const int q = item / p.Hkv;
+  w.seq = q % p.num_seqs;
+  w.split = q / p.num_seqs;
   w.q_start = r.q0;
   w.q_len = r.q1 - r.q0;
   w.seq_len = r.seq_len;
@@ -137,119 +139,17 @@ __device__ __forceinline__ int dec_fill(const DecParams& p, DecItem& w, const De
   if (p.window > 0) kv_lo = max(0, w.ctx - p.window + 1);
   const int tile_lo = kv_lo >> 7, tile_hi = (w.seq_len + 127) >> 7;
   w.kept = p.window > 0 ? min(tile_lo, (p.keep_first + 127) >> 7) : 0;
-  w.t0 = tile_lo - w.kept;
-  return w.kept + tile_hi - tile_lo;
+  const int n_all = w.kept + tile_hi - tile_lo;
+  const int per_split = (n_all + p.num_splits - 1) / p.num_splits;
+  w.first = w.split * per_split;
+  w.t0 = tile_lo - w.kept + w.first;
+  w.n = w.q_len > 0 ? max(0, min(n_all, w.first + per_split) - w.first) : 0;
+  return w;
 }
 
-// The items of a CTA, one after the other; every role walks them by itself.
-// Even parts: items are (sequence, KV head, part of its tiles), CTA b takes items b, b + gridDim.x, ...
-// Stretches: the tiles of all (sequence, KV head) pairs lie on one line, and CTA b takes the b-th of equal stretches of it, whatever pairs it
-// cuts: a pair's pieces are its splits.  Even parts of ragged sequences, dealt out in turn, leave a CTA with more or longer parts than
-// another: 33 sequences of 2300 keys, 8 KV heads, two splits 63 us, stretches 56; 48 of 1024 keys, 4 KV heads 30.4 and 29.1 us.
-// Finding the stretch takes about a microsecond, which few sequences do not give back.  us, even parts and stretches, 4 KV heads: 1 sequence of 1024
-// keys 9.1 and 9.7, 4 13.6 and 13.4, 8 17.2 and 15.0, 16 22.2 and 18.9, 64 42.3 and 38.8; 8 of 300 keys 9.7 and 10.4 (and a merge of 3.9 each).
-// A stretch is long enough that no pair is cut into more than num_splits pieces: n tiles meet at most (n - 2) / stretch + 2 stretches.
-// A pair without keys counts as one tile; sequences without query rows have no items.
-struct DecWalk {
-  int next;                        // even parts: the next item
-  int seq, h, first, split, left;  // stretches: the next piece and the tiles left in the stretch
-  DecRaw raw, ahead;               // words of the next item's sequence and of the one behind it
-
-  // called by whole warps
-  __device__ __forceinline__ void start(const DecParams& p) {
-    next = blockIdx.x;
-    seq = h = first = split = left = 0;
-    raw = ahead = {0, 0, 0};
-    if (!p.stretches) {
-      if (next < p.num_items) raw = dec_load(p, (next / p.Hkv) % p.num_seqs);
-      return;
-    }
-    const int lane = threadIdx.x & 31;
-    auto weight = [&](int s) {
-      DecItem w;
-      const int n = s < p.num_seqs ? dec_fill(p, w, dec_load(p, s)) : 0;
-      return s < p.num_seqs && w.q_len > 0 ? max(n, 1) : 0;
-    };
-    int total = 0, most = 2;
-    for (int s = lane; s < p.num_seqs; s += 32) {
-      const int n = weight(s);
-      total += n;
-      most = max(most, n);
-    }
-    total = __reduce_add_sync(0xffffffffu, total) * p.Hkv;
-    most = __reduce_max_sync(0xffffffffu, most);
-    const int grid = gridDim.x, len = max((total + grid - 1) / grid, (most - 2) / (p.num_splits - 1) + 1);
-    const long from = (long)blockIdx.x * len;
-    if (from >= total) return;
-    const int at = (int)from;
-    int base = 0;
-#pragma unroll 1
-    for (int s0 = 0; s0 < p.num_seqs; s0 += 32) {
-      const int n = weight(s0 + lane);
-      int incl = n * p.Hkv;
-      for (int d = 1; d < 32; d <<= 1) {
-        const int o = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += o;
-      }
-      const unsigned past = __ballot_sync(0xffffffffu, at < base + incl);
-      if (past) {
-        const int k = __ffs(past) - 1, nk = __shfl_sync(0xffffffffu, n, k);
-        const int off = at - base - (__shfl_sync(0xffffffffu, incl, k) - nk * p.Hkv);
-        seq = s0 + k;
-        h = off / nk;
-        first = off - h * nk;
-        split = (int)blockIdx.x - (at - first) / len;
-        left = min(len, total - at);
-        break;
-      }
-      base += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (left > 0) {
-      raw = dec_load(p, seq);
-      if (seq + 1 < p.num_seqs) ahead = dec_load(p, seq + 1);
-    }
-  }
-
-  __device__ __forceinline__ bool step(const DecParams& p, DecItem& w) {
-    if (!p.stretches) {
-      if (next >= p.num_items) return false;
-      w.h = next % p.Hkv;
-      w.seq = (next / p.Hkv) % p.num_seqs;
-      w.split = next / p.Hkv / p.num_seqs;
-      const int n_all = dec_fill(p, w, raw), per_split = (n_all + p.num_splits - 1) / p.num_splits;
-      w.first = w.split * per_split;
-      w.t0 += w.first;
-      w.n = w.q_len > 0 ? max(0, min(n_all, w.first + per_split) - w.first) : 0;
-      w.unused_end = w.split + 1;
-      next += gridDim.x;
-      if (next < p.num_items) raw = dec_load(p, (next / p.Hkv) % p.num_seqs);
-      return true;
-    }
-    if (left <= 0) return false;
-    w.h = h;
-    w.seq = seq;
-    const int n_all = dec_fill(p, w, raw), take = min(max(n_all, 1) - first, left);
-    w.split = split;
-    w.first = first;
-    w.t0 += first;
-    w.n = n_all > 0 ? take : 0;
-    first += take;
-    left -= take;
-    w.unused_end = 0;
-    if (first >= n_all) {
-      w.unused_end = p.num_splits;
-      first = split = 0;
-      if (++h == p.Hkv && left > 0) {
-        h = 0;
-        do {
-          raw = ahead;
-          if (++seq + 1 < p.num_seqs) ahead = dec_load(p, seq + 1);
-        } while (raw.q1 <= raw.q0 && seq + 1 < p.num_seqs);
-      }
-    }
-    return true;
-  }
-};
+__device__ __forceinline__ DecItem dec_item(const DecParams& p, int item) {
+  return dec_make(p, item, dec_load(p, item));
+}
 
 template <int D, int NVT, bool VAR>
 __global__ void __launch_bounds__(DEC_THREADS, 1)
@@ -336,8 +236,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = warp_uniform(*tmem_ptr);
-  DecWalk walk;
-  walk.start(p);
+  const int num_items = p.num_items;
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
@@ -354,12 +253,20 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
       return p.block_table[(long)d.seq * p.max_blocks + min(key0, d.seq_len - 1) / p.block_size];
     };
     DecItem w_next;
+    DecRaw raw_next = {0, 0, 0};          // words of the item after the next one
     int blk_first_next = 0;
-    bool more = walk.step(p, w_next);
-    if (more) blk_first_next = first_blk(w_next);
-    auto advance = [&]() {
-      more = walk.step(p, w_next);
-      if (more) blk_first_next = first_blk(w_next);
+    w_next.n = 0;
+    if ((int)blockIdx.x < num_items) {
+      w_next = dec_item(p, blockIdx.x);
+      blk_first_next = first_blk(w_next);
+      if ((int)(blockIdx.x + gridDim.x) < num_items) raw_next = dec_load(p, blockIdx.x + gridDim.x);
+    }
+    auto advance = [&](int item_after) {
+      if (item_after < num_items) {
+        w_next = dec_make(p, item_after, raw_next);
+        blk_first_next = first_blk(w_next);
+        if (item_after + (int)gridDim.x < num_items) raw_next = dec_load(p, item_after + gridDim.x);
+      }
     };
     // The query rows of an item go into Q buffer (its index among the non-empty items) & 1; the
     // buffer of the item after the current one is free (its last reader was two items ago), so
@@ -378,12 +285,13 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
     };
     bool q_ahead = false;                // the next non-empty item's Q load was already issued
 #pragma unroll 1
-    while (more) {
+    for (int item = blockIdx.x; item < num_items; item += gridDim.x) {
       const DecItem w = w_next;
       const int hk = VAR ? w.h * p.key_heads / p.Hkv : w.h;
       int blk_cur = blk_first_next;
+      const int item_after = item + gridDim.x;
       if (w.n <= 0) {
-        advance();
+        advance(item_after);
         continue;
       }
       const int* bt = p.block_table + (long)w.seq * p.max_blocks;
@@ -470,10 +378,10 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
           __syncwarp();
         }
         blk_cur = blk_next;
-        if (j == 0) advance();                 // after this item's first tile is on its way
+        if (j == 0) advance(item_after);       // after this item's first tile is on its way
         // third tile: its stage was freed by the last S MMA of the previous item, so the Q buffer
         // of the next item (last read by that MMA) is free as well and load_q does not wait
-        if (j == min(2, w.n - 1) && more && w_next.n > 0) {
+        if (j == min(2, w.n - 1) && item_after < num_items && w_next.n > 0) {
           if (!load_q(it + 1, w_next)) goto done;
           q_ahead = true;
         }
@@ -489,9 +397,12 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
       // A of the second product: 16 keys of V^T (two 64-wide d atoms DEC_HALF apart, 8-key groups 1024 B apart)
       const uint64_t dv0 = make_smem_desc(smem_u32(Vs), DEC_HALF, 1024, kLayoutSw128), dp0 = make_smem_desc(smem_u32(Ps), 16, 1024, kLayoutSw128);
       uint32_t gt = 0, it = 0;
-      DecItem w;
+      DecRaw raw_next = {0, 0, 0};
+      if ((int)blockIdx.x < num_items) raw_next = dec_load(p, blockIdx.x);
 #pragma unroll 1
-      while (walk.step(p, w)) {
+      for (int item = blockIdx.x; item < num_items; item += gridDim.x) {
+        const DecItem w = dec_make(p, item, raw_next);
+        if (item + (int)gridDim.x < num_items) raw_next = dec_load(p, item + gridDim.x);
         if (w.n <= 0) continue;
         const int qb = it & 1;
         const uint64_t dq = dq0 + (uint32_t)(qb * (Cfg::Q_BYTES >> 4));
@@ -558,19 +469,21 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q,
     int* redi = reinterpret_cast<int*>(red);        // [2 tiles][4 warps][16]
     const int col = lane & (NVT - 1), col_tok = col / G, col_head = col - col_tok * G;      // the column this lane finishes
     uint32_t gt = 0, it = 0;
-    DecItem w;
+    DecRaw raw_next = {0, 0, 0};
+    if ((int)blockIdx.x < num_items) raw_next = dec_load(p, blockIdx.x);
 #pragma unroll 1
-    while (walk.step(p, w)) {
+    for (int item = blockIdx.x; item < num_items; item += gridDim.x) {
+      const DecItem w = dec_make(p, item, raw_next);
+      if (item + (int)gridDim.x < num_items) raw_next = dec_load(p, item + gridDim.x);
       const int nv = w.q_len * G;                   // valid columns (<= 16)
-      if (p.num_splits > 1) {                   // splits without keys have no weight in the merge
-        const int s0 = w.split + (w.n > 0 ? 1 : 0), count = (w.unused_end - s0) * nv;
-        for (int i = tid; i < count; i += 128) {
-          const int c = i % nv;
-          p.partial_lse[((long)(w.q_start + c / G) * p.Hq + (w.h * G + c % G)) * p.num_splits + s0 + i / nv] = -INFINITY;
-        }
-      }
       if (w.n <= 0) {
-        if (p.num_splits == 1 && p.lse_out && w.q_len > 0) {
+        if (p.num_splits > 1 && w.q_len > 0) {      // an empty split still owns its partial slots
+          for (int c = tid; c < nv; c += 128) {
+            const long pidx =
+                ((long)(w.q_start + c / G) * p.Hq + (w.h * G + c % G)) * p.num_splits + w.split;
+            p.partial_lse[pidx] = -INFINITY;        // the merge reads no sums behind the last split with keys
+          }
+        } else if (p.num_splits == 1 && p.lse_out && w.q_len > 0) {
           // a caller that merges partial results of several ranks needs a defined (zero-weight)
           // result for a sequence none of whose keys live here
           for (int c = 0; c < nv; c++) {
@@ -819,15 +732,14 @@ static int launch_decode_nv(const CUtensorMap& tq, const CUtensorMap& tk, const 
   return B200_CHECK_LAUNCH();
 }
 
-// fills in the item count; ncols: columns that can be valid; even_parts: no stretches, whose cuts depend on all lengths of the batch
+// fills in the item count; ncols: columns that can be valid
 template <bool VAR>
 static int launch_decode(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tk32,
-                         const CUtensorMap& tv32, DecParams& p, int ncols, bool even_parts, cudaStream_t stream) {
+                         const CUtensorMap& tv32, DecParams& p, int ncols, cudaStream_t stream) {
   const long items = (long)p.Hkv * p.num_seqs * p.num_splits;
   if (items > 0x7fffffffL) return 9125;
   if (ncols > DEC_NQ) return 9126;
   p.num_items = (int)items;
-  p.stretches = p.num_splits > 1 && !even_parts && p.num_seqs >= DEC_STRETCH_SEQS;
   static int sm_count[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 9127;
@@ -858,14 +770,13 @@ B200_API int b200_attn_decode_set_l2_prefetch(int tiles) {
 // scratch needs b200_attn_scratch_bytes(T, Hq, D, num_splits) bytes when num_splits > 1.
 // lse_out (optional, fp32 [T, Hq]): log-sum-exp of every (token, head) over the keys this call saw,
 // for callers that merge the results of several calls (context-parallel ranks).
-// even_parts: the splits are even parts of every sequence by itself, whatever the others' lengths.
 B200_API int b200_attn_decode_tc_lse(const void* q, long q_stride, long T, const void* k_cache,
                                      const void* v_cache, long num_blocks, int block_size,
                                      const void* query_start_loc, const void* seq_lens,
                                      const void* block_table, int max_blocks, int num_seqs, int Hq,
                                      int Hkv, int D, float scale, int window, int num_splits,
                                      int max_q_len, void* out, long out_stride, void* scratch,
-                                     int kv_layout, void* lse_out, int even_parts,
+                                     int kv_layout, void* lse_out,
                                      int* status, void* timeline, cudaStream_t stream) {
   using namespace b200;
   if (num_seqs <= 0 || T <= 0) return 0;
@@ -937,7 +848,7 @@ B200_API int b200_attn_decode_tc_lse(const void* q, long q_stride, long T, const
   p.l2_prefetch = g_dec_l2_prefetch;
   p.keep_first = 0;
   {
-    const int lrc = launch_decode<false>(tq, tk, tv, tk32, tv32, p, max_q_len * G, even_parts != 0, stream);
+    const int lrc = launch_decode<false>(tq, tk, tv, tk32, tv32, p, max_q_len * G, stream);
     if (lrc) return lrc;
   }
   if (num_splits > 1)
@@ -957,7 +868,7 @@ B200_API int b200_attn_decode_tc(const void* q, long q_stride, long T, const voi
   return b200_attn_decode_tc_lse(q, q_stride, T, k_cache, v_cache, num_blocks, block_size,
                                  query_start_loc, seq_lens, block_table, max_blocks, num_seqs, Hq,
                                  Hkv, D, scale, window, num_splits, max_q_len, out, out_stride,
-                                 scratch, kv_layout, nullptr, 0, status, timeline, stream);
+                                 scratch, kv_layout, nullptr, status, timeline, stream);
 }
 
 // Options as in AttnVariantArgs; one query token per sequence (row b of q belongs to sequence b), bf16, D and Dv
@@ -1020,7 +931,7 @@ B200_API int b200_attention_variant_decode(const b200::AttnVariantArgs* a, int* 
   p.bias = a->bias; p.sink = a->sink;
   p.gate = (const __nv_bfloat16*)a->gate;
   p.gate_stride = a->gate_stride;
-  int rc = launch_decode<true>(tq, tkv[0], tkv[1], tkv32[0], tkv32[1], p, G, a->even_parts != 0, stream);
+  int rc = launch_decode<true>(tq, tkv[0], tkv[1], tkv32[0], tkv32[1], p, G, stream);
   if (rc) return rc;
   if (a->num_splits > 1)
     return launch_merge_splits(p.partial_o, p.partial_lse, a->num_seqs, a->Hq, a->num_splits, a->Dv, a->out,

@@ -552,7 +552,7 @@ def paged_attention_decode_tc(q: torch.Tensor, k_cache: torch.Tensor, v_cache: t
         meta.block_table.stride(0), num_seqs, Hq, Hkv, D, scale, int(window), num_splits,
         max_q_len if max_q_len else min(meta.max_query_len, 16 // (Hq // Hkv)), out.data_ptr(),
         out.stride(0), _native.ptr(scratch), kv_layout(k_cache), _native.ptr(lse_out),
-        int(fixed_sums()), _native.status_word(q.device).data_ptr(), _native.ptr(timeline), _native.stream_ptr())
+        _native.status_word(q.device).data_ptr(), _native.ptr(timeline), _native.stream_ptr())
     _native.check(rc, "attn_decode_tc")
     launch_counter[0] += 1 + (1 if num_splits > 1 else 0)
     return out
