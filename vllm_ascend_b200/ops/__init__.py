@@ -66,8 +66,8 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float,
     H = x.shape[-1]
     if x.stride(-1) != 1:
         x = x.contiguous()
-    x2 = x if x.dim() == 2 else x.reshape(-1, H)
-    T = x2.shape[0]
+    x2 = x if x.dim() == 2 and H else x.reshape(-1, H)      # rows without columns are refused there
+    T, given = x2.shape[0], out
     if out is None:
         out = x2.new_empty((T, H))
     if residual is not None:
@@ -77,7 +77,7 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float,
                                      out.stride(0), _native.stream_ptr())
     _native.check(rc, "rms_norm")
     launch_counter[0] += 1
-    return out if x2 is x else out.view(x.shape), residual
+    return out if x2 is x and given is None else out.view(x.shape), residual
 
 
 def layer_norm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], eps: float) -> torch.Tensor:
@@ -172,8 +172,8 @@ def qknorm_rope_kvwrite(qkv: torch.Tensor, positions: torch.Tensor, cos_sin: tor
 
 # ---------------------------------------------------------------- GEMM
 def _dense_rows(x: torch.Tensor, K: int) -> torch.Tensor:
-    """x as [rows, K] with adjacent columns and rows on 16-byte boundaries apart, as the GEMM kernels take it."""
-    x2 = x if x.dim() == 2 else x.reshape(-1, K)
+    """x as [rows, K] with adjacent columns and rows on 16-byte boundaries apart, as the GEMM kernels take it; none for K = 0."""
+    x2 = x if x.dim() == 2 and K else x.reshape(-1, K)
     return x2 if x2.stride(1) == 1 and x2.stride(0) % 8 == 0 else x2.contiguous()
 
 
@@ -195,6 +195,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         if residual is not None:
             y = y + residual.view(M, N)
         return y.view(*x.shape[:-1], N)
+    given = out
     if out is None:
         out = x2.new_empty((M, N))
     if M == 0:
@@ -217,7 +218,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
             _native.status_word(x.device).data_ptr(), 0, _native.stream_ptr())
     _native.check(rc, "gemm_bf16")
     launch_counter[0] += 1
-    return out if x.dim() == 2 else out.view(*x.shape[:-1], N)
+    return out if x.dim() == 2 and given is None else out.view(*x.shape[:-1], N)
 
 
 def linear_fp32(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
@@ -303,7 +304,7 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Ten
         return silu_and_mul(y) if limit is None else activation(y.contiguous(), "swiglu_oai", True, CLAMPED_GATE_ALPHA, limit)
     alpha, limit = (0.0, 0.0) if limit is None else (CLAMPED_GATE_ALPHA, float(limit))
     x2 = _dense_rows(x, K)
-    M = x2.shape[0]
+    M, given = x2.shape[0], out
     if out is None:
         out = x2.new_empty((M, I))
     min2 = envs.VLLM_B200_GEMM_2CTA_MIN_M
@@ -319,7 +320,7 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Ten
             alpha, limit, _native.status_word(x.device).data_ptr(), _native.stream_ptr())
         _native.check(rc, "gemm_swiglu")
         launch_counter[0] += 1
-    return out if x.dim() == 2 else out.view(*x.shape[:-1], I)
+    return out if x.dim() == 2 and given is None else out.view(*x.shape[:-1], I)
 
 
 #: most rows of the few-row GEMM
