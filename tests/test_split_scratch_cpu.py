@@ -23,3 +23,10 @@ def test_a_captured_buffer_stays(monkeypatch, get):
     more = get(5 << 20)                             # a later eager step
     assert more.numel() >= 5 << 20 and more.data_ptr() != held
     assert get(1).data_ptr() == held and get(3 << 20).data_ptr() == held
+
+
+@pytest.mark.parametrize("get", [lambda n: ops._get_scratch(torch.device("cpu"), n), lambda n: mla._split_scratch(torch.device("cpu"), n)],
+                         ids=["attention", "latent"])
+def test_a_buffer_of_inference_mode_serves_others(get):
+    with torch.inference_mode():
+        assert not get(6 << 20).is_inference()

@@ -22,7 +22,8 @@ class Scratch:
         key, capturing = (device.type, index), torch.cuda.is_initialized() and torch.cuda.is_current_stream_capturing()
         buf = self._shared.get(key)
         if buf is None or buf.numel() < numel:
-            own = torch.empty(max(numel, 1 << 20), dtype=self._dtype, device=device)
+            with torch.inference_mode(False):      # calls inside and outside of that mode share it
+                own = torch.empty(max(numel, 1 << 20), dtype=self._dtype, device=device)
             if capturing or key in self._captured:
                 return own
             self._shared[key] = buf = own
