@@ -292,9 +292,9 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmap_a,
 #pragma unroll
           for (int i = 0; i < 32; i++) acc[32 + i] = fmaf(__uint_as_float(r1[i]), sc, acc[32 + i]);
         } else {
-          // 640 threads have 96 registers: eight columns at a time leave the accumulators and the loop their own.  With sixteen, what was
-          // spilled around the loop cost as much as the loads (2048 x 57344 x 8192 with loads of scales 1010 us, with scales from shared
-          // memory 1100, and 940 so)
+          // 640 threads have 96 registers: eight columns at a time leave the accumulators and the loop their own (2048 x 57344 x 8192 by itself:
+          // 1074 us with sixteen and a load of scales in every thread, 937 to 960 so; sixteen with scales from shared memory were no gain, for what
+          // was then spilled around the loop)
 #pragma unroll
           for (int c0 = 0; c0 < F8_COLS; c0 += 8) {
             uint32_t r[8];

@@ -137,7 +137,9 @@ def _fp8_few_rows_faster(M: int, N: int, K: int) -> bool:
 
     up to 32 rows   K of 1024 and more: 32 rows of 8192 x 2048 11 -> 8, 57344 x 8192 89 -> 78
     33..64 rows     64 rows of 4096 x 4096 14 -> 12, 10240 x 4096 15.4 -> 16.0 (three splits) and x 8192 25 -> 23, 14336 x 4096 16 -> 19 and x 8192
-                    26 -> 28 (two); of K = 2048 2048 columns 9.0 -> 7.2, 6144 10.1 -> 10.5, 8192 10 -> 11
+                    26 -> 28 (two); of K = 2048 2048 columns 9.0 -> 7.2, 6144 10.1 -> 10.5, 8192 10 -> 11.  The line was drawn when the general
+                    kernel was slower, and gives 10240 x 4096, 14336 x 8192 and 6144 x 2048 to the few-row kernel, 4 to 8 % behind by now: another
+                    kernel sums K in another order, which the next layer's quantisation carries on
     65..128 rows    one block per SM, and its promotion takes as long as the general kernel's: 128 rows of 4096 x 4096 15.6 -> 13.8 (four), 8192 x 4096
                     16 -> 18, x 8192 25.6 -> 26.6 and x 28672 73 -> 82 (two), 28672 x 8192 50 -> 91 (one)
     """
